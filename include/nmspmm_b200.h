@@ -195,6 +195,17 @@ int nmspmm_gemm_row_major_16(const nmspmm_gemm_desc* desc, int dtype,
 /* n values (n % 4 == 0) of `dtype` at src_dev (8-byte aligned) -> FP32 at dst_dev (16-byte aligned). */
 int nmspmm_widen_device(int dtype, const void* src_dev, float* dst_dev, size_t n, void* stream);
 
+/* Backward of y = x . B (no counterpart in the reference, which has no training path): in FP32
+ * whatever path the forward took.  desc gives M, N, K and n_keep (16, 12, 8 or 4 of 32); x is
+ * M x K row-major and grad_y M x N row-major, both of `dtype`; B the compressed values and DT_dev
+ * the raw window-local indices [W][N/32].  grad_x_dev (M x K, of dtype) receives
+ * grad_y . B^T, grad_B_dev ([W][N], float) x^T . grad_y at the kept positions; either may be NULL
+ * (then B resp. x may be too).  The workspace needs no initial contents. */
+size_t nmspmm_linear_grad_workspace_bytes(const nmspmm_gemm_desc* desc, int dtype, int want_x, int want_values);
+int nmspmm_linear_grad(const nmspmm_gemm_desc* desc, int dtype, const void* x_rows_dev, const void* grad_y_dev,
+                       const float* B_dev, const int* DT_dev, void* grad_x_dev, float* grad_B_dev,
+                       void* workspace_dev, size_t workspace_bytes, void* stream);
+
 /* The multiply of one rank of a column-sharded B fused with the all-gather of C (no
  * counterpart in the reference, which runs on one GPU).  The rank's problem is
  * desc (N = the columns of its slab); every finished tile is stored, inside the multiply

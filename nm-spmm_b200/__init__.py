@@ -40,7 +40,7 @@ C_ABI_SYMBOLS = (
     "nmspmm_test_short_fill", "nmspmm_set_tile_band", "nmspmm_tuned_plan_set", "nmspmm_tuned_plan_load", "nmspmm_tuned_plan_clear",
     "nmspmm_tuned_plan_count", "nmspmm_gemm_workspace_bytes", "nmspmm_gemm", "nmspmm_gemm_row_major",
     "nmspmm_gemm_row_major_workspace_bytes", "nmspmm_gemm_row_major_16", "nmspmm_gemm_row_major_16_workspace_bytes",
-    "nmspmm_widen_device", "nmspmm_gemm_with_cached_workspace", "nmspmm_device_status",
+    "nmspmm_linear_grad", "nmspmm_linear_grad_workspace_bytes", "nmspmm_widen_device", "nmspmm_gemm_with_cached_workspace", "nmspmm_device_status",
     "nmspmm_gemm_plan", "nmspmm_gemm_host", "nmspmm_release_cached", "nmspmm_measure_ffma_peak",
     "nmspmm_gemm_static_scratch", "nmspmm_gemm_gather", "nmspmm_prune_device",
 )
@@ -102,6 +102,9 @@ def load_library():
     lib.nmspmm_gemm_row_major_16_workspace_bytes.argtypes = [ctypes.POINTER(GemmDesc)]
     lib.nmspmm_gemm_row_major_16.argtypes = [ctypes.POINTER(GemmDesc), ctypes.c_int, vp, vp, vp, vp, vp, vp, sz, vp]
     lib.nmspmm_widen_device.argtypes = [ctypes.c_int, vp, vp, sz, vp]
+    lib.nmspmm_linear_grad_workspace_bytes.restype = sz
+    lib.nmspmm_linear_grad_workspace_bytes.argtypes = [ctypes.POINTER(GemmDesc), ci, ci, ci]
+    lib.nmspmm_linear_grad.argtypes = [ctypes.POINTER(GemmDesc), ci, vp, vp, vp, vp, vp, vp, vp, sz, vp]
     lib.nmspmm_gemm_with_cached_workspace.argtypes = [ctypes.POINTER(GemmDesc), vp, vp, vp, vp, vp, vp]
     lib.nmspmm_gemm_static_scratch.argtypes = [ctypes.POINTER(GemmDesc), vp, vp, vp, vp, vp, vp]
     lib.nmspmm_prune_device.argtypes = [vp, vp, vp, ci, ci, ci, ci, vp]

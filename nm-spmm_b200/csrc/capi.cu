@@ -920,6 +920,63 @@ int nmspmm_widen_device(int dtype, const void* src_dev, float* dst_dev, size_t n
     return e == cudaSuccess ? NMSPMM_OK : cuda_fail(e);
 }
 
+// ---- backward of the linear layer ------------------------------------------------------------
+static size_t linear_grad_bytes(const nmspmm_gemm_desc* d, int dtype, bool want_x, bool want_b, int sms)
+{
+    // the two gradients run one after the other on a stream and share the scratch
+    const size_t wide = dtype == NMSPMM_DTYPE_F32 ? 0 : round256(static_cast<size_t>(d->M) * d->N * sizeof(float));
+    const size_t x = want_x ? grad_input_scratch_bytes(d->M, d->N, d->K, d->n_keep, sms) : 0;
+    const size_t b = want_b ? grad_values_scratch_bytes(d->M, d->N, d->K, d->n_keep, sms) : 0;
+    return round256(wide + (x > b ? x : b)) + 256;
+}
+
+static int check_linear_grad(const nmspmm_gemm_desc* d, int dtype)
+{
+    if (!d || d->M <= 0 || d->N <= 0 || d->K <= 0 || d->N % kVecLenHost != 0 || d->K % 32 != 0) return NMSPMM_INVALID_ARGUMENT;
+    if (dtype != NMSPMM_DTYPE_F32 && dtype != NMSPMM_DTYPE_F16 && dtype != NMSPMM_DTYPE_BF16) return NMSPMM_INVALID_ARGUMENT;
+    return linear_grad_supported(d->n_keep) ? NMSPMM_OK : NMSPMM_UNSUPPORTED;
+}
+
+size_t nmspmm_linear_grad_workspace_bytes(const nmspmm_gemm_desc* desc, int dtype, int want_x, int want_values)
+{
+    if (check_linear_grad(desc, dtype) != NMSPMM_OK) return 0;
+    return linear_grad_bytes(desc, dtype, want_x != 0, want_values != 0, sm_count());
+}
+
+int nmspmm_linear_grad(const nmspmm_gemm_desc* desc, int dtype, const void* x_rows_dev, const void* grad_y_dev, const float* B_dev,
+                       const int* DT_dev, void* grad_x_dev, float* grad_B_dev, void* workspace_dev, size_t workspace_bytes,
+                       void* stream)
+{
+    int rc = check_linear_grad(desc, dtype);
+    if (rc != NMSPMM_OK) return rc;
+    if (!grad_y_dev || !DT_dev || !workspace_dev || !aligned16(workspace_dev)) return NMSPMM_INVALID_ARGUMENT;
+    if ((grad_x_dev && (!B_dev || !aligned16(B_dev) || !aligned16(grad_x_dev))) || (grad_B_dev && (!x_rows_dev || !aligned16(grad_B_dev))))
+        return NMSPMM_INVALID_ARGUMENT;
+    if (!aligned16(grad_y_dev)) return NMSPMM_INVALID_ARGUMENT;
+    DeviceInfo* di = nullptr;
+    rc = device_info(&di);
+    if (rc != NMSPMM_OK) return rc;
+    if (workspace_bytes < linear_grad_bytes(desc, dtype, grad_x_dev != nullptr, grad_B_dev != nullptr, di->sms)) return NMSPMM_WORKSPACE_TOO_SMALL;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    unsigned char* ws = static_cast<unsigned char*>(workspace_dev);
+    const float* g = static_cast<const float*>(grad_y_dev);
+    cudaError_t e = cudaSuccess;
+    if (dtype != NMSPMM_DTYPE_F32) {
+        const size_t n = static_cast<size_t>(desc->M) * desc->N;
+        e = launch_widen(dtype, grad_y_dev, reinterpret_cast<float*>(ws), n, st);
+        if (e != cudaSuccess) return cuda_fail(e);
+        g = reinterpret_cast<const float*>(ws);
+        ws += round256(n * sizeof(float));
+    }
+    if (grad_x_dev)
+        e = launch_grad_input(dtype, g, B_dev, DT_dev, grad_x_dev, desc->M, desc->N, desc->K, desc->n_keep, di->sms,
+                              reinterpret_cast<float*>(ws), di->status_word, st);
+    if (e == cudaSuccess && grad_B_dev)
+        e = launch_grad_values(dtype, x_rows_dev, g, DT_dev, grad_B_dev, desc->M, desc->N, desc->K, desc->n_keep, di->sms,
+                               reinterpret_cast<float*>(ws), di->status_word, st);
+    return e == cudaSuccess ? NMSPMM_OK : cuda_fail(e);
+}
+
 int nmspmm_gemm_gather(const nmspmm_gemm_desc* desc, const float* A_dev, const float* B_dev, const int* D_dev,
                        const int* column_info_dev, float* const* C_all, int n_out, long long ldc, int col0,
                        void* workspace_dev, size_t workspace_bytes, void* stream)

@@ -21,6 +21,16 @@ cudaError_t launch_transpose_rows_16(int dtype, const void* in, float* out, int 
 cudaError_t launch_narrow(int dtype, const float* in, void* out, size_t n, cudaStream_t st);
 cudaError_t launch_widen(int dtype, const void* in, float* out, size_t n, cudaStream_t st);
 
+// Backward of the linear layer (linear_grad.cu): gradients of the kept values and of x, ratios
+// 16 / 12 / 8 / 4 of 32, DT raw window-local indices, grad_y float, x and grad_x of dtype.
+bool linear_grad_supported(int n_keep);
+size_t grad_values_scratch_bytes(int M, int N, int K, int n_keep, int sms);
+size_t grad_input_scratch_bytes(int M, int N, int K, int n_keep, int sms);
+cudaError_t launch_grad_values(int dtype, const void* x, const float* grad_y, const int* DT, float* grad_B, int M, int N, int K,
+                               int n_keep, int sms, float* scratch, int* status, cudaStream_t st);
+cudaError_t launch_grad_input(int dtype, const float* grad_y, const float* B, const int* DT, void* grad_x, int M, int N, int K,
+                              int n_keep, int sms, float* scratch, int* status, cudaStream_t st);
+
 // One compiled FFMA kernel variant.
 struct FfmaVariant {
     int tile_id;        // nmspmm_tile
@@ -38,7 +48,8 @@ const FfmaVariant* find_ffma_variant(int tile_id, int n_keep, int mode);
 
 // Row-major 2-D float tensor [rows][cols] (cols innermost) with a box_cols x box_rows box;
 // swizzle128 = 0: rows land unswizzled, 1: 32-byte chunks swizzled within 128-byte rows
-// (CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B; box_cols * 4 must be 128).
+// (CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B), 2: 16-byte chunks (CU_TENSOR_MAP_SWIZZLE_128B); box_cols * 4
+// must be 128 for both.
 // Elements outside the tensor are delivered as zeros.
 cudaError_t encode_tensor_map_2d(CUtensorMap* map, const float* base, int cols, int rows, int box_cols, int box_rows,
                                  int swizzle128 = 0);

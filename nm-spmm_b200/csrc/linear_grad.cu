@@ -1,0 +1,601 @@
+// Backward of y = x . B for a vector-wise N:M sparse B, in FP32 like the exact forward path:
+//
+//     grad_B[w][n] = sum_m x[m][k(w, n/32)] grad_y[m][n]            (the kept positions only)
+//     grad_x[m][k] = sum over the kept (w, n) with k(w, n/32) = k of grad_y[m][n] B[w][n]
+//
+// Both are 2 M N W useful FLOPs, n_keep / 32 of the dense products they replace (an expanded
+// B or an M x K x N product of which most is thrown away), and both are bound by the FP32
+// FMA pipe: 17.2 GFLOP at M = 2048, N = K = 4096, 8:32, against 0.1 GB of operands.  Measured
+// there: grad_B 331 us (51.8 TFLOP/s of the 74 the pipe has), grad_x 454 us (37.9), against 1169 and
+// 1136 us of the dense FP32 products (and 70 us of expanding B and picking the kept positions); at
+// 16:32 647 and 851 us, at 4:32 207 and 249 us.
+//
+// The indices are the raw window-local ones, [W][N/32].  Every wait is bounded; one that
+// gives up raises the device status word and nothing of its tile is stored.
+#include <cuda.h>
+#include <cuda_bf16.h>
+#include <cuda_fp16.h>
+
+#include "common.cuh"
+#include "kernels.h"
+
+namespace nmspmm {
+
+struct GradArgs {
+    const int* DT;          // [W][N/32] window-local k of every kept row
+    const float* xq;        // grad_B: [M4/4][K][4], the rows of x in groups of four
+    const float* B;         // grad_x: the launcher's (the kernel reads it through a tensor map)
+    void* out;              // grad_B [W][N] float, or grad_x [M][K] of dtype
+    float* partial;         // slots of split tiles
+    int* status;
+    int M, N, K, W;
+    int tiles_x;            // tiles along the fast tile dimension
+    int n_whole, slices;    // the first n_whole tiles are computed by one CTA each, the others in `slices` pieces
+    int dtype;
+};
+
+template <typename T> __device__ __forceinline__ float to_float(T v);
+template <> __device__ __forceinline__ float to_float<float>(float v) { return v; }
+template <> __device__ __forceinline__ float to_float<__half>(__half v) { return __half2float(v); }
+template <> __device__ __forceinline__ float to_float<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
+
+__device__ __forceinline__ void store_as(void* out, size_t at, float v, int dtype)
+{
+    if (dtype == kDtypeF32) static_cast<float*>(out)[at] = v;
+    else if (dtype == kDtypeF16) static_cast<__half*>(out)[at] = __float2half_rn(v);
+    else static_cast<__nv_bfloat16*>(out)[at] = __float2bfloat16_rn(v);
+}
+
+// Rows of x in groups of four: out[m / 4][k][m % 4], rows past M zero.  A thread reads one k of
+// four rows (coalesced along k) and writes one float4 (coalesced): no shared memory.
+template <typename T>
+__global__ void __launch_bounds__(256) quad_rows_kernel(const T* __restrict__ x, float4* __restrict__ out, int M, int K)
+{
+    const size_t n = static_cast<size_t>((M + 3) / 4) * K;
+    for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n; i += static_cast<size_t>(gridDim.x) * blockDim.x) {
+        const int mq = static_cast<int>(i / K), k = static_cast<int>(i - static_cast<size_t>(mq) * K);
+        float v[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int m = mq * 4 + j;
+            v[j] = m < M ? to_float<T>(x[static_cast<size_t>(m) * K + k]) : 0.f;
+        }
+        out[i] = make_float4(v[0], v[1], v[2], v[3]);
+    }
+}
+
+// ------------------------------------------------------------------------- grad of the kept values
+// One CTA: RW kept rows x 128 columns (four vectors, a warp each) over a range of m.  Thread tile
+// TW rows x 8 columns, eight row groups x four column groups.  A step stages MC rows of
+// grad_y ([MC][128], TMA) and of x over the k range the rows come from ([MC/4][KT][4], bulk
+// copies): a row's four m of one k are one 128-bit load at a k offset the thread keeps in a
+// register for the whole launch, so the gather costs no index traffic.  Lanes: a 128-bit shared
+// load takes one wavefront per eight lanes, and two such groups share one where lane i reads the
+// address of lane i ^ 1 (the loads of x: lane bit 0 is a column bit) or of lane i ^ 2 (the loads of
+// grad_y: bit 1 is a row bit).  A half warp then reads x at four unrelated k, which meet in a bank
+// now and then; with lane / 4 and lane % 4 the kernel took 3.7 wavefronts per load.
+template <int NKEEP>
+struct GradValuesCfg {
+    static constexpr int TW = (NKEEP == 12) ? 6 : 8;
+    static constexpr int RW = 8 * TW;
+    static constexpr int KT = RW / NKEEP * 32;
+    static constexpr int MC = (NKEEP == 4) ? 8 : 16;
+    static constexpr int THREADS = 128;
+    static constexpr int X_BYTES = MC * KT * 4, G_BYTES = MC * 128 * 4, STAGE_BYTES = X_BYTES + G_BYTES;
+    static constexpr int STAGES = 3;
+    static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 128 + 128;
+    static_assert(RW % NKEEP == 0, "whole windows");
+};
+
+template <int NKEEP>
+__global__ void __launch_bounds__(128, 3)
+nm_grad_values_kernel(const GradArgs a, const __grid_constant__ CUtensorMap map_g)
+{
+    using Cfg = GradValuesCfg<NKEEP>;
+    constexpr int TW = Cfg::TW, RW = Cfg::RW, KT = Cfg::KT, MC = Cfg::MC, STAGES = Cfg::STAGES;
+    extern __shared__ unsigned char smem_raw[];
+    const uint32_t ring = (smem_u32(smem_raw) + 127u) & ~127u;
+    const uint32_t bars = ring + STAGES * Cfg::STAGE_BYTES, abort_word = bars + STAGES * 8;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int ng = (lane & 1) | ((lane >> 1) & 2), wg = ((lane >> 1) & 1) | ((lane >> 2) & 6);      // see above
+
+    const bool sliced = static_cast<int>(blockIdx.x) >= a.n_whole;
+    const int S = sliced ? a.slices : 1, slot = static_cast<int>(blockIdx.x) - a.n_whole;
+    const int tile = sliced ? a.n_whole + slot / S : static_cast<int>(blockIdx.x);
+    const int tw = tile / a.tiles_x, tn = tile - tw * a.tiles_x;
+    const int w0 = tw * RW, n0 = tn * 128, k0 = w0 / NKEEP * 32;
+    const int n_steps_all = (a.M + MC - 1) / MC;
+    int first, n_steps;
+    slice_range(n_steps_all, S, sliced ? slot % S : 0, first, n_steps);
+    const uint32_t row_bytes = static_cast<uint32_t>(min(KT, a.K - k0)) * 16u;      // one group of four m, the tile's k
+    const int n_quads = (a.M + 3) / 4;
+
+    if (tid == 0) {
+        prefetch_tensor_map(&map_g);
+        for (int s = 0; s < STAGES; ++s) mbar_init(bars + s * 8, 1);
+        sts_volatile_s32(abort_word, 0);
+        mbar_init_fence();
+    }
+    __syncthreads();
+    grid_dependency_wait();
+
+    auto fill = [&](int it) {                              // one thread
+        const uint32_t dst = ring + (it % STAGES) * Cfg::STAGE_BYTES, full = bars + (it % STAGES) * 8;
+        const int mq0 = (first + it) * (MC / 4), quads = min(MC / 4, n_quads - mq0);
+        mbar_arrive_expect_tx(full, Cfg::G_BYTES + quads * row_bytes);
+        for (int q = 0; q < quads; ++q)
+            bulk_g2s(dst + q * (KT * 16), a.xq + (static_cast<size_t>(mq0 + q) * a.K + k0) * 4, row_bytes, full);
+        tma_load_2d(dst + Cfg::X_BYTES, &map_g, n0, (first + it) * MC, full);       // rows past M arrive as zeros
+    };
+    if (tid == 0)
+        for (int it = 0; it < STAGES - 1 && it < n_steps; ++it) fill(it);
+
+    const int v = (n0 >> 5) + warp;                        // this warp's vector
+    const bool live = v * 32 < a.N;
+    int off[TW];
+#pragma unroll
+    for (int r = 0; r < TW; ++r) {
+        const int w = w0 + wg * TW + r;
+        const int k = (live && w < a.W) ? (__ldg(a.DT + static_cast<size_t>(w) * (a.N >> 5) + v) & 31) + (wg * TW + r) / NKEEP * 32 : 0;
+        off[r] = k * 16;
+    }
+    float2 acc[TW][4];
+#pragma unroll
+    for (int r = 0; r < TW; ++r)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) acc[r][c] = make_float2(0.f, 0.f);
+
+    bool alive = true;
+    for (int it = 0; it < n_steps; ++it) {
+        // the barrier frees the slot of the step before, which takes the step STAGES - 1 ahead
+        __syncthreads();
+        if (tid == 0 && it + STAGES - 1 < n_steps && alive) {
+            fence_proxy_async();
+            fill(it + STAGES - 1);
+        }
+        __syncwarp();
+        const int s = it % STAGES;
+        alive = __all_sync(0xffffffffu, mbar_wait_bounded(bars + s * 8, (it / STAGES) & 1, abort_word)) && alive;
+        if (!live || !alive) continue;
+        const uint32_t xs = ring + s * Cfg::STAGE_BYTES, gs = xs + Cfg::X_BYTES + warp * 128 + ng * 16;
+        const int quads = min(MC / 4, n_quads - (first + it) * (MC / 4));       // the ragged last step holds fewer
+#pragma unroll 1
+        for (int q = 0; q < quads; ++q) {
+            float4 x4[TW];
+#pragma unroll
+            for (int r = 0; r < TW; ++r) x4[r] = lds_f4(xs + q * (KT * 16) + off[r]);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float4 g0 = lds_f4(gs + (q * 4 + j) * 512), g1 = lds_f4(gs + (q * 4 + j) * 512 + 64);
+                const float2 p0 = make_float2(g0.x, g0.y), p1 = make_float2(g0.z, g0.w);
+                const float2 p2 = make_float2(g1.x, g1.y), p3 = make_float2(g1.z, g1.w);
+#pragma unroll
+                for (int r = 0; r < TW; ++r) {
+                    const float xv = j == 0 ? x4[r].x : (j == 1 ? x4[r].y : (j == 2 ? x4[r].z : x4[r].w));
+                    const float2 xx = make_float2(xv, xv);
+                    acc[r][0] = __ffma2_rn(xx, p0, acc[r][0]);
+                    acc[r][1] = __ffma2_rn(xx, p1, acc[r][1]);
+                    acc[r][2] = __ffma2_rn(xx, p2, acc[r][2]);
+                    acc[r][3] = __ffma2_rn(xx, p3, acc[r][3]);
+                }
+            }
+        }
+    }
+    __syncthreads();
+    grid_launch_dependents();
+    if (lds_volatile_s32(abort_word) != 0) {
+        if (tid == 0) atomicMax(a.status, kDevTimeoutFull);
+        return;
+    }
+    if (!live) return;
+#pragma unroll
+    for (int r = 0; r < TW; ++r) {
+        const int w = wg * TW + r;
+        if (w0 + w >= a.W) continue;
+        float* p = sliced ? a.partial + (static_cast<size_t>(slot) * RW + w) * 128 + warp * 32 + ng * 4
+                          : static_cast<float*>(a.out) + static_cast<size_t>(w0 + w) * a.N + n0 + warp * 32 + ng * 4;
+        *reinterpret_cast<float4*>(p) = make_float4(acc[r][0].x, acc[r][0].y, acc[r][1].x, acc[r][1].y);
+        *reinterpret_cast<float4*>(p + 16) = make_float4(acc[r][2].x, acc[r][2].y, acc[r][3].x, acc[r][3].y);
+    }
+}
+
+// -------------------------------------------------------------------------------- grad of the input
+// One CTA: MT rows x KT k of grad_x over a range of vectors.  A vector adds to n_keep of every 32
+// k, a different set for every vector, so the accumulators that last are in shared memory
+// ([KT][MT] floats, 128 KB) and the registers hold one vector's contribution: a warp multiplies
+// 64 rows of grad_y by 32 (24) kept rows of B over the vector's 32 columns (thread tile 8 x 8, both
+// operands read 128 bits along n, so the packed FMA takes its pairs from the loads as they are
+// and sums even and odd columns apart), then adds the result to the rows of the accumulator
+// that its index list names: 16 + 16 shared accesses of 128 bits after 1024 packed FMAs.
+// Shared memory is the second bound: 128 loads of two wavefronts and the 128 of the additions
+// against 512 cycles of the FMA pipe.  (Thread tile 8 x 4 on sixteen warps: 65 % of the
+// shared-memory wavefronts there are, 481 us at M = 2048, N = K = 4096, 8:32.)
+// The accumulator is what limits the warps: 32 KB of it per warp at 8:32.  At 8:32 and 4:32 two
+// and four groups of warps therefore share it, each taking every second / fourth vector; a
+// token per patch of the accumulator hands it from group to group in vector order, so that the
+// sums have one order and the groups compute while others add.
+template <int NKEEP>
+struct GradInputCfg {
+    static constexpr int MT = (NKEEP == 4) ? 64 : 128, KT = (NKEEP == 4) ? 512 : 256;
+    static constexpr int WT = KT / 32 * NKEEP;             // kept rows under the tile
+    static constexpr int TR = (NKEEP == 12) ? 6 : 8;       // kept rows per thread: a warp's 4 TR rows are whole windows
+    static constexpr int MH = MT / 64, AREAS = MH * (WT / (4 * TR));
+    static constexpr int GROUPS = 8 / AREAS;
+    static constexpr int WARPS = AREAS * GROUPS, THREADS = WARPS * 32;
+    static constexpr int G_BYTES = MT * 128, B_BYTES = WT * 128, STAGE_BYTES = G_BYTES + B_BYTES;
+    static constexpr int ACC_BYTES = KT * MT * 4;
+    static constexpr int STAGES = (227 * 1024 - 2048 - ACC_BYTES) / STAGE_BYTES;
+    static constexpr int CTRL_BYTES = 512;
+    static constexpr int SMEM_BYTES = ACC_BYTES + STAGES * STAGE_BYTES + CTRL_BYTES + 1024;
+    static_assert(STAGES >= 3 && STAGES >= GROUPS, "a stage for every group at least");
+    static_assert(STAGES * 12 + AREAS * GROUPS * 8 + 4 <= CTRL_BYTES, "control block");
+    static_assert(SMEM_BYTES <= 227 * 1024, "shared memory");
+};
+
+template <int NKEEP>
+__global__ void __launch_bounds__((GradInputCfg<NKEEP>::THREADS), 1)
+nm_grad_input_kernel(const GradArgs a, const __grid_constant__ CUtensorMap map_g, const __grid_constant__ CUtensorMap map_b)
+{
+    using Cfg = GradInputCfg<NKEEP>;
+    constexpr int MT = Cfg::MT, KT = Cfg::KT, MH = Cfg::MH, AREAS = Cfg::AREAS, GROUPS = Cfg::GROUPS, STAGES = Cfg::STAGES;
+    constexpr int TR = Cfg::TR;
+    extern __shared__ unsigned char smem_raw[];
+    const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u;       // 128-byte swizzle: 1024-byte alignment
+    const uint32_t sums = ring + STAGES * Cfg::STAGE_BYTES;
+    const uint32_t bars = sums + Cfg::ACC_BYTES, tokens = bars + STAGES * 8, reads = tokens + AREAS * GROUPS * 8;
+    const uint32_t abort_word = reads + STAGES * 4;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int mg = (lane >> 1) & 7, wg = (lane & 1) | ((lane >> 3) & 2);      // both operands' loads pair up (see grad_values)
+    const int group = warp / AREAS, area = warp % AREAS, mh = area % MH, wq = area / MH;
+
+    const bool sliced = static_cast<int>(blockIdx.x) >= a.n_whole;
+    const int S = sliced ? a.slices : 1, slot = static_cast<int>(blockIdx.x) - a.n_whole;
+    const int tile = sliced ? a.n_whole + slot / S : static_cast<int>(blockIdx.x);
+    const int tm = tile / a.tiles_x, tk = tile - tm * a.tiles_x;
+    const int m0 = tm * MT, k0 = tk * KT, w0 = k0 / 32 * NKEEP;
+    int v0, T;                                             // this CTA's vectors: v0 .. v0 + T - 1
+    slice_range(a.N >> 5, S, sliced ? slot % S : 0, v0, T);
+
+    if (tid == 0) {
+        prefetch_tensor_map(&map_g);
+        prefetch_tensor_map(&map_b);
+        for (int s = 0; s < STAGES; ++s) {
+            mbar_init(bars + s * 8, 1);
+            sts_s32(reads + s * 4, 0);
+        }
+        for (int i = 0; i < AREAS * GROUPS; ++i) mbar_init(tokens + i * 8, 1);
+        sts_volatile_s32(abort_word, 0);
+        mbar_init_fence();
+    }
+    for (int o = tid * 16; o < Cfg::ACC_BYTES; o += Cfg::THREADS * 16) sts_f4(sums + o, make_float4(0.f, 0.f, 0.f, 0.f));
+    __syncthreads();
+    grid_dependency_wait();
+
+    auto fill = [&](int t) {                               // one thread: vector v0 + t into stage t % STAGES
+        const uint32_t dst = ring + (t % STAGES) * Cfg::STAGE_BYTES, full = bars + (t % STAGES) * 8;
+        mbar_arrive_expect_tx(full, Cfg::STAGE_BYTES);     // rows past M or W arrive as zeros
+        tma_load_2d(dst, &map_g, (v0 + t) * 32, m0, full);
+        tma_load_2d(dst + Cfg::G_BYTES, &map_b, (v0 + t) * 32, w0, full);
+    };
+    if (tid == 0)
+        for (int t = 0; t < STAGES && t < T; ++t) fill(t);
+
+    // kept rows of this thread: wq * (4 * TR) + r * 4 + wg, so that the four row groups of a warp fall
+    // into different 16-byte chunks of the swizzled rows; rows of grad_y: mh * 64 + i * 8 + mg.
+    const int nv = a.N >> 5;
+    const int* dt = a.DT + static_cast<size_t>(w0 + wq * (4 * TR) + wg) * nv + v0;
+    auto index_of = [&](int t, int r) {                    // k within the window, -1: no such row
+        return (w0 + wq * (4 * TR) + r * 4 + wg < a.W && t < T) ? (__ldg(dt + static_cast<size_t>(r * 4) * nv + t) & 31) : -1;
+    };
+    int k_next[TR];
+#pragma unroll
+    for (int r = 0; r < TR; ++r) k_next[r] = index_of(group, r);
+
+    const uint32_t g_rel = (mh * 64 + mg) * 128, b_rel = Cfg::G_BYTES + (wq * (4 * TR) + wg) * 128;
+    for (int t = group; t < T; t += GROUPS) {
+        int k_of[TR];
+#pragma unroll
+        for (int r = 0; r < TR; ++r) {
+            k_of[r] = k_next[r];
+            k_next[r] = index_of(t + GROUPS, r);
+        }
+        const int s = t % STAGES;
+        if (!__all_sync(0xffffffffu, mbar_wait_bounded(bars + s * 8, (t / STAGES) & 1, abort_word))) break;
+        const uint32_t gs = ring + s * Cfg::STAGE_BYTES + g_rel, bs = ring + s * Cfg::STAGE_BYTES + b_rel;
+        float2 acc[8][TR];                                  // (even columns, odd columns)
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int r = 0; r < TR; ++r) acc[i][r] = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {                      // four columns at a time
+            float4 b[TR];
+#pragma unroll
+            for (int r = 0; r < TR; ++r) b[r] = lds_f4(bs + r * 512 + ((c ^ (((wq * TR + r) & 1) * 4 + wg)) << 4));
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const float4 g = lds_f4(gs + i * 1024 + ((c ^ mg) << 4));
+#pragma unroll
+                for (int r = 0; r < TR; ++r) acc[i][r] = __ffma2_rn(make_float2(g.x, g.y), make_float2(b[r].x, b[r].y), acc[i][r]);
+#pragma unroll
+                for (int r = 0; r < TR; ++r) acc[i][r] = __ffma2_rn(make_float2(g.z, g.w), make_float2(b[r].z, b[r].w), acc[i][r]);
+            }
+        }
+        // the stage has been read by this warp; the last warp to say so refills it
+        __syncwarp();
+        if (lane == 0) {
+            __threadfence_block();
+            unsigned old;
+            asm volatile("atom.shared.add.u32 %0, [%1], 1;" : "=r"(old) : "r"(reads + s * 4) : "memory");
+            if (old == static_cast<unsigned>(AREAS * (t / STAGES + 1) - 1) && t + STAGES < T) {
+                __threadfence_block();
+                fence_proxy_async();
+                fill(t + STAGES);
+            }
+        }
+        __syncwarp();
+        // this patch of the accumulator, after the vector before has been added to it
+        if (GROUPS > 1 && t > 0) {
+            const int from = (t - 1) % GROUPS;
+            if (!__all_sync(0xffffffffu, mbar_wait_bounded(tokens + (area * GROUPS + from) * 8, ((t - 1) / GROUPS) & 1, abort_word))) break;
+        }
+        if (GROUPS == 1) __syncwarp();
+#pragma unroll
+        for (int r = 0; r < TR; ++r) {
+            if (k_of[r] >= 0) {
+                const int k = (wq * (4 * TR) + r * 4 + wg) / NKEEP * 32 + k_of[r];
+                const uint32_t p = sums + k * (MT * 4) + mh * 256 + ((mg ^ (k & 7)) << 4);
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    float4 x = lds_f4(p + h * 128);
+                    x.x += acc[4 * h][r].x + acc[4 * h][r].y;
+                    x.y += acc[4 * h + 1][r].x + acc[4 * h + 1][r].y;
+                    x.z += acc[4 * h + 2][r].x + acc[4 * h + 2][r].y;
+                    x.w += acc[4 * h + 3][r].x + acc[4 * h + 3][r].y;
+                    sts_f4(p + h * 128, x);
+                }
+            }
+        }
+        __syncwarp();
+        if (GROUPS > 1 && lane == 0) mbar_arrive(tokens + (area * GROUPS + group) * 8);
+    }
+    __syncthreads();
+    grid_launch_dependents();
+    if (lds_volatile_s32(abort_word) != 0) {
+        if (tid == 0) atomicMax(a.status, kDevTimeoutFull);
+        return;
+    }
+    // a warp per row of the tile, lanes along k (four lanes of a load meet in a bank: 1.5 % of a tile's time)
+    for (int m = warp; m < MT; m += Cfg::WARPS) {
+        if (m0 + m >= a.M) continue;
+        const int h = (m >> 5) & 1, x = (m >> 3) & 3;      // i = (m % 64) / 8 = 4 h + x
+        for (int k = lane; k < KT; k += 32) {
+            if (k0 + k >= a.K) break;
+            const float val = __uint_as_float(lds_u32(sums + k * (MT * 4) + (m >> 6) * 256 + h * 128 + (((m & 7) ^ (k & 7)) << 4) + x * 4));
+            if (sliced) a.partial[(static_cast<size_t>(slot) * MT + m) * KT + k] = val;
+            else store_as(a.out, static_cast<size_t>(m0 + m) * a.K + k0 + k, val, a.dtype);
+        }
+    }
+}
+
+// Adds the slices of split tiles (slots of rows x cols floats, one after the other) in order and
+// writes the elements that exist.  One float4 per thread.
+__global__ void __launch_bounds__(256) nm_grad_reduce_kernel(const GradArgs a, int rows, int cols, int out_rows, int out_cols)
+{
+    const int per_row = cols / 4, ctas = (rows * per_row + 255) / 256;
+    const int i = blockIdx.x / ctas, e = (blockIdx.x - i * ctas) * 256 + threadIdx.x;
+    const int tile = a.n_whole + i, ty = tile / a.tiles_x, tx = tile - ty * a.tiles_x;
+    const int r = e / per_row, c = (e - r * per_row) * 4;
+    grid_dependency_wait();
+    if (*reinterpret_cast<volatile int*>(a.status) != 0) return;       // a wait gave up: the slices are incomplete
+    if (r >= rows || ty * rows + r >= out_rows || tx * cols + c >= out_cols) return;
+    const float4* src = reinterpret_cast<const float4*>(a.partial + (static_cast<size_t>(i) * a.slices * rows + r) * cols + c);
+    const size_t step = static_cast<size_t>(rows) * cols / 4;
+    float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int z = 0; z < a.slices; z += 4) {
+        float4 x[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (z + u < a.slices) x[u] = __ldcg(src + (z + u) * step);
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (z + u < a.slices) { sum.x += x[u].x; sum.y += x[u].y; sum.z += x[u].z; sum.w += x[u].w; }
+    }
+    const size_t at = static_cast<size_t>(ty * rows + r) * out_cols + tx * cols + c;
+    if (a.dtype == kDtypeF32) {
+        *reinterpret_cast<float4*>(static_cast<float*>(a.out) + at) = sum;
+    } else {
+        store_as(a.out, at, sum.x, a.dtype);
+        store_as(a.out, at + 1, sum.y, a.dtype);
+        store_as(a.out, at + 2, sum.z, a.dtype);
+        store_as(a.out, at + 3, sum.w, a.dtype);
+    }
+}
+
+// ---------------------------------------------------------------------------------------- host side
+// How a grid of equal tiles over `steps` contraction steps is cut: whole tiles while they fill
+// rounds of `slots` CTAs, the rest in S slices each.  S minimises the rounds of the rest, in
+// units of a whole tile, plus what a slice costs besides (its scratch slot written and read back
+// by the reduction: `slot_cost`, as a share of a tile's time).
+static void cut_tiles(int tiles, int slots, int steps, int least_steps, double slot_cost, int* whole, int* slices)
+{
+    *whole = tiles / slots * slots;
+    const int rest = tiles - *whole;
+    *slices = 1;
+    if (rest == 0) return;
+    double best = 1.0;
+    for (int s = 2; s <= 32 && steps / s >= least_steps; ++s) {
+        const long long ctas = static_cast<long long>(rest) * s;
+        const double cost = static_cast<double>((ctas + slots - 1) / slots) / s + slot_cost * (static_cast<double>(ctas) / slots);
+        if (cost < best * 0.98) {
+            best = cost;
+            *slices = s;
+        }
+    }
+    if (*slices == 1) *whole = tiles;
+}
+
+struct GradPlan {
+    int tiles_x = 0, tiles = 0, whole = 0, slices = 1, rows = 0, cols = 0;
+    size_t partial_floats() const { return slices > 1 ? static_cast<size_t>(tiles - whole) * slices * rows * cols : 0; }
+    int ctas() const { return whole + (tiles - whole) * slices; }
+};
+
+template <int NKEEP>
+static GradPlan plan_values(int M, int N, int W, int sms)
+{
+    using Cfg = GradValuesCfg<NKEEP>;
+    GradPlan p;
+    p.rows = Cfg::RW;
+    p.cols = 128;
+    p.tiles_x = (N + 127) / 128;
+    p.tiles = p.tiles_x * ((W + Cfg::RW - 1) / Cfg::RW);
+    cut_tiles(p.tiles, sms * 3, (M + Cfg::MC - 1) / Cfg::MC, 4, 10.0 / (M > 10 ? M : 10), &p.whole, &p.slices);
+    return p;
+}
+
+template <int NKEEP>
+static GradPlan plan_input(int M, int N, int K, int sms)
+{
+    using Cfg = GradInputCfg<NKEEP>;
+    GradPlan p;
+    p.rows = Cfg::MT;
+    p.cols = Cfg::KT;
+    p.tiles_x = (K + Cfg::KT - 1) / Cfg::KT;
+    p.tiles = p.tiles_x * ((M + Cfg::MT - 1) / Cfg::MT);
+    cut_tiles(p.tiles, sms, N / 32, 4, 4.0 / (N / 32 > 4 ? N / 32 : 4), &p.whole, &p.slices);
+    return p;
+}
+
+template <typename Kernel>
+static cudaError_t allow_smem(Kernel kernel, int bytes, bool* configured)
+{
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess || dev >= 64 || configured[dev]) return e;
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess) configured[dev] = true;
+    return e;
+}
+
+static cudaError_t launch_quad_rows(int dtype, const void* x, float* out, int M, int K, cudaStream_t st)
+{
+    const size_t n = static_cast<size_t>((M + 3) / 4) * K, want = (n + 255) / 256;
+    const unsigned blocks = static_cast<unsigned>(want < 148 * 32 ? want : 148 * 32);
+    float4* o = reinterpret_cast<float4*>(out);
+    if (dtype == kDtypeF32) quad_rows_kernel<float><<<blocks, 256, 0, st>>>(static_cast<const float*>(x), o, M, K);
+    else if (dtype == kDtypeF16) quad_rows_kernel<__half><<<blocks, 256, 0, st>>>(static_cast<const __half*>(x), o, M, K);
+    else quad_rows_kernel<__nv_bfloat16><<<blocks, 256, 0, st>>>(static_cast<const __nv_bfloat16*>(x), o, M, K);
+    return cudaGetLastError();
+}
+
+static cudaError_t launch_grad_reduce(const GradArgs& a, const GradPlan& p, int out_rows, int out_cols, cudaStream_t st)
+{
+    const int ctas = (p.rows * p.cols / 4 + 255) / 256;
+    return launch_overlapped(nm_grad_reduce_kernel, (p.tiles - p.whole) * ctas, 256, 0, st, a, p.rows, p.cols, out_rows, out_cols);
+}
+
+template <int NKEEP>
+static cudaError_t launch_values(GradArgs a, const GradPlan& p, const float* grad_y, cudaStream_t st)
+{
+    using Cfg = GradValuesCfg<NKEEP>;
+    static bool configured[64] = {};
+    cudaError_t e = allow_smem(nm_grad_values_kernel<NKEEP>, Cfg::SMEM_BYTES, configured);
+    if (e != cudaSuccess) return e;
+    CUtensorMap map_g;
+    e = encode_tensor_map_2d(&map_g, grad_y, a.N, a.M, 128, Cfg::MC, 0);
+    if (e != cudaSuccess) return e;
+    a.tiles_x = p.tiles_x;
+    a.n_whole = p.whole;
+    a.slices = p.slices;
+    a.dtype = kDtypeF32;
+    e = launch_overlapped(nm_grad_values_kernel<NKEEP>, p.ctas(), Cfg::THREADS, Cfg::SMEM_BYTES, st, a, map_g);
+    if (e == cudaSuccess && p.slices > 1) e = launch_grad_reduce(a, p, a.W, a.N, st);
+    return e;
+}
+
+template <int NKEEP>
+static cudaError_t launch_input(GradArgs a, const GradPlan& p, const float* grad_y, cudaStream_t st)
+{
+    using Cfg = GradInputCfg<NKEEP>;
+    static bool configured[64] = {};
+    cudaError_t e = allow_smem(nm_grad_input_kernel<NKEEP>, Cfg::SMEM_BYTES, configured);
+    if (e != cudaSuccess) return e;
+    CUtensorMap map_g, map_b;
+    e = encode_tensor_map_2d(&map_g, grad_y, a.N, a.M, 32, Cfg::MT, 2);
+    if (e != cudaSuccess) return e;
+    e = encode_tensor_map_2d(&map_b, a.B, a.N, a.W, 32, Cfg::WT, 2);
+    if (e != cudaSuccess) return e;
+    a.tiles_x = p.tiles_x;
+    a.n_whole = p.whole;
+    a.slices = p.slices;
+    e = launch_overlapped(nm_grad_input_kernel<NKEEP>, p.ctas(), Cfg::THREADS, Cfg::SMEM_BYTES, st, a, map_g, map_b);
+    if (e == cudaSuccess && p.slices > 1) e = launch_grad_reduce(a, p, a.M, a.K, st);
+    return e;
+}
+
+#define NMSPMM_BY_RATIO(call)                       \
+    switch (n_keep) {                               \
+    case 16: return call(16);                       \
+    case 12: return call(12);                       \
+    case 8: return call(8);                         \
+    case 4: return call(4);                         \
+    default: break;                                 \
+    }
+
+bool linear_grad_supported(int n_keep) { return n_keep == 16 || n_keep == 12 || n_keep == 8 || n_keep == 4; }
+
+size_t grad_values_scratch_bytes(int M, int N, int K, int n_keep, int sms)
+{
+    const size_t quads = static_cast<size_t>((M + 3) / 4) * 4 * K;
+    const int W = K / 32 * n_keep;
+#define NMSPMM_CALL(R) (quads + plan_values<R>(M, N, W, sms).partial_floats()) * sizeof(float)
+    NMSPMM_BY_RATIO(NMSPMM_CALL)
+#undef NMSPMM_CALL
+    return 0;
+}
+
+size_t grad_input_scratch_bytes(int M, int N, int K, int n_keep, int sms)
+{
+#define NMSPMM_CALL(R) plan_input<R>(M, N, K, sms).partial_floats() * sizeof(float)
+    NMSPMM_BY_RATIO(NMSPMM_CALL)
+#undef NMSPMM_CALL
+    return 0;
+}
+
+cudaError_t launch_grad_values(int dtype, const void* x, const float* grad_y, const int* DT, float* grad_B, int M, int N, int K,
+                               int n_keep, int sms, float* scratch, int* status, cudaStream_t st)
+{
+    cudaError_t e = launch_quad_rows(dtype, x, scratch, M, K, st);
+    if (e != cudaSuccess) return e;
+    GradArgs a {};
+    a.DT = DT;
+    a.xq = scratch;
+    a.out = grad_B;
+    a.partial = scratch + static_cast<size_t>((M + 3) / 4) * 4 * K;
+    a.status = status;
+    a.M = M; a.N = N; a.K = K; a.W = K / 32 * n_keep;
+#define NMSPMM_CALL(R) launch_values<R>(a, plan_values<R>(M, N, a.W, sms), grad_y, st)
+    NMSPMM_BY_RATIO(NMSPMM_CALL)
+#undef NMSPMM_CALL
+    return cudaErrorInvalidValue;
+}
+
+cudaError_t launch_grad_input(int dtype, const float* grad_y, const float* B, const int* DT, void* grad_x, int M, int N, int K,
+                              int n_keep, int sms, float* scratch, int* status, cudaStream_t st)
+{
+    GradArgs a {};
+    a.DT = DT;
+    a.B = B;
+    a.out = grad_x;
+    a.partial = scratch;
+    a.status = status;
+    a.dtype = dtype;
+    a.M = M; a.N = N; a.K = K; a.W = K / 32 * n_keep;
+#define NMSPMM_CALL(R) launch_input<R>(a, plan_input<R>(M, N, K, sms), grad_y, st)
+    NMSPMM_BY_RATIO(NMSPMM_CALL)
+#undef NMSPMM_CALL
+    return cudaErrorInvalidValue;
+}
+
+}  // namespace nmspmm

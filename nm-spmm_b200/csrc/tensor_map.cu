@@ -30,7 +30,7 @@ static EncodeTiledFn encode_fn()
 // host thread are kept, keyed by everything that goes into them.
 struct MapKey {
     const void* base;
-    int cols, rows, box_a, box_b, kind;       // kind: 0 plain 2-D, 1 swizzled 2-D, 2 blocks of 32 columns
+    int cols, rows, box_a, box_b, kind;       // kind: 0 plain 2-D, 1 / 3 swizzled 2-D (32- / 16-byte chunks), 2 blocks of 32 columns
     bool operator==(const MapKey& o) const
     {
         return base == o.base && cols == o.cols && rows == o.rows && box_a == o.box_a && box_b == o.box_b && kind == o.kind;
@@ -64,7 +64,7 @@ static thread_local MapCache tl_maps;
 cudaError_t encode_tensor_map_2d(CUtensorMap* map, const float* base, int cols, int rows, int box_cols, int box_rows,
                                  int swizzle128)
 {
-    const MapKey mk { base, cols, rows, box_cols, box_rows, swizzle128 ? 1 : 0 };
+    const MapKey mk { base, cols, rows, box_cols, box_rows, swizzle128 == 2 ? 3 : swizzle128 };
     if (tl_maps.find(mk, map)) return cudaSuccess;
     EncodeTiledFn fn = encode_fn();
     if (!fn) return cudaErrorNotSupported;
@@ -73,7 +73,9 @@ cudaError_t encode_tensor_map_2d(CUtensorMap* map, const float* base, int cols, 
     const cuuint32_t box[2] = { static_cast<cuuint32_t>(box_cols), static_cast<cuuint32_t>(box_rows) };
     const cuuint32_t elem[2] = { 1, 1 };
     const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(base), dims, strides, box, elem,
-                          CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B : CU_TENSOR_MAP_SWIZZLE_NONE,
+                          CU_TENSOR_MAP_INTERLEAVE_NONE,
+                          swizzle128 == 2 ? CU_TENSOR_MAP_SWIZZLE_128B
+                                          : (swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B : CU_TENSOR_MAP_SWIZZLE_NONE),
                           CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r == CUDA_SUCCESS) tl_maps.put(mk, *map);

@@ -10,9 +10,12 @@ multiply); nothing is padded or transposed in eager PyTorch.  float16 / bfloat16
 give a result of the same dtype (``nmspmm_gemm_row_major_16``: widened exactly inside the
 transposition, summed in FP32, rounded once at the end); the compressed weights are FP32.
 
+The backward pass runs on the compressed weight too (``nmspmm_linear_grad``: both gradients in
+FP32, n_keep / 32 of the work of the dense products); an unpruned weight (32 of 32) and a
+backward that is itself to be differentiated take torch's own products.
+
 The reference has no framework binding (its only caller is its test driver,
-tests/test_nmspmm.cu:8-160).  The backward pass is a convenience, not a tuned path: it
-expands the compressed weight to dense and uses torch's own products.
+tests/test_nmspmm.cu:8-160).
 """
 import ctypes
 from typing import Optional
@@ -31,6 +34,27 @@ def _dense_rows(raw_indices, n_keep: int):
     torch = _torch()
     win = torch.arange(raw_indices.shape[0], device=raw_indices.device) // n_keep
     return (raw_indices.to(torch.int64) + (win * 32)[:, None]).repeat_interleave(32, dim=1)
+
+
+def _sparse_grads(pkg, x, values, raw_indices, n_keep: int, grad_y, want_x: bool, want_values: bool):
+    """(grad_x, grad_values) by nmspmm_linear_grad, None where not wanted."""
+    torch = _torch()
+    lib = pkg.load_library()
+    x, values, grad_y = x.contiguous(), values.contiguous(), grad_y.to(x.dtype).contiguous()
+    if grad_y.data_ptr() % 16 != 0:
+        grad_y = grad_y.clone()                                           # a view into the middle of a buffer: TMA wants 16 bytes
+    dtype = pkg.dtype_id(x.dtype)
+    d = pkg.make_desc(x.shape[0], values.shape[1], x.shape[1], n_keep, pkg.FORMAT_LOW, 32)
+    grad_x = torch.empty_like(x) if want_x else None
+    grad_values = torch.empty_like(values) if want_values else None
+    need = int(lib.nmspmm_linear_grad_workspace_bytes(ctypes.byref(d), dtype, int(want_x), int(want_values)))
+    ws = torch.empty(need, dtype=torch.uint8, device=x.device)
+    ptr = lambda t: ctypes.c_void_p(0 if t is None else t.data_ptr())  # noqa: E731
+    rc = lib.nmspmm_linear_grad(ctypes.byref(d), dtype, ptr(x), ptr(grad_y), ptr(values), ptr(raw_indices), ptr(grad_x), ptr(grad_values),
+                                ptr(ws), need, ctypes.c_void_p(torch.cuda.current_stream(x.device).cuda_stream))
+    if rc != pkg.OK:
+        raise pkg.NMSpMMError("nmspmm_linear_grad", rc)
+    return grad_x, grad_values
 
 
 def register_ops(pkg):
@@ -83,14 +107,18 @@ def register_ops(pkg):
 
     def backward(ctx, grad_y):
         x, values, raw_indices = ctx.saved_tensors
+        want_x, want_values = ctx.needs_input_grad[0], ctx.needs_input_grad[1]
+        # (with create_graph the formula has to be differentiable itself: the dense products below)
+        if ctx.n_keep in (16, 12, 8, 4) and not torch.is_grad_enabled():
+            return (*_sparse_grads(pkg, x, values, raw_indices, ctx.n_keep, grad_y, want_x, want_values), *[None] * 8)
         rows = _dense_rows(raw_indices, ctx.n_keep)                       # (W, N) global k of every kept value
         grad_x = grad_values = None
         g32 = grad_y.to(torch.float32)
-        if ctx.needs_input_grad[0]:
+        if want_x:
             dense = torch.zeros((x.shape[1], values.shape[1]), dtype=torch.float32, device=values.device)
             dense.scatter_(0, rows, values)                               # B with explicit zeros, (K, N)
             grad_x = (g32 @ dense.t()).to(x.dtype)
-        if ctx.needs_input_grad[1]:
+        if want_values:
             grad_values = (x.to(torch.float32).t() @ g32).gather(0, rows)  # d/dB restricted to the kept positions
         return grad_x, grad_values, None, None, None, None, None, None, None, None
 
