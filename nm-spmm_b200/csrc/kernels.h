@@ -96,11 +96,11 @@ cudaError_t launch_reduce_slices(int ns, const GemmArgs& args, const GemmOutputs
 // finishing.  Every kernel launched this way executes griddepcontrol.wait before its first
 // access to global memory.
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_overlapped(void (*kernel)(KArgs...), unsigned blocks, unsigned threads, size_t smem_bytes,
+inline cudaError_t launch_overlapped(void (*kernel)(KArgs...), dim3 blocks, unsigned threads, size_t smem_bytes,
                                      cudaStream_t st, Args... args)
 {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(blocks);
+    cfg.gridDim = blocks;
     cfg.blockDim = dim3(threads);
     cfg.dynamicSmemBytes = smem_bytes;
     cfg.stream = st;

@@ -42,17 +42,20 @@ __global__ void __launch_bounds__(256) retile_kernel(const int* __restrict__ DT,
 }
 
 // PreProcessing_high_sparsity (src/preprocessing.cu:17-78), optionally with
-// transIndex folded in.  A CTA handles one merged window (pn rows) of up to 32
+// transIndex folded in.  A CTA handles one merged window (pn rows) of up to 8
 // index blocks: the window's rows are read coalesced into shared memory, then each
-// warp takes blocks in turn: it ORs a 64-bit mask of the local columns its block
+// warp takes one block: it ORs a 64-bit mask of the local columns its block
 // uses, writes the ascending list (-1 padded) to column_info and each index's rank
 // (population count of the mask below it) to the re-tiled D.
 //   pn, pm: merged window (rows kept / width, pm <= 64).  fuse != 0: DT holds raw
 //   0..pm/2-1 indices and rows x >= pn/2 of a window belong to its odd half.
-constexpr int kHighBlocksPerCta = 32;
+// Latency-bound (3 MB at 4096 x 11008, 4 of 32): a block per warp and no second pass over a CTA's
+// blocks -- with 32 blocks per CTA, four per warp, the packing took 7.8 us there and the
+// separate launch that filled the list's tail 1.8.
+constexpr int kHighBlocksPerCta = 8;
 __global__ void __launch_bounds__(256) preprocess_high_kernel(const int* __restrict__ DT, int* __restrict__ D,
                                                               int* __restrict__ cinfo, int pm, int pn, int W, int Q,
-                                                              int Qs, int fuse)
+                                                              int Qs, int fuse, int tail_ints)
 {
     extern __shared__ int rows[];                  // [pn][kHighBlocksPerCta * Qs + Qs]: padded, see pitch
     const int win = blockIdx.x;
@@ -63,6 +66,9 @@ __global__ void __launch_bounds__(256) preprocess_high_kernel(const int* __restr
     // a warp reads one block's [pn][Qs] indices, Qs from each row: Qs extra ints per row
     // put consecutive rows Qs banks apart (an unpadded pitch made that an 8-way conflict)
     const int pitch = kHighBlocksPerCta * Qs + Qs;
+    grid_dependency_wait();
+    if (blockIdx.x == 0 && blockIdx.y == 0)                // the extra window behind the last list: all -1
+        for (int t = threadIdx.x; t < tail_ints; t += blockDim.x) cinfo[static_cast<size_t>(nblk_total) * gridDim.x * pm + t] = -1;
     for (int t = threadIdx.x; t < pn * width; t += blockDim.x) {
         const int x = t / width, c = t % width;
         int v = DT[static_cast<size_t>(win * pn + x) * Q + blk0 * Qs + c];
@@ -97,12 +103,6 @@ __global__ void __launch_bounds__(256) preprocess_high_kernel(const int* __restr
     }
 }
 
-__global__ void fill_kernel(int* p, int n, int value)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) p[i] = value;
-}
-
 cudaError_t launch_trans_index(int* DT, int W, int Q, int pruning_N, int pruning_M, cudaStream_t st)
 {
     const long long total = static_cast<long long>(W) * Q;
@@ -128,14 +128,7 @@ cudaError_t launch_preprocess_high(const int* DT, int* D, int* cinfo, int pm, in
     const int nblk = Q / Qs, nwin = W / pn;
     dim3 grid(nwin, (nblk + kHighBlocksPerCta - 1) / kHighBlocksPerCta);
     const size_t smem = static_cast<size_t>(pn) * (kHighBlocksPerCta * Qs + Qs) * sizeof(int);
-    preprocess_high_kernel<<<grid, 256, smem, st>>>(DT, D, cinfo, pm, pn, W, Q, Qs, fuse);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    if (tail_ints > 0) {
-        fill_kernel<<<(tail_ints + 255) / 256, 256, 0, st>>>(cinfo + static_cast<size_t>(nblk) * nwin * pm, tail_ints, -1);
-        e = cudaGetLastError();
-    }
-    return e;
+    return launch_overlapped(preprocess_high_kernel, grid, 256, smem, st, DT, D, cinfo, pm, pn, W, Q, Qs, fuse, tail_ints);
 }
 
 // Row-major activations [M][K] -> the reference's col-major A, i.e. [K][ld] with ld >= M,

@@ -101,6 +101,17 @@ def test_prune_device_matches_the_host_generator(pkg, n_keep, vec_len):
     assert np.array_equal(BT.cpu().numpy(), want_BT)
 
 
+@pytest.mark.parametrize("K,N,vec_len", [(32, 32, 32), (32, 96, 32), (64, 32 * 9, 32), (32, 64, 64), (96, 64 * 5, 64)])
+@pytest.mark.parametrize("n_keep", [1, 8, 31])
+def test_prune_device_with_few_and_uneven_units(pkg, K, N, vec_len, n_keep):
+    """Fewer (window, vector) units than a CTA has warps, and counts that leave its last warps idle."""
+    Bd = np.random.default_rng(K * N + n_keep).standard_normal((K, N)).astype(np.float32)
+    BT, DT = pkg.prune_device(torch.from_numpy(Bd).cuda(), n_keep, vec_len)
+    want_BT, want_DT = pkg.formats.prune_magnitude(Bd, n_keep, vec_len)
+    assert np.array_equal(DT.cpu().numpy(), want_DT)
+    assert np.array_equal(BT.cpu().numpy(), want_BT)
+
+
 @pytest.mark.parametrize("vec_len", [32, 64])
 def test_prune_device_against_an_independent_statement_of_the_rule(pkg, vec_len):
     """The LLM-linear weight (4096 x 11008, N(0, 0.02^2)) pruned on the GPU, checked against the
