@@ -144,15 +144,30 @@ static int check_desc(const nmspmm_gemm_desc* d, int* mode_out, bool any_rows = 
     return NMSPMM_OK;
 }
 
+// Whether the exact path stages this shape's 16:32 / 12:32 windows in pairs on tile 128 x 128.
+static bool staged_in_pairs(const nmspmm_gemm_desc* d)
+{
+    return d->format == NMSPMM_FORMAT_LOW && (d->n_keep == 16 || d->n_keep == 12) && d->K >= 512;      // short K keeps the finer windows for splitting
+}
+
+// Tile of the exact path.  Over 64 rows: 64 x 128 where it pads fewer rows than 128 x 128 does.
+// The pairs of windows that 16:32 and 12:32 have on 128 x 128 alone are worth more than the
+// padding except between 128 and 192 rows (256 padded rows count as 213): at 5760 columns, K = 2080,
+// 12:32, 776 / 1032 / 320 / 192 rows take 159 / 202 / 82 / 59 us on it, 172 / 212 / 82 / 53 on 64 x 128; at
+// 4096 x 4096, 16:32, 904 / 448 / 192 rows 311 / 166 / 88 against 346 / 173 / 81.
 static int pick_tile(const nmspmm_gemm_desc* d, int sms)
 {
     (void)sms;
     if (d->M <= 16) return kTile16x128;
     if (d->M <= 32) return kTile32x128;
     if (d->M <= 64) return kTile64x128;
-    const int pad128 = (d->M + 127) / 128 * 128, pad64 = (d->M + 63) / 64 * 64;
-    return (pad64 < pad128) ? kTile64x128 : kTile128x128;
+    const long long pad128 = (static_cast<long long>(d->M) + 127) / 128 * 128, pad64 = (static_cast<long long>(d->M) + 63) / 64 * 64;
+    return (pad64 * 100 < pad128 * (staged_in_pairs(d) ? 83 : 100)) ? kTile64x128 : kTile128x128;
 }
+
+// Least share of the CTA slots, in per cent, that slices of equal length have to keep busy to be
+// taken over ranges that cross tiles (below).
+constexpr int kEvenSlicesPercent = 95;
 
 // ---- tuned plans ------------------------------------------------------------------
 // (M, N, K, n_keep, format, path, vec_len) -> tile and split_k found by measurement
@@ -445,9 +460,9 @@ static int make_plan(const nmspmm_gemm_desc* d_in, int sms, Plan* p, bool any_ro
     const int tile = d->tile ? d->tile : pick_tile(d, sms);
     const FfmaVariant* v = find_ffma_variant(tile, d->n_keep, mode);
     if (!v) return NMSPMM_UNSUPPORTED;
-    // 16:32 and 12:32 on the 128 x 128 tile: two 32-k windows per stage when K allows it
-    // (half as many CTA barriers per k: 1.232 -> 1.190 ms at 4096^3, 16:32)
-    if (mode == kModeLow && tile == kTile128x128 && d->K % 64 == 0 && d->K >= 512) {      // short K keeps the finer windows for splitting
+    // 16:32 and 12:32 on the 128 x 128 tile: two 32-k windows per stage (half as many CTA barriers
+    // per k: 1.232 -> 1.190 ms at 4096^3, 16:32); the last pair of an odd number holds one window
+    if (tile == kTile128x128 && staged_in_pairs(d)) {
         if (d->n_keep == 16 && kFfma_low16p_count > 0) v = &kFfma_low16p[0];
         if (d->n_keep == 12 && kFfma_low12p_count > 0) v = &kFfma_low12p[0];
     }
@@ -455,7 +470,7 @@ static int make_plan(const nmspmm_gemm_desc* d_in, int sms, Plan* p, bool any_ro
     p->ws = v->ws;
     const int ws = v->ws;
     p->W = d->K / 32 * d->n_keep;
-    p->n_win = p->W / ws;
+    p->n_win = (p->W + ws - 1) / ws;                       // (a pair at the end may hold one window)
     p->tiles_x = (d->N + v->ns - 1) / v->ns;
     p->tiles_y = (d->M + v->ms - 1) / v->ms;
     const long long n_tiles = static_cast<long long>(p->tiles_x) * p->tiles_y;
@@ -497,6 +512,14 @@ static int make_plan(const nmspmm_gemm_desc* d_in, int sms, Plan* p, bool any_ro
             if (n_sk > by_length) n_sk = by_length;
             if (n_sk > tail_units) n_sk = tail_units;
             if (n_sk < 1) n_sk = 1;
+            // A problem of less than one wave: ranges that are a whole number of slices of each tile
+            // where they keep nearly all of the CTA slots busy: no CTA then holds pieces of two tiles, and one slice per tile
+            // needs no scratch.  585 tiles on 592 slots (776 x 5760, K = 2048, 8:32): 117 -> 106 us, 288 on
+            // 296 (1032 x 4096 x 4096): 198 -> 188; at 86 to 91 % of the slots it gains at 4:32 and
+            // loses up to 9 % at 16:32, below it loses everywhere.  (Behind whole waves the choice
+            // moves nothing: the tail is short.)
+            const long long even = n_sk / tail_tiles * tail_tiles;
+            if (n_dp == 0 && even * 100 >= n_sk * kEvenSlicesPercent) n_sk = even;
         }
         p->split_k = 0;
         p->n_dp = static_cast<int>(n_dp);

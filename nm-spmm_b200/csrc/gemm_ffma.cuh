@@ -43,7 +43,7 @@ namespace nmspmm {
 template <int MS, int NS, int WM, int WS, int KS_, int MODE>
 struct FfmaCfg {
     static constexpr int KS = KS_;                       // rows of A staged per window: 32, or 64 (a merged HIGH window)
-    static constexpr bool PAIR = (MODE == kModeLow && KS_ == 64);    // LOW staged as pairs of 32-k windows (WS = 2 n_keep)
+    static constexpr bool PAIR = (MODE == kModeLow && KS_ == 64);    // LOW staged as pairs of 32-k windows (WS = 2 n_keep); the last may hold one
     static constexpr bool BANDED = (MODE == kModeLow && WS % 16 == 0);   // 16:32 and unpruned: the tile order may be banded (see tile_position)
     static_assert(KS_ == 64 || (MODE == kModeLow && KS_ == 32), "LOW windows are 32 k wide, staged singly or in pairs; HIGH windows are 64 k wide");
     static constexpr int QT = NS / kVecLen;              // vectors per tile
@@ -151,15 +151,29 @@ __device__ __forceinline__ void nm_gemm_ffma_body(const GemmArgs& g, const CUten
         const int lb0 = bj >> layout_shift;                // first packed index block under the tile
         const int nlb = ((bj + cols - 1) >> layout_shift) - lb0 + 1;
         const uint32_t as = ring + s * Cfg::STAGE_BYTES, bs = as + Cfg::A_BYTES, ds = bs + Cfg::B_BYTES;
+        uint32_t i_bytes = d_bytes;                        // index bytes of one block that exist
+        if constexpr (Cfg::PAIR) {
+            // The last pair of an odd number of windows: its second window's rows of A and B
+            // arrive as zeros; its indices do not exist and become 0, a row inside the stage.
+            const int rows = g.W - win * WS;
+            if (rows < WS) {
+                i_bytes = static_cast<uint32_t>(rows << qs_shift) * 4u;
+                for (int o = lane; o < nlb * (d_chunk >> 1); o += 32) {
+                    const int b = o / (d_chunk >> 1);
+                    sts_s32(ds + b * d_bytes + i_bytes + (o - b * (d_chunk >> 1)) * 4, 0);
+                }
+                __syncwarp();
+            }
+        }
         if (lane == 0) {
-            mbar_arrive_expect_tx(full, Cfg::TX_FIXED + nlb * (d_bytes + (MODE == kModeHigh ? 256u : 0u)));
+            mbar_arrive_expect_tx(full, Cfg::TX_FIXED + nlb * (i_bytes + (MODE == kModeHigh ? 256u : 0u)));
             tma_load_2d(as, &map_a, bi, win * KS, full);      // rows/columns past the tensor arrive as zeros
             tma_load_2d(bs, &map_b, bj, win * WS, full);
         }
         __syncwarp();
         if (lane < nlb) {
             const int* src = g.D + ((static_cast<size_t>(lb0 + lane) * g.W) << qs_shift) + static_cast<size_t>(win) * d_chunk;
-            bulk_g2s(ds + lane * d_bytes, src, d_bytes, full);
+            bulk_g2s(ds + lane * d_bytes, src, i_bytes, full);
             if (MODE == kModeHigh) {
                 // one list per merged 64-k window
                 const int* ci = g.cinfo + (static_cast<size_t>(lb0 + lane) * g.sched.n_win + win) * 64;
@@ -426,7 +440,8 @@ cudaError_t launch_ffma(const GemmArgs& a, const GemmOutputs& outs, int grid, cu
         configured[dev] = true;
     }
     CUtensorMap map_a, map_b;
-    e = encode_tensor_map_2d(&map_a, a.A, outs.lda ? outs.lda : a.M, a.sched.n_win * Cfg::KS, MS, Cfg::KS);
+    const int K = Cfg::PAIR ? a.W / (WS / 2) * 32 : a.sched.n_win * Cfg::KS;     // the last pair may hold one window only
+    e = encode_tensor_map_2d(&map_a, a.A, outs.lda ? outs.lda : a.M, K, MS, Cfg::KS);
     if (e != cudaSuccess) return e;
     // (test hook: a box one row short delivers fewer bytes than the stage's barrier expects,
     // so that the kernel's bounded waits run out; see nmspmm_test_short_fill)

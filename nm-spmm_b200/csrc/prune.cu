@@ -15,9 +15,9 @@
 // lane = row on the global loads every instruction touched 32 lines and the L1's tag look-ups were
 // the bound (4096 x 11008, 4 of 32: 66 us, 2.8 TB/s of the 203 MB it moves).  Then lane = row: a lane
 // adds up its row's squares, ranks them against the other 31 (broadcast shared loads), and the kept
-// rows go out the way they came in.  A patch per warp and no register holds the tile, so that 48
+// rows go out the way they came in.  A patch per warp and no register holds the tile, so that 32
 // warps' copies are in flight on an SM.  Pruning and packing
-// together, 4096 x 11008, 4 of 32: 75.8 us with the former loads, 41.1 with these (232 MB, 5.6 TB/s).
+// together, 4096 x 11008, 4 of 32: 75.8 us with the former loads, 41.1 with these (206 MB, 5.0 TB/s).
 #include <cuda_runtime.h>
 #include <stdint.h>
 

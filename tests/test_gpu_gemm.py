@@ -57,6 +57,17 @@ def test_every_compiled_tile(pkg, orc, tile, n_keep, fmt, layout):
     assert rel_err(run(pkg, p, layout_ns=layout, fmt=fmt, tile=tile), want) <= FP32_TOL
 
 
+@pytest.mark.parametrize("windows", [17, 19, 33])
+@pytest.mark.parametrize("n_keep", [16, 12])
+@pytest.mark.parametrize("layout", [32, 64, 128])
+@pytest.mark.parametrize("split_k", [0, 3])
+def test_pairs_of_windows_with_an_odd_number_of_windows(pkg, orc, windows, n_keep, layout, split_k):
+    """16:32 and 12:32 on tile 128 x 128 stage two windows at a time; the last pair here holds one."""
+    p = pkg.formats.make_random(136, 384, 32 * windows, n_keep, seed=70 + windows)
+    want = orc.nm_gemm_f32(p.A_km, p.B_col, p.D_col)
+    assert rel_err(run(pkg, p, layout_ns=layout, tile=1, split_k=split_k), want) <= FP32_TOL
+
+
 @pytest.mark.parametrize("split_k", [2, 3, 5, 8, 64])
 @pytest.mark.parametrize("n_keep", [16, 8])
 def test_split_k_is_exact_and_deterministic(pkg, orc, n_keep, split_k):

@@ -272,3 +272,20 @@ def test_few_rows_plans(pkg):
     assert lib.nmspmm_gemm_workspace_bytes(ctypes.byref(too_few)) == 0   # 1024 windows per slice: refused
     # left to the library, the same split goes to the 128-row tiles instead
     assert pkg.plan(pkg.make_desc(16, 1024, 131072, 4, pkg.FORMAT_HIGH, 128, pkg.PATH_TF32, 2)).tile_m == 128
+
+
+def test_slices_of_equal_length_where_they_fill_the_slots(pkg):
+    """The last partial wave is cut into whole slices per tile when those keep 95 % of the CTA slots busy
+    (148 SMs), into ranges that cross tiles otherwise."""
+    whole = pkg.plan(pkg.make_desc(776, 5760, 2048, 8, 1, 128))                # 13 x 45 = 585 of 592: one slice per tile
+    assert (whole.tile_m, whole.n_dp, whole.n_virtual) == (64, 0, 585)
+    assert pkg.workspace_bytes(pkg.make_desc(776, 5760, 2048, 8, 1, 128)) == 0
+    assert pkg.plan(pkg.make_desc(1536, 1536, 8192, 8, 1, 128)).n_virtual == 288   # 144 tiles, two slices each
+    ranges = pkg.plan(pkg.make_desc(256, 4096, 4096, 8, 1, 128))               # 64 tiles: four slices each would leave 40 of 296 idle
+    assert ranges.n_virtual == 296
+
+
+@pytest.mark.parametrize("M,K,n_keep,tile_m", [(192, 2080, 12, 64), (320, 2080, 12, 128), (776, 2080, 16, 128), (320, 480, 12, 64),
+                                               (320, 2048, 8, 64), (192, 4096, 16, 64), (1032, 4096, 12, 128)])
+def test_tile_of_the_exact_path_follows_padding_and_pairs(pkg, M, K, n_keep, tile_m):
+    assert pkg.plan(pkg.make_desc(M, 4096, K, n_keep, pkg.format_of(n_keep), 128)).tile_m == tile_m
