@@ -784,13 +784,13 @@ int nmspmm_gemm_plan(const nmspmm_gemm_desc* desc, nmspmm_gemm_plan_info* out)
 // The multiply with its outputs spelled out: n_out buffers, row stride ldc, first column col0.
 static int gemm_launch(const nmspmm_gemm_desc* desc, const float* A_dev, const float* B_dev, const int* D_dev,
                        const int* column_info_dev, float* const* C_out, int n_out, long long ldc, int col0,
-                       void* workspace_dev, size_t workspace_bytes, void* stream, int lda = 0)
+                       void* workspace_dev, size_t workspace_bytes, void* stream, int lda = 0, int a_rows = 0, int c_dtype = kDtypeF32)
 {
     DeviceInfo* di = nullptr;
     int rc = device_info(&di);
     if (rc != NMSPMM_OK) return rc;
     Plan p;
-    rc = make_plan(desc, di->sms, &p, lda != 0);
+    rc = make_plan(desc, di->sms, &p, lda != 0 || a_rows != 0);
     if (rc != NMSPMM_OK) return rc;
     if (lda != 0 && (lda < desc->M || lda % 4 != 0)) return NMSPMM_INVALID_ARGUMENT;
     if (!A_dev || !B_dev || !D_dev || !C_out || n_out < 1 || n_out > kMaxOutputs) return NMSPMM_INVALID_ARGUMENT;
@@ -804,13 +804,15 @@ static int gemm_launch(const nmspmm_gemm_desc* desc, const float* A_dev, const f
     a.cinfo = column_info_dev;
     GemmOutputs outs {};
     for (int o = 0; o < n_out; ++o) {
-        if (!C_out[o] || !aligned16(C_out[o])) return NMSPMM_INVALID_ARGUMENT;
+        if (!C_out[o] || (c_dtype == kDtypeF32 && !aligned16(C_out[o]))) return NMSPMM_INVALID_ARGUMENT;
         if (o == 0) a.C = C_out[o]; else outs.C_more[o - 1] = C_out[o];
     }
     outs.n_out = n_out;
     outs.ldc = ldc;
     outs.col0 = col0;
     outs.lda = lda;
+    outs.a_rows = a_rows;
+    outs.c_dtype = c_dtype;
     a.status = di->status_word;
     a.M = desc->M;
     a.N = desc->N;
@@ -869,6 +871,10 @@ static size_t row_major_head_bytes(const Plan& p)
     return own > 0 ? own : kCounterBlock;
 }
 
+// The few-rows kernels read row-major activations as they are, through a tensor map (so they want
+// them on 16 bytes); the others get a col-major copy.
+static bool reads_rows(const Plan& p, const void* A_rows) { return p.tv && p.tv->form == 2 && aligned16(A_rows); }
+
 size_t nmspmm_gemm_row_major_workspace_bytes(const nmspmm_gemm_desc* desc)
 {
     Plan p;
@@ -886,10 +892,13 @@ int nmspmm_gemm_row_major(const nmspmm_gemm_desc* desc, const float* A_rows_dev,
     const size_t copy_bytes = row_major_copy_bytes(desc), own = p.counters_bytes + p.partial_bytes, head = row_major_head_bytes(p);
     if (workspace_bytes < head + copy_bytes) return NMSPMM_WORKSPACE_TOO_SMALL;
     const int ld = (desc->M + 3) / 4 * 4;
+    float* out[1] = { C_dev };
+    if (reads_rows(p, A_rows_dev))
+        return gemm_launch(desc, A_rows_dev, B_dev, D_dev, column_info_dev, out, 1, desc->N, 0, own ? workspace_dev : nullptr, own, stream, 0,
+                           1 + kDtypeF32);
     float* A_cols = reinterpret_cast<float*>(static_cast<unsigned char*>(workspace_dev) + head);
     cudaError_t e = launch_transpose_rows(A_rows_dev, A_cols, desc->M, desc->K, ld, static_cast<cudaStream_t>(stream));
     if (e != cudaSuccess) return cuda_fail(e);
-    float* out[1] = { C_dev };
     return gemm_launch(desc, A_cols, B_dev, D_dev, column_info_dev, out, 1, desc->N, 0, own ? workspace_dev : nullptr, own, stream, ld);
 }
 
@@ -925,8 +934,16 @@ int nmspmm_gemm_row_major_16(const nmspmm_gemm_desc* desc, int dtype, const void
     unsigned char* ws = static_cast<unsigned char*>(workspace_dev);
     float* A_cols = reinterpret_cast<float*>(ws + head);
     float* C32 = reinterpret_cast<float*>(ws + head + copy_bytes);
+    // The tensor-core path's kernels store C in 16 bits themselves; the exact path's, at the edge of
+    // their registers, leave that to a pass over an FP32 C.
+    float* const direct[1] = { static_cast<float*>(C_dev) };
+    if (reads_rows(p, A_rows_dev))
+        return gemm_launch(desc, static_cast<const float*>(A_rows_dev), B_dev, D_dev, column_info_dev, direct, 1, desc->N, 0,
+                           own ? ws : nullptr, own, stream, 0, 1 + dtype, dtype);
     cudaError_t e = launch_transpose_rows_16(dtype, A_rows_dev, A_cols, desc->M, desc->K, ld, st);
     if (e != cudaSuccess) return cuda_fail(e);
+    if (p.tv)
+        return gemm_launch(desc, A_cols, B_dev, D_dev, column_info_dev, direct, 1, desc->N, 0, own ? ws : nullptr, own, stream, ld, 0, dtype);
     float* out[1] = { C32 };
     rc = gemm_launch(desc, A_cols, B_dev, D_dev, column_info_dev, out, 1, desc->N, 0, own ? ws : nullptr, own, stream, ld);
     if (rc != NMSPMM_OK) return rc;

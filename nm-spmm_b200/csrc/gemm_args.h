@@ -11,6 +11,7 @@
 namespace nmspmm {
 
 enum { kModeLow = 0, kModeHigh = 1 };
+enum { kDtypeF32 = 0, kDtypeF16 = 1, kDtypeBF16 = 2 };   // nmspmm_dtype
 constexpr int kVecLenHost = 32;   // columns per vector (VEC_LEN of the reference API)
 
 // CTA tiles compiled into the library (rows x columns of C).
@@ -68,6 +69,8 @@ struct GemmOutputs {
     int col0;
     long long ldc;
     int lda;               // host side only (tensor-map encoding): floats between consecutive k rows of A; 0 = M
+    int c_dtype;           // type C is stored in (kDtype*): FP32 wherever there is more than one output
+    int a_rows;            // host side only: 0 = A is col-major, else A is row-major [M][K] of type a_rows - 1 (few-rows kernels)
 };
 NMSPMM_HD float* output_of(const GemmArgs& a, const GemmOutputs& o, int i) { return i == 0 ? a.C : o.C_more[i - 1]; }
 

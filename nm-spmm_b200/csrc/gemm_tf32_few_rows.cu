@@ -22,6 +22,12 @@
 //   * The k of every kept row of the CTA's windows (through column_info on the 64-k formats)
 //     is resolved once, before the loop, into shared memory: a window's arithmetic is far
 //     shorter than a trip to L2.
+//   * Row-major A (activations as a layer has them: FP32, half or bfloat16) is read as it lies in
+//     memory: a window is a box of MS rows x KS columns whose 16-byte chunks are swizzled within the
+//     rows, the fragment loads take one value each and widen it (exactly), and C is written in the
+//     activations' type.  A transposing launch ahead of the multiply and a rounding one behind it
+//     cost 2.9 + 2.6 us of 20 (and two launches) at 1 x 4096 x 4096.  The layer's
+//     whole pass there: 50.1 -> 43.3 us, the rest of it host time.
 //   * K slices of a tile leave their accumulators in scratch slots of MS x 128 floats and
 //     nm_reduce_slices_kernel adds them in k order; a tile computed by one CTA is stored
 //     directly (to every output buffer when the caller gathers).
@@ -31,16 +37,22 @@
 #include "common.cuh"
 #include "gemm_args.h"
 #include "kernels.h"
+#include "store16.cuh"
 
 namespace nmspmm {
 
-template <int MS_, int WS_, int KS_, int MODE_>
+// Where the fragments of A come from: col-major FP32 (blocks of 32-bit k rows), or row-major rows of
+// FP32 / half / bfloat16.
+enum { kSrcCols = 0, kSrcRows32 = 1, kSrcRowsF16 = 2, kSrcRowsBF16 = 3 };
+
+template <int MS_, int WS_, int KS_, int MODE_, int SRC_>
 struct FewRowsCfg {
     static constexpr int MS = MS_, NS = 128, WS = WS_, KS = KS_, MODE = MODE_;
     static constexpr int THREADS = 128, MB = MS / 16, GROUPS = WS / 8;
-    static constexpr bool A_PLAIN = (MS == 16);              // 16 rows: [KS][16] as it lies in memory; else swizzled blocks of 32 rows
+    static constexpr int SRC = SRC_;
+    static constexpr bool A_PLAIN = (SRC == kSrcCols && MS == 16);              // 16 rows: [KS][16] as it lies in memory; else swizzled blocks of 32 rows
     static constexpr int ABLK = (MS + 31) / 32;
-    static constexpr int A_BYTES = A_PLAIN ? KS * 64 : ABLK * KS * 128;
+    static constexpr int A_BYTES = SRC >= kSrcRowsF16 ? MS * KS * 2 : ((SRC == kSrcRows32 || A_PLAIN) ? MS * KS * 4 : ABLK * KS * 128);
     static constexpr int B_BYTES = 4 * WS * 128;             // [4 vectors][WS][32]
     static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
     static constexpr int STAGES = (MS == 16) ? 4 : ((MS == 32) ? 3 : 2);   // four CTAs per SM in every case
@@ -61,12 +73,34 @@ __device__ __forceinline__ void mma_tf32_16x8x8(float (&c)[4], const uint32_t (&
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-template <int MS_, int WS_, int KS_, int MODE_>
-__global__ void __launch_bounds__(128, (FewRowsCfg<MS_, WS_, KS_, MODE_>::MIN_BLOCKS))
+// Byte offset of element (m, k) in a window of row-major A: FP32 blocks of 32 k, or rows of KS
+// 16-bit values; 16-byte chunks swizzled by the row within 128-byte (KS = 32, 16 bits: 64-byte) rows.
+template <int SRC, int MS, int KS>
+__device__ __forceinline__ uint32_t row_element(int m, int k)
+{
+    if constexpr (SRC == kSrcRows32) return (k >> 5) * (MS * 128) + m * 128 + ((((k & 31) >> 2) ^ (m & 7)) << 4) + (k & 3) * 4;
+    else if constexpr (KS == 64) return m * 128 + (((k >> 3) ^ (m & 7)) << 4) + (k & 7) * 2;
+    else return m * 64 + (((k >> 3) ^ ((m >> 1) & 3)) << 4) + (k & 7) * 2;
+}
+template <int SRC>
+__device__ __forceinline__ uint32_t load_element(uint32_t addr)      // as an FP32 bit pattern
+{
+    if constexpr (SRC == kSrcRows32) {
+        return lds_u32(addr);
+    } else {
+        unsigned short h;
+        asm volatile("ld.shared.u16 %0, [%1];" : "=h"(h) : "r"(addr));
+        if constexpr (SRC == kSrcRowsBF16) return static_cast<uint32_t>(h) << 16;
+        else return __float_as_uint(__half2float(__ushort_as_half(h)));
+    }
+}
+
+template <int MS_, int WS_, int KS_, int MODE_, int SRC_>
+__global__ void __launch_bounds__(128, (FewRowsCfg<MS_, WS_, KS_, MODE_, SRC_>::MIN_BLOCKS))
 nm_gemm_tf32_few_rows_kernel(const GemmArgs g, const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                            const GemmOutputs outs, const int a_blocked)
 {
-    using Cfg = FewRowsCfg<MS_, WS_, KS_, MODE_>;
+    using Cfg = FewRowsCfg<MS_, WS_, KS_, MODE_, SRC_>;
     constexpr int MS = Cfg::MS, NS = Cfg::NS, WS = Cfg::WS, KS = Cfg::KS, MB = Cfg::MB, STAGES = Cfg::STAGES;
 
     extern __shared__ unsigned char smem_raw[];
@@ -96,7 +130,11 @@ nm_gemm_tf32_few_rows_kernel(const GemmArgs g, const __grid_constant__ CUtensorM
         const int s = it % STAGES;
         const uint32_t dst = ring + s * Cfg::STAGE_BYTES, full = bar_full + s * 8;
         mbar_arrive_expect_tx(full, Cfg::STAGE_BYTES);
-        if (Cfg::A_PLAIN) {
+        if (Cfg::SRC == kSrcRows32) {                      // blocks of 32 k, [MS][32] each
+            for (int blk = 0; blk < KS / 32; ++blk) tma_load_2d(dst + blk * (MS * 128), &map_a, (win0 + it) * KS + blk * 32, 0, full);
+        } else if (Cfg::SRC >= kSrcRowsF16) {
+            tma_load_2d(dst, &map_a, (win0 + it) * KS, 0, full);
+        } else if (Cfg::A_PLAIN) {
             tma_load_2d(dst, &map_a, 0, (win0 + it) * KS, full);
         } else if (a_blocked) {
             tma_load_3d(dst, &map_a, 0, (win0 + it) * KS, 0, full);
@@ -160,8 +198,20 @@ nm_gemm_tf32_few_rows_kernel(const GemmArgs g, const __grid_constant__ CUtensorM
                 const int w0 = grp * 8 + t, w1 = w0 + 4;   // kept rows behind fragment columns t and t + 4
                 const int k0 = lds_s32(kl + w0 * 4), k1 = lds_s32(kl + w1 * 4);
                 uint32_t a[MB][4];
+                if constexpr (Cfg::SRC != kSrcCols) {
+                    // element (m, k) of the window, m % 8 = gq for every row this lane reads
+                    const uint32_t p0 = as + row_element<Cfg::SRC, MS, KS>(gq, k0), p1 = as + row_element<Cfg::SRC, MS, KS>(gq, k1);
+                    constexpr int PITCH8 = 8 * (Cfg::SRC == kSrcRows32 ? 128 : KS * 2);      // eight rows further
 #pragma unroll
-                for (int mb = 0; mb < MB; ++mb) {
+                    for (int mb = 0; mb < MB; ++mb) {
+                        a[mb][0] = load_element<Cfg::SRC>(p0 + (2 * mb) * PITCH8);
+                        a[mb][1] = load_element<Cfg::SRC>(p0 + (2 * mb + 1) * PITCH8);
+                        a[mb][2] = load_element<Cfg::SRC>(p1 + (2 * mb) * PITCH8);
+                        a[mb][3] = load_element<Cfg::SRC>(p1 + (2 * mb + 1) * PITCH8);
+                    }
+                }
+#pragma unroll
+                for (int mb = 0; Cfg::SRC == kSrcCols && mb < MB; ++mb) {
                     if (Cfg::A_PLAIN) {                    // rows of 64 bytes: the four k of a fragment column meet in pairs of banks at worst
                         a[mb][0] = lds_u32(as + k0 * 64 + gq * 4);
                         a[mb][1] = lds_u32(as + k0 * 64 + (gq + 8) * 4);
@@ -209,25 +259,26 @@ nm_gemm_tf32_few_rows_kernel(const GemmArgs g, const __grid_constant__ CUtensorM
             }
     } else {
         for (int o = 0; o < outs.n_out; ++o) {
-            float* C = output_of(g, outs, o) + outs.col0 + bj + col;
+            float* C = output_of(g, outs, o);
+            const size_t c0 = static_cast<size_t>(outs.col0) + bj + col;
 #pragma unroll
             for (int mb = 0; mb < MB; ++mb) {
                 const int r0 = mb * 16 + gq, r1 = r0 + 8;
 #pragma unroll
                 for (int nb = 0; nb < 4; ++nb) {
-                    if (r0 < g.M) *reinterpret_cast<float2*>(C + static_cast<size_t>(r0) * outs.ldc + nb * 8) = make_float2(acc[mb][nb][0], acc[mb][nb][1]);
-                    if (r1 < g.M) *reinterpret_cast<float2*>(C + static_cast<size_t>(r1) * outs.ldc + nb * 8) = make_float2(acc[mb][nb][2], acc[mb][nb][3]);
+                    if (r0 < g.M) store_c2(C, c0 + static_cast<size_t>(r0) * outs.ldc + nb * 8, make_float2(acc[mb][nb][0], acc[mb][nb][1]), outs.c_dtype);
+                    if (r1 < g.M) store_c2(C, c0 + static_cast<size_t>(r1) * outs.ldc + nb * 8, make_float2(acc[mb][nb][2], acc[mb][nb][3]), outs.c_dtype);
                 }
             }
         }
     }
 }
 
-template <int MS, int WS, int KS, int MODE>
-static cudaError_t launch_few_rows(const GemmArgs& a, const GemmOutputs& outs, int ctas, cudaStream_t st)
+template <int MS, int WS, int KS, int MODE, int SRC>
+static cudaError_t launch_few_rows_from(const GemmArgs& a, const GemmOutputs& outs, int ctas, cudaStream_t st)
 {
-    using Cfg = FewRowsCfg<MS, WS, KS, MODE>;
-    auto kernel = nm_gemm_tf32_few_rows_kernel<MS, WS, KS, MODE>;
+    using Cfg = FewRowsCfg<MS, WS, KS, MODE, SRC>;
+    auto kernel = nm_gemm_tf32_few_rows_kernel<MS, WS, KS, MODE, SRC>;
     static bool configured[64] = {};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -240,18 +291,34 @@ static cudaError_t launch_few_rows(const GemmArgs& a, const GemmOutputs& outs, i
     CUtensorMap map_a, map_b;
     const int K = a.sched.n_win * KS;
     const int lda = outs.lda ? outs.lda : a.M;
-    const int a_blocked = (!Cfg::A_PLAIN && lda % 32 == 0) ? 1 : 0;    // columns past lda read as zeros either way
-    e = Cfg::A_PLAIN ? encode_tensor_map_2d(&map_a, a.A, lda, K, 16, KS, 0)
-                     : (a_blocked ? encode_tensor_map_blocks32(&map_a, a.A, lda, K, KS, Cfg::ABLK)
-                                  : encode_tensor_map_2d(&map_a, a.A, lda, K, 32, KS, 1));
+    const int a_blocked = (SRC == kSrcCols && !Cfg::A_PLAIN && lda % 32 == 0) ? 1 : 0;    // columns past lda read as zeros either way
+    if (SRC >= kSrcRowsF16) e = encode_tensor_map_rows16(&map_a, a.A, K, a.M, KS, MS);     // rows past M read as zeros
+    else if (SRC == kSrcRows32) e = encode_tensor_map_2d(&map_a, a.A, K, a.M, 32, MS, 2);
+    else
+        e = Cfg::A_PLAIN ? encode_tensor_map_2d(&map_a, a.A, lda, K, 16, KS, 0)
+                         : (a_blocked ? encode_tensor_map_blocks32(&map_a, a.A, lda, K, KS, Cfg::ABLK)
+                                      : encode_tensor_map_2d(&map_a, a.A, lda, K, 32, KS, 1));
     if (e != cudaSuccess) return e;
     e = encode_tensor_map_blocks32(&map_b, a.B, a.N, a.W, WS - (g_test_short_fill ? 1 : 0), 4);   // (test hook, see kernels.h)
     if (e != cudaSuccess) return e;
     return launch_overlapped(kernel, ctas, Cfg::THREADS, Cfg::SMEM_BYTES, st, a, map_a, map_b, outs, a_blocked);
 }
 
+template <int MS, int WS, int KS, int MODE>
+static cudaError_t launch_few_rows(const GemmArgs& a, const GemmOutputs& outs, int ctas, cudaStream_t st)
+{
+    switch (outs.a_rows) {
+    case 0: return launch_few_rows_from<MS, WS, KS, MODE, kSrcCols>(a, outs, ctas, st);
+    case 1 + kDtypeF32: return launch_few_rows_from<MS, WS, KS, MODE, kSrcRows32>(a, outs, ctas, st);
+    case 1 + kDtypeF16: return launch_few_rows_from<MS, WS, KS, MODE, kSrcRowsF16>(a, outs, ctas, st);
+    case 1 + kDtypeBF16: return launch_few_rows_from<MS, WS, KS, MODE, kSrcRowsBF16>(a, outs, ctas, st);
+    default: return cudaErrorInvalidValue;
+    }
+}
+
+// (the plan is the same whatever A's form: shared memory as the col-major form has it)
 #define NMSPMM_FEW_ROWS_VARIANT(NKEEP, MS, WS, KS, MODE)                                                               \
-    { NKEEP, WS, KS, MODE, 128, 32, FewRowsCfg<MS, WS, KS, MODE>::SMEM_BYTES, FewRowsCfg<MS, WS, KS, MODE>::STAGES, 128, \
+    { NKEEP, WS, KS, MODE, 128, 32, FewRowsCfg<MS, WS, KS, MODE, kSrcCols>::SMEM_BYTES, FewRowsCfg<MS, WS, KS, MODE, kSrcCols>::STAGES, 128, \
       &launch_few_rows<MS, WS, KS, MODE>, 2, MS }
 
 extern const SlicedVariant kTf32FewRowsVariants[] = {

@@ -16,7 +16,6 @@ cudaError_t launch_transpose_rows(const float* in, float* out, int M, int K, int
 
 // 16-bit storage (convert16.cu): the same transposition from half / bfloat16 rows, n floats
 // rounded to 16 bits, n 16-bit values widened (n % 4 == 0).
-enum { kDtypeF32 = 0, kDtypeF16 = 1, kDtypeBF16 = 2 };
 cudaError_t launch_transpose_rows_16(int dtype, const void* in, float* out, int M, int K, int ld, cudaStream_t st);
 cudaError_t launch_narrow(int dtype, const float* in, void* out, size_t n, cudaStream_t st);
 cudaError_t launch_widen(int dtype, const void* in, float* out, size_t n, cudaStream_t st);
@@ -58,6 +57,10 @@ cudaError_t encode_tensor_map_2d(CUtensorMap* map, const float* base, int cols, 
 // box_blocks blocks x box_rows rows lands block after block, each [box_rows][32] swizzled like
 // encode_tensor_map_2d's swizzle128 form.
 cudaError_t encode_tensor_map_blocks32(CUtensorMap* map, const float* base, int cols, int rows, int box_rows, int box_blocks);
+
+// Row-major [rows][cols] tensor of 16-bit values, box of 64 or 32 columns x box_rows, 16-byte chunks swizzled
+// within the box's rows (CU_TENSOR_MAP_SWIZZLE_128B / 64B).
+cudaError_t encode_tensor_map_rows16(CUtensorMap* map, const void* base, int cols, int rows, int box_cols, int box_rows);
 
 // One compiled variant of the kernels that cut K into whole slices per tile and leave the
 // slices in scratch slots for nm_reduce_slices_kernel: the TF32 tensor-core kernels (tile

@@ -11,6 +11,7 @@
 #include "common.cuh"
 #include "gemm_args.h"
 #include "kernels.h"
+#include "store16.cuh"
 
 namespace nmspmm {
 
@@ -175,7 +176,7 @@ __global__ void __launch_bounds__(256) nm_reduce_slices_kernel(const GemmArgs g,
                 if (z + u < S) { sum.x += x[u].x; sum.y += x[u].y; sum.z += x[u].z; sum.w += x[u].w; }
         }
         const size_t at = static_cast<size_t>(bi + row) * outs.ldc + outs.col0 + bj + c4 * 4;
-        for (int o = 0; o < outs.n_out; ++o) *reinterpret_cast<float4*>(output_of(g, outs, o) + at) = sum;
+        for (int o = 0; o < outs.n_out; ++o) store_c4(output_of(g, outs, o), at, sum, outs.c_dtype);
     }
 }
 
@@ -189,7 +190,7 @@ cudaError_t launch_reduce_slices(int ns, const GemmArgs& a, const GemmOutputs& o
     if (ns == 128 && ms == 128)
         return many ? launch_after_multiply(nm_reduce_slices_kernel<128, 1>, n_tiles * 16, 256, st, a, outs, first_tile)
                     : launch_after_multiply(nm_reduce_slices_kernel<128, 4>, n_tiles * 4, 256, st, a, outs, first_tile);
-    // the few-row tiles of gemm_tf32_skinny.cu: slots of ms x 128
+    // the few-row tiles of gemm_tf32_few_rows.cu: slots of ms x 128
     if (ns == 128 && ms == 64) return launch_after_multiply(nm_reduce_slices_kernel<128, 1, 64>, n_tiles * 8, 256, st, a, outs, first_tile);
     if (ns == 128 && ms == 32) return launch_after_multiply(nm_reduce_slices_kernel<128, 1, 32>, n_tiles * 4, 256, st, a, outs, first_tile);
     if (ns == 128 && ms == 16) return launch_after_multiply(nm_reduce_slices_kernel<128, 1, 16>, n_tiles * 2, 256, st, a, outs, first_tile);

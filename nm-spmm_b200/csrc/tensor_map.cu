@@ -30,7 +30,7 @@ static EncodeTiledFn encode_fn()
 // host thread are kept, keyed by everything that goes into them.
 struct MapKey {
     const void* base;
-    int cols, rows, box_a, box_b, kind;       // kind: 0 plain 2-D, 1 / 3 swizzled 2-D (32- / 16-byte chunks), 2 blocks of 32 columns
+    int cols, rows, box_a, box_b, kind;       // kind: 0 plain 2-D, 1 / 3 swizzled 2-D (32- / 16-byte chunks), 2 blocks of 32 columns, 4 swizzled 2-D of 16-bit values
     bool operator==(const MapKey& o) const
     {
         return base == o.base && cols == o.cols && rows == o.rows && box_a == o.box_a && box_b == o.box_b && kind == o.kind;
@@ -102,6 +102,24 @@ cudaError_t encode_tensor_map_blocks32(CUtensorMap* map, const float* base, int 
     const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float*>(base), dims, strides, box, elem,
                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B,
                           CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r == CUDA_SUCCESS) tl_maps.put(mk, *map);
+    return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
+}
+
+cudaError_t encode_tensor_map_rows16(CUtensorMap* map, const void* base, int cols, int rows, int box_cols, int box_rows)
+{
+    const MapKey mk { base, cols, rows, box_cols, box_rows, 4 };
+    if (tl_maps.find(mk, map)) return cudaSuccess;
+    EncodeTiledFn fn = encode_fn();
+    if (!fn) return cudaErrorNotSupported;
+    if (box_cols != 64 && box_cols != 32) return cudaErrorInvalidValue;
+    const cuuint64_t dims[2] = { static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows) };
+    const cuuint64_t strides[1] = { static_cast<cuuint64_t>(cols) * 2 };
+    const cuuint32_t box[2] = { static_cast<cuuint32_t>(box_cols), static_cast<cuuint32_t>(box_rows) };
+    const cuuint32_t elem[2] = { 1, 1 };
+    const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, const_cast<void*>(base), dims, strides, box, elem,
+                          CU_TENSOR_MAP_INTERLEAVE_NONE, box_cols == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
+                          CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r == CUDA_SUCCESS) tl_maps.put(mk, *map);
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }

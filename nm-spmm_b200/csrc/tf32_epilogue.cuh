@@ -3,6 +3,7 @@
 #pragma once
 #include "common.cuh"
 #include "gemm_args.h"
+#include "store16.cuh"
 #include "tcgen05.cuh"
 
 namespace nmspmm {
@@ -45,6 +46,13 @@ __device__ __forceinline__ void tf32_store_vectors(uint32_t tmem, int quad, int 
         float4 val[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) val[i] = lds_f4(patch + (4 * i + r_sub) * 144 + c4 * 4);
+        if (!sliced && outs.c_dtype != kDtypeF32) {        // one private 16-bit C
+            const size_t at = static_cast<size_t>(base - g.C);
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                if (4 * i < rows_left) store_c4(g.C, at + static_cast<size_t>(4 * i) * row_step, val[i], outs.c_dtype);
+            continue;
+        }
 #pragma unroll
         for (int i = 0; i < 8; ++i)
             if (4 * i < rows_left) *reinterpret_cast<float4*>(base + static_cast<size_t>(4 * i) * row_step) = val[i];

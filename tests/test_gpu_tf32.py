@@ -280,3 +280,31 @@ def test_tf32_tiles_walked_in_bands_of_columns(pkg, orc, n_keep, fmt, tile, M, N
     assert pkg.device_status() == 0
     assert torch.equal(banded, plain)
     assert rel_err(banded.cpu().numpy(), orc.nm_gemm_f64(p.A_km, p.B_col, p.D_col)) <= TF32_TOL
+
+
+@pytest.mark.parametrize("dtype,tol", [(torch.float32, 1e-5), (torch.float16, 5e-4), (torch.bfloat16, 4e-3)])
+@pytest.mark.parametrize("M", [1, 17, 33, 64, 65, 130])
+@pytest.mark.parametrize("N", [128, 448])
+@pytest.mark.parametrize("n_keep,vec_len", [(4, 32), (8, 32), (12, 32), (16, 32), (32, 32), (4, 64), (8, 64), (12, 64), (16, 64)])
+def test_row_major_activations_match_the_col_major_route(pkg, dtype, tol, M, N, n_keep, vec_len):
+    """The tensor-core kernels that read row-major activations as they are, in each type, against the
+    same multiply of the same values given col-major (rows of A filled up to a multiple of 4): both cut
+    the operands to TF32 and add in FP32, so they differ by the order of the sums and, for 16-bit
+    results, one rounding (2^-9 and 2^-12 of a value).  The activations off a 16-byte boundary take the
+    transposing route and agree too."""
+    fmt = 0 if n_keep > 8 or (n_keep == 8 and vec_len == 32 and N == 448) else 1      # 8:32 in both formats
+    K = 640 if fmt else 608
+    p = pkg.formats.make_random(4, N, K, n_keep, seed=900 + n_keep + N, vec_len=vec_len)
+    op = pkg.NMSpMM.from_problem(p, layout_ns=64, fmt=fmt)
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(M)
+    x = (torch.rand((M, K), device="cuda", generator=gen) * 2 - 1).to(dtype)
+    A = torch.zeros((K, (M + 3) // 4 * 4), device="cuda")
+    A[:, :M] = x.float().t()
+    want = op.matmul(A, path=pkg.PATH_TF32)[:M].double()
+    shifted = torch.empty(M * K + 1, dtype=dtype, device="cuda")[1:].view(M, K).copy_(x)
+    for rows in (x, shifted):
+        got = op.matmul_rows(rows, path=pkg.PATH_TF32)
+        assert got.dtype == dtype
+        assert float((got.double() - want).norm() / want.norm()) <= tol
+    assert pkg.device_status() == 0
