@@ -38,6 +38,13 @@
 // n_keep = 32 (nothing pruned) has the identity as its index list and multiplies A_window by
 // the B rows directly.  12:32 gathers 16 columns per vector of which 4 are zero (P has no
 // entry for them), and loads 16 rows of B per vector of which the last 4 meet those zeros.
+//
+// Row-major A (activations as a layer has them) is read as it lies in memory: a window is 128 rows x
+// KW columns, a K-major operand.  FP32 rows change nothing else.  Half and bfloat16 rows are
+// gathered in their own type (kind::f16, one-hot P of that type, FP32 result: exact), K = 16 per
+// instruction: half as many gather instructions per step and half of A's bytes, no transposing and
+// widening launch ahead of the multiply, and C is stored in the activations' type.
+// 256 x 11008 x 4096, bfloat16, 8:32: the pass takes 50.8 us, 59.5 with a transposing and a rounding launch.
 // Every wait is bounded; a wait that gives up raises the device status word.
 #include <cuda.h>
 
@@ -70,24 +77,30 @@ __device__ unsigned long long g_tf32_profile[16];
 #define TF_OUT(i, v)
 #endif
 
-template <int NKEEP, int KW_, int MODE, int QT_, int VL_ = 32>
+// How A is read: col-major FP32, or row-major FP32 / 16-bit values (half or bfloat16 by launch).
+enum { kTf32Cols = 0, kTf32Rows32 = 1, kTf32Rows16 = 2 };
+
+template <int NKEEP, int KW_, int MODE, int QT_, int VL_ = 32, int SRC_ = kTf32Cols>
 struct Tf32Cfg {
+    static constexpr int SRC = SRC_;
+    static constexpr int EB = (SRC == kTf32Rows16) ? 2 : 4;  // bytes of a value of A and of P
     static constexpr int MS = 128, QT = QT_, NS = QT * 32;   // QT = 8: one CTA per SM; QT = 4: two
     static constexpr int KW = KW_;                           // k per step
     static constexpr int WS = NKEEP * (KW / 32);             // rows of B per step
     static constexpr int WSP = (WS + 7) / 8 * 8;             // gathered columns per vector (K of the products)
     static constexpr bool DIRECT = (NKEEP == 32);            // identity index list: no gather
     static constexpr int G = WSP / 8;                        // product instructions per vector and step
-    static constexpr int NKS = KW / 8;                       // gather instructions per step
+    static constexpr int NKS = KW * EB / 32;                 // gather instructions per step (32 bytes of K each)
     static constexpr int VL = VL_;                           // columns that share an index list: 32, or 64 (two adjacent equal lists)
     static constexpr int QV = NS / VL;                       // vectors per tile
     static constexpr int N1 = QV * WSP;                      // gathered columns per step
     static_assert(VL == 32 || (VL == 64 && NKEEP != 32), "vectors of 32 or 64 columns");
     static_assert(DIRECT || N1 <= 128, "one builder thread per gathered column");
     static_assert(MODE == kModeHigh || KW == 32, "only the 64-k format has merged windows");
-    static constexpr int A_BYTES = KW * 512;                 // [4 blocks of 32 rows of the tile][KW][32]
+    static_assert(!(DIRECT && SRC == kTf32Rows16), "the direct product multiplies A by FP32 rows of B");
+    static constexpr int A_BYTES = 128 * KW * EB;            // col-major: [4 blocks of 32 rows of the tile][KW][32]; rows: [128][<= 128 bytes], blocks of 32 k if FP32
     static constexpr int B_BYTES = QT * WSP * 128;           // [QT][WSP][32]
-    static constexpr int P_BYTES = DIRECT ? 0 : N1 * KW * 4; // [N1 / 32][KW][32]
+    static constexpr int P_BYTES = DIRECT ? 0 : N1 * KW * EB;  // [N1 / 32][KW][32]; 16 bits: K-major, [N1][KW]
     static constexpr int STAGE_BYTES = A_BYTES + B_BYTES + P_BYTES;
     static_assert(A_BYTES % 1024 == 0 && B_BYTES % 1024 == 0 && P_BYTES % 1024 == 0, "swizzle atoms stay aligned");
     static constexpr int CTAS_PER_SM = (QT == 8) ? 1 : 2;
@@ -124,12 +137,23 @@ __device__ __forceinline__ uint32_t p_offset(int n, int k)
     return static_cast<uint32_t>(nb * (KW * 128) + k * 128 + ((((c >> 3) ^ (k & 3)) << 5) | ((c & 7) << 2)));
 }
 
-template <int NKEEP, int KW_, int MODE, int QT_, int VL_>
-__global__ void __launch_bounds__((Tf32Cfg<NKEEP, KW_, MODE, QT_, VL_>::THREADS), (Tf32Cfg<NKEEP, KW_, MODE, QT_, VL_>::CTAS_PER_SM))
-nm_gemm_tf32_kernel(const GemmArgs g, const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                    const GemmOutputs outs, const int a_blocked)
+// The same for a P of 16-bit values (K-major, [N1][KW], 16-byte chunks swizzled within the rows).
+template <int KW>
+__device__ __forceinline__ uint32_t p16_offset(int n, int k)
 {
-    using Cfg = Tf32Cfg<NKEEP, KW_, MODE, QT_, VL_>;
+    return static_cast<uint32_t>(n * (KW * 2) + (((k >> 3) ^ (KW == 64 ? (n & 7) : ((n >> 1) & 3))) << 4) + (k & 7) * 2);
+}
+__device__ __forceinline__ void sts_u16(uint32_t addr, unsigned v)
+{
+    asm volatile("st.shared.u16 [%0], %1;" ::"r"(addr), "h"(static_cast<unsigned short>(v)) : "memory");
+}
+
+template <int NKEEP, int KW_, int MODE, int QT_, int VL_, int SRC_>
+__global__ void __launch_bounds__((Tf32Cfg<NKEEP, KW_, MODE, QT_, VL_, SRC_>::THREADS), (Tf32Cfg<NKEEP, KW_, MODE, QT_, VL_, SRC_>::CTAS_PER_SM))
+nm_gemm_tf32_kernel(const GemmArgs g, const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+                    const GemmOutputs outs, const int a_form)     // col-major: 1 where the rows of A are whole blocks of 32; 16 bits: the type
+{
+    using Cfg = Tf32Cfg<NKEEP, KW_, MODE, QT_, VL_, SRC_>;
     constexpr int MS = Cfg::MS, NS = Cfg::NS, QT = Cfg::QT, KW = Cfg::KW, WS = Cfg::WS, WSP = Cfg::WSP;
     constexpr int VL = Cfg::VL, QV = Cfg::QV, BPV = VL / 32;              // 32-column blocks per vector
     constexpr int STAGES = Cfg::STAGES, NBUF = Cfg::NBUF, RING = Cfg::RING, PD = Cfg::PD;
@@ -212,7 +236,11 @@ nm_gemm_tf32_kernel(const GemmArgs g, const __grid_constant__ CUtensorMap map_a,
             const uint32_t st = ring + s * Cfg::STAGE_BYTES, full = bar_full + s * 8;
             if (elect_one()) {
                 mbar_arrive_expect_tx(full, Cfg::A_BYTES + Cfg::B_BYTES);
-                if (a_blocked) {
+                if constexpr (Cfg::SRC == kTf32Rows32) {
+                    for (int kb = 0; kb < KW / 32; ++kb) tma_load_2d(st + kb * 16384, &map_a, (win0 + it) * KW + kb * 32, bi, full);
+                } else if constexpr (Cfg::SRC == kTf32Rows16) {
+                    tma_load_2d(st, &map_a, (win0 + it) * KW, bi, full);
+                } else if (a_form) {
                     tma_load_3d(st, &map_a, 0, (win0 + it) * KW, bi >> 5, full);
                 } else {                                   // rows not a multiple of 32: four boxes of 32 rows, the ragged one zero-filled
                     for (int mb = 0; mb < 4; ++mb) tma_load_2d(st + mb * (KW * 128), &map_a, bi + mb * 32, (win0 + it) * KW, full);
@@ -226,8 +254,16 @@ nm_gemm_tf32_kernel(const GemmArgs g, const __grid_constant__ CUtensorMap map_a,
 #endif
     } else if (warp == 1) {
         // ------------------------------------------------------------------ gather issuer
-        constexpr uint32_t idesc_gather = umma_idesc_tf32(128, DIRECT ? 32 : Cfg::N1, true);
-        const uint32_t idesc_direct = umma_idesc_tf32(128, live_vecs * 32, true);
+        constexpr bool COLS = (Cfg::SRC == kTf32Cols);
+        const uint32_t idesc_gather = Cfg::SRC == kTf32Rows16 ? umma_idesc_16(128, DIRECT ? 32 : Cfg::N1, a_form == kDtypeBF16)
+                                                              : umma_idesc_tf32(128, DIRECT ? 32 : Cfg::N1, COLS);
+        const uint32_t idesc_direct = umma_idesc_tf32(128, live_vecs * 32, COLS);
+        // A's descriptor for the ks-th 32 bytes of K (col-major: the ks-th eight rows of k)
+        auto a_desc = [](uint32_t st, int ks) {
+            if constexpr (Cfg::SRC == kTf32Cols) return umma_desc_mn_tf32(st + ks * 1024, KW * 128, 512);
+            else if constexpr (Cfg::SRC == kTf32Rows32) return umma_desc_k_major<128>(st + (ks >> 2) * 16384 + (ks & 3) * 32);
+            else return umma_desc_k_major<KW * 2>(st + ks * 32);
+        };
         bool alive = true;
         TF_DECL(m_full = 0, m_free = 0, m_issue = 0);
         TF_T(m_start);
@@ -248,17 +284,20 @@ nm_gemm_tf32_kernel(const GemmArgs g, const __grid_constant__ CUtensorMap map_a,
                 if (DIRECT) {
 #pragma unroll
                     for (int ks = 0; ks < Cfg::NKS; ++ks)
-                        umma_tf32_ss(tmem_addr(tmem, 0, 0), umma_desc_mn_tf32(st + ks * 1024, KW * 128, 512),
+                        umma_tf32_ss(tmem_addr(tmem, 0, 0), a_desc(st, ks),
                                      umma_desc_mn_tf32(st + Cfg::A_BYTES + ks * 1024, WSP * 128, 512), idesc_direct,
                                      (t | ks) != 0);
                     tc_commit(bar_empty + s * 8);
                 } else {
                     const uint32_t gbuf = tmem_addr(tmem, 0, Cfg::ACOL0 + (t % NBUF) * Cfg::N1);
 #pragma unroll
-                    for (int ks = 0; ks < Cfg::NKS; ++ks)
-                        umma_tf32_ss(gbuf, umma_desc_mn_tf32(st + ks * 1024, KW * 128, 512),
-                                     umma_desc_mn_tf32(st + Cfg::A_BYTES + Cfg::B_BYTES + ks * 1024, KW * 128, 512),
-                                     idesc_gather, ks != 0);
+                    for (int ks = 0; ks < Cfg::NKS; ++ks) {
+                        const uint32_t p = st + Cfg::A_BYTES + Cfg::B_BYTES;
+                        if constexpr (Cfg::SRC == kTf32Rows16)
+                            umma_f16_ss(gbuf, a_desc(st, ks), umma_desc_k_major<KW * 2>(p + ks * 32), idesc_gather, ks != 0);
+                        else
+                            umma_tf32_ss(gbuf, a_desc(st, ks), umma_desc_mn_tf32(p + ks * 1024, KW * 128, 512), idesc_gather, ks != 0);
+                    }
                     tc_commit(bar_gdone + (t % NBUF) * 8);
                 }
             }
@@ -372,8 +411,13 @@ nm_gemm_tf32_kernel(const GemmArgs g, const __grid_constant__ CUtensorMap map_a,
                 if (has) {
                     const uint32_t ps = ring + s * Cfg::STAGE_BYTES + Cfg::A_BYTES + Cfg::B_BYTES;
                     const int old = lds_s32(my_prev + s * 512);
-                    if (old >= 0) sts_f32(ps + p_offset<KW>(e, old), 0.f);
-                    sts_f32(ps + p_offset<KW>(e, k), 1.f);
+                    if constexpr (Cfg::SRC == kTf32Rows16) {
+                        if (old >= 0) sts_u16(ps + p16_offset<KW>(e, old), 0u);
+                        sts_u16(ps + p16_offset<KW>(e, k), a_form == kDtypeBF16 ? 0x3F80u : 0x3C00u);      // 1.0
+                    } else {
+                        if (old >= 0) sts_f32(ps + p_offset<KW>(e, old), 0.f);
+                        sts_f32(ps + p_offset<KW>(e, k), 1.f);
+                    }
                     sts_s32(my_prev + s * 512, k);
                 }
                 fence_proxy_async();                       // the tensor core reads P through the asynchronous proxy
@@ -412,11 +456,11 @@ nm_gemm_tf32_kernel(const GemmArgs g, const __grid_constant__ CUtensorMap map_a,
     }
 }
 
-template <int NKEEP, int KW, int MODE, int QT, int VL>
-static cudaError_t launch_tf32(const GemmArgs& a, const GemmOutputs& outs, int tiles, cudaStream_t st)
+template <int NKEEP, int KW, int MODE, int QT, int VL, int SRC>
+static cudaError_t launch_tf32_from(const GemmArgs& a, const GemmOutputs& outs, int tiles, cudaStream_t st)
 {
-    using Cfg = Tf32Cfg<NKEEP, KW, MODE, QT, VL>;
-    auto kernel = nm_gemm_tf32_kernel<NKEEP, KW, MODE, QT, VL>;
+    using Cfg = Tf32Cfg<NKEEP, KW, MODE, QT, VL, SRC>;
+    auto kernel = nm_gemm_tf32_kernel<NKEEP, KW, MODE, QT, VL, SRC>;
     static bool configured[64] = {};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -429,13 +473,28 @@ static cudaError_t launch_tf32(const GemmArgs& a, const GemmOutputs& outs, int t
     CUtensorMap map_a, map_b;
     const int K = a.sched.n_win * KW;
     const int lda = outs.lda ? outs.lda : a.M;             // a row-major caller's transposed copy is padded to 4 columns
-    const int a_blocked = (lda % 32 == 0) ? 1 : 0;
-    e = a_blocked ? encode_tensor_map_blocks32(&map_a, a.A, lda, K, KW, 4)
-                  : encode_tensor_map_2d(&map_a, a.A, lda, K, 32, KW, 1);
+    int a_form = (lda % 32 == 0) ? 1 : 0;
+    if (SRC == kTf32Rows16) {
+        a_form = outs.a_rows - 1;
+        e = encode_tensor_map_rows16(&map_a, a.A, K, a.M, KW, 128);       // rows past M read as zeros
+    } else if (SRC == kTf32Rows32) {
+        e = encode_tensor_map_2d(&map_a, a.A, K, a.M, 32, 128, 2);
+    } else {
+        e = a_form ? encode_tensor_map_blocks32(&map_a, a.A, lda, K, KW, 4) : encode_tensor_map_2d(&map_a, a.A, lda, K, 32, KW, 1);
+    }
     if (e != cudaSuccess) return e;
     e = encode_tensor_map_blocks32(&map_b, a.B, a.N, a.W, Cfg::WSP - (g_test_short_fill ? 1 : 0), QT);   // (test hook, see kernels.h)
     if (e != cudaSuccess) return e;
-    return launch_overlapped(kernel, tiles, Cfg::THREADS, Cfg::SMEM_BYTES, st, a, map_a, map_b, outs, a_blocked);
+    return launch_overlapped(kernel, tiles, Cfg::THREADS, Cfg::SMEM_BYTES, st, a, map_a, map_b, outs, a_form);
+}
+
+template <int NKEEP, int KW, int MODE, int QT, int VL>
+static cudaError_t launch_tf32(const GemmArgs& a, const GemmOutputs& outs, int tiles, cudaStream_t st)
+{
+    if (outs.a_rows == 0) return launch_tf32_from<NKEEP, KW, MODE, QT, VL, kTf32Cols>(a, outs, tiles, st);
+    if (outs.a_rows == 1 + kDtypeF32) return launch_tf32_from<NKEEP, KW, MODE, QT, VL, kTf32Rows32>(a, outs, tiles, st);
+    if constexpr (NKEEP != 32) return launch_tf32_from<NKEEP, KW, MODE, QT, VL, kTf32Rows16>(a, outs, tiles, st);
+    else return cudaErrorInvalidValue;
 }
 
 #define NMSPMM_TF32_VARIANT(NKEEP, KW, MODE, QT, VL)                                                                   \

@@ -76,6 +76,28 @@ __device__ __forceinline__ uint64_t umma_desc_mn_tf32(uint32_t smem_addr, uint32
     return d;
 }
 
+// Shared-memory descriptor of a K-major operand in rows of 64 or 128 bytes whose 16-byte chunks are
+// swizzled within the row (what a TMA copy with CU_TENSOR_MAP_SWIZZLE_64B / 128B writes): groups of
+// eight rows follow one another.  The next 32 bytes of K are at smem_addr + 32.  The operand itself
+// starts on 512 / 1024 bytes.
+template <int ROW_BYTES>
+__device__ __forceinline__ uint64_t umma_desc_k_major(uint32_t smem_addr)
+{
+    static_assert(ROW_BYTES == 64 || ROW_BYTES == 128, "one swizzle atom per row");
+    uint64_t d = static_cast<uint64_t>((smem_addr >> 4) & 0x3FFFu);
+    d |= 1ull << 16;                                  // leading byte offset: not used by the swizzled K-major layouts
+    d |= static_cast<uint64_t>((8 * ROW_BYTES) >> 4) << 32;         // stride byte offset: next eight rows
+    d |= 1ull << 46;
+    d |= (ROW_BYTES == 128 ? 2ull : 4ull) << 61;      // SWIZZLE_128B / SWIZZLE_64B
+    return d;
+}
+
+// Instruction descriptor of kind::f16: FP32 accumulate, A and B both half (or both bfloat16), both K-major.
+__host__ __device__ constexpr uint32_t umma_idesc_16(int m, int n, bool bf16)
+{
+    return (1u << 4) | (bf16 ? (1u << 7) | (1u << 10) : 0u) | (static_cast<uint32_t>(n >> 3) << 17) | (static_cast<uint32_t>(m >> 4) << 24);
+}
+
 // Instruction descriptor of kind::tf32: FP32 accumulate, A and B TF32, B MN-major (n
 // contiguous in shared memory), M x N tile.  A is K-major when it comes from Tensor Memory;
 // a_mn_major = true for an A taken from shared memory with m contiguous.
@@ -106,6 +128,19 @@ __device__ __forceinline__ void umma_tf32_ss(uint32_t d_tmem, uint64_t a_desc, u
         ".reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t"
+        "}\n"
+        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate ? 1u : 0u)
+        : "memory");
+}
+
+// One thread: D[tmem] (+)= A[smem] * B[smem], M x N x 16 half or bfloat16.
+__device__ __forceinline__ void umma_f16_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, bool accumulate)
+{
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
         "}\n"
         ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate ? 1u : 0u)
         : "memory");
