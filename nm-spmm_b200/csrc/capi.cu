@@ -901,7 +901,7 @@ int nmspmm_gemm_row_major(const nmspmm_gemm_desc* desc, const float* A_rows_dev,
         return gemm_launch(desc, A_rows_dev, B_dev, D_dev, column_info_dev, out, 1, desc->N, 0, own ? workspace_dev : nullptr, own, stream, 0,
                            1 + kDtypeF32);
     float* A_cols = reinterpret_cast<float*>(static_cast<unsigned char*>(workspace_dev) + head);
-    cudaError_t e = launch_transpose_rows(A_rows_dev, A_cols, desc->M, desc->K, ld, static_cast<cudaStream_t>(stream));
+    cudaError_t e = launch_transpose_rows(kDtypeF32, A_rows_dev, A_cols, desc->M, desc->K, ld, static_cast<cudaStream_t>(stream));
     if (e != cudaSuccess) return cuda_fail(e);
     return gemm_launch(desc, A_cols, B_dev, D_dev, column_info_dev, out, 1, desc->N, 0, own ? workspace_dev : nullptr, own, stream, ld);
 }
@@ -944,7 +944,7 @@ int nmspmm_gemm_row_major_16(const nmspmm_gemm_desc* desc, int dtype, const void
     if (reads_rows(p, A_rows_dev, dtype))
         return gemm_launch(desc, static_cast<const float*>(A_rows_dev), B_dev, D_dev, column_info_dev, direct, 1, desc->N, 0,
                            own ? ws : nullptr, own, stream, 0, 1 + dtype, dtype);
-    cudaError_t e = launch_transpose_rows_16(dtype, A_rows_dev, A_cols, desc->M, desc->K, ld, st);
+    cudaError_t e = launch_transpose_rows(dtype, A_rows_dev, A_cols, desc->M, desc->K, ld, st);
     if (e != cudaSuccess) return cuda_fail(e);
     if (p.tv)
         return gemm_launch(desc, A_cols, B_dev, D_dev, column_info_dev, direct, 1, desc->N, 0, own ? ws : nullptr, own, stream, ld, 0, dtype);

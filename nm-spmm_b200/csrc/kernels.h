@@ -11,12 +11,10 @@ cudaError_t launch_retile(const int* DT, int* D, int W, int Q, int Qs, cudaStrea
 cudaError_t launch_preprocess_high(const int* DT, int* D, int* cinfo, int pm, int pn, int W, int Q, int Qs,
                                    int fuse, int tail_ints, cudaStream_t st);
 
-// in [M][K] row-major -> out [K][ld] (ld >= M, the extra columns zero).
-cudaError_t launch_transpose_rows(const float* in, float* out, int M, int K, int ld, cudaStream_t st);
+// in [M][K] row-major, FP32 / half / bfloat16 -> out [K][ld] (ld >= M a multiple of 4, the extra columns zero).
+cudaError_t launch_transpose_rows(int dtype, const void* in, float* out, int M, int K, int ld, cudaStream_t st);
 
-// 16-bit storage (convert16.cu): the same transposition from half / bfloat16 rows, n floats
-// rounded to 16 bits, n 16-bit values widened (n % 4 == 0).
-cudaError_t launch_transpose_rows_16(int dtype, const void* in, float* out, int M, int K, int ld, cudaStream_t st);
+// 16-bit storage (convert16.cu): n floats rounded to 16 bits, n 16-bit values widened (n % 4 == 0).
 cudaError_t launch_narrow(int dtype, const float* in, void* out, size_t n, cudaStream_t st);
 cudaError_t launch_widen(int dtype, const void* in, float* out, size_t n, cudaStream_t st);
 
