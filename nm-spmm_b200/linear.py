@@ -21,6 +21,7 @@ import ctypes
 from typing import Optional
 
 _registered = None
+_library = None         # the torch.library.Library that holds the operator (it lives as long as this object)
 _workspaces = {}        # per device: the operator's scratch (zero when made: the multiply wants its counter block zero)
 
 
@@ -64,39 +65,47 @@ def register_ops(pkg):
         return _registered
     torch = _torch()
 
-    @torch.library.custom_op("nmspmm_b200::sparse_linear", mutates_args=())
-    def sparse_linear(x: torch.Tensor, values: torch.Tensor, packed: torch.Tensor, column_info: Optional[torch.Tensor],
-                      raw_indices: torch.Tensor, n_keep: int, fmt: int, layout_ns: int, vec_len: int, path: int) -> torch.Tensor:
+    # Defined through torch.library.Library rather than the custom_op decorator: the decorator's wrapper
+    # around the body cost 7 us of host time a call, as much as the multiply of one token.
+    global _library
+    _library = torch.library.Library("nmspmm_b200", "FRAGMENT")
+    name = "nmspmm_b200::sparse_linear"
+    _library.define("sparse_linear(Tensor x, Tensor values, Tensor packed, Tensor? column_info, Tensor raw_indices, SymInt n_keep, "
+                    "SymInt fmt, SymInt layout_ns, SymInt vec_len, SymInt path) -> Tensor", tags=(torch.Tag.pt2_compliant_tag,))
+
+    def sparse_linear(x, values, packed, column_info, raw_indices, n_keep, fmt, layout_ns, vec_len, path):
         """x (M, K) row-major float32 / float16 / bfloat16 . B (K, N) in N:M form -> (M, N) of x's dtype.  ``values`` (W, N) are the
         compressed weights, ``packed`` / ``column_info`` the packed indices the kernels read,
         ``raw_indices`` (W, N/32) the unpacked ones (used by the backward formula only)."""
         lib = pkg.load_library()
+        if x.device != values.device:                                     # (a host x beside CUDA weights is dispatched here too)
+            raise TypeError(f"x: expected a tensor on {values.device}, got one on {x.device}")
         x = x.contiguous()
         M, K = x.shape
         N = values.shape[1]
         dtype = pkg.dtype_id(x.dtype)
-        d = pkg.make_desc(M, N, K, n_keep, fmt, layout_ns, path, 0, 0, vec_len)
+        d = ctypes.byref(pkg.GemmDesc(M, N, K, n_keep, fmt, layout_ns, path, 0, 0, vec_len))
         wide = dtype == pkg.DTYPE_F32
-        need = int((lib.nmspmm_gemm_row_major_workspace_bytes if wide else lib.nmspmm_gemm_row_major_16_workspace_bytes)(ctypes.byref(d)))
+        need = lib.nmspmm_gemm_row_major_workspace_bytes(d) if wide else lib.nmspmm_gemm_row_major_16_workspace_bytes(d)
         if need == 0:
             raise pkg.NMSpMMError("nmspmm_gemm_row_major_workspace_bytes", pkg.UNSUPPORTED)
         ws = _workspaces.get(x.device)
         if ws is None or ws.numel() < need:
             ws = _workspaces[x.device] = torch.zeros(need, dtype=torch.uint8, device=x.device)
-        y = torch.empty((M, N), dtype=x.dtype, device=x.device)
-        ci = ctypes.c_void_p(column_info.data_ptr()) if column_info is not None else ctypes.c_void_p(0)
-        ptrs = (ctypes.c_void_p(x.data_ptr()), ctypes.c_void_p(values.data_ptr()), ctypes.c_void_p(packed.data_ptr()), ci,
-                ctypes.c_void_p(y.data_ptr()), ctypes.c_void_p(ws.data_ptr()), ws.numel(),
-                ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+        y = x.new_empty((M, N))
+        ptrs = (x.data_ptr(), values.data_ptr(), packed.data_ptr(), None if column_info is None else column_info.data_ptr(),
+                y.data_ptr(), ws.data_ptr(), ws.numel(), pkg._stream_ptr())
         if wide:
-            rc, where = lib.nmspmm_gemm_row_major(ctypes.byref(d), *ptrs), "nmspmm_gemm_row_major"
+            rc, where = lib.nmspmm_gemm_row_major(d, *ptrs), "nmspmm_gemm_row_major"
         else:
-            rc, where = lib.nmspmm_gemm_row_major_16(ctypes.byref(d), dtype, *ptrs), "nmspmm_gemm_row_major_16"
+            rc, where = lib.nmspmm_gemm_row_major_16(d, dtype, *ptrs), "nmspmm_gemm_row_major_16"
         if rc != pkg.OK:
             raise pkg.NMSpMMError(where, rc)
         return y
 
-    @sparse_linear.register_fake
+    _library.impl("sparse_linear", sparse_linear, "CUDA")
+
+    @torch.library.register_fake(name, lib=_library)
     def _(x, values, packed, column_info, raw_indices, n_keep, fmt, layout_ns, vec_len, path):
         return x.new_empty((x.shape[0], values.shape[1]))
 
@@ -122,9 +131,9 @@ def register_ops(pkg):
             grad_values = (x.to(torch.float32).t() @ g32).gather(0, rows)  # d/dB restricted to the kept positions
         return grad_x, grad_values, None, None, None, None, None, None, None, None
 
-    sparse_linear.register_autograd(backward, setup_context=setup_context)
-    _registered = sparse_linear
-    return sparse_linear
+    torch.library.register_autograd(name, backward, setup_context=setup_context, lib=_library)
+    _registered = torch.ops.nmspmm_b200.sparse_linear.default
+    return _registered
 
 
 class NMSparseLinear:
@@ -152,15 +161,24 @@ class NMSparseLinear:
 
     def __call__(self, x):
         torch = _torch()
+        flat = x.dim() == 2 and x.shape[1] == self.in_features
         lead = x.shape[:-1]
-        x2 = x.reshape(-1, self.in_features)
+        x2 = x if flat else x.reshape(-1, self.in_features)
         if x2.dtype not in (torch.float32, torch.float16, torch.bfloat16):
             x2 = x2.to(torch.float32)
-        y = self._op(x2, self.values, self.op.D, self.op.column_info, self.raw_indices, self.n_keep, self.op.format,
-                     self.op.layout_ns, self.vec_len, self.path)
+        op = self.op
+        args = (x2, self.values, op.D, op.column_info, self.raw_indices, self.n_keep, op.format, op.layout_ns, self.vec_len, self.path)
+        if torch.is_grad_enabled() or torch.compiler.is_compiling():
+            y = self._op(*args)
+        else:
+            # Nothing to record: straight to the operator's kernel, past the Python function behind its
+            # autograd key, which would call it again just so (4 us).  Everything above that key --
+            # tracing, functorch, dispatch modes, tensor subclasses -- still sees the call.
+            with torch._C._AutoDispatchBelowAutograd():
+                y = self._op(*args)
         if self.bias is not None:
             y = y + self.bias.to(y.dtype)
-        return y.reshape(*lead, self.out_features)
+        return y if flat else y.reshape(*lead, self.out_features)
 
     def dense_weight(self):
         """The pruned weight as a dense (out_features, in_features) tensor (zeros where pruned),

@@ -85,6 +85,32 @@ def test_custom_op_is_registered_with_fake_kernel_and_autograd(pkg):
         assert op(*fake).shape == (8, 256)
 
 
+def test_forward_without_gradients_takes_the_same_operator(pkg):
+    """Under no_grad the layer goes past the operator's autograd key only: the result is the recorded
+    call's, dispatch modes see the call, and host tensors are refused."""
+    from torch.utils._python_dispatch import TorchDispatchMode
+    seen = []
+
+    class Log(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            seen.append(str(func))
+            return func(*args, **(kwargs or {}))
+
+    layer = pkg.linear.NMSparseLinear(pkg, torch.randn(256, 128, device="cuda") * 0.1, 8)
+    x = torch.randn(2, 3, 128, device="cuda", requires_grad=True)
+    recorded = layer(x)
+    assert recorded.requires_grad and recorded.shape == (2, 3, 256)
+    with torch.no_grad():
+        plain = layer(x)
+        assert not plain.requires_grad and torch.equal(plain, recorded)
+        assert torch.equal(layer(x.reshape(6, 128)).reshape(2, 3, 256), recorded)
+        with Log():
+            layer(x)
+    assert any("sparse_linear" in name for name in seen)
+    with pytest.raises(TypeError):
+        layer(torch.randn(4, 128))
+
+
 # ---------------------------------------------------------------------------- 16-bit storage
 
 def _round_to(t, dtype):
