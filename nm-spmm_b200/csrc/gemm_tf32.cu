@@ -31,7 +31,7 @@
 //               the result buffer.  One thread issues a tcgen05.mma every 26 cycles at best
 //               (measured), and a step has 12 to 20 of them: three issuing threads keep the
 //               tensor pipe, not the issue slot, the bound.
-//   warps 4-7   one thread per (vector, kept row): fetches its index two to four steps ahead
+//   warps 4-11  (4-7 on the 128-column tile) one thread per (vector, kept row) and turn: fetches its index two to four steps ahead
 //               with cp.async (through column_info on the 64-k format), keeps P's one-hot
 //               entry current, and after the last step reads the accumulators (tcgen05.ld),
 //               transposes them through shared memory and stores C in 128-byte row pieces.
@@ -95,7 +95,7 @@ struct Tf32Cfg {
     static constexpr int QV = NS / VL;                       // vectors per tile
     static constexpr int N1 = QV * WSP;                      // gathered columns per step
     static_assert(VL == 32 || (VL == 64 && NKEEP != 32), "vectors of 32 or 64 columns");
-    static_assert(DIRECT || N1 <= 128, "one builder thread per gathered column");
+    static_assert(DIRECT || (N1 <= 128 && N1 % 32 == 0), "one builder thread per gathered column, whole warps");
     static_assert(MODE == kModeHigh || KW == 32, "only the 64-k format has merged windows");
     static_assert(!(DIRECT && SRC == kTf32Rows16), "the direct product multiplies A by FP32 rows of B");
     static constexpr int A_BYTES = 128 * KW * EB;            // col-major: [4 blocks of 32 rows of the tile][KW][32]; rows: [128][<= 128 bytes], blocks of 32 k if FP32
@@ -107,15 +107,25 @@ struct Tf32Cfg {
     static constexpr int TMEM_COLS = 512 / CTAS_PER_SM;      // each resident CTA allocates its share
     static constexpr int PD = 2;                             // index prefetch distance, in steps, per look-up
     static constexpr int RING = 4 * PD;                      // slots of the per-thread index rings
-    static constexpr int BUILDERS = 128;
+    // One thread keeps one gathered column; the builder warps form GROUPS groups of N1 threads that take
+    // turns with the steps.  A step is a chain of some 600 cycles for the warp that builds it (index
+    // arrived, stage free, old entry, new entry, proxy fence, arrival): with one group that chain,
+    // not the tensor pipe, was part of what an 8:32 step waited for: 4096 x 4096 x 11008, 8:32, 417 -> 404 us,
+    // with bfloat16 activations 444 -> 405; 4096 x 28672 x 2048 with 64-wide vectors 667 -> 636 and 632 -> 578.
+    static constexpr int BUILDERS = (QT == 8) ? 256 : 128;
+    static constexpr int GROUP_WARPS = N1 / 32;
     static constexpr int PRODUCT_WARPS = 2;
     static constexpr int THREADS = (2 + PRODUCT_WARPS) * 32 + BUILDERS;
-    static constexpr int AUX_BYTES = (2 * RING + 8) * BUILDERS * 4;    // index rings + previous one-hot per stage (<= 8 stages)
+    static constexpr int AUX_BYTES = 2 * RING * BUILDERS * 4 + 8 * 128 * 4;      // index rings; previous one-hot per stage (<= 8 stages) and column
     static constexpr int CTRL_BYTES = 256;
     static constexpr int SMEM_LIMIT = (CTAS_PER_SM == 1 ? 227 : 113) * 1024;
     static constexpr int ST0 = (SMEM_LIMIT - 1024 - AUX_BYTES - CTRL_BYTES) / STAGE_BYTES;
     static constexpr int STAGES = ST0 > 6 ? 6 : ST0;
     static_assert(STAGES >= 2, "at least two stages");
+    // A group that has built step i - GROUPS knows that step i - GROUPS - STAGES has been consumed; its
+    // wait for the stage of step i tells one phase from the next only if step i - 2 STAGES has been.
+    static constexpr int GROUPS = DIRECT ? 1 : (BUILDERS / N1 < STAGES ? BUILDERS / N1 : STAGES);
+    static_assert(GROUPS >= 1 && GROUPS <= STAGES, "see above");
     // Ring of gather results beside the accumulators.  A gather's result is complete (and its
     // commit arrives) some hundreds of cycles after issue, and the products that free the
     // buffer again take as long: the loop gather -> products -> gather is latency-bound
@@ -123,7 +133,7 @@ struct Tf32Cfg {
     static constexpr int NBUF0 = DIRECT ? 1 : (TMEM_COLS - NS) / N1;
     static constexpr int NBUF = NBUF0 > 4 ? 4 : NBUF0;
     static_assert(NBUF >= 1, "no room for a gather result beside the accumulators");
-    static constexpr int EPI_BYTES = 4 * kTf32PatchBytes;    // four warps' transposition patches
+    static constexpr int EPI_BYTES = BUILDERS / 32 * kTf32PatchBytes;    // the builder warps' transposition patches
     static_assert(EPI_BYTES <= STAGES * STAGE_BYTES, "the epilogue reuses the stage ring");
     static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + AUX_BYTES + CTRL_BYTES + 1024;   // + alignment slack
     static constexpr int ACOL0 = NS;                         // first gather-result column
@@ -162,9 +172,10 @@ nm_gemm_tf32_kernel(const GemmArgs g, const __grid_constant__ CUtensorMap map_a,
 
     extern __shared__ unsigned char smem_raw[];
     const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u;          // swizzle atoms want 1024-byte alignment
-    const uint32_t idx_ring = ring + STAGES * Cfg::STAGE_BYTES;           // [RING][128] raw index (rank on the 64-k format)
-    const uint32_t k_ring = idx_ring + RING * 512;                        // [RING][128] k after the column_info look-up
-    const uint32_t prev_k = k_ring + RING * 512;                          // [STAGES][128] one-hot entry now set in the stage
+    const uint32_t idx_ring = ring + STAGES * Cfg::STAGE_BYTES;           // [RING][BUILDERS] raw index (rank on the 64-k format)
+    constexpr int SLOT = Cfg::BUILDERS * 4;
+    const uint32_t k_ring = idx_ring + RING * SLOT;                       // [RING][BUILDERS] k after the column_info look-up
+    const uint32_t prev_k = k_ring + RING * SLOT;                         // [STAGES][128] one-hot entry of each column now set in the stage
     const uint32_t bars = ring + STAGES * Cfg::STAGE_BYTES + Cfg::AUX_BYTES;
     const uint32_t bar_full = bars, bar_empty = bars + STAGES * 8;
     const uint32_t bar_gdone = bar_empty + STAGES * 8, bar_gfree = bar_gdone + 4 * 8, bar_acc = bar_gfree + 4 * 8;
@@ -192,7 +203,7 @@ nm_gemm_tf32_kernel(const GemmArgs g, const __grid_constant__ CUtensorMap map_a,
         prefetch_tensor_map(&map_a);
         prefetch_tensor_map(&map_b);
         for (int s = 0; s < STAGES; ++s) {
-            mbar_init(bar_full + s * 8, DIRECT ? 1 : 1 + Cfg::BUILDERS / 32);   // the TMA bytes + the builder warps
+            mbar_init(bar_full + s * 8, DIRECT ? 1 : 1 + Cfg::GROUP_WARPS);     // the TMA bytes + the warps that build the step
             mbar_init(bar_empty + s * 8, DIRECT ? 1 : Cfg::PRODUCT_WARPS);      // the commits behind the step's products
         }
         for (int b = 0; b < 4; ++b) {
@@ -205,6 +216,7 @@ nm_gemm_tf32_kernel(const GemmArgs g, const __grid_constant__ CUtensorMap map_a,
     }
     if (warp == 1) tmem_alloc(tmem_word, Cfg::TMEM_COLS);
     if (!DIRECT) {
+        for (int o = tid * 4; o < 8 * 512; o += Cfg::THREADS * 4) sts_s32(prev_k + o, -1);
         // P starts as all zeros; 12:32 also wants the never-set columns of every vector zero
         const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
         for (int s = 0; s < STAGES; ++s)
@@ -365,42 +377,43 @@ nm_gemm_tf32_kernel(const GemmArgs g, const __grid_constant__ CUtensorMap map_a,
         }
     } else {
         // ------------------------------------------------------------------ one-hot builders
-        const int e = tid - FIRST_BUILDER * 32;            // gathered column this thread keeps
+        const int b = tid - FIRST_BUILDER * 32;
         const int quad = warp & 3;                         // TMEM lane quadrant this warp may touch
         bool alive = true;
         if (!DIRECT) {
+            constexpr int GROUPS = Cfg::GROUPS;
+            const int group = b / Cfg::N1, e = b % Cfg::N1;          // this thread keeps gathered column e of steps group, group + GROUPS, ...
             const int v = e / WSP, j = e % WSP;
-            const bool has = e < Cfg::N1 && j < WS && v * BPV < live_vecs;
+            const bool has = j < WS && v * BPV < live_vecs;
             const int q = (bj >> 5) + v * BPV, qs_shift = g.qs_shift;       // the (first) 32-column index list of vector v
             const int* dptr = g.D + ((static_cast<size_t>(q >> qs_shift) * g.W) << qs_shift) + (q & ((1 << qs_shift) - 1)) +
                               (static_cast<size_t>(j) << qs_shift);
             const int n_merged = (KW == 64) ? g.sched.n_win : (g.sched.n_win >> 1);
             const int* ciptr = (MODE == kModeHigh) ? g.cinfo + static_cast<size_t>(q >> qs_shift) * n_merged * 64 : nullptr;
-            const uint32_t my_idx = idx_ring + e * 4, my_k = k_ring + e * 4, my_prev = prev_k + e * 4;
-            for (int s = 0; s < STAGES; ++s) sts_s32(my_prev + s * 512, -1);
+            const uint32_t my_idx = idx_ring + b * 4, my_k = k_ring + b * 4, my_prev = prev_k + e * 4;
             TF_DECL(b_cp = 0, b_empty = 0);
             TF_T(b_start);
-            for (int i = -2 * PD; i < n_win; ++i) {
+            for (int turn = -2 * PD, i = group - 2 * PD * GROUPS; group < GROUPS && i < n_win; ++turn, i += GROUPS) {
                 TF_T(t0);
-                cp_async_wait<PD - 1>();                   // the copies issued PD iterations ago and earlier have landed
+                cp_async_wait<PD - 1>();                   // the copies issued PD turns ago and earlier have landed
                 TF_ADD(b_cp, t0);
                 int k = 0;
-                if (has && i >= 0) {
-                    k = lds_s32((MODE == kModeHigh ? my_k : my_idx) + (i & (RING - 1)) * 512);
+                if (has && turn >= 0) {
+                    k = lds_s32((MODE == kModeHigh ? my_k : my_idx) + (turn & (RING - 1)) * SLOT);
                     if (MODE == kModeHigh && KW == 32) k -= ((win0 + i) & 1) * 32;
                 }
                 if (has) {
-                    const int i2 = i + 2 * PD, i1 = i + PD;
+                    const int i2 = i + 2 * PD * GROUPS, i1 = i + PD * GROUPS;
                     if (i2 < n_win)
-                        cp_async_4(my_idx + (i2 & (RING - 1)) * 512, dptr + ((static_cast<size_t>(win0 + i2) * WS) << qs_shift));
-                    if (MODE == kModeHigh && i1 >= 0 && i1 < n_win) {
-                        const int rank = lds_s32(my_idx + (i1 & (RING - 1)) * 512);
+                        cp_async_4(my_idx + ((turn + 2 * PD) & (RING - 1)) * SLOT, dptr + ((static_cast<size_t>(win0 + i2) * WS) << qs_shift));
+                    if (MODE == kModeHigh && turn >= -PD && i1 < n_win) {
+                        const int rank = lds_s32(my_idx + ((turn + PD) & (RING - 1)) * SLOT);
                         const int m = (KW == 64) ? (win0 + i1) : ((win0 + i1) >> 1);
-                        cp_async_4(my_k + (i1 & (RING - 1)) * 512, ciptr + static_cast<size_t>(m) * 64 + rank);
+                        cp_async_4(my_k + ((turn + PD) & (RING - 1)) * SLOT, ciptr + static_cast<size_t>(m) * 64 + rank);
                     }
                 }
                 cp_async_commit();
-                if (i < 0) continue;
+                if (turn < 0) continue;
                 const int s = i % STAGES;
                 if (i >= STAGES) {
                     TF_T(t1);
@@ -439,13 +452,15 @@ nm_gemm_tf32_kernel(const GemmArgs g, const __grid_constant__ CUtensorMap map_a,
             tc_fence_after_sync();
             // every MMA has completed, so every TMA copy has landed and been read: the
             // stage ring is free and serves as the transposition patches
-            tf32_store_vectors<NS>(tmem, quad, lane, 0, live_vecs, ring + (warp - FIRST_BUILDER) * kTf32PatchBytes, g, outs, bi, bj,
-                                   sliced, slot);
+            constexpr int SHARES = Cfg::BUILDERS / 128, VPW = QT / SHARES;     // the warps of a quadrant share the vectors
+            const int v0 = (warp - FIRST_BUILDER) / 4 * VPW;
+            tf32_store_vectors<NS>(tmem, quad, lane, v0, min(v0 + VPW, live_vecs), ring + (warp - FIRST_BUILDER) * kTf32PatchBytes, g, outs,
+                                   bi, bj, sliced, slot);
         } else if (lane == 0) {
             atomicMax(g.status, kDevTimeoutMma);
         }
 #ifdef NMSPMM_TF32_PROFILE
-        if (e == 0) { TF_OUT(13, e_go - e_start); TF_OUT(14, clock64() - e_go); }
+        if (b == 0) { TF_OUT(13, e_go - e_start); TF_OUT(14, clock64() - e_go); }
 #endif
     }
     tc_fence_before_sync();
