@@ -116,11 +116,16 @@ struct Tf32Cfg {
     static constexpr int GROUP_WARPS = N1 / 32;
     static constexpr int PRODUCT_WARPS = 2;
     static constexpr int THREADS = (2 + PRODUCT_WARPS) * 32 + BUILDERS;
-    static constexpr int AUX_BYTES = 2 * RING * BUILDERS * 4 + 8 * 128 * 4;      // index rings; previous one-hot per stage (<= 8 stages) and column
+    // Every stage counts: a step's way through its stage -- copies, one-hot entries, gather, products and the
+    // barriers between them -- takes some 2400 cycles even with nothing to compute (bfloat16 activations,
+    // 2048 x 9472 x 4096, 8:32, four / six / eight stages: 202 / 185 / 171 us).  FP32 stages are larger; a seventh where
+    // it fits (64-wide vectors, 8:32) measured 2 % slower.
+    static constexpr int MAX_STAGES = (SRC == kTf32Rows16) ? 8 : 6;
+    static constexpr int AUX_BYTES = 2 * RING * BUILDERS * 4 + MAX_STAGES * 128 * 4;      // index rings; previous one-hot per stage and column
     static constexpr int CTRL_BYTES = 256;
     static constexpr int SMEM_LIMIT = (CTAS_PER_SM == 1 ? 227 : 113) * 1024;
     static constexpr int ST0 = (SMEM_LIMIT - 1024 - AUX_BYTES - CTRL_BYTES) / STAGE_BYTES;
-    static constexpr int STAGES = ST0 > 6 ? 6 : ST0;
+    static constexpr int STAGES = ST0 > MAX_STAGES ? MAX_STAGES : ST0;
     static_assert(STAGES >= 2, "at least two stages");
     // A group that has built step i - GROUPS knows that step i - GROUPS - STAGES has been consumed; its
     // wait for the stage of step i tells one phase from the next only if step i - 2 STAGES has been.
@@ -131,7 +136,8 @@ struct Tf32Cfg {
     // buffer again take as long: the loop gather -> products -> gather is latency-bound
     // unless several steps are in flight, so the ring is as deep as Tensor Memory allows.
     static constexpr int NBUF0 = DIRECT ? 1 : (TMEM_COLS - NS) / N1;
-    static constexpr int NBUF = NBUF0 > 4 ? 4 : NBUF0;
+    static constexpr int NBUF1 = NBUF0 > 4 ? 4 : NBUF0;
+    static constexpr int NBUF = NBUF1 > STAGES ? STAGES : NBUF1;     // (the barrier that frees a step's stage frees its buffer too)
     static_assert(NBUF >= 1, "no room for a gather result beside the accumulators");
     static constexpr int EPI_BYTES = BUILDERS / 32 * kTf32PatchBytes;    // the builder warps' transposition patches
     static_assert(EPI_BYTES <= STAGES * STAGE_BYTES, "the epilogue reuses the stage ring");
@@ -178,9 +184,9 @@ nm_gemm_tf32_kernel(const GemmArgs g, const __grid_constant__ CUtensorMap map_a,
     const uint32_t prev_k = k_ring + RING * SLOT;                         // [STAGES][128] one-hot entry of each column now set in the stage
     const uint32_t bars = ring + STAGES * Cfg::STAGE_BYTES + Cfg::AUX_BYTES;
     const uint32_t bar_full = bars, bar_empty = bars + STAGES * 8;
-    const uint32_t bar_gdone = bar_empty + STAGES * 8, bar_gfree = bar_gdone + 4 * 8, bar_acc = bar_gfree + 4 * 8;
+    const uint32_t bar_gdone = bar_empty + STAGES * 8, bar_acc = bar_gdone + 4 * 8;
     const uint32_t tmem_word = bar_acc + 8, abort_word = tmem_word + 4;
-    static_assert((2 * 6 + 2 * 4 + 1) * 8 + 8 <= Cfg::CTRL_BYTES, "control block");
+    static_assert((2 * Cfg::MAX_STAGES + 4 + 1) * 8 + 8 <= Cfg::CTRL_BYTES, "control block");
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     // The first n_dp CTAs take one whole tile each.  The remaining tiles (the partial last
@@ -206,17 +212,14 @@ nm_gemm_tf32_kernel(const GemmArgs g, const __grid_constant__ CUtensorMap map_a,
             mbar_init(bar_full + s * 8, DIRECT ? 1 : 1 + Cfg::GROUP_WARPS);     // the TMA bytes + the warps that build the step
             mbar_init(bar_empty + s * 8, DIRECT ? 1 : Cfg::PRODUCT_WARPS);      // the commits behind the step's products
         }
-        for (int b = 0; b < 4; ++b) {
-            mbar_init(bar_gdone + b * 8, 1);                                    // the commit behind a gather
-            mbar_init(bar_gfree + b * 8, Cfg::PRODUCT_WARPS);                   // the commits behind the products that read it
-        }
+        for (int b = 0; b < 4; ++b) mbar_init(bar_gdone + b * 8, 1);            // the commit behind a gather
         mbar_init(bar_acc, DIRECT ? 1 : Cfg::PRODUCT_WARPS);
         sts_volatile_s32(abort_word, 0);
         mbar_init_fence();
     }
     if (warp == 1) tmem_alloc(tmem_word, Cfg::TMEM_COLS);
     if (!DIRECT) {
-        for (int o = tid * 4; o < 8 * 512; o += Cfg::THREADS * 4) sts_s32(prev_k + o, -1);
+        for (int o = tid * 4; o < Cfg::MAX_STAGES * 512; o += Cfg::THREADS * 4) sts_s32(prev_k + o, -1);
         // P starts as all zeros; 12:32 also wants the never-set columns of every vector zero
         const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
         for (int s = 0; s < STAGES; ++s)
@@ -285,8 +288,10 @@ nm_gemm_tf32_kernel(const GemmArgs g, const __grid_constant__ CUtensorMap map_a,
             bool ok = mbar_wait_bounded(bar_full + s * 8, (t / STAGES) & 1, abort_word);
             TF_ADD(m_full, t0);
             TF_T(t1);
-            if (!DIRECT && t >= NBUF)                      // the result buffer is free once the products of step t - NBUF are done
-                ok = ok && mbar_wait_bounded(bar_gfree + (t % NBUF) * 8, ((t / NBUF) - 1) & 1, abort_word);
+            // the result buffer is free once the products of step t - NBUF are done, which is when that
+            // step's stage is (the stage's next phase ends with step t - NBUF + STAGES, not before this one)
+            if (!DIRECT && t >= NBUF)
+                ok = ok && mbar_wait_bounded(bar_empty + ((t - NBUF) % STAGES) * 8, ((t - NBUF) / STAGES) & 1, abort_word);
             TF_ADD(m_free, t1);
             if (!__all_sync(0xffffffffu, ok)) { alive = false; break; }
             TF_T(t2);
@@ -356,11 +361,9 @@ nm_gemm_tf32_kernel(const GemmArgs g, const __grid_constant__ CUtensorMap map_a,
                                              umma_desc_mn_tf32(bs + v * (BPV * WSP * 128) + gi * 1024, WSP * 128, 512),
                                              idesc_product, (u | gi) != 0);
                         }
-                        tc_commit(bar_empty + s * 8);      // this half of the step's products has read the stage
-                        tc_commit(bar_gfree + b * 8);      // and the gather result
+                        tc_commit(bar_empty + s * 8);      // this half of the step's products has read the stage and the gather result
                     } else {
                         mbar_arrive(bar_empty + s * 8);    // no vector of this half exists; the gather itself has completed
-                        mbar_arrive(bar_gfree + b * 8);
                     }
                 }
                 __syncwarp();
