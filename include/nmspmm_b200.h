@@ -167,9 +167,10 @@ int nmspmm_gemm(const nmspmm_gemm_desc* desc,
                 float* C_dev, void* workspace_dev, size_t workspace_bytes, void* stream);
 
 /* The multiply for activations stored row-major, A[i*K + k] (no counterpart in the reference,
- * whose A is col-major, include/utils.h:34-38; a linear layer's input is not).  A first kernel
- * on `stream` writes the col-major copy (its k rows padded to a multiple of 4 floats, so M
- * may be any positive number here) into the workspace, the multiply follows.
+ * whose A is col-major, include/utils.h:34-38; a linear layer's input is not).  M may be any
+ * positive number here.  The TF32 path's kernels read A as it lies in memory where it starts on
+ * 16 bytes; for the exact path (and an A that does not) a first kernel on `stream` writes the
+ * col-major copy, its k rows padded to a multiple of 4 floats, into the workspace.
  * C is row-major M x N as everywhere.  The workspace holds what nmspmm_gemm needs (first, so
  * that the counter block keeps its place when the same workspace serves different M) and then
  * that copy: ask nmspmm_gemm_row_major_workspace_bytes. */
@@ -184,9 +185,10 @@ int nmspmm_gemm_row_major(const nmspmm_gemm_desc* desc,
  * are widened once, nmspmm_widen_device, before they are compressed).  Every half and
  * bfloat16 value is a TF32 value, so on NMSPMM_PATH_TF32 the products of widened operands
  * are exact and only the FP32 sums and the final rounding of y (to nearest even) separate the
- * result from the real one; NMSPMM_PATH_FP32 is exact in the same sense.  One kernel widens
- * and transposes x, the multiply follows, one kernel rounds y; the workspace holds what the
- * multiply needs and the two FP32 copies. */
+ * result from the real one; NMSPMM_PATH_FP32 is exact in the same sense.  The TF32 path reads x
+ * and writes y in `dtype` (x on 16 bytes; an unpruned B excepted); otherwise one kernel widens
+ * and transposes x, and on the exact path one rounds y.  The workspace holds what the
+ * multiply needs and room for the two FP32 copies. */
 enum nmspmm_dtype { NMSPMM_DTYPE_F32 = 0, NMSPMM_DTYPE_F16 = 1, NMSPMM_DTYPE_BF16 = 2 };
 size_t nmspmm_gemm_row_major_16_workspace_bytes(const nmspmm_gemm_desc* desc);
 int nmspmm_gemm_row_major_16(const nmspmm_gemm_desc* desc, int dtype,

@@ -2,13 +2,14 @@
 weight pruned to ``n_keep``:32 (per-vector L2 magnitude), compressed and packed on the GPU
 once, and every forward one call of the multiply.
 
-The forward is registered with ``torch.library`` as the custom operator
+The forward is registered with ``torch.library`` as the operator
 ``nmspmm_b200::sparse_linear`` (with a fake kernel for tracing and an autograd formula), so
 the layer can be traced, compiled around and differentiated.  Activations are taken
-row-major as they come (``nmspmm_gemm_row_major`` transposes on the GPU ahead of the
-multiply); nothing is padded or transposed in eager PyTorch.  float16 / bfloat16 activations
-give a result of the same dtype (``nmspmm_gemm_row_major_16``: widened exactly inside the
-transposition, summed in FP32, rounded once at the end); the compressed weights are FP32.
+row-major as they come (``nmspmm_gemm_row_major``: the tensor-core path reads them so, the exact
+path transposes on the GPU ahead of the multiply); nothing is padded or transposed in eager
+PyTorch.  float16 / bfloat16 activations give a result of the same dtype
+(``nmspmm_gemm_row_major_16``: widened exactly, summed in FP32, rounded once at the end); the
+compressed weights are FP32.
 
 The backward pass runs on the compressed weight too (``nmspmm_linear_grad``: both gradients in
 FP32, n_keep / 32 of the work of the dense products); an unpruned weight (32 of 32) and a
