@@ -110,6 +110,21 @@ def register_ops(pkg):
     def _(x, values, packed, column_info, raw_indices, n_keep, fmt, layout_ns, vec_len, path):
         return x.new_empty((x.shape[0], values.shape[1]))
 
+    # The backward's kernels behind an operator of their own: whatever traces, batches or compiles a backward pass sees
+    # one opaque call with a fake kernel.  A gradient that is not wanted comes back with no elements.
+    _library.define("sparse_linear_grad(Tensor x, Tensor values, Tensor raw_indices, Tensor grad_y, SymInt n_keep, bool want_x, "
+                    "bool want_values) -> (Tensor, Tensor)", tags=(torch.Tag.pt2_compliant_tag,))
+
+    def sparse_linear_grad(x, values, raw_indices, grad_y, n_keep, want_x, want_values):
+        grad_x, grad_values = _sparse_grads(pkg, x, values, raw_indices, n_keep, grad_y, want_x, want_values)
+        return x.new_empty(0) if grad_x is None else grad_x, values.new_empty(0) if grad_values is None else grad_values
+
+    _library.impl("sparse_linear_grad", sparse_linear_grad, "CUDA")
+
+    @torch.library.register_fake("nmspmm_b200::sparse_linear_grad", lib=_library)
+    def _(x, values, raw_indices, grad_y, n_keep, want_x, want_values):
+        return x.new_empty(x.shape if want_x else (0,)), values.new_empty(values.shape if want_values else (0,))
+
     def setup_context(ctx, inputs, output):
         x, values, _packed, _ci, raw_indices, n_keep = inputs[:6]
         ctx.n_keep = n_keep
@@ -120,7 +135,8 @@ def register_ops(pkg):
         want_x, want_values = ctx.needs_input_grad[0], ctx.needs_input_grad[1]
         # (with create_graph the formula has to be differentiable itself: the dense products below)
         if ctx.n_keep in (16, 12, 8, 4) and not torch.is_grad_enabled():
-            return (*_sparse_grads(pkg, x, values, raw_indices, ctx.n_keep, grad_y, want_x, want_values), *[None] * 8)
+            grad_x, grad_values = torch.ops.nmspmm_b200.sparse_linear_grad(x, values, raw_indices, grad_y, ctx.n_keep, want_x, want_values)
+            return (grad_x if want_x else None, grad_values if want_values else None, *[None] * 8)
         rows = _dense_rows(raw_indices, ctx.n_keep)                       # (W, N) global k of every kept value
         grad_x = grad_values = None
         g32 = grad_y.to(torch.float32)

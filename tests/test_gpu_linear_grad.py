@@ -68,3 +68,33 @@ def test_backward_that_is_differentiated_again(pkg):
     (gx,) = torch.autograd.grad(layer(x).square().sum(), x, create_graph=True)
     (second,) = torch.autograd.grad(gx.square().sum(), layer.values)
     assert torch.isfinite(second).all() and float(second.norm()) > 0
+
+
+def test_backward_is_an_operator(pkg):
+    """Traced, compiled and batched backward passes reach the same kernels as a plain one."""
+    from torch.fx.experimental.proxy_tensor import make_fx
+    torch.manual_seed(4)
+    layer = pkg.linear.NMSparseLinear(pkg, torch.randn(256, 128, device="cuda"), 8)
+    layer.values.requires_grad_(True)
+    x = torch.randn(8, 128, device="cuda", requires_grad=True)
+    args = (x, layer.values, layer.op.D, layer.op.column_info, layer.raw_indices, 8, layer.op.format, layer.op.layout_ns, 32, 0)
+    torch.library.opcheck(torch.ops.nmspmm_b200.sparse_linear, args)
+    torch.library.opcheck(torch.ops.nmspmm_b200.sparse_linear_grad,
+                          (x.detach(), layer.values.detach(), layer.raw_indices, torch.randn(8, 256, device="cuda"), 8, True, False))
+
+    def step(x):
+        x = x.detach().requires_grad_()
+        return torch.autograd.grad(layer(x).square().sum(), (x, layer.values))
+
+    want = step(x)
+    for got in (make_fx(step)(x)(x), step(x)):
+        assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+    torch._dynamo.reset()
+    xc = x.detach().clone().requires_grad_()
+    torch.compile(lambda x: layer(x).square().sum(), backend="aot_eager")(xc).backward()
+    assert torch.equal(xc.grad, want[0]) and torch.equal(layer.values.grad, want[1])
+    y, c = layer(x), torch.randn(3, 8, 256, device="cuda")
+    batched = torch.autograd.grad(y, (x, layer.values), c, is_grads_batched=True, retain_graph=True)
+    for i in range(3):
+        one = torch.autograd.grad(y, (x, layer.values), c[i], retain_graph=True)
+        assert torch.equal(batched[0][i], one[0]) and torch.equal(batched[1][i], one[1])
