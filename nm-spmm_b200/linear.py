@@ -43,6 +43,7 @@ def _sparse_grads(pkg, x, values, raw_indices, n_keep: int, grad_y, want_x: bool
     torch = _torch()
     lib = pkg.load_library()
     x, values, grad_y = x.contiguous(), values.contiguous(), grad_y.to(x.dtype).contiguous()
+    raw_indices = raw_indices.to(torch.int32).contiguous()                # the kernels read (W, N/32) int32 as it lies
     if grad_y.data_ptr() % 16 != 0:
         grad_y = grad_y.clone()                                           # a view into the middle of a buffer: TMA wants 16 bytes
     dtype = pkg.dtype_id(x.dtype)

@@ -98,3 +98,12 @@ def test_backward_is_an_operator(pkg):
     for i in range(3):
         one = torch.autograd.grad(y, (x, layer.values), c[i], retain_graph=True)
         assert torch.equal(batched[0][i], one[0]) and torch.equal(batched[1][i], one[1])
+
+
+def test_raw_indices_of_any_integer_type_and_stride(pkg):
+    values, DT, gen = _operand(pkg, 256, 128, 8, seed=5)
+    x, g = torch.randn((9, 128), device="cuda", generator=gen), torch.randn((9, 256), device="cuda", generator=gen)
+    want = pkg.linear._sparse_grads(pkg, x, values, DT, 8, g, True, True)
+    for raw in (DT.long(), DT.to(torch.uint8), DT.t().contiguous().t()):
+        got = pkg.linear._sparse_grads(pkg, x, values, raw, 8, g, True, True)
+        assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
