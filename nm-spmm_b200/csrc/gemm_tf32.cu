@@ -165,7 +165,8 @@ __device__ __forceinline__ void sts_u16(uint32_t addr, unsigned v)
     asm volatile("st.shared.u16 [%0], %1;" ::"r"(addr), "h"(static_cast<unsigned short>(v)) : "memory");
 }
 
-template <int NKEEP, int KW_, int MODE, int QT_, int VL_, int SRC_>
+// C16: C is stored in 16 bits (a parameter: see gemm_tf32_few_rows.cu).
+template <int NKEEP, int KW_, int MODE, int QT_, int VL_, int SRC_, bool C16>
 __global__ void __launch_bounds__((Tf32Cfg<NKEEP, KW_, MODE, QT_, VL_, SRC_>::THREADS), (Tf32Cfg<NKEEP, KW_, MODE, QT_, VL_, SRC_>::CTAS_PER_SM))
 nm_gemm_tf32_kernel(const GemmArgs g, const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                     const GemmOutputs outs, const int a_form)     // col-major: 1 where the rows of A are whole blocks of 32; 16 bits: the type
@@ -458,8 +459,8 @@ nm_gemm_tf32_kernel(const GemmArgs g, const __grid_constant__ CUtensorMap map_a,
             // stage ring is free and serves as the transposition patches
             constexpr int SHARES = Cfg::BUILDERS / 128, VPW = QT / SHARES;     // the warps of a quadrant share the vectors
             const int v0 = (warp - FIRST_BUILDER) / 4 * VPW;
-            tf32_store_vectors<NS>(tmem, quad, lane, v0, min(v0 + VPW, live_vecs), ring + (warp - FIRST_BUILDER) * kTf32PatchBytes, g, outs,
-                                   bi, bj, sliced, slot);
+            tf32_store_vectors<NS, C16>(tmem, quad, lane, v0, min(v0 + VPW, live_vecs), ring + (warp - FIRST_BUILDER) * kTf32PatchBytes, g,
+                                        outs, bi, bj, sliced, slot);
         } else if (lane == 0) {
             atomicMax(g.status, kDevTimeoutMma);
         }
@@ -475,11 +476,11 @@ nm_gemm_tf32_kernel(const GemmArgs g, const __grid_constant__ CUtensorMap map_a,
     }
 }
 
-template <int NKEEP, int KW, int MODE, int QT, int VL, int SRC>
+template <int NKEEP, int KW, int MODE, int QT, int VL, int SRC, bool C16>
 static cudaError_t launch_tf32_from(const GemmArgs& a, const GemmOutputs& outs, int tiles, cudaStream_t st)
 {
     using Cfg = Tf32Cfg<NKEEP, KW, MODE, QT, VL, SRC>;
-    auto kernel = nm_gemm_tf32_kernel<NKEEP, KW, MODE, QT, VL, SRC>;
+    auto kernel = nm_gemm_tf32_kernel<NKEEP, KW, MODE, QT, VL, SRC, C16>;
     static bool configured[64] = {};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -510,10 +511,17 @@ static cudaError_t launch_tf32_from(const GemmArgs& a, const GemmOutputs& outs, 
 template <int NKEEP, int KW, int MODE, int QT, int VL>
 static cudaError_t launch_tf32(const GemmArgs& a, const GemmOutputs& outs, int tiles, cudaStream_t st)
 {
-    if (outs.a_rows == 0) return launch_tf32_from<NKEEP, KW, MODE, QT, VL, kTf32Cols>(a, outs, tiles, st);
-    if (outs.a_rows == 1 + kDtypeF32) return launch_tf32_from<NKEEP, KW, MODE, QT, VL, kTf32Rows32>(a, outs, tiles, st);
-    if constexpr (NKEEP != 32) return launch_tf32_from<NKEEP, KW, MODE, QT, VL, kTf32Rows16>(a, outs, tiles, st);
-    else return cudaErrorInvalidValue;
+    const bool c16 = outs.c_dtype != kDtypeF32;
+    if (c16 && outs.n_out != 1) return cudaErrorInvalidValue;
+    if (outs.a_rows == 0)                                  // 16-bit C: activations that had to be transposed ahead
+        return c16 ? launch_tf32_from<NKEEP, KW, MODE, QT, VL, kTf32Cols, true>(a, outs, tiles, st)
+                   : launch_tf32_from<NKEEP, KW, MODE, QT, VL, kTf32Cols, false>(a, outs, tiles, st);
+    if (outs.a_rows == 1 + kDtypeF32)
+        return c16 ? cudaErrorInvalidValue : launch_tf32_from<NKEEP, KW, MODE, QT, VL, kTf32Rows32, false>(a, outs, tiles, st);
+    if constexpr (NKEEP != 32)
+        return c16 ? launch_tf32_from<NKEEP, KW, MODE, QT, VL, kTf32Rows16, true>(a, outs, tiles, st) : cudaErrorInvalidValue;
+    else
+        return cudaErrorInvalidValue;
 }
 
 #define NMSPMM_TF32_VARIANT(NKEEP, KW, MODE, QT, VL)                                                                   \

@@ -74,7 +74,7 @@ __device__ __forceinline__ int ldg_stream_s32(const int* p)
     return v;
 }
 
-template <int NKEEP>
+template <int NKEEP, bool C16>
 __global__ void __launch_bounds__(Tf32ExpandCfg<NKEEP>::THREADS, 1)
 nm_gemm_tf32_expand_kernel(const GemmArgs g, const __grid_constant__ CUtensorMap map_a, const GemmOutputs outs, const int a_blocked)
 {
@@ -280,7 +280,7 @@ nm_gemm_tf32_expand_kernel(const GemmArgs g, const __grid_constant__ CUtensorMap
             // rings are free and serve as the transposition patches.  Two warps share a TMEM
             // lane quadrant (warp % 4); each takes half of the tile's vectors.
             const int half = v >> 2;
-            tf32_store_vectors<NS>(tmem, warp & 3, lane, min(half * (QT / 2), live_vecs), min((half + 1) * (QT / 2), live_vecs),
+            tf32_store_vectors<NS, C16>(tmem, warp & 3, lane, min(half * (QT / 2), live_vecs), min((half + 1) * (QT / 2), live_vecs),
                                    ring_a + v * kTf32PatchBytes, g, outs, bi, bj, sliced, slot);
         } else if (lane == 0) {
             atomicMax(g.status, kDevTimeoutMma);
@@ -294,11 +294,11 @@ nm_gemm_tf32_expand_kernel(const GemmArgs g, const __grid_constant__ CUtensorMap
     }
 }
 
-template <int NKEEP>
-static cudaError_t launch_tf32_expand(const GemmArgs& a, const GemmOutputs& outs, int tiles, cudaStream_t st)
+template <int NKEEP, bool C16>
+static cudaError_t launch_tf32_expand_to(const GemmArgs& a, const GemmOutputs& outs, int tiles, cudaStream_t st)
 {
     using Cfg = Tf32ExpandCfg<NKEEP>;
-    auto kernel = nm_gemm_tf32_expand_kernel<NKEEP>;
+    auto kernel = nm_gemm_tf32_expand_kernel<NKEEP, C16>;
     static bool configured[64] = {};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -317,6 +317,13 @@ static cudaError_t launch_tf32_expand(const GemmArgs& a, const GemmOutputs& outs
                   : encode_tensor_map_2d(&map_a, a.A, lda, K, 32, box_rows, 1);
     if (e != cudaSuccess) return e;
     return launch_overlapped(kernel, tiles, Cfg::THREADS, Cfg::SMEM_BYTES, st, a, map_a, outs, a_blocked);
+}
+
+template <int NKEEP>
+static cudaError_t launch_tf32_expand(const GemmArgs& a, const GemmOutputs& outs, int tiles, cudaStream_t st)
+{
+    if (outs.c_dtype == kDtypeF32) return launch_tf32_expand_to<NKEEP, false>(a, outs, tiles, st);
+    return outs.n_out == 1 ? launch_tf32_expand_to<NKEEP, true>(a, outs, tiles, st) : cudaErrorInvalidValue;
 }
 
 #define NMSPMM_TF32_EXPAND_VARIANT(NKEEP)                                                                              \

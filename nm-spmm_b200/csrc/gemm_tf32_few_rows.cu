@@ -95,10 +95,12 @@ __device__ __forceinline__ uint32_t load_element(uint32_t addr)      // as an FP
     }
 }
 
-template <int MS_, int WS_, int KS_, int MODE_, int SRC_>
+// C16: C is stored in 16 bits.  A parameter of the kernel, not a branch of its stores: with the type read
+// at run time the 64-row tiles, at the 128 registers that four CTAs per SM leave, spilled 96 bytes.
+template <int MS_, int WS_, int KS_, int MODE_, int SRC_, bool C16>
 __global__ void __launch_bounds__(128, (FewRowsCfg<MS_, WS_, KS_, MODE_, SRC_>::MIN_BLOCKS))
 nm_gemm_tf32_few_rows_kernel(const GemmArgs g, const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                           const GemmOutputs outs, const int a_blocked)
+                           const __grid_constant__ GemmOutputs outs, const int a_blocked)
 {
     using Cfg = FewRowsCfg<MS_, WS_, KS_, MODE_, SRC_>;
     constexpr int MS = Cfg::MS, NS = Cfg::NS, WS = Cfg::WS, KS = Cfg::KS, MB = Cfg::MB, STAGES = Cfg::STAGES;
@@ -258,27 +260,34 @@ nm_gemm_tf32_few_rows_kernel(const GemmArgs g, const __grid_constant__ CUtensorM
                 __stcg(reinterpret_cast<float2*>(p + 8 * NS), make_float2(acc[mb][nb][2], acc[mb][nb][3]));
             }
     } else {
-        for (int o = 0; o < outs.n_out; ++o) {
-            float* C = output_of(g, outs, o);
-            const size_t c0 = static_cast<size_t>(outs.col0) + bj + col;
+        auto store_tile = [&](auto* C, auto pair) {        // C at this lane's first column of the tile's first row
 #pragma unroll
             for (int mb = 0; mb < MB; ++mb) {
                 const int r0 = mb * 16 + gq, r1 = r0 + 8;
 #pragma unroll
                 for (int nb = 0; nb < 4; ++nb) {
-                    if (r0 < g.M) store_c2(C, c0 + static_cast<size_t>(r0) * outs.ldc + nb * 8, make_float2(acc[mb][nb][0], acc[mb][nb][1]), outs.c_dtype);
-                    if (r1 < g.M) store_c2(C, c0 + static_cast<size_t>(r1) * outs.ldc + nb * 8, make_float2(acc[mb][nb][2], acc[mb][nb][3]), outs.c_dtype);
+                    if (r0 < g.M) pair(C + static_cast<size_t>(r0) * outs.ldc + nb * 8, acc[mb][nb][0], acc[mb][nb][1]);
+                    if (r1 < g.M) pair(C + static_cast<size_t>(r1) * outs.ldc + nb * 8, acc[mb][nb][2], acc[mb][nb][3]);
                 }
             }
+        };
+        const size_t c0 = static_cast<size_t>(outs.col0) + bj + col;
+        if constexpr (C16) {                               // one private C
+            const int dtype = Cfg::SRC == kSrcRowsF16 ? kDtypeF16 : (Cfg::SRC == kSrcRowsBF16 ? kDtypeBF16 : outs.c_dtype);
+            store_tile(reinterpret_cast<uint16_t*>(g.C) + c0,
+                       [&](uint16_t* p, float lo, float hi) { *reinterpret_cast<uint32_t*>(p) = round_pair(lo, hi, dtype); });
+        } else {
+            for (int o = 0; o < outs.n_out; ++o)
+                store_tile(output_of(g, outs, o) + c0, [](float* p, float lo, float hi) { *reinterpret_cast<float2*>(p) = make_float2(lo, hi); });
         }
     }
 }
 
-template <int MS, int WS, int KS, int MODE, int SRC>
+template <int MS, int WS, int KS, int MODE, int SRC, bool C16>
 static cudaError_t launch_few_rows_from(const GemmArgs& a, const GemmOutputs& outs, int ctas, cudaStream_t st)
 {
     using Cfg = FewRowsCfg<MS, WS, KS, MODE, SRC>;
-    auto kernel = nm_gemm_tf32_few_rows_kernel<MS, WS, KS, MODE, SRC>;
+    auto kernel = nm_gemm_tf32_few_rows_kernel<MS, WS, KS, MODE, SRC, C16>;
     static bool configured[64] = {};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -307,11 +316,18 @@ static cudaError_t launch_few_rows_from(const GemmArgs& a, const GemmOutputs& ou
 template <int MS, int WS, int KS, int MODE>
 static cudaError_t launch_few_rows(const GemmArgs& a, const GemmOutputs& outs, int ctas, cudaStream_t st)
 {
+    const bool c16 = outs.c_dtype != kDtypeF32;
+    if (c16 && outs.n_out != 1) return cudaErrorInvalidValue;
     switch (outs.a_rows) {
-    case 0: return launch_few_rows_from<MS, WS, KS, MODE, kSrcCols>(a, outs, ctas, st);
-    case 1 + kDtypeF32: return launch_few_rows_from<MS, WS, KS, MODE, kSrcRows32>(a, outs, ctas, st);
-    case 1 + kDtypeF16: return launch_few_rows_from<MS, WS, KS, MODE, kSrcRowsF16>(a, outs, ctas, st);
-    case 1 + kDtypeBF16: return launch_few_rows_from<MS, WS, KS, MODE, kSrcRowsBF16>(a, outs, ctas, st);
+    case 0:                                                // 16-bit C: activations off a 16-byte boundary, transposed ahead
+        return c16 ? launch_few_rows_from<MS, WS, KS, MODE, kSrcCols, true>(a, outs, ctas, st)
+                   : launch_few_rows_from<MS, WS, KS, MODE, kSrcCols, false>(a, outs, ctas, st);
+    case 1 + kDtypeF32:
+        return c16 ? cudaErrorInvalidValue : launch_few_rows_from<MS, WS, KS, MODE, kSrcRows32, false>(a, outs, ctas, st);
+    case 1 + kDtypeF16:
+        return outs.c_dtype == kDtypeF16 ? launch_few_rows_from<MS, WS, KS, MODE, kSrcRowsF16, true>(a, outs, ctas, st) : cudaErrorInvalidValue;
+    case 1 + kDtypeBF16:
+        return outs.c_dtype == kDtypeBF16 ? launch_few_rows_from<MS, WS, KS, MODE, kSrcRowsBF16, true>(a, outs, ctas, st) : cudaErrorInvalidValue;
     default: return cudaErrorInvalidValue;
     }
 }

@@ -54,7 +54,7 @@ constexpr int kReduceInFlight = 16;   // loads of one thread that are issued bef
 // case of a handful of pieces, where the launch is what costs.
 template <int MS, int NS, int WM, int CTAS_PER_ROW>
 __global__ void __launch_bounds__((FragmentMap<MS, NS, WM>::NCT))
-nm_reduce_pieces_kernel(const GemmArgs g, const GemmOutputs outs, int first_tile)
+nm_reduce_pieces_kernel(const GemmArgs g, const __grid_constant__ GemmOutputs outs, int first_tile)
 {
     using Map = FragmentMap<MS, NS, WM>;
     constexpr int NCT = Map::NCT, MT = Map::MT;
@@ -144,8 +144,9 @@ cudaError_t launch_reduce_pieces(int tile_id, const GemmArgs& a, const GemmOutpu
 // flight for tiles of many slices (deep K: every round of loads is a trip to L2); EPT = 4 with
 // four in flight otherwise (fewer CTAs of fewer registers, more of which are resident before
 // the multiply ends: the launch is what costs there).
-template <int NS, int EPT, int MS = 128>
-__global__ void __launch_bounds__(256) nm_reduce_slices_kernel(const GemmArgs g, const GemmOutputs outs, int first_tile)
+// C16: one C, in 16 bits.  (A parameter: with C's type read per store every sum of slices took 0.3 us longer.)
+template <int NS, int EPT, int MS, bool C16>
+__global__ void __launch_bounds__(256) nm_reduce_slices_kernel(const GemmArgs g, const __grid_constant__ GemmOutputs outs, int first_tile)
 {
     constexpr int V4 = NS / 4;                             // float4 words per tile row; MS = rows of a slot
     constexpr int FLIGHT = (EPT == 1) ? kReduceInFlight : 4;   // loads in flight per thread
@@ -176,8 +177,21 @@ __global__ void __launch_bounds__(256) nm_reduce_slices_kernel(const GemmArgs g,
                 if (z + u < S) { sum.x += x[u].x; sum.y += x[u].y; sum.z += x[u].z; sum.w += x[u].w; }
         }
         const size_t at = static_cast<size_t>(bi + row) * outs.ldc + outs.col0 + bj + c4 * 4;
-        for (int o = 0; o < outs.n_out; ++o) store_c4(output_of(g, outs, o), at, sum, outs.c_dtype);
+        if constexpr (C16) {
+            store_four_16(g.C, at, sum, outs.c_dtype);
+        } else {
+            for (int o = 0; o < outs.n_out; ++o) *reinterpret_cast<float4*>(output_of(g, outs, o) + at) = sum;
+        }
     }
+}
+
+template <int NS, int EPT, int MS>
+static cudaError_t launch_slices(const GemmArgs& a, const GemmOutputs& outs, int first_tile, int n_tiles, cudaStream_t st)
+{
+    const int grid = n_tiles * (MS * NS / 4 / (256 * EPT));
+    if (outs.c_dtype == kDtypeF32) return launch_after_multiply(nm_reduce_slices_kernel<NS, EPT, MS, false>, grid, 256, st, a, outs, first_tile);
+    if (outs.n_out != 1) return cudaErrorInvalidValue;
+    return launch_after_multiply(nm_reduce_slices_kernel<NS, EPT, MS, true>, grid, 256, st, a, outs, first_tile);
 }
 
 cudaError_t launch_reduce_slices(int ns, const GemmArgs& a, const GemmOutputs& outs, int first_tile, int n_tiles, cudaStream_t st, int ms)
@@ -185,15 +199,13 @@ cudaError_t launch_reduce_slices(int ns, const GemmArgs& a, const GemmOutputs& o
     if (n_tiles <= 0) return cudaSuccess;
     const bool many = a.sched.split_k > kReduceInFlight / 2;
     if (ns == 256 && ms == 128)
-        return many ? launch_after_multiply(nm_reduce_slices_kernel<256, 1>, n_tiles * 32, 256, st, a, outs, first_tile)
-                    : launch_after_multiply(nm_reduce_slices_kernel<256, 4>, n_tiles * 8, 256, st, a, outs, first_tile);
+        return many ? launch_slices<256, 1, 128>(a, outs, first_tile, n_tiles, st) : launch_slices<256, 4, 128>(a, outs, first_tile, n_tiles, st);
     if (ns == 128 && ms == 128)
-        return many ? launch_after_multiply(nm_reduce_slices_kernel<128, 1>, n_tiles * 16, 256, st, a, outs, first_tile)
-                    : launch_after_multiply(nm_reduce_slices_kernel<128, 4>, n_tiles * 4, 256, st, a, outs, first_tile);
+        return many ? launch_slices<128, 1, 128>(a, outs, first_tile, n_tiles, st) : launch_slices<128, 4, 128>(a, outs, first_tile, n_tiles, st);
     // the few-row tiles of gemm_tf32_few_rows.cu: slots of ms x 128
-    if (ns == 128 && ms == 64) return launch_after_multiply(nm_reduce_slices_kernel<128, 1, 64>, n_tiles * 8, 256, st, a, outs, first_tile);
-    if (ns == 128 && ms == 32) return launch_after_multiply(nm_reduce_slices_kernel<128, 1, 32>, n_tiles * 4, 256, st, a, outs, first_tile);
-    if (ns == 128 && ms == 16) return launch_after_multiply(nm_reduce_slices_kernel<128, 1, 16>, n_tiles * 2, 256, st, a, outs, first_tile);
+    if (ns == 128 && ms == 64) return launch_slices<128, 1, 64>(a, outs, first_tile, n_tiles, st);
+    if (ns == 128 && ms == 32) return launch_slices<128, 1, 32>(a, outs, first_tile, n_tiles, st);
+    if (ns == 128 && ms == 16) return launch_slices<128, 1, 16>(a, outs, first_tile, n_tiles, st);
     return cudaErrorInvalidValue;
 }
 

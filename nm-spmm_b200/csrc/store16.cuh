@@ -1,4 +1,4 @@
-// Stores of FP32 results into a C of FP32, half or bfloat16 (rounded to nearest even).
+// Stores of FP32 results into a C of half or bfloat16 (rounded to nearest even).
 #pragma once
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -18,16 +18,10 @@ __device__ __forceinline__ uint32_t round_pair(float lo, float hi, int dtype)
     return *reinterpret_cast<const uint32_t*>(&h);
 }
 
-// Four / two adjacent elements from element `at` of C on.
-__device__ __forceinline__ void store_c4(float* C, size_t at, float4 v, int dtype)
+// Four adjacent elements from element `at` of a 16-bit C on (C as GemmArgs holds it).
+__device__ __forceinline__ void store_four_16(float* C, size_t at, float4 v, int dtype)
 {
-    if (dtype == kDtypeF32) *reinterpret_cast<float4*>(C + at) = v;
-    else *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(C) + at) = make_uint2(round_pair(v.x, v.y, dtype), round_pair(v.z, v.w, dtype));
-}
-__device__ __forceinline__ void store_c2(float* C, size_t at, float2 v, int dtype)
-{
-    if (dtype == kDtypeF32) *reinterpret_cast<float2*>(C + at) = v;
-    else *reinterpret_cast<uint32_t*>(reinterpret_cast<uint16_t*>(C) + at) = round_pair(v.x, v.y, dtype);
+    *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(C) + at) = make_uint2(round_pair(v.x, v.y, dtype), round_pair(v.z, v.w, dtype));
 }
 
 }  // namespace nmspmm

@@ -17,8 +17,8 @@ constexpr int kTf32PatchBytes = 32 * 144;   // one warp's 32 x 32 transposition 
 // bytes per store instruction.  The eight shared loads of a vector are issued ahead of its
 // eight global stores (as a chain of load -> store pairs the same work took three times as
 // long).  The peers' copies (fused all-gather) have a loop of their own so that the common
-// single-output case is a plain unrolled run.
-template <int NS>
+// single-output case is a plain unrolled run.  C16: one private C in 16 bits.
+template <int NS, bool C16 = false>
 __device__ __forceinline__ void tf32_store_vectors(uint32_t tmem, int quad, int lane, int v_begin, int v_end, uint32_t patch,
                                                    const GemmArgs& g, const GemmOutputs& outs, int bi, int bj, bool sliced,
                                                    int slot)
@@ -46,17 +46,19 @@ __device__ __forceinline__ void tf32_store_vectors(uint32_t tmem, int quad, int 
         float4 val[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) val[i] = lds_f4(patch + (4 * i + r_sub) * 144 + c4 * 4);
-        if (!sliced && outs.c_dtype != kDtypeF32) {        // one private 16-bit C
-            const size_t at = static_cast<size_t>(base - g.C);
+        if constexpr (C16) {
+            if (!sliced) {
+                const size_t at = static_cast<size_t>(base - g.C);
 #pragma unroll
-            for (int i = 0; i < 8; ++i)
-                if (4 * i < rows_left) store_c4(g.C, at + static_cast<size_t>(4 * i) * row_step, val[i], outs.c_dtype);
-            continue;
+                for (int i = 0; i < 8; ++i)
+                    if (4 * i < rows_left) store_four_16(g.C, at + static_cast<size_t>(4 * i) * row_step, val[i], outs.c_dtype);
+                continue;
+            }
         }
 #pragma unroll
         for (int i = 0; i < 8; ++i)
             if (4 * i < rows_left) *reinterpret_cast<float4*>(base + static_cast<size_t>(4 * i) * row_step) = val[i];
-        if (!sliced && outs.n_out > 1) {
+        if (!C16 && !sliced && outs.n_out > 1) {
             for (int o = 1; o < outs.n_out; ++o) {         // peers' copies of C when gathering
                 float* const pb = outs.C_more[o - 1] + (base - g.C);
 #pragma unroll
