@@ -289,3 +289,12 @@ def test_slices_of_equal_length_where_they_fill_the_slots(pkg):
                                                (320, 2048, 8, 64), (192, 4096, 16, 64), (1032, 4096, 12, 128)])
 def test_tile_of_the_exact_path_follows_padding_and_pairs(pkg, M, K, n_keep, tile_m):
     assert pkg.plan(pkg.make_desc(M, 4096, K, n_keep, pkg.format_of(n_keep), 128)).tile_m == tile_m
+
+
+def test_the_few_rows_kernels_do_not_spill(pkg_host):
+    """What ptxas said when the library was built: the 64-row tiles have 128 registers for four CTAs per SM."""
+    report = os.path.join(pkg_host.build.OBJ, "gemm_tf32_few_rows.cu.o.ptxas.txt")
+    if not os.path.exists(report):
+        pytest.skip("built without ptxas' report")
+    spills = [int(n) for n in re.findall(r"(\d+) bytes spill stores", open(report).read())]
+    assert len(spills) >= 12 and not any(spills)
