@@ -168,6 +168,8 @@ static int pick_tile(const nmspmm_gemm_desc* d, int sms)
 // Least share of the CTA slots, in per cent, that slices of equal length have to keep busy to be
 // taken over ranges that cross tiles (below).
 constexpr int kEvenSlicesPercent = 95;
+// What such slices save, in kept rows of a tile.
+constexpr int kEvenSlicesRows = 100;
 
 // ---- tuned plans ------------------------------------------------------------------
 // (M, N, K, n_keep, format, path, vec_len) -> tile and split_k found by measurement
@@ -513,13 +515,21 @@ static int make_plan(const nmspmm_gemm_desc* d_in, int sms, Plan* p, bool any_ro
             if (n_sk > tail_units) n_sk = tail_units;
             if (n_sk < 1) n_sk = 1;
             // A problem of less than one wave: ranges that are a whole number of slices of each tile
-            // where they keep nearly all of the CTA slots busy: no CTA then holds pieces of two tiles, and one slice per tile
-            // needs no scratch.  585 tiles on 592 slots (776 x 5760, K = 2048, 8:32): 117 -> 106 us, 288 on
-            // 296 (1032 x 4096 x 4096): 198 -> 188; at 86 to 91 % of the slots it gains at 4:32 and
-            // loses up to 9 % at 16:32, below it loses everywhere.  (Behind whole waves the choice
-            // moves nothing: the tail is short.)
+            // where that pays: no CTA then holds pieces of two tiles, and one slice per tile needs
+            // no scratch.  What it saves is about the time of 100 kept rows per tile, shared by the tile's
+            // slices; what it costs is the slots it leaves idle for the time of a slice.  So: idle share x
+            // kept rows of a tile <= 100.  739 plans that keep 95 % of the slots, 16 to 1536 rows, 4:32 to 16:32,
+            // K to 131072, B from HBM, slices against ranges: 0.95 to 1.44 times the speed; where this
+            // line takes them 1.027 in the mean over all plans, 0.987 the least (585 tiles on 592 slots,
+            // 776 x 5760, K = 2048, 8:32: 117 -> 106 us; refused: 564 of 592, 192 x 24064 x 22016, 16:32, 2099 -> 2182).
+            // Few-row tiles only where the rows of A are whole 64 bytes: there B is streamed, slices that
+            // start together read the same lines of A at the same time, and of other rows (4, 12 and 20 rows
+            // measured) each of those reads touches more lines: 4 x 24960 x 5120, 4:32, 36.8 -> 53.7 us,
+            // 12 x 24448 x 1536 16.8 -> 20.9.  (Behind whole waves the choice moves nothing: the tail is short.)
             const long long even = n_sk / tail_tiles * tail_tiles;
-            if (n_dp == 0 && even * 100 >= n_sk * kEvenSlicesPercent) n_sk = even;
+            const bool rows_suit = d->M > 64 || d->M % 16 == 0;
+            if (n_dp == 0 && rows_suit && even * 100 >= n_sk * kEvenSlicesPercent && (n_sk - even) * p->W <= kEvenSlicesRows * n_sk)
+                n_sk = even;
         }
         p->split_k = 0;
         p->n_dp = static_cast<int>(n_dp);

@@ -285,6 +285,16 @@ def test_slices_of_equal_length_where_they_fill_the_slots(pkg):
     assert ranges.n_virtual == 296
 
 
+@pytest.mark.parametrize("M,N,K,n_keep,n_virtual", [
+    (4, 12032, 2048, 12, 592), (4, 24960, 5120, 4, 592), (12, 24448, 1536, 4, 592), (20, 24704, 1536, 4, 592),   # rows of A not whole 64 bytes
+    (16, 24320, 4096, 4, 570), (32, 14848, 1024, 12, 580), (64, 10752, 4096, 16, 588),     # little left idle
+    (48, 12032, 22016, 16, 592), (192, 24064, 22016, 16, 592), (128, 6016, 14336, 16, 296), (256, 640, 120128, 8, 296)])  # too much left idle for too long
+def test_slices_of_equal_length_only_where_they_pay(pkg, M, N, K, n_keep, n_virtual):
+    """Plans of less than a wave whose equal slices would keep 95 % of the slots: taken where the idle share times
+    the kept rows is at most 100, and on few-row tiles where M is a multiple of 16."""
+    assert pkg.plan(pkg.make_desc(M, N, K, n_keep, pkg.format_of(n_keep), 128)).n_virtual == n_virtual
+
+
 @pytest.mark.parametrize("M,K,n_keep,tile_m", [(192, 2080, 12, 64), (320, 2080, 12, 128), (776, 2080, 16, 128), (320, 480, 12, 64),
                                                (320, 2048, 8, 64), (192, 4096, 16, 64), (1032, 4096, 12, 128)])
 def test_tile_of_the_exact_path_follows_padding_and_pairs(pkg, M, K, n_keep, tile_m):
