@@ -170,7 +170,8 @@ int nmspmm_gemm(const nmspmm_gemm_desc* desc,
  * whose A is col-major, include/utils.h:34-38; a linear layer's input is not).  M may be any
  * positive number here.  The TF32 path's kernels read A as it lies in memory where it starts on
  * 16 bytes; for the exact path (and an A that does not) a first kernel on `stream` writes the
- * col-major copy, its k rows padded to a multiple of 4 floats, into the workspace.
+ * col-major copy, its k rows padded to a multiple of 4 floats, into the workspace.  The same
+ * copy is made where C overlaps A: the result may overwrite the activations.
  * C is row-major M x N as everywhere.  The workspace holds what nmspmm_gemm needs (first, so
  * that the counter block keeps its place when the same workspace serves different M) and then
  * that copy: ask nmspmm_gemm_row_major_workspace_bytes. */
@@ -186,8 +187,8 @@ int nmspmm_gemm_row_major(const nmspmm_gemm_desc* desc,
  * bfloat16 value is a TF32 value, so on NMSPMM_PATH_TF32 the products of widened operands
  * are exact and only the FP32 sums and the final rounding of y (to nearest even) separate the
  * result from the real one; NMSPMM_PATH_FP32 is exact in the same sense.  The TF32 path reads x
- * and writes y in `dtype` (x on 16 bytes; an unpruned B excepted); otherwise one kernel widens
- * and transposes x, and on the exact path one rounds y.  The workspace holds what the
+ * and writes y in `dtype` (x on 16 bytes and apart from y; an unpruned B excepted); otherwise one
+ * kernel widens and transposes x, and on the exact path one rounds y.  The workspace holds what the
  * multiply needs and room for the two FP32 copies. */
 enum nmspmm_dtype { NMSPMM_DTYPE_F32 = 0, NMSPMM_DTYPE_F16 = 1, NMSPMM_DTYPE_BF16 = 2 };
 size_t nmspmm_gemm_row_major_16_workspace_bytes(const nmspmm_gemm_desc* desc);
@@ -202,7 +203,7 @@ int nmspmm_widen_device(int dtype, const void* src_dev, float* dst_dev, size_t n
  * M x K row-major and grad_y M x N row-major, both of `dtype`; B the compressed values and DT_dev
  * the raw window-local indices [W][N/32].  grad_x_dev (M x K, of dtype) receives
  * grad_y . B^T, grad_B_dev ([W][N], float) x^T . grad_y at the kept positions; either may be NULL
- * (then B resp. x may be too).  The workspace needs no initial contents. */
+ * (then B resp. x may be too).  No result may overlap an operand.  The workspace needs no initial contents. */
 size_t nmspmm_linear_grad_workspace_bytes(const nmspmm_gemm_desc* desc, int dtype, int want_x, int want_values);
 int nmspmm_linear_grad(const nmspmm_gemm_desc* desc, int dtype, const void* x_rows_dev, const void* grad_y_dev,
                        const float* B_dev, const int* DT_dev, void* grad_x_dev, float* grad_B_dev,

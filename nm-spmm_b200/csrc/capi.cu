@@ -881,12 +881,21 @@ static size_t row_major_head_bytes(const Plan& p)
     return own > 0 ? own : kCounterBlock;
 }
 
+static bool overlap(const void* a, size_t a_bytes, const void* b, size_t b_bytes)
+{
+    const uintptr_t x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
+    return x < y + b_bytes && y < x + a_bytes;
+}
+
 // The tensor-core path's kernels read row-major activations as they are, through a tensor map (so
 // they want them on 16 bytes); the others -- the exact path, the expanding form, and 16-bit rows of
-// an unpruned weight, whose product takes A and B in one type -- get a col-major copy.
-static bool reads_rows(const Plan& p, const void* A_rows, int dtype)
+// an unpruned weight, whose product takes A and B in one type -- get a col-major copy.  So does a
+// call whose result overwrites its activations: the copy is complete before C is written.
+static bool reads_rows(const Plan& p, const nmspmm_gemm_desc* d, const void* A_rows, const void* C, int dtype)
 {
-    return p.tv && p.tv->form != 1 && aligned16(A_rows) && (dtype == kDtypeF32 || p.tv->n_keep != 32);
+    const size_t size = dtype == kDtypeF32 ? 4 : 2;
+    return p.tv && p.tv->form != 1 && aligned16(A_rows) && (dtype == kDtypeF32 || p.tv->n_keep != 32) &&
+           !overlap(A_rows, size * d->M * d->K, C, size * d->M * d->N);
 }
 
 size_t nmspmm_gemm_row_major_workspace_bytes(const nmspmm_gemm_desc* desc)
@@ -907,7 +916,7 @@ int nmspmm_gemm_row_major(const nmspmm_gemm_desc* desc, const float* A_rows_dev,
     if (workspace_bytes < head + copy_bytes) return NMSPMM_WORKSPACE_TOO_SMALL;
     const int ld = (desc->M + 3) / 4 * 4;
     float* out[1] = { C_dev };
-    if (reads_rows(p, A_rows_dev, kDtypeF32))
+    if (reads_rows(p, desc, A_rows_dev, C_dev, kDtypeF32))
         return gemm_launch(desc, A_rows_dev, B_dev, D_dev, column_info_dev, out, 1, desc->N, 0, own ? workspace_dev : nullptr, own, stream, 0,
                            1 + kDtypeF32);
     float* A_cols = reinterpret_cast<float*>(static_cast<unsigned char*>(workspace_dev) + head);
@@ -951,7 +960,7 @@ int nmspmm_gemm_row_major_16(const nmspmm_gemm_desc* desc, int dtype, const void
     // The tensor-core path's kernels store C in 16 bits themselves; the exact path's, at the edge of
     // their registers, leave that to a pass over an FP32 C.
     float* const direct[1] = { static_cast<float*>(C_dev) };
-    if (reads_rows(p, A_rows_dev, dtype))
+    if (reads_rows(p, desc, A_rows_dev, C_dev, dtype))
         return gemm_launch(desc, static_cast<const float*>(A_rows_dev), B_dev, D_dev, column_info_dev, direct, 1, desc->N, 0,
                            own ? ws : nullptr, own, stream, 0, 1 + dtype, dtype);
     cudaError_t e = launch_transpose_rows(dtype, A_rows_dev, A_cols, desc->M, desc->K, ld, st);

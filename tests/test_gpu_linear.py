@@ -182,3 +182,22 @@ def test_one_workspace_serves_row_major_calls_of_different_row_counts(pkg, orc):
             tol = 1e-5 if dt == torch.float32 else 4e-3
             assert float((y.to(torch.float32) - ref).norm() / ref.norm()) <= tol, (M, dt)
     assert pkg.device_status() == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("path", [0, 1])
+@pytest.mark.parametrize("M,N,K", [(5, 256, 256), (33, 256, 256), (300, 256, 512), (2, 512, 256)])
+def test_the_result_may_overwrite_the_activations(pkg, dtype, path, M, N, K):
+    """x and y in one buffer: y at its head (same start, N <, =, > K), or starting inside x."""
+    p = pkg.formats.make_random(4, N, K, 8, seed=530 + M)
+    op = pkg.NMSpMM.from_problem(p)
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(M)
+    x = (torch.rand((M, K), device="cuda", generator=gen) * 2 - 1).to(dtype)
+    want = op.matmul_rows(x, path=path)
+    for at in (0, M * K // 2 // 16 * 16):                                # y's first element, on 16 bytes
+        buffer = torch.zeros(M * (K + N) + 16, dtype=dtype, device="cuda")
+        inside = buffer[:M * K].view(M, K).copy_(x)
+        y = buffer[at:at + M * N].view(M, N)
+        assert op.matmul_rows(inside, path=path, out=y) is y
+        assert float((y.double() - want.double()).norm() / want.double().norm()) <= (1e-5 if dtype == torch.float32 else 4e-3)
