@@ -70,6 +70,11 @@ def register_ops(pkg):
     # Defined through torch.library.Library rather than the custom_op decorator: the decorator's wrapper
     # around the body cost 7 us of host time a call, as much as the multiply of one token.
     global _library
+    if torch._C._dispatch_has_kernel("nmspmm_b200::sparse_linear"):
+        # Another copy of this package in the process (loaded under a second name) holds the operators: they
+        # take everything they need as arguments.
+        _registered = torch.ops.nmspmm_b200.sparse_linear.default
+        return _registered
     _library = torch.library.Library("nmspmm_b200", "FRAGMENT")
     name = "nmspmm_b200::sparse_linear"
     _library.define("sparse_linear(Tensor x, Tensor values, Tensor packed, Tensor? column_info, Tensor raw_indices, SymInt n_keep, "

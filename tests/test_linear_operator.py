@@ -93,3 +93,19 @@ def test_backward_on_meta_tensors(op, operand):
     y = op(x, values, torch.zeros(4, dtype=torch.int32, device="meta"), None, raw, N_KEEP, 1, 128, 32, 0)
     gx, gv = torch.autograd.grad(y.sum(), (x, values))
     assert gx.shape == x.shape and gv.shape == values.shape
+
+
+def test_a_second_copy_of_the_package_shares_the_operator(op, pkg_host):
+    import importlib.util
+    import os
+    import sys
+    here = os.path.dirname(pkg_host.__file__)
+    spec = importlib.util.spec_from_file_location("nm_spmm_second", os.path.join(here, "__init__.py"), submodule_search_locations=[here])
+    second = importlib.util.module_from_spec(spec)
+    sys.modules["nm_spmm_second"] = second
+    try:
+        spec.loader.exec_module(second)
+        assert second.linear.register_ops(second) is pkg_host.linear.register_ops(pkg_host)
+    finally:
+        for name in [n for n in sys.modules if n.split(".")[0] == "nm_spmm_second"]:
+            del sys.modules[name]
