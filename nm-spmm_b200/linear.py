@@ -12,8 +12,9 @@ PyTorch.  float16 / bfloat16 activations give a result of the same dtype
 compressed weights are FP32.
 
 The backward pass runs on the compressed weight too (``nmspmm_linear_grad``: both gradients in
-FP32, n_keep / 32 of the work of the dense products); an unpruned weight (32 of 32) and a
-backward that is itself to be differentiated take torch's own products.
+FP32, n_keep / 32 of the work of the dense products); an unpruned weight (32 of 32), a
+backward that is itself to be differentiated and large calls of a program that allows torch TF32
+products take torch's own.
 
 The reference has no framework binding (its only caller is its test driver,
 tests/test_nmspmm.cu:8-160).
@@ -36,6 +37,17 @@ def _dense_rows(raw_indices, n_keep: int):
     torch = _torch()
     win = torch.arange(raw_indices.shape[0], device=raw_indices.device) // n_keep
     return (raw_indices.to(torch.int64) + (win * 32)[:, None]).repeat_interleave(32, dim=1)
+
+
+def _dense_tf32_pays(M: int, N: int, K: int, n_keep: int) -> bool:
+    """Whether the backward takes torch's dense products: only where the caller has allowed torch TF32
+    matrix products, which are 32 / n_keep times the work at some twenty times the FP32 rate, and where
+    the call is large enough for the expansion of B to pay.  Both gradients, B200, us: 4096 x 4096 x 4096 at
+    4 / 8 / 16:32 832 / 1493 / 2934 by the kernels, 419 / 444 / 495 dense in TF32; 1024 rows 241 / 416 / 819
+    against 177 / 202 / 254; 256 rows 90 / 127 / 226 against 123 / 147 / 200; 1024 x 1024 x 1024 at 8:32 56 against 109.
+    (Dense in FP32 loses everywhere.)"""
+    return (_torch().backends.cuda.matmul.fp32_precision == "tf32"        # whichever of torch's switches set it
+            and M * n_keep >= 3000 and M * N * K * n_keep >= 3.4e10)
 
 
 def _sparse_grads(pkg, x, values, raw_indices, n_keep: int, grad_y, want_x: bool, want_values: bool):
@@ -140,7 +152,8 @@ def register_ops(pkg):
         x, values, raw_indices = ctx.saved_tensors
         want_x, want_values = ctx.needs_input_grad[0], ctx.needs_input_grad[1]
         # (with create_graph the formula has to be differentiable itself: the dense products below)
-        if ctx.n_keep in (16, 12, 8, 4) and not torch.is_grad_enabled():
+        if (ctx.n_keep in (16, 12, 8, 4) and not torch.is_grad_enabled()
+                and not _dense_tf32_pays(x.shape[0], values.shape[1], x.shape[1], ctx.n_keep)):
             grad_x, grad_values = torch.ops.nmspmm_b200.sparse_linear_grad(x, values, raw_indices, grad_y, ctx.n_keep, want_x, want_values)
             return (grad_x if want_x else None, grad_values if want_values else None, *[None] * 8)
         rows = _dense_rows(raw_indices, ctx.n_keep)                       # (W, N) global k of every kept value

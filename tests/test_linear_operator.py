@@ -109,3 +109,25 @@ def test_a_second_copy_of_the_package_shares_the_operator(op, pkg_host):
     finally:
         for name in [n for n in sys.modules if n.split(".")[0] == "nm_spmm_second"]:
             del sys.modules[name]
+
+
+@pytest.mark.parametrize("allowed,rows,kernels", [(False, 4096, True), (True, 4096, False), (True, 128, True)])
+def test_large_backward_follows_torchs_tf32_switch(op, pkg_host, allowed, rows, kernels):
+    """With TF32 products allowed a large backward is faster on torch's dense ones; otherwise it takes the kernels."""
+    from torch.fx.experimental.proxy_tensor import make_fx
+    size, raw = 4096, torch.zeros(4096 // 32 * N_KEEP, 4096 // 32, dtype=torch.int32, device="meta")
+
+    def step(x, values):
+        x, values = x.detach().requires_grad_(), values.detach().requires_grad_()
+        y = op(x, values, torch.zeros(4, dtype=torch.int32, device="meta"), None, raw, N_KEEP, 1, 128, 32, 0)
+        return torch.autograd.grad(y.square().sum(), (x, values))
+
+    before = torch.backends.cuda.matmul.allow_tf32
+    torch.backends.cuda.matmul.allow_tf32 = allowed
+    try:
+        graph = make_fx(step)(torch.empty(rows, size, device="meta"), torch.empty(size // 32 * N_KEEP, size, device="meta"))
+    finally:
+        torch.backends.cuda.matmul.allow_tf32 = before
+    called = [n.target for n in graph.graph.nodes]
+    assert (torch.ops.nmspmm_b200.sparse_linear_grad.default in called) == kernels
+    assert (torch.ops.aten.mm.default in called) != kernels
