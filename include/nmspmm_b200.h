@@ -152,6 +152,9 @@ typedef struct nmspmm_gemm_desc {
  * multiply (a CTA that gave up did not arrive at its counter). */
 #define NMSPMM_COUNTER_BYTES (64u << 10)
 size_t nmspmm_gemm_workspace_bytes(const nmspmm_gemm_desc* desc);
+/* How many bytes at the head of a workspace that no multiply has used yet have to be zero for this
+ * description (any M; 0 for most): what a caller with fresh memory per call clears instead of all of it. */
+size_t nmspmm_gemm_counter_bytes(const nmspmm_gemm_desc* desc);
 
 /* Replaces the eight nmGEMM_*_matrices_{low,high}_sparsity launchers
  * (src/kernel_*.cu).  C is overwritten with A.B for every split_k.  The pieces of a tile

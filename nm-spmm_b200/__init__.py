@@ -14,6 +14,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import threading
 from typing import Optional
 
 import numpy as np
@@ -38,7 +39,7 @@ C_ABI_SYMBOLS = (
     "nmspmm_trans_index_device", "nmspmm_preprocess_low_device", "nmspmm_preprocess_high_device",
     "nmspmm_trans_index_host", "nmspmm_preprocess_low_host", "nmspmm_preprocess_high_host",
     "nmspmm_test_short_fill", "nmspmm_set_tile_band", "nmspmm_tuned_plan_set", "nmspmm_tuned_plan_load", "nmspmm_tuned_plan_clear",
-    "nmspmm_tuned_plan_count", "nmspmm_gemm_workspace_bytes", "nmspmm_gemm", "nmspmm_gemm_row_major",
+    "nmspmm_tuned_plan_count", "nmspmm_gemm_workspace_bytes", "nmspmm_gemm_counter_bytes", "nmspmm_gemm", "nmspmm_gemm_row_major",
     "nmspmm_gemm_row_major_workspace_bytes", "nmspmm_gemm_row_major_16", "nmspmm_gemm_row_major_16_workspace_bytes",
     "nmspmm_linear_grad", "nmspmm_linear_grad_workspace_bytes", "nmspmm_widen_device", "nmspmm_gemm_with_cached_workspace", "nmspmm_device_status",
     "nmspmm_gemm_plan", "nmspmm_gemm_host", "nmspmm_release_cached", "nmspmm_measure_ffma_peak",
@@ -102,6 +103,8 @@ def load_library():
     lib.nmspmm_gemm_row_major_16_workspace_bytes.argtypes = [ctypes.POINTER(GemmDesc)]
     lib.nmspmm_gemm_row_major_16.argtypes = [ctypes.POINTER(GemmDesc), ctypes.c_int, vp, vp, vp, vp, vp, vp, sz, vp]
     lib.nmspmm_widen_device.argtypes = [ctypes.c_int, vp, vp, sz, vp]
+    lib.nmspmm_gemm_counter_bytes.restype = sz
+    lib.nmspmm_gemm_counter_bytes.argtypes = [ctypes.POINTER(GemmDesc)]
     lib.nmspmm_linear_grad_workspace_bytes.restype = sz
     lib.nmspmm_linear_grad_workspace_bytes.argtypes = [ctypes.POINTER(GemmDesc), ci, ci, ci]
     lib.nmspmm_linear_grad.argtypes = [ctypes.POINTER(GemmDesc), ci, vp, vp, vp, vp, vp, vp, vp, sz, vp]
@@ -123,17 +126,63 @@ def _check(where: str, status: int) -> None:
         raise NMSpMMError(where, status)
 
 
+_torch_module = None
+
+
 def _torch():
-    import torch
-    return torch
+    global _torch_module
+    if _torch_module is None:
+        import torch
+        _torch_module = torch
+    return _torch_module
+
+
+def _raw_stream() -> int:
+    """torch.cuda.current_stream().cuda_stream without the Stream object around it (3 us of host time)."""
+    torch = _torch()
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def _stream_ptr(stream=None):
-    torch = _torch()
-    if stream is None:
-        # torch.cuda.current_stream().cuda_stream without the Stream object around it (3 us of host time)
-        return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
-    return ctypes.c_void_p(stream.cuda_stream)
+    return ctypes.c_void_p(_raw_stream() if stream is None else stream.cuda_stream)
+
+
+class Scratch:
+    """The multiply's workspaces of one owner: a kept one per host thread, device and stream, because two
+    calls that overlap on the GPU, or whose launches two threads interleave, would write the same
+    slots.  Kept: the ``SLOTS`` newest, of at most ``KEEP_BYTES`` each (a dropped one goes back to torch's
+    allocator, which gives it out again in its stream's order); a copied or pickled owner starts with none.  A larger workspace, and any under
+    CUDA-graph capture, where the memory has to be the graph's own, is fresh for the call."""
+
+    SLOTS, KEEP_BYTES = 8, 64 << 20
+    _lock = threading.Lock()
+
+    def __init__(self):
+        self._kept = {}
+
+    def __reduce__(self):
+        return Scratch, ()
+
+    def get(self, nbytes: int, desc, like, stream: int):
+        """(address, bytes, tensor) of at least ``nbytes`` on the device of the tensor ``like`` for a multiply of ``desc``
+        (by reference) on ``stream``, the current one.  The tensor has to outlive the launch."""
+        if nbytes <= self.KEEP_BYTES and (stream == 0 or not _torch().cuda.is_current_stream_capturing()):   # 0 is never captured
+            key = (threading.get_ident(), like.get_device(), stream)
+            kept = self._kept.get(key)
+            if kept is None or kept[1] < nbytes:
+                ws = _torch().zeros(nbytes, dtype=_torch().uint8, device=like.device)
+                kept = (ws.data_ptr(), nbytes, ws)
+                with self._lock:
+                    self._kept.pop(key, None)
+                    while len(self._kept) >= self.SLOTS:
+                        del self._kept[next(iter(self._kept))]
+                    self._kept[key] = kept
+            return kept
+        ws = _torch().empty(nbytes, dtype=_torch().uint8, device=like.device)
+        counters = load_library().nmspmm_gemm_counter_bytes(desc)
+        if counters:
+            ws[:counters].zero_()
+        return ws.data_ptr(), nbytes, ws
 
 
 def _dev_ptr(t, dtype, name: str):
@@ -457,11 +506,16 @@ def bind_host_to_gpu(device_index: int) -> bool:
     return True
 
 
+_dtype_ids = {}
+
+
 def dtype_id(torch_dtype) -> int:
     """nmspmm_dtype of a torch dtype (float32, float16, bfloat16)."""
-    torch = _torch()
+    if not _dtype_ids:
+        torch = _torch()
+        _dtype_ids.update({torch.float32: DTYPE_F32, torch.float16: DTYPE_F16, torch.bfloat16: DTYPE_BF16})
     try:
-        return {torch.float32: DTYPE_F32, torch.float16: DTYPE_F16, torch.bfloat16: DTYPE_BF16}[torch_dtype]
+        return _dtype_ids[torch_dtype]
     except KeyError:
         raise NMSpMMError("dtype_id", UNSUPPORTED) from None
 
@@ -513,7 +567,7 @@ class NMSpMM:
             self.D, self.column_info = preprocess_high_device(raw, 32, n_keep, layout_ns, fuse_trans_index=True)
         else:
             self.D, self.column_info = preprocess_low_device(raw, layout_ns), None
-        self._workspace = None
+        self._scratch = Scratch()
 
     @classmethod
     def from_problem(cls, p: "formats.NMProblem", layout_ns: int = 128, fmt: Optional[int] = None, device=None):
@@ -529,13 +583,9 @@ class NMSpMM:
     def desc(self, M: int, path: int = PATH_FP32, split_k: int = 0, tile: int = 0) -> GemmDesc:
         return make_desc(M, self.N, self.K, self.n_keep, self.format, self.layout_ns, path, split_k, tile, self.vec_len)
 
-    def _scratch(self, nbytes: int):
-        torch = _torch()
-        if nbytes == 0:
-            return None
-        if self._workspace is None or self._workspace.numel() < nbytes:
-            self._workspace = torch.zeros(nbytes, dtype=torch.uint8, device=self.B.device)
-        return self._workspace
+    def _workspace(self, desc):
+        need = workspace_bytes(desc)
+        return self._scratch.get(need, ctypes.byref(desc), self.B, _raw_stream())[2] if need else None
 
     def matmul(self, A, path: int = PATH_FP32, split_k: int = 0, tile: int = 0, out=None):
         """C (M, N) = A . B for ``A`` given as a (K, M) float32 CUDA tensor."""
@@ -544,7 +594,7 @@ class NMSpMM:
         assert K == self.K
         d = self.desc(M, path, split_k, tile)
         C = torch.empty((M, self.N), dtype=torch.float32, device=A.device) if out is None else out
-        gemm(d, A, self.B, self.D, self.column_info, C, self._scratch(workspace_bytes(d)))
+        gemm(d, A, self.B, self.D, self.column_info, C, self._workspace(d))
         return C
 
     def matmul_rows(self, x, path: int = PATH_FP32, split_k: int = 0, tile: int = 0, out=None):
@@ -562,12 +612,13 @@ class NMSpMM:
         need = int(sizer(ctypes.byref(d)))
         if need == 0:
             raise NMSpMMError("nmspmm_gemm_row_major_workspace_bytes", UNSUPPORTED)
-        ws = self._scratch(need)
+        stream = _raw_stream()
+        ws, ws_bytes, _held = self._scratch.get(need, ctypes.byref(d), self.B, stream)
         C = torch.empty((M, self.N), dtype=x.dtype, device=x.device) if out is None else out
         assert C.dtype == x.dtype and C.is_contiguous()
         col = ctypes.c_void_p(self.column_info.data_ptr()) if self.column_info is not None else ctypes.c_void_p(0)
         ptrs = (ctypes.c_void_p(x.data_ptr()), ctypes.c_void_p(self.B.data_ptr()), ctypes.c_void_p(self.D.data_ptr()), col,
-                ctypes.c_void_p(C.data_ptr()), ctypes.c_void_p(ws.data_ptr()), ws.numel(), _stream_ptr())
+                ctypes.c_void_p(C.data_ptr()), ctypes.c_void_p(ws), ws_bytes, ctypes.c_void_p(stream))
         if dtype == DTYPE_F32:
             _check("nmspmm_gemm_row_major", lib.nmspmm_gemm_row_major(ctypes.byref(d), *ptrs))
         else:
@@ -581,4 +632,4 @@ class NMSpMM:
         K, M = A.shape
         assert K == self.K
         d = self.desc(M, path, split_k, tile)
-        gemm_gather(d, A, self.B, self.D, self.column_info, out_ptrs, ldc, col0, self._scratch(workspace_bytes(d)))
+        gemm_gather(d, A, self.B, self.D, self.column_info, out_ptrs, ldc, col0, self._workspace(d))

@@ -766,6 +766,13 @@ size_t nmspmm_gemm_workspace_bytes(const nmspmm_gemm_desc* desc)
     return p.counters_bytes + p.partial_bytes;
 }
 
+size_t nmspmm_gemm_counter_bytes(const nmspmm_gemm_desc* desc)
+{
+    Plan p;
+    if (make_plan(desc, sm_count(), &p, true) != NMSPMM_OK || !p.v || p.slots == 0 || p.deferred) return 0;
+    return round256(static_cast<size_t>(p.n_tiles) * sizeof(unsigned));
+}
+
 int nmspmm_gemm_plan(const nmspmm_gemm_desc* desc, nmspmm_gemm_plan_info* out)
 {
     if (!out) return NMSPMM_INVALID_ARGUMENT;

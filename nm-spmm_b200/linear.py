@@ -24,12 +24,18 @@ from typing import Optional
 
 _registered = None
 _library = None         # the torch.library.Library that holds the operator (it lives as long as this object)
-_workspaces = {}        # per device: the operator's scratch (zero when made: the multiply wants its counter block zero)
+_scratch = None         # the operator's workspaces (pkg.Scratch)
+
+
+_torch_module = None
 
 
 def _torch():
-    import torch
-    return torch
+    global _torch_module
+    if _torch_module is None:
+        import torch
+        _torch_module = torch
+    return _torch_module
 
 
 def _dense_rows(raw_indices, n_keep: int):
@@ -74,10 +80,11 @@ def _sparse_grads(pkg, x, values, raw_indices, n_keep: int, grad_y, want_x: bool
 
 def register_ops(pkg):
     """Defines ``torch.ops.nmspmm_b200.sparse_linear`` once per process and returns it."""
-    global _registered
+    global _registered, _scratch
     if _registered is not None:
         return _registered
     torch = _torch()
+    scratch = _scratch = pkg.Scratch()
 
     # Defined through torch.library.Library rather than the custom_op decorator: the decorator's wrapper
     # around the body cost 7 us of host time a call, as much as the multiply of one token.
@@ -108,12 +115,11 @@ def register_ops(pkg):
         need = lib.nmspmm_gemm_row_major_workspace_bytes(d) if wide else lib.nmspmm_gemm_row_major_16_workspace_bytes(d)
         if need == 0:
             raise pkg.NMSpMMError("nmspmm_gemm_row_major_workspace_bytes", pkg.UNSUPPORTED)
-        ws = _workspaces.get(x.device)
-        if ws is None or ws.numel() < need:
-            ws = _workspaces[x.device] = torch.zeros(need, dtype=torch.uint8, device=x.device)
+        stream = pkg._raw_stream()
+        ws, ws_bytes, _held = scratch.get(need, d, x, stream)
         y = x.new_empty((M, N))
         ptrs = (x.data_ptr(), values.data_ptr(), packed.data_ptr(), None if column_info is None else column_info.data_ptr(),
-                y.data_ptr(), ws.data_ptr(), ws.numel(), pkg._stream_ptr())
+                y.data_ptr(), ws, ws_bytes, stream)
         if wide:
             rc, where = lib.nmspmm_gemm_row_major(d, *ptrs), "nmspmm_gemm_row_major"
         else:

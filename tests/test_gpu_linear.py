@@ -201,3 +201,52 @@ def test_the_result_may_overwrite_the_activations(pkg, dtype, path, M, N, K):
         y = buffer[at:at + M * N].view(M, N)
         assert op.matmul_rows(inside, path=path, out=y) is y
         assert float((y.double() - want.double()).norm() / want.double().norm()) <= (1e-5 if dtype == torch.float32 else 4e-3)
+
+
+@pytest.mark.parametrize("path", [0, 1])
+def test_layers_on_two_streams_at_once(pkg, path):
+    """Calls that overlap on the GPU: each stream's scratch is its own, the operator's and an operand's."""
+    torch.manual_seed(9)
+    layer = pkg.linear.NMSparseLinear(pkg, torch.randn(4096, 2048, device="cuda") * 0.02, 8, path=path)
+    xs = [torch.randn(m, 2048, device="cuda") for m in (16, 40, 130, 200)]
+    calls = (layer, lambda x: layer.op.matmul_rows(x, path=path))
+    with torch.no_grad():
+        want = [[call(x) for x in xs] for call in calls]
+        streams = [torch.cuda.Stream() for _ in range(3)]
+        torch.cuda.synchronize()
+        got = [[] for _ in streams]
+        for turn in range(20):
+            for s, stream in enumerate(streams):
+                with torch.cuda.stream(stream):
+                    at = (turn + s) % len(xs), turn % 2
+                    got[s].append((at, calls[at[1]](xs[at[0]])))
+        torch.cuda.synchronize()
+    for per_stream in got:
+        for (i, c), y in per_stream:
+            assert torch.equal(y, want[c][i])
+    assert pkg.device_status() == 0
+
+
+@pytest.mark.parametrize("path", [0, 1])
+def test_captured_layers_and_eager_ones(pkg, path):
+    """A graph's calls have memory of the graph: replays are right after eager calls, between them, and before
+    any eager call on the capture's stream."""
+    torch.manual_seed(10)
+    layer = pkg.linear.NMSparseLinear(pkg, torch.randn(1024, 512, device="cuda") * 0.02, 16, path=path)
+    x = torch.randn(136, 512, device="cuda")
+    with torch.no_grad():
+        want = layer(x)
+        graphs = []
+        for _ in range(2):
+            g, at = torch.cuda.CUDAGraph(), torch.zeros_like(x)
+            with torch.cuda.graph(g):
+                y = layer(at)
+            graphs.append((g, at, y))
+        for g, at, y in reversed(graphs):                                # the later graph first
+            at.copy_(x)
+            g.replay()
+            big = layer(torch.randn(2048, 512, device="cuda"))           # the kept scratch grows meanwhile
+            g.replay()
+            torch.cuda.synchronize()
+            assert torch.equal(y, want) and big.shape == (2048, 1024)
+    assert pkg.device_status() == 0

@@ -308,3 +308,12 @@ def test_the_few_rows_kernels_do_not_spill(pkg_host):
         pytest.skip("built without ptxas' report")
     spills = [int(n) for n in re.findall(r"(\d+) bytes spill stores", open(report).read())]
     assert len(spills) >= 12 and not any(spills)
+
+
+def test_counter_bytes_are_asked_for_only_by_plans_that_use_counters(pkg):
+    def counters(*args):
+        return pkg.load_library().nmspmm_gemm_counter_bytes(ctypes.byref(pkg.make_desc(*args)))
+    assert counters(128, 256, 2048, 16, 0, 128, 0, 2) == 256             # two pieces per tile, added by the last to arrive
+    assert counters(128, 256, 2048, 16, 0, 128, 0, 8) == 0               # eight: the reduction kernel
+    assert counters(128, 256, 2048, 16, 0, 128, 0, 1) == 0               # whole tiles
+    assert counters(3, 11008, 4096, 8, 1, 128, 1) == 0                   # TF32, any row count
