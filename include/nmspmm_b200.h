@@ -177,8 +177,11 @@ int nmspmm_gemm(const nmspmm_gemm_desc* desc,
  * copy is made where C overlaps A: the result may overwrite the activations.
  * C is row-major M x N as everywhere.  The workspace holds what nmspmm_gemm needs (first, so
  * that the counter block keeps its place when the same workspace serves different M) and then
- * that copy: ask nmspmm_gemm_row_major_workspace_bytes. */
+ * that copy: nmspmm_gemm_row_major_workspace_bytes has room for it whatever A is.  A caller that asks
+ * per call (nmspmm_gemm_row_major_call_bytes: the type of A and C and both addresses) learns what that very
+ * call takes, without the copy where there is none; the entries accept that much. */
 size_t nmspmm_gemm_row_major_workspace_bytes(const nmspmm_gemm_desc* desc);
+size_t nmspmm_gemm_row_major_call_bytes(const nmspmm_gemm_desc* desc, int dtype, const void* A_rows_dev, const void* C_dev);
 int nmspmm_gemm_row_major(const nmspmm_gemm_desc* desc,
                           const float* A_rows_dev, const float* B_dev, const int* D_dev, const int* column_info_dev,
                           float* C_dev, void* workspace_dev, size_t workspace_bytes, void* stream);
@@ -192,7 +195,7 @@ int nmspmm_gemm_row_major(const nmspmm_gemm_desc* desc,
  * result from the real one; NMSPMM_PATH_FP32 is exact in the same sense.  The TF32 path reads x
  * and writes y in `dtype` (x on 16 bytes and apart from y; an unpruned B excepted); otherwise one
  * kernel widens and transposes x, and on the exact path one rounds y.  The workspace holds what the
- * multiply needs and room for the two FP32 copies. */
+ * multiply needs, room for the FP32 copy of x and, on the exact path, for that of y. */
 enum nmspmm_dtype { NMSPMM_DTYPE_F32 = 0, NMSPMM_DTYPE_F16 = 1, NMSPMM_DTYPE_BF16 = 2 };
 size_t nmspmm_gemm_row_major_16_workspace_bytes(const nmspmm_gemm_desc* desc);
 int nmspmm_gemm_row_major_16(const nmspmm_gemm_desc* desc, int dtype,

@@ -40,7 +40,7 @@ C_ABI_SYMBOLS = (
     "nmspmm_trans_index_host", "nmspmm_preprocess_low_host", "nmspmm_preprocess_high_host",
     "nmspmm_test_short_fill", "nmspmm_set_tile_band", "nmspmm_tuned_plan_set", "nmspmm_tuned_plan_load", "nmspmm_tuned_plan_clear",
     "nmspmm_tuned_plan_count", "nmspmm_gemm_workspace_bytes", "nmspmm_gemm_counter_bytes", "nmspmm_gemm", "nmspmm_gemm_row_major",
-    "nmspmm_gemm_row_major_workspace_bytes", "nmspmm_gemm_row_major_16", "nmspmm_gemm_row_major_16_workspace_bytes",
+    "nmspmm_gemm_row_major_workspace_bytes", "nmspmm_gemm_row_major_call_bytes", "nmspmm_gemm_row_major_16", "nmspmm_gemm_row_major_16_workspace_bytes",
     "nmspmm_linear_grad", "nmspmm_linear_grad_workspace_bytes", "nmspmm_widen_device", "nmspmm_gemm_with_cached_workspace", "nmspmm_device_status",
     "nmspmm_gemm_plan", "nmspmm_gemm_host", "nmspmm_release_cached", "nmspmm_measure_ffma_peak",
     "nmspmm_gemm_static_scratch", "nmspmm_gemm_gather", "nmspmm_prune_device",
@@ -103,6 +103,8 @@ def load_library():
     lib.nmspmm_gemm_row_major_16_workspace_bytes.argtypes = [ctypes.POINTER(GemmDesc)]
     lib.nmspmm_gemm_row_major_16.argtypes = [ctypes.POINTER(GemmDesc), ctypes.c_int, vp, vp, vp, vp, vp, vp, sz, vp]
     lib.nmspmm_widen_device.argtypes = [ctypes.c_int, vp, vp, sz, vp]
+    lib.nmspmm_gemm_row_major_call_bytes.restype = sz
+    lib.nmspmm_gemm_row_major_call_bytes.argtypes = [ctypes.POINTER(GemmDesc), ci, vp, vp]
     lib.nmspmm_gemm_counter_bytes.restype = sz
     lib.nmspmm_gemm_counter_bytes.argtypes = [ctypes.POINTER(GemmDesc)]
     lib.nmspmm_linear_grad_workspace_bytes.restype = sz
@@ -598,24 +600,23 @@ class NMSpMM:
         return C
 
     def matmul_rows(self, x, path: int = PATH_FP32, split_k: int = 0, tile: int = 0, out=None):
-        """C (M, N) = x . B for ``x`` given row-major as an (M, K) CUDA tensor (any M >= 1): the
-        library transposes on the GPU ahead of the multiply (nmspmm_gemm_row_major).  ``x`` may
-        be float32, or float16 / bfloat16: then the result has that dtype too, the widening is
-        part of the transposition and one pass rounds the result (nmspmm_gemm_row_major_16)."""
+        """C (M, N) = x . B for ``x`` given row-major as an (M, K) CUDA tensor (any M >= 1;
+        nmspmm_gemm_row_major): the tensor-core path reads the rows as they lie, the exact path transposes on the GPU
+        ahead of the multiply.  ``x`` may be float32, or float16 / bfloat16: then the result has that dtype too, widened
+        exactly, summed in FP32 and rounded once (nmspmm_gemm_row_major_16).  ``out`` may overlap ``x``."""
         torch = _torch()
         M, K = x.shape
         assert K == self.K and x.is_contiguous()
         dtype = dtype_id(x.dtype)
         lib = load_library()
         d = self.desc(M, path, split_k, tile)
-        sizer = lib.nmspmm_gemm_row_major_workspace_bytes if dtype == DTYPE_F32 else lib.nmspmm_gemm_row_major_16_workspace_bytes
-        need = int(sizer(ctypes.byref(d)))
-        if need == 0:
-            raise NMSpMMError("nmspmm_gemm_row_major_workspace_bytes", UNSUPPORTED)
-        stream = _raw_stream()
-        ws, ws_bytes, _held = self._scratch.get(need, ctypes.byref(d), self.B, stream)
         C = torch.empty((M, self.N), dtype=x.dtype, device=x.device) if out is None else out
         assert C.dtype == x.dtype and C.is_contiguous()
+        need = lib.nmspmm_gemm_row_major_call_bytes(ctypes.byref(d), dtype, x.data_ptr(), C.data_ptr())
+        if need == 0:
+            raise NMSpMMError("nmspmm_gemm_row_major_call_bytes", UNSUPPORTED)
+        stream = _raw_stream()
+        ws, ws_bytes, _held = self._scratch.get(need, ctypes.byref(d), self.B, stream)
         col = ctypes.c_void_p(self.column_info.data_ptr()) if self.column_info is not None else ctypes.c_void_p(0)
         ptrs = (ctypes.c_void_p(x.data_ptr()), ctypes.c_void_p(self.B.data_ptr()), ctypes.c_void_p(self.D.data_ptr()), col,
                 ctypes.c_void_p(C.data_ptr()), ctypes.c_void_p(ws), ws_bytes, ctypes.c_void_p(stream))

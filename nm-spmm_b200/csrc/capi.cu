@@ -905,11 +905,30 @@ static bool reads_rows(const Plan& p, const nmspmm_gemm_desc* d, const void* A_r
            !overlap(A_rows, size * d->M * d->K, C, size * d->M * d->N);
 }
 
+static size_t result_copy_bytes(const nmspmm_gemm_desc* d)
+{
+    return round256(static_cast<size_t>(d->M) * d->N * sizeof(float));
+}
+
+// What one row-major call writes into its workspace: the multiply's scratch, the col-major copy of A
+// unless the kernels read the rows, and an FP32 C for the exact path to round from.
+static size_t row_major_bytes(const Plan& p, const nmspmm_gemm_desc* d, int dtype, bool copy_a)
+{
+    return row_major_head_bytes(p) + (copy_a ? row_major_copy_bytes(d) : 0) + (dtype != kDtypeF32 && !p.tv ? result_copy_bytes(d) : 0);
+}
+
 size_t nmspmm_gemm_row_major_workspace_bytes(const nmspmm_gemm_desc* desc)
 {
     Plan p;
     if (!desc || make_plan(desc, sm_count(), &p, true) != NMSPMM_OK) return 0;
-    return row_major_head_bytes(p) + row_major_copy_bytes(desc);
+    return row_major_bytes(p, desc, kDtypeF32, true);
+}
+
+size_t nmspmm_gemm_row_major_call_bytes(const nmspmm_gemm_desc* desc, int dtype, const void* A_rows_dev, const void* C_dev)
+{
+    Plan p;
+    if (!desc || make_plan(desc, sm_count(), &p, true) != NMSPMM_OK) return 0;
+    return row_major_bytes(p, desc, dtype, !reads_rows(p, desc, A_rows_dev, C_dev, dtype));
 }
 
 int nmspmm_gemm_row_major(const nmspmm_gemm_desc* desc, const float* A_rows_dev, const float* B_dev, const int* D_dev,
@@ -919,11 +938,12 @@ int nmspmm_gemm_row_major(const nmspmm_gemm_desc* desc, const float* A_rows_dev,
     Plan p;
     int rc = make_plan(desc, sm_count(), &p, true);
     if (rc != NMSPMM_OK) return rc;
-    const size_t copy_bytes = row_major_copy_bytes(desc), own = p.counters_bytes + p.partial_bytes, head = row_major_head_bytes(p);
-    if (workspace_bytes < head + copy_bytes) return NMSPMM_WORKSPACE_TOO_SMALL;
+    const bool rows = reads_rows(p, desc, A_rows_dev, C_dev, kDtypeF32);
+    if (workspace_bytes < row_major_bytes(p, desc, kDtypeF32, !rows)) return NMSPMM_WORKSPACE_TOO_SMALL;
+    const size_t own = p.counters_bytes + p.partial_bytes, head = row_major_head_bytes(p);
     const int ld = (desc->M + 3) / 4 * 4;
     float* out[1] = { C_dev };
-    if (reads_rows(p, desc, A_rows_dev, C_dev, kDtypeF32))
+    if (rows)
         return gemm_launch(desc, A_rows_dev, B_dev, D_dev, column_info_dev, out, 1, desc->N, 0, own ? workspace_dev : nullptr, own, stream, 0,
                            1 + kDtypeF32);
     float* A_cols = reinterpret_cast<float*>(static_cast<unsigned char*>(workspace_dev) + head);
@@ -935,16 +955,11 @@ int nmspmm_gemm_row_major(const nmspmm_gemm_desc* desc, const float* A_rows_dev,
 // ---- activations and result in 16-bit storage ---------------------------------------------
 static_assert(NMSPMM_DTYPE_F16 == kDtypeF16 && NMSPMM_DTYPE_BF16 == kDtypeBF16, "the public dtype ids are the library's");
 
-static size_t result_copy_bytes(const nmspmm_gemm_desc* d)
-{
-    return round256(static_cast<size_t>(d->M) * d->N * sizeof(float));
-}
-
 size_t nmspmm_gemm_row_major_16_workspace_bytes(const nmspmm_gemm_desc* desc)
 {
     Plan p;
     if (!desc || make_plan(desc, sm_count(), &p, true) != NMSPMM_OK) return 0;
-    return row_major_head_bytes(p) + row_major_copy_bytes(desc) + result_copy_bytes(desc);
+    return row_major_bytes(p, desc, kDtypeF16, true);
 }
 
 int nmspmm_gemm_row_major_16(const nmspmm_gemm_desc* desc, int dtype, const void* A_rows_dev, const float* B_dev, const int* D_dev,
@@ -956,18 +971,18 @@ int nmspmm_gemm_row_major_16(const nmspmm_gemm_desc* desc, int dtype, const void
     Plan p;
     int rc = make_plan(desc, sm_count(), &p, true);
     if (rc != NMSPMM_OK) return rc;
-    const size_t copy_bytes = row_major_copy_bytes(desc), c_bytes = result_copy_bytes(desc);
+    const bool rows = reads_rows(p, desc, A_rows_dev, C_dev, dtype);
+    if (workspace_bytes < row_major_bytes(p, desc, dtype, !rows)) return NMSPMM_WORKSPACE_TOO_SMALL;
     const size_t own = p.counters_bytes + p.partial_bytes, head = row_major_head_bytes(p);
-    if (workspace_bytes < head + copy_bytes + c_bytes) return NMSPMM_WORKSPACE_TOO_SMALL;
     const int ld = (desc->M + 3) / 4 * 4;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     unsigned char* ws = static_cast<unsigned char*>(workspace_dev);
     float* A_cols = reinterpret_cast<float*>(ws + head);
-    float* C32 = reinterpret_cast<float*>(ws + head + copy_bytes);
+    float* C32 = reinterpret_cast<float*>(ws + head + row_major_copy_bytes(desc));      // exact path only
     // The tensor-core path's kernels store C in 16 bits themselves; the exact path's, at the edge of
     // their registers, leave that to a pass over an FP32 C.
     float* const direct[1] = { static_cast<float*>(C_dev) };
-    if (reads_rows(p, desc, A_rows_dev, C_dev, dtype))
+    if (rows)
         return gemm_launch(desc, static_cast<const float*>(A_rows_dev), B_dev, D_dev, column_info_dev, direct, 1, desc->N, 0,
                            own ? ws : nullptr, own, stream, 0, 1 + dtype, dtype);
     cudaError_t e = launch_transpose_rows(dtype, A_rows_dev, A_cols, desc->M, desc->K, ld, st);

@@ -112,12 +112,12 @@ def register_ops(pkg):
         dtype = pkg.dtype_id(x.dtype)
         d = ctypes.byref(pkg.GemmDesc(M, N, K, n_keep, fmt, layout_ns, path, 0, 0, vec_len))
         wide = dtype == pkg.DTYPE_F32
-        need = lib.nmspmm_gemm_row_major_workspace_bytes(d) if wide else lib.nmspmm_gemm_row_major_16_workspace_bytes(d)
+        y = x.new_empty((M, N))
+        need = lib.nmspmm_gemm_row_major_call_bytes(d, dtype, x.data_ptr(), y.data_ptr())
         if need == 0:
-            raise pkg.NMSpMMError("nmspmm_gemm_row_major_workspace_bytes", pkg.UNSUPPORTED)
+            raise pkg.NMSpMMError("nmspmm_gemm_row_major_call_bytes", pkg.UNSUPPORTED)
         stream = pkg._raw_stream()
         ws, ws_bytes, _held = scratch.get(need, d, x, stream)
-        y = x.new_empty((M, N))
         ptrs = (x.data_ptr(), values.data_ptr(), packed.data_ptr(), None if column_info is None else column_info.data_ptr(),
                 y.data_ptr(), ws, ws_bytes, stream)
         if wide:

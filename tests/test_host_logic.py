@@ -317,3 +317,26 @@ def test_counter_bytes_are_asked_for_only_by_plans_that_use_counters(pkg):
     assert counters(128, 256, 2048, 16, 0, 128, 0, 8) == 0               # eight: the reduction kernel
     assert counters(128, 256, 2048, 16, 0, 128, 0, 1) == 0               # whole tiles
     assert counters(3, 11008, 4096, 8, 1, 128, 1) == 0                   # TF32, any row count
+
+
+def test_row_major_scratch_is_what_the_call_writes(pkg):
+    """The tensor-core path reads rows and stores 16 bits itself: no FP32 copies of A or C are asked for, unless A
+    is off a 16-byte boundary, C overlaps A, or the weight is unpruned."""
+    lib, base = pkg.load_library(), 1 << 20
+    M, N, K = 8192, 28672, 8192
+    tf32 = ctypes.byref(pkg.make_desc(M, N, K, 8, 1, 128, pkg.PATH_TF32, 0, 0, 64))
+    exact = ctypes.byref(pkg.make_desc(M, N, K, 8, 1, 128, pkg.PATH_FP32))
+    dense = ctypes.byref(pkg.make_desc(M, N, K, 32, 0, 128, pkg.PATH_TF32))
+    far, copy_a, copy_c = base + 4 * M * K, 4 * M * K, 4 * M * N
+
+    def call(desc, dtype, a=base, c=far):
+        return lib.nmspmm_gemm_row_major_call_bytes(desc, dtype, a, c)
+
+    for dtype in (pkg.DTYPE_F32, pkg.DTYPE_F16, pkg.DTYPE_BF16):
+        own = call(tf32, dtype)
+        assert 0 < own < 32 << 20
+        assert call(tf32, dtype, a=base + 8) == call(tf32, dtype, c=base + 4096) == own + copy_a
+        assert call(exact, dtype) >= copy_a + (0 if dtype == pkg.DTYPE_F32 else copy_c)
+    assert call(dense, pkg.DTYPE_F16) >= copy_a > call(dense, pkg.DTYPE_F32)
+    assert lib.nmspmm_gemm_row_major_16_workspace_bytes(tf32) == own + copy_a       # whatever A is, without an FP32 C
+    assert lib.nmspmm_gemm_row_major_workspace_bytes(tf32) == own + copy_a
