@@ -308,3 +308,30 @@ def test_row_major_activations_match_the_col_major_route(pkg, dtype, tol, M, N, 
         assert got.dtype == dtype
         assert float((got.double() - want).norm() / want.norm()) <= tol
     assert pkg.device_status() == 0
+
+
+@pytest.mark.parametrize("dtype,tol", [(torch.float32, 1e-5), (torch.float16, 5e-4), (torch.bfloat16, 4e-3)])
+@pytest.mark.parametrize("M,tile", [(1, 0), (17, 0), (33, 0), (64, 0), (64, 1), (130, 0), (130, 1), (300, 0), (300, 9)])
+@pytest.mark.parametrize("n_keep,vec_len,fmt", [(4, 32, 1), (8, 32, 1), (8, 32, 0), (12, 32, 0), (16, 32, 0), (32, 32, 0),
+                                                (4, 64, 1), (8, 64, 1), (12, 64, 0), (16, 64, 0)])
+def test_row_major_activations_unsplit(pkg, dtype, tol, M, tile, n_keep, vec_len, fmt):
+    """One CTA per tile over 2048 k: C goes from the accumulators straight to its own type, and every stage ring
+    wraps several times (32 or 64 steps; the deepest has 8 stages), so that one-hot entries are cleared and the
+    builder groups meet stages that others used.  Against the col-major route cut into slices, as above."""
+    if tile == 9 and (fmt == 1 or n_keep in (4, 32) or vec_len == 64):
+        pytest.skip("no expanding form")
+    N, K = 448, 2048
+    p = pkg.formats.make_random(4, N, K, n_keep, seed=950 + n_keep + vec_len, vec_len=vec_len)
+    op = pkg.NMSpMM.from_problem(p, layout_ns=64, fmt=fmt)
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(M)
+    x = (torch.rand((M, K), device="cuda", generator=gen) * 2 - 1).to(dtype)
+    A = torch.zeros((K, (M + 3) // 4 * 4), device="cuda")
+    A[:, :M] = x.float().t()
+    want = op.matmul(A, path=pkg.PATH_TF32)[:M].double()
+    shifted = torch.empty(M * K + 1, dtype=dtype, device="cuda")[1:].view(M, K).copy_(x)
+    for rows in (x, shifted):
+        got = op.matmul_rows(rows, path=pkg.PATH_TF32, split_k=1, tile=tile)
+        assert got.dtype == dtype
+        assert float((got.double() - want).norm() / want.norm()) <= tol
+    assert pkg.device_status() == 0
