@@ -70,7 +70,7 @@ struct GemmOutputs {
     long long ldc;
     int lda;               // host side only (tensor-map encoding): floats between consecutive k rows of A; 0 = M
     int c_dtype;           // type C is stored in (kDtype*): FP32 wherever there is more than one output
-    int a_rows;            // host side only: 0 = A is col-major, else A is row-major [M][K] of type a_rows - 1 (few-rows kernels)
+    int a_rows;            // host side only: 0 = A is col-major, else A is row-major [M][K] of type a_rows - 1 (tensor-core path)
 };
 NMSPMM_HD float* output_of(const GemmArgs& a, const GemmOutputs& o, int i) { return i == 0 ? a.C : o.C_more[i - 1]; }
 

@@ -154,7 +154,7 @@ __device__ __forceinline__ void nm_gemm_ffma_body(const GemmArgs& g, const CUten
         uint32_t i_bytes = d_bytes;                        // index bytes of one block that exist
         if constexpr (Cfg::PAIR) {
             // The last pair of an odd number of windows: its second window's rows of A and B
-            // arrive as zeros; its indices do not exist and become 0, a row inside the stage.
+            // arrive as zeros; its indices do not exist and become 0, the first of those rows of A.
             const int rows = g.W - win * WS;
             if (rows < WS) {
                 i_bytes = static_cast<uint32_t>(rows << qs_shift) * 4u;

@@ -31,7 +31,8 @@
 //               the result buffer.  One thread issues a tcgen05.mma every 26 cycles at best
 //               (measured), and a step has 12 to 20 of them: three issuing threads keep the
 //               tensor pipe, not the issue slot, the bound.
-//   warps 4-11  (4-7 on the 128-column tile and at 16:32, 12:32 and 32:32) one thread per (vector, kept row) and turn: fetches its index two to four steps ahead
+//   warps 4-11  (4-7 on the 128-column tile, at 16:32 and 12:32 with 32-wide vectors, and at 32:32) one
+//               thread per (vector, kept row) and turn: fetches its index two to four steps ahead
 //               with cp.async (through column_info on the 64-k format), keeps P's one-hot
 //               entry current, and after the last step reads the accumulators (tcgen05.ld),
 //               transposes them through shared memory and stores C in 128-byte row pieces.
@@ -44,7 +45,8 @@
 // gathered in their own type (kind::f16, one-hot P of that type, FP32 result: exact), K = 16 per
 // instruction: half as many gather instructions per step and half of A's bytes, no transposing and
 // widening launch ahead of the multiply, and C is stored in the activations' type.
-// 256 x 11008 x 4096, bfloat16, 8:32: the pass takes 50.8 us, 59.5 with a transposing and a rounding launch.
+// 256 x 11008 x 4096, bfloat16, 8:32: 59.5 us with a transposing and a rounding launch, 50.8 without, 42.5 with the
+// builder groups and stages below.
 // Every wait is bounded; a wait that gives up raises the device status word.
 #include <cuda.h>
 
@@ -112,7 +114,7 @@ struct Tf32Cfg {
     // arrived, stage free, old entry, new entry, proxy fence, arrival): with one group that chain,
     // not the tensor pipe, was part of what an 8:32 step waited for: 4096 x 4096 x 11008, 8:32, 417 -> 404 us,
     // with bfloat16 activations 444 -> 405; 4096 x 28672 x 2048 with 64-wide vectors 667 -> 636 and 632 -> 578.
-    // (16:32 and 12:32 fill one group of 128: a second one gained nothing there, their steps are longer.)
+    // (16:32 and 12:32 with 32-wide vectors fill one group of 128: a second one gained nothing there, their steps are longer.)
     static constexpr int BUILDERS = (QT == 8 && N1 < 128) ? 256 : 128;
     static constexpr int GROUP_WARPS = N1 / 32;
     static constexpr int PRODUCT_WARPS = 2;

@@ -26,8 +26,7 @@
 //     memory: a window is a box of MS rows x KS columns whose 16-byte chunks are swizzled within the
 //     rows, the fragment loads take one value each and widen it (exactly), and C is written in the
 //     activations' type.  A transposing launch ahead of the multiply and a rounding one behind it
-//     cost 2.9 + 2.6 us of 20 (and two launches) at 1 x 4096 x 4096.  The layer's
-//     whole pass there: 50.1 -> 43.3 us, the rest of it host time.
+//     cost 2.9 + 2.6 us of 20 (and two launches) at 1 x 4096 x 4096.
 //   * K slices of a tile leave their accumulators in scratch slots of MS x 128 floats and
 //     nm_reduce_slices_kernel adds them in k order; a tile computed by one CTA is stored
 //     directly (to every output buffer when the caller gathers).

@@ -73,7 +73,7 @@ __global__ void __launch_bounds__(256) quad_rows_kernel(const T* __restrict__ x,
 // load takes one wavefront per eight lanes, and two such groups share one where lane i reads the
 // address of lane i ^ 1 (the loads of x: lane bit 0 is a column bit) or of lane i ^ 2 (the loads of
 // grad_y: bit 1 is a row bit).  A half warp then reads x at four unrelated k, which meet in a bank
-// now and then; with lane / 4 and lane % 4 the kernel took 3.7 wavefronts per load.
+// now and then: 2.7 wavefronts per load in all, the FMA pipe active 74 % of the time.
 template <int NKEEP>
 struct GradValuesCfg {
     static constexpr int TW = (NKEEP == 12) ? 6 : 8;
@@ -207,9 +207,9 @@ nm_grad_values_kernel(const GradArgs a, const __grid_constant__ CUtensorMap map_
 // operands read 128 bits along n, so the packed FMA takes its pairs from the loads as they are
 // and sums even and odd columns apart), then adds the result to the rows of the accumulator
 // that its index list names: 16 + 16 shared accesses of 128 bits after 1024 packed FMAs.
-// Shared memory is the second bound: 128 loads of two wavefronts and the 128 of the additions
-// against 512 cycles of the FMA pipe.  (Thread tile 8 x 4 on sixteen warps: 65 % of the
-// shared-memory wavefronts there are, 481 us at M = 2048, N = K = 4096, 8:32.)
+// Nothing is saturated: at M = 2048, N = K = 4096, 8:32 the FMA pipe is active 56 % of the time and half of the
+// shared-memory wavefronts there are go by, on two warps per scheduler whose own fixed latencies are the
+// largest stall.  (Thread tile 8 x 4 on sixteen warps took 481 us there.)
 // The accumulator is what limits the warps: 32 KB of it per warp at 8:32.  At 8:32 and 4:32 two
 // and four groups of warps therefore share it, each taking every second / fourth vector; a
 // token per patch of the accumulator hands it from group to group in vector order, so that the
