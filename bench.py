@@ -310,7 +310,7 @@ def run_ours(args, rank: int, world: int, local_rank: int):
     C_sets = [torch.empty((M, n_local), dtype=torch.float32, device="cuda") for _ in range(SETS)]
     path = pkg.PATH_TF32 if (args.kernel_only and args.path == "tf32") else pkg.PATH_FP32
     desc = op.desc(M, path=path, tile=args.tile, split_k=args.split_k)
-    plan = pkg.plan(desc)
+    plan = pkg.call_plan(desc)
 
     def step(i):
         op.matmul(A_sets[i % SETS], out=C_sets[i % SETS], path=path, tile=args.tile, split_k=args.split_k)
@@ -685,13 +685,14 @@ def measure_workload(pkg, torch, name: str, tile: int = 0, split_k: int = 0, ste
             continue
         fns = [lambda o=o, c=c: o.matmul(A, out=c, path=path, tile=tile, split_k=split_k) for o, c in zip(ops, Cs)]
         ms = graph_time(fns)
-        plan = pkg.plan(ops[0].desc(M, path=path, tile=tile, split_k=split_k))
+        plan = pkg.call_plan(ops[0].desc(M, path=path, tile=tile, split_k=split_k))
         err = sampled_rows_error(p.A_km, p.BT, p.DT, n_keep, Cs[0][torch.as_tensor(rows, device="cuda")].cpu().numpy(), rows,
                                  f64=(pname == "tf32"))
         out[pname] = {"ms": ms, "useful_tflops": useful / (ms * 1e-3) / 1e12, "bytes_per_s_gbs": abytes / (ms * 1e-3) / 1e9,
                       "roofline_frac": max(useful / peak, abytes / hbm) / (ms * 1e-3),
                       "bound": "hbm" if abytes / hbm > useful / peak else "flops",
-                      "kernel": ("nm_gemm_ffma_kernel" if pname == "fp32" else
+                      "kernel": (("nm_gemm_wide_kernel" if plan.tile in (pkg.TILE_128x256, pkg.TILE_256x128, pkg.TILE_64x512) else "nm_gemm_ffma_kernel")
+                                 if pname == "fp32" else
                                  ("nm_gemm_tf32_few_rows_kernel" if plan.tile_m < 128 else "nm_gemm_tf32_kernel")),
                       "tile": [plan.tile_m, plan.tile_n], "ctas": plan.grid, "whole_tiles": plan.n_dp,
                       "rel_err_rows": err, "parity": bool(err <= (1e-5 if pname == "fp32" else 2e-3))}

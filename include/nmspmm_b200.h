@@ -106,7 +106,7 @@ int nmspmm_preprocess_high_host(int* column_info_host, int pruning_M, int prunin
 
 /* ------------------------------------------------------------------ the multiply */
 
-/* CTA tiles compiled into the library (rows x columns of C).  The exact path has all of 1..7;
+/* CTA tiles compiled into the library (rows x columns of C).  The exact path has all of 1..7, 10 and 11;
  * the TF32 path 128 x 128 and 128 x 256, the latter in two forms: the tensor core gathers the
  * kept rows of A (every format and ratio), or B is expanded with zeros and the A window is
  * multiplied whole (32-k formats with 16, 12 or 8 kept rows).  NMSPMM_TILE_128x256 leaves the
@@ -123,7 +123,9 @@ enum nmspmm_tile_id {
     NMSPMM_TILE_16x256 = 6,
     NMSPMM_TILE_32x256 = 7,
     NMSPMM_TILE_128x256_GATHER = 8,   /* TF32 path only */
-    NMSPMM_TILE_128x256_EXPAND = 9    /* TF32 path only */
+    NMSPMM_TILE_128x256_EXPAND = 9,   /* TF32 path only */
+    NMSPMM_TILE_256x128 = 10,         /* exact path only */
+    NMSPMM_TILE_64x512 = 11           /* exact path only */
 };
 
 typedef struct nmspmm_gemm_desc {
@@ -152,6 +154,12 @@ typedef struct nmspmm_gemm_desc {
  * multiply (a CTA that gave up did not arrive at its counter). */
 #define NMSPMM_COUNTER_BYTES (64u << 10)
 size_t nmspmm_gemm_workspace_bytes(const nmspmm_gemm_desc* desc);
+/* Scratch with which a call runs its fastest form.  On the exact path, where tile and split_k are left to
+ * the library and no tuned entry names them, a call may run one of the wide tiles (ids 5, 10 and 11: one CTA per SM)
+ * instead of the tile that nmspmm_gemm_plan names, wherever the scratch it is handed holds that tile's
+ * pieces; with nmspmm_gemm_workspace_bytes alone (never more than this) it runs the named one.  The wide
+ * tiles write no counters. */
+size_t nmspmm_gemm_call_workspace_bytes(const nmspmm_gemm_desc* desc);
 /* How many bytes at the head of a workspace that no multiply has used yet have to be zero for this
  * description (any M; 0 for most): what a caller with fresh memory per call clears instead of all of it. */
 size_t nmspmm_gemm_counter_bytes(const nmspmm_gemm_desc* desc);
@@ -288,6 +296,8 @@ typedef struct nmspmm_gemm_plan_info {
     int stages;
 } nmspmm_gemm_plan_info;
 int nmspmm_gemm_plan(const nmspmm_gemm_desc* desc, nmspmm_gemm_plan_info* out);
+/* What a call of nmspmm_gemm with workspace_bytes of scratch runs (see nmspmm_gemm_call_workspace_bytes). */
+int nmspmm_gemm_call_plan(const nmspmm_gemm_desc* desc, size_t workspace_bytes, nmspmm_gemm_plan_info* out);
 
 /* End-to-end form on HOST buffers: copies A, B, the raw DT [W][Q] and nothing else
  * to the device, packs the indices there, multiplies and copies C back.  Device

@@ -28,7 +28,7 @@ LIB_PATH = os.environ.get("NMSPMM_LIBRARY") or os.path.join(_HERE, "libnmspmm_b2
 OK, INVALID_ARGUMENT, UNSUPPORTED, CUDA_ERROR, WORKSPACE_TOO_SMALL, DEVICE_TIMEOUT = range(6)
 PATH_FP32, PATH_TF32 = 0, 1
 (TILE_AUTO, TILE_128x128, TILE_64x128, TILE_32x128, TILE_16x128, TILE_128x256, TILE_16x256, TILE_32x256,
- TILE_128x256_GATHER, TILE_128x256_EXPAND) = range(10)   # nmspmm_tile_id
+ TILE_128x256_GATHER, TILE_128x256_EXPAND, TILE_256x128, TILE_64x512) = range(12)   # nmspmm_tile_id
 FORMAT_LOW, FORMAT_HIGH = 0, 1
 DTYPE_F32, DTYPE_F16, DTYPE_BF16 = 0, 1, 2               # nmspmm_dtype
 VEC_LEN = 32
@@ -39,7 +39,7 @@ C_ABI_SYMBOLS = (
     "nmspmm_trans_index_device", "nmspmm_preprocess_low_device", "nmspmm_preprocess_high_device",
     "nmspmm_trans_index_host", "nmspmm_preprocess_low_host", "nmspmm_preprocess_high_host",
     "nmspmm_test_short_fill", "nmspmm_set_tile_band", "nmspmm_tuned_plan_set", "nmspmm_tuned_plan_load", "nmspmm_tuned_plan_clear",
-    "nmspmm_tuned_plan_count", "nmspmm_gemm_workspace_bytes", "nmspmm_gemm_counter_bytes", "nmspmm_gemm", "nmspmm_gemm_row_major",
+    "nmspmm_tuned_plan_count", "nmspmm_gemm_workspace_bytes", "nmspmm_gemm_call_workspace_bytes", "nmspmm_gemm_call_plan", "nmspmm_gemm_counter_bytes", "nmspmm_gemm", "nmspmm_gemm_row_major",
     "nmspmm_gemm_row_major_workspace_bytes", "nmspmm_gemm_row_major_call_bytes", "nmspmm_gemm_row_major_16", "nmspmm_gemm_row_major_16_workspace_bytes",
     "nmspmm_linear_grad", "nmspmm_linear_grad_workspace_bytes", "nmspmm_widen_device", "nmspmm_gemm_with_cached_workspace", "nmspmm_device_status",
     "nmspmm_gemm_plan", "nmspmm_gemm_host", "nmspmm_release_cached", "nmspmm_measure_ffma_peak",
@@ -93,6 +93,9 @@ def load_library():
     lib.nmspmm_preprocess_high_host.argtypes = [vp, ci, ci, vp, ci, ci, ci, ci]
     lib.nmspmm_gemm_workspace_bytes.restype = sz
     lib.nmspmm_gemm_workspace_bytes.argtypes = [ctypes.POINTER(GemmDesc)]
+    lib.nmspmm_gemm_call_workspace_bytes.restype = sz
+    lib.nmspmm_gemm_call_workspace_bytes.argtypes = [ctypes.POINTER(GemmDesc)]
+    lib.nmspmm_gemm_call_plan.argtypes = [ctypes.POINTER(GemmDesc), sz, ctypes.POINTER(PlanInfo)]
     lib.nmspmm_gemm.argtypes = [ctypes.POINTER(GemmDesc), vp, vp, vp, vp, vp, vp, sz, vp]
     lib.nmspmm_tuned_plan_set.argtypes = [ctypes.POINTER(GemmDesc), ci, ci]
     lib.nmspmm_tuned_plan_load.argtypes = [ctypes.c_char_p]
@@ -294,6 +297,19 @@ def plan(desc: GemmDesc) -> PlanInfo:
 
 def workspace_bytes(desc: GemmDesc) -> int:
     return int(load_library().nmspmm_gemm_workspace_bytes(ctypes.byref(desc)))
+
+
+def call_workspace_bytes(desc: GemmDesc) -> int:
+    """nmspmm_gemm_call_workspace_bytes: scratch with which a call runs its fastest form."""
+    return int(load_library().nmspmm_gemm_call_workspace_bytes(ctypes.byref(desc)))
+
+
+def call_plan(desc: GemmDesc, scratch_bytes: Optional[int] = None) -> PlanInfo:
+    """nmspmm_gemm_call_plan: what a call with that much scratch (default: call_workspace_bytes) runs."""
+    info = PlanInfo()
+    have = call_workspace_bytes(desc) if scratch_bytes is None else scratch_bytes
+    _check("nmspmm_gemm_call_plan", load_library().nmspmm_gemm_call_plan(ctypes.byref(desc), have, ctypes.byref(info)))
+    return info
 
 
 def gemm(desc: GemmDesc, A, B, D, column_info, C, workspace=None, stream=None) -> None:
@@ -586,7 +602,7 @@ class NMSpMM:
         return make_desc(M, self.N, self.K, self.n_keep, self.format, self.layout_ns, path, split_k, tile, self.vec_len)
 
     def _workspace(self, desc):
-        need = workspace_bytes(desc)
+        need = call_workspace_bytes(desc)
         return self._scratch.get(need, ctypes.byref(desc), self.B, _raw_stream())[2] if need else None
 
     def matmul(self, A, path: int = PATH_FP32, split_k: int = 0, tile: int = 0, out=None):

@@ -150,19 +150,69 @@ static bool staged_in_pairs(const nmspmm_gemm_desc* d)
     return d->format == NMSPMM_FORMAT_LOW && (d->n_keep == 16 || d->n_keep == 12) && d->K >= 512;      // short K keeps the finer windows for splitting
 }
 
-// Tile of the exact path.  Over 64 rows: 64 x 128 where it pads fewer rows than 128 x 128 does.
+// The 64 / 128-row (up to 32 rows: 16 / 32-row) tile of the exact path.  Over 64 rows: 64 x 128 where it pads fewer rows than 128 x 128 does.
 // The pairs of windows that 16:32 and 12:32 have on 128 x 128 alone are worth more than the
 // padding except between 128 and 192 rows (256 padded rows count as 213): at 5760 columns, K = 2080,
 // 12:32, 776 / 1032 / 320 / 192 rows take 159 / 202 / 82 / 59 us on it, 172 / 212 / 82 / 53 on 64 x 128; at
 // 4096 x 4096, 16:32, 904 / 448 / 192 rows 311 / 166 / 88 against 346 / 173 / 81.
-static int pick_tile(const nmspmm_gemm_desc* d, int sms)
+static int pick_tile(const nmspmm_gemm_desc* d)
 {
-    (void)sms;
     if (d->M <= 16) return kTile16x128;
     if (d->M <= 32) return kTile32x128;
     if (d->M <= 64) return kTile64x128;
     const long long pad128 = (static_cast<long long>(d->M) + 127) / 128 * 128, pad64 = (static_cast<long long>(d->M) + 63) / 64 * 64;
     return (pad64 * 100 < pad128 * (staged_in_pairs(d) ? 83 : 100)) ? kTile64x128 : kTile128x128;
+}
+
+// About how long the busiest CTA of a tile's schedule multiplies, in microseconds at the peak
+// FMA rate of an SM (128 per cycle, 1.965 GHz), whole padded tiles.
+static double busiest_cta_us(const nmspmm_gemm_desc* d, const FfmaVariant* v, int sms)
+{
+    const double tiles = static_cast<double>((d->M + v->ms - 1) / v->ms) * ((d->N + v->ns - 1) / v->ns);
+    const double n_win = (d->K / 32 * d->n_keep + v->ws - 1) / v->ws, units = tiles * n_win;
+    double n = static_cast<double>(sms) * v->min_blocks, share = v->min_blocks;    // CTAs, and how many of them share an SM
+    if (tiles < n) {
+        double most = units / 4 > tiles ? units / 4 : tiles;
+        if (most < n) {
+            n = most;
+            share = n / sms > 1 ? n / sms : 1;
+        }
+    }
+    return units / n * share * v->ms * v->ns * v->ws / (128.0 * 1965.0);
+}
+
+// The wide tile (gemm_ffma_wide.cuh) a call should run instead of pick_tile's, or kTileAuto.  They
+// multiply faster -- microseconds per microsecond at the peak, least squares over 186 shapes of more than 32
+// rows: 1.31 / 1.22 / 1.24 / 1.19 at 4 / 8 / 12 / 16 of 32 against 1.64 / 1.40 / 1.35 / 1.28 on 128 x 128 and 1.78 / 1.51 / 1.66 / 1.52 on
+// 64 x 128, 64 x 512 4 % slower than the other two -- but have one CTA per SM: nothing hides a tile's
+// stores (about 1.5 us for 128 x 256) or a launch's first copies and last pieces (about 2 us more).
+// So the wide tile with the least predicted time is taken where it is 2 % under the other's, a
+// call's 15 us included.  Under 224 kept rows per column the stores weigh more than this line knows
+// (5440 x 1792 x 640, 8:32: 78 us on 64 x 128, 90 on 128 x 256).  8:32 on the 32-k format counts as 4:32 (eight
+// rows a window); an unpruned weight gains nothing (51 shapes: 0.92 to 1.06).  Over the 186 shapes calls take
+// 1 / 1.080 of the time in the mean (with the best tile of each 1 / 1.107), none longer than before by more than 0.1 %.
+static int pick_wide_tile(const nmspmm_gemm_desc* d, int mode, int sms)
+{
+    const int W = d->K / 32 * d->n_keep, square = pick_tile(d);
+    if (d->M <= 32 || W < 224 || d->n_keep == 32) return kTileAuto;
+    const FfmaVariant* sv = find_ffma_variant(square, d->n_keep, mode);
+    if (!sv) return kTileAuto;
+    const int r = (d->n_keep == 4 || (d->n_keep == 8 && mode == kModeLow)) ? 0 : (d->n_keep == 8 ? 1 : (d->n_keep == 12 ? 2 : 3));
+    static const double kWide[4] = { 1.31, 1.22, 1.24, 1.19 }, k128[4] = { 1.64, 1.40, 1.35, 1.28 }, k64[4] = { 1.78, 1.51, 1.66, 1.52 };
+    const double call = 15.0;
+    double best = (call + (square == kTile128x128 ? k128 : k64)[r] * busiest_cta_us(d, sv, sms)) / 1.02;
+    int tile = kTileAuto;
+    for (int t : { kTile128x256, kTile256x128, kTile64x512 }) {
+        const FfmaVariant* v = find_ffma_variant(t, d->n_keep, mode);
+        if (!v) continue;
+        const double tiles = static_cast<double>((d->M + v->ms - 1) / v->ms) * ((d->N + v->ns - 1) / v->ns);
+        const double us = call + 2.0 + kWide[r] * (t == kTile64x512 ? 1.04 : 1.0) * busiest_cta_us(d, v, sms) + 1.5 * tiles / sms;
+        if (us < best) {
+            best = us;
+            tile = t;
+        }
+    }
+    return tile;
 }
 
 // Least share of the CTA slots, in per cent, that slices of equal length have to keep busy to be
@@ -267,7 +317,8 @@ static bool tuned_lookup(const nmspmm_gemm_desc* d, int* tile, int* split_k)
 static_assert(NMSPMM_TILE_128x128 == kTile128x128 && NMSPMM_TILE_64x128 == kTile64x128 && NMSPMM_TILE_32x128 == kTile32x128 &&
                   NMSPMM_TILE_16x128 == kTile16x128 && NMSPMM_TILE_128x256 == kTile128x256 && NMSPMM_TILE_16x256 == kTile16x256 &&
                   NMSPMM_TILE_32x256 == kTile32x256 && NMSPMM_TILE_128x256_GATHER == kTile128x256Gather &&
-                  NMSPMM_TILE_128x256_EXPAND == kTile128x256Expand && NMSPMM_TILE_128x256_EXPAND + 1 == kTileCount,
+                  NMSPMM_TILE_128x256_EXPAND == kTile128x256Expand && NMSPMM_TILE_256x128 == kTile256x128 &&
+                  NMSPMM_TILE_64x512 == kTile64x512 && NMSPMM_TILE_64x512 + 1 == kTileCount,
               "the public tile ids are the library's");
 
 // Whether the TF32 path should expand B rather than gather A when the caller leaves the choice
@@ -459,7 +510,7 @@ static int make_plan(const nmspmm_gemm_desc* d_in, int sms, Plan* p, bool any_ro
         return NMSPMM_OK;
     }
     if (d->path != NMSPMM_PATH_FP32) return NMSPMM_UNSUPPORTED;
-    const int tile = d->tile ? d->tile : pick_tile(d, sms);
+    const int tile = d->tile ? d->tile : pick_tile(d);
     const FfmaVariant* v = find_ffma_variant(tile, d->n_keep, mode);
     if (!v) return NMSPMM_UNSUPPORTED;
     // 16:32 and 12:32 on the 128 x 128 tile: two 32-k windows per stage (half as many CTA barriers
@@ -482,6 +533,7 @@ static int make_plan(const nmspmm_gemm_desc* d_in, int sms, Plan* p, bool any_ro
     if (mode == kModeLow && v->ws % 16 == 0)              // the variants compiled with the banded order (FfmaCfg::BANDED)
         p->band = tile_band(d, p->W, v->ns, p->tiles_x, p->tiles_y);
     const int resident = sms * v->min_blocks;
+    const bool wide = v->min_blocks == 1;                  // the wide tiles leave every split to the reduction kernel, and no SM runs a lone CTA faster
     if (d->split_k > 0) {
         // Explicit K slices: one unit range per (tile, slice); a single slice stores directly.
         int s = d->split_k < p->n_win ? d->split_k : p->n_win;
@@ -489,7 +541,7 @@ static int make_plan(const nmspmm_gemm_desc* d_in, int sms, Plan* p, bool any_ro
         p->split_k = s;
         p->n_virtual = static_cast<int>(n_tiles * s);
         p->slots = (s > 1) ? p->n_virtual : 0;
-        p->deferred = s > kDeferPieces;
+        p->deferred = s > kDeferPieces || wide;
         p->first_split_tile = 0;
         p->n_split_tiles = p->n_tiles;
     } else {
@@ -503,7 +555,7 @@ static int make_plan(const nmspmm_gemm_desc* d_in, int sms, Plan* p, bool any_ro
         // few tiles would each hold an SM for a whole tile's time, and cutting them over all
         // the slots pays (8192 x 3584 x 8192, one rank's slab of eight: 1792 tiles = 6.05 waves).
         const long long full_waves = n_tiles / resident * resident;
-        const bool sparse_tail = (n_tiles - full_waves) * 4 <= resident;
+        const bool sparse_tail = wide || (n_tiles - full_waves) * 4 <= resident;
         const long long n_dp = (n_tiles >= 2LL * resident && !sparse_tail) ? n_tiles : full_waves;
         const long long tail_tiles = n_tiles - n_dp;
         long long n_sk = 0;
@@ -537,7 +589,7 @@ static int make_plan(const nmspmm_gemm_desc* d_in, int sms, Plan* p, bool any_ro
         // equal ranges that coincide with whole tiles need no scratch
         const bool aligned = (n_sk == 0) || (n_sk == tail_tiles);
         p->slots = aligned ? 0 : static_cast<int>(2 * n_sk);
-        p->deferred = !aligned && n_sk > static_cast<long long>(kDeferPieces - 1) * tail_tiles;   // a tile sees up to n_sk / tail_tiles + 1 pieces
+        p->deferred = !aligned && (wide || n_sk > static_cast<long long>(kDeferPieces - 1) * tail_tiles);   // a tile sees up to n_sk / tail_tiles + 1 pieces
         p->first_split_tile = p->n_dp;
         p->n_split_tiles = static_cast<int>(tail_tiles);
     }
@@ -547,6 +599,24 @@ static int make_plan(const nmspmm_gemm_desc* d_in, int sms, Plan* p, bool any_ro
         p->partial_bytes = static_cast<size_t>(p->slots) * v->ms * v->ns * sizeof(float);
     }
     return NMSPMM_OK;
+}
+
+static size_t scratch_bytes(const Plan& p) { return p.counters_bytes + p.partial_bytes; }
+
+// The plan a call runs that has `workspace_bytes` of scratch: make_plan's, or on the exact path, where the
+// description leaves tile and split to the library and no tuned entry names them, a wide tile's
+// (pick_wide_tile) if its scratch fits.
+static int plan_call(const nmspmm_gemm_desc* d, int sms, size_t workspace_bytes, Plan* p, bool any_rows = false)
+{
+    const int rc = make_plan(d, sms, p, any_rows);
+    if (rc != NMSPMM_OK || !p->v || d->tile != 0 || d->split_k != 0) return rc;
+    int tuned_tile, tuned_split;
+    if (tuned_lookup(d, &tuned_tile, &tuned_split)) return rc;
+    nmspmm_gemm_desc w = *d;
+    w.tile = pick_wide_tile(d, p->v->mode, sms);
+    Plan wp;
+    if (w.tile != kTileAuto && make_plan(&w, sms, &wp, any_rows) == NMSPMM_OK && scratch_bytes(wp) <= workspace_bytes) *p = wp;
+    return rc;
 }
 
 static int sm_count()
@@ -763,7 +833,15 @@ size_t nmspmm_gemm_workspace_bytes(const nmspmm_gemm_desc* desc)
 {
     Plan p;
     if (make_plan(desc, sm_count(), &p) != NMSPMM_OK) return 0;
-    return p.counters_bytes + p.partial_bytes;
+    return scratch_bytes(p);
+}
+
+// The larger of what the description's plan and what the call's need.
+size_t nmspmm_gemm_call_workspace_bytes(const nmspmm_gemm_desc* desc)
+{
+    Plan p, c;
+    if (make_plan(desc, sm_count(), &p) != NMSPMM_OK || plan_call(desc, sm_count(), SIZE_MAX, &c) != NMSPMM_OK) return 0;
+    return scratch_bytes(p) > scratch_bytes(c) ? scratch_bytes(p) : scratch_bytes(c);
 }
 
 size_t nmspmm_gemm_counter_bytes(const nmspmm_gemm_desc* desc)
@@ -773,12 +851,8 @@ size_t nmspmm_gemm_counter_bytes(const nmspmm_gemm_desc* desc)
     return round256(static_cast<size_t>(p.n_tiles) * sizeof(unsigned));
 }
 
-int nmspmm_gemm_plan(const nmspmm_gemm_desc* desc, nmspmm_gemm_plan_info* out)
+static void describe_plan(const Plan& p, nmspmm_gemm_plan_info* out)
 {
-    if (!out) return NMSPMM_INVALID_ARGUMENT;
-    Plan p;
-    int rc = make_plan(desc, sm_count(), &p);
-    if (rc != NMSPMM_OK) return rc;
     out->tile = p.v ? p.v->tile_id
                     : (p.tv->form == 2 ? (p.tv->ms == 16 ? kTile16x128 : (p.tv->ms == 32 ? kTile32x128 : kTile64x128))
                                        : (p.tv->ns == 128 ? kTile128x128 : (p.tv->form == 1 ? kTile128x256Expand : kTile128x256)));
@@ -795,7 +869,24 @@ int nmspmm_gemm_plan(const nmspmm_gemm_desc* desc, nmspmm_gemm_plan_info* out)
     out->threads = p.v ? p.v->threads : p.tv->threads;
     out->smem_bytes = p.v ? p.v->smem_bytes : p.tv->smem_bytes;
     out->stages = p.v ? p.v->stages : p.tv->stages;
-    return NMSPMM_OK;
+}
+
+int nmspmm_gemm_plan(const nmspmm_gemm_desc* desc, nmspmm_gemm_plan_info* out)
+{
+    if (!out) return NMSPMM_INVALID_ARGUMENT;
+    Plan p;
+    const int rc = make_plan(desc, sm_count(), &p);
+    if (rc == NMSPMM_OK) describe_plan(p, out);
+    return rc;
+}
+
+int nmspmm_gemm_call_plan(const nmspmm_gemm_desc* desc, size_t workspace_bytes, nmspmm_gemm_plan_info* out)
+{
+    if (!out) return NMSPMM_INVALID_ARGUMENT;
+    Plan p;
+    const int rc = plan_call(desc, sm_count(), workspace_bytes, &p);
+    if (rc == NMSPMM_OK) describe_plan(p, out);
+    return rc;
 }
 
 // The multiply with its outputs spelled out: n_out buffers, row stride ldc, first column col0.
@@ -807,7 +898,7 @@ static int gemm_launch(const nmspmm_gemm_desc* desc, const float* A_dev, const f
     int rc = device_info(&di);
     if (rc != NMSPMM_OK) return rc;
     Plan p;
-    rc = make_plan(desc, di->sms, &p, lda != 0 || a_rows != 0);
+    rc = plan_call(desc, di->sms, aligned16(workspace_dev) && workspace_dev ? workspace_bytes : 0, &p, lda != 0 || a_rows != 0);
     if (rc != NMSPMM_OK) return rc;
     if (lda != 0 && (lda < desc->M || lda % 4 != 0)) return NMSPMM_INVALID_ARGUMENT;
     if (!A_dev || !B_dev || !D_dev || !C_out || n_out < 1 || n_out > kMaxOutputs) return NMSPMM_INVALID_ARGUMENT;
@@ -843,7 +934,7 @@ static int gemm_launch(const nmspmm_gemm_desc* desc, const float* A_dev, const f
     a.qs_shift = desc->layout_ns == 128 ? 2 : (desc->layout_ns == 64 ? 1 : 0);
     if (p.slots > 0) {
         if (!workspace_dev || !aligned16(workspace_dev)) return NMSPMM_INVALID_ARGUMENT;
-        if (workspace_bytes < p.counters_bytes + p.partial_bytes) return NMSPMM_WORKSPACE_TOO_SMALL;
+        if (workspace_bytes < scratch_bytes(p)) return NMSPMM_WORKSPACE_TOO_SMALL;
         a.counters = p.deferred ? nullptr : static_cast<unsigned*>(workspace_dev);
         a.partial = reinterpret_cast<float*>(static_cast<unsigned char*>(workspace_dev) + p.counters_bytes);
         if (a.counters && (p.counters_bytes > kCounterBlock || g_timeout_seen)) {
@@ -884,7 +975,7 @@ static size_t row_major_copy_bytes(const nmspmm_gemm_desc* d)
 // with; a plan that needs nothing still leaves the block's bytes alone.  The copies follow.
 static size_t row_major_head_bytes(const Plan& p)
 {
-    const size_t own = p.counters_bytes + p.partial_bytes;
+    const size_t own = scratch_bytes(p);
     return own > 0 ? own : kCounterBlock;
 }
 
@@ -917,18 +1008,32 @@ static size_t row_major_bytes(const Plan& p, const nmspmm_gemm_desc* d, int dtyp
     return row_major_head_bytes(p) + (copy_a ? row_major_copy_bytes(d) : 0) + (dtype != kDtypeF32 && !p.tv ? result_copy_bytes(d) : 0);
 }
 
-size_t nmspmm_gemm_row_major_workspace_bytes(const nmspmm_gemm_desc* desc)
+// The larger of what the description's plan and what the call's takes (plan_call); copy_a < 0: by the addresses.
+static size_t row_major_bytes_any(const nmspmm_gemm_desc* d, int dtype, int copy_a, const void* A_rows = nullptr, const void* C = nullptr)
 {
-    Plan p;
-    if (!desc || make_plan(desc, sm_count(), &p, true) != NMSPMM_OK) return 0;
-    return row_major_bytes(p, desc, kDtypeF32, true);
+    Plan p, c;
+    if (!d || make_plan(d, sm_count(), &p, true) != NMSPMM_OK || plan_call(d, sm_count(), SIZE_MAX, &c, true) != NMSPMM_OK) return 0;
+    const bool copy = copy_a < 0 ? !reads_rows(p, d, A_rows, C, dtype) : copy_a != 0;
+    const size_t x = row_major_bytes(p, d, dtype, copy), y = row_major_bytes(c, d, dtype, copy);
+    return x > y ? x : y;
 }
+
+// The plan a row-major call with this much workspace runs.
+static int plan_row_major(const nmspmm_gemm_desc* d, const void* A_rows, const void* C, int dtype, size_t workspace_bytes, Plan* p)
+{
+    int rc = plan_call(d, sm_count(), SIZE_MAX, p, true);
+    if (rc == NMSPMM_OK && workspace_bytes < row_major_bytes(*p, d, dtype, !reads_rows(*p, d, A_rows, C, dtype))) {
+        rc = make_plan(d, sm_count(), p, true);
+        if (rc == NMSPMM_OK && workspace_bytes < row_major_bytes(*p, d, dtype, !reads_rows(*p, d, A_rows, C, dtype))) rc = NMSPMM_WORKSPACE_TOO_SMALL;
+    }
+    return rc;
+}
+
+size_t nmspmm_gemm_row_major_workspace_bytes(const nmspmm_gemm_desc* desc) { return row_major_bytes_any(desc, kDtypeF32, 1); }
 
 size_t nmspmm_gemm_row_major_call_bytes(const nmspmm_gemm_desc* desc, int dtype, const void* A_rows_dev, const void* C_dev)
 {
-    Plan p;
-    if (!desc || make_plan(desc, sm_count(), &p, true) != NMSPMM_OK) return 0;
-    return row_major_bytes(p, desc, dtype, !reads_rows(p, desc, A_rows_dev, C_dev, dtype));
+    return row_major_bytes_any(desc, dtype, -1, A_rows_dev, C_dev);
 }
 
 int nmspmm_gemm_row_major(const nmspmm_gemm_desc* desc, const float* A_rows_dev, const float* B_dev, const int* D_dev,
@@ -936,11 +1041,10 @@ int nmspmm_gemm_row_major(const nmspmm_gemm_desc* desc, const float* A_rows_dev,
 {
     if (!desc || !A_rows_dev || !workspace_dev || !aligned16(workspace_dev)) return NMSPMM_INVALID_ARGUMENT;
     Plan p;
-    int rc = make_plan(desc, sm_count(), &p, true);
+    const int rc = plan_row_major(desc, A_rows_dev, C_dev, kDtypeF32, workspace_bytes, &p);
     if (rc != NMSPMM_OK) return rc;
     const bool rows = reads_rows(p, desc, A_rows_dev, C_dev, kDtypeF32);
-    if (workspace_bytes < row_major_bytes(p, desc, kDtypeF32, !rows)) return NMSPMM_WORKSPACE_TOO_SMALL;
-    const size_t own = p.counters_bytes + p.partial_bytes, head = row_major_head_bytes(p);
+    const size_t own = scratch_bytes(p), head = row_major_head_bytes(p);
     const int ld = (desc->M + 3) / 4 * 4;
     float* out[1] = { C_dev };
     if (rows)
@@ -955,12 +1059,7 @@ int nmspmm_gemm_row_major(const nmspmm_gemm_desc* desc, const float* A_rows_dev,
 // ---- activations and result in 16-bit storage ---------------------------------------------
 static_assert(NMSPMM_DTYPE_F16 == kDtypeF16 && NMSPMM_DTYPE_BF16 == kDtypeBF16, "the public dtype ids are the library's");
 
-size_t nmspmm_gemm_row_major_16_workspace_bytes(const nmspmm_gemm_desc* desc)
-{
-    Plan p;
-    if (!desc || make_plan(desc, sm_count(), &p, true) != NMSPMM_OK) return 0;
-    return row_major_bytes(p, desc, kDtypeF16, true);
-}
+size_t nmspmm_gemm_row_major_16_workspace_bytes(const nmspmm_gemm_desc* desc) { return row_major_bytes_any(desc, kDtypeF16, 1); }
 
 int nmspmm_gemm_row_major_16(const nmspmm_gemm_desc* desc, int dtype, const void* A_rows_dev, const float* B_dev, const int* D_dev,
                              const int* column_info_dev, void* C_dev, void* workspace_dev, size_t workspace_bytes, void* stream)
@@ -969,11 +1068,10 @@ int nmspmm_gemm_row_major_16(const nmspmm_gemm_desc* desc, int dtype, const void
     if (dtype != NMSPMM_DTYPE_F16 && dtype != NMSPMM_DTYPE_BF16) return NMSPMM_INVALID_ARGUMENT;
     if ((reinterpret_cast<uintptr_t>(C_dev) & 7u) != 0) return NMSPMM_INVALID_ARGUMENT;
     Plan p;
-    int rc = make_plan(desc, sm_count(), &p, true);
+    int rc = plan_row_major(desc, A_rows_dev, C_dev, dtype, workspace_bytes, &p);
     if (rc != NMSPMM_OK) return rc;
     const bool rows = reads_rows(p, desc, A_rows_dev, C_dev, dtype);
-    if (workspace_bytes < row_major_bytes(p, desc, dtype, !rows)) return NMSPMM_WORKSPACE_TOO_SMALL;
-    const size_t own = p.counters_bytes + p.partial_bytes, head = row_major_head_bytes(p);
+    const size_t own = scratch_bytes(p), head = row_major_head_bytes(p);
     const int ld = (desc->M + 3) / 4 * 4;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     unsigned char* ws = static_cast<unsigned char*>(workspace_dev);
@@ -1089,7 +1187,7 @@ int nmspmm_device_status(int* status_out, int clear)
 int nmspmm_gemm_with_cached_workspace(const nmspmm_gemm_desc* desc, const float* A_dev, const float* B_dev,
                                       const int* D_dev, const int* column_info_dev, float* C_dev, void* stream)
 {
-    const size_t need = nmspmm_gemm_workspace_bytes(desc);
+    const size_t need = nmspmm_gemm_call_workspace_bytes(desc);
     void* ws = nullptr;
     size_t have = 0;
     if (need > 0) {
@@ -1187,10 +1285,8 @@ int nmspmm_gemm_host(const nmspmm_gemm_desc* desc, const float* A_host, const fl
     for (int c = 0; c < n_chunks; ++c) {
         nmspmm_gemm_desc dc = *desc;
         dc.M = (c + 1 < n_chunks) ? chunk_rows : M - c * chunk_rows;
-        Plan pc;
-        rc = make_plan(&dc, di->sms, &pc);
-        if (rc != NMSPMM_OK) return rc;
-        if (pc.counters_bytes + pc.partial_bytes > ws_need) ws_need = pc.counters_bytes + pc.partial_bytes;
+        const size_t need = nmspmm_gemm_call_workspace_bytes(&dc);
+        if (need > ws_need) ws_need = need;
     }
 
     const size_t a_b = round256(sizeof(float) * M * static_cast<size_t>(K));

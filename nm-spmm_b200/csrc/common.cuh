@@ -85,6 +85,22 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity)
     return ok != 0;
 }
 
+// The same, letting the hardware suspend the thread for up to about `ns` nanoseconds.
+__device__ __forceinline__ bool mbar_try_wait_for(uint32_t bar, uint32_t parity, uint32_t ns)
+{
+    uint32_t ok;
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n"
+        "selp.u32 %0, 1, 0, p;\n"
+        "}\n"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity), "r"(ns)
+        : "memory");
+    return ok != 0;
+}
+
 __device__ __forceinline__ int lds_volatile_s32(uint32_t addr)
 {
     int v;
@@ -114,6 +130,22 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity,
                 sts_volatile_s32(abort_word, 1);
                 return false;
             }
+        }
+    }
+    return true;
+}
+
+// Same contract again, for warps that spend most of their time here beside warps that compute:
+// a poll takes issue slots, so the thread sleeps through the wait in the hardware.
+__device__ __forceinline__ bool mbar_sleep_bounded(uint32_t bar, uint32_t parity, uint32_t abort_word)
+{
+    if (mbar_try_wait(bar, parity)) return true;
+    const long long t0 = clock64();
+    while (!mbar_try_wait_for(bar, parity, 10000u)) {
+        if (lds_volatile_s32(abort_word)) return false;
+        if (clock64() - t0 > kWaitCycleLimit) {
+            sts_volatile_s32(abort_word, 1);
+            return false;
         }
     }
     return true;

@@ -26,6 +26,8 @@ enum nmspmm_tile {
     kTile32x256 = 7,
     kTile128x256Gather = 8,   // TF32 path only: tile 128 x 256, the form that gathers A with the tensor core
     kTile128x256Expand = 9,   // TF32 path only: tile 128 x 256, the form that expands B with zeros (32-k formats, 16 / 12 / 8 kept)
+    kTile256x128 = 10,    // exact path only
+    kTile64x512 = 11,     // exact path only
     kTileCount
 };
 

@@ -465,7 +465,6 @@ cudaError_t launch_ffma(const GemmArgs& a, const GemmOutputs& outs, int grid, cu
     NMSPMM_FFMA_VARIANT(kTile64x128, NKEEP, 64, 128, 64, WS, KS, MODE),   \
     NMSPMM_FFMA_VARIANT(kTile32x128, NKEEP, 32, 128, 32, WS, KS, MODE),   \
     NMSPMM_FFMA_VARIANT(kTile16x128, NKEEP, 16, 128, 16, WS, KS, MODE),   \
-    NMSPMM_FFMA_VARIANT(kTile128x256, NKEEP, 128, 256, 64, WS, KS, MODE), \
     NMSPMM_FFMA_VARIANT(kTile16x256, NKEEP, 16, 256, 16, WS, KS, MODE),   \
     NMSPMM_FFMA_VARIANT(kTile32x256, NKEEP, 32, 256, 32, WS, KS, MODE)
 

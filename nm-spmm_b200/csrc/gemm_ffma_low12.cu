@@ -5,8 +5,9 @@
 // holding the window's twelve row offsets itself the compiler fits them (24 bytes).
 #define NMSPMM_IDX_SHFL 0
 #include "gemm_ffma.cuh"
+#include "gemm_ffma_wide.cuh"
 
 namespace nmspmm {
-extern const FfmaVariant kFfma_low12[] = { NMSPMM_FFMA_TILES(12, 12, 32, kModeLow) };
+extern const FfmaVariant kFfma_low12[] = { NMSPMM_FFMA_TILES(12, 12, 32, kModeLow), NMSPMM_WIDE_TILES(12, 12, 32, kModeLow) };
 extern const int kFfma_low12_count = sizeof(kFfma_low12) / sizeof(kFfma_low12[0]);
 }  // namespace nmspmm

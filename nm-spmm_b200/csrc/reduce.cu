@@ -31,17 +31,37 @@ static cudaError_t launch_after_multiply(void (*kernel)(KArgs...), unsigned bloc
 // WM x 32: thread tid holds rows row(i), i < MT, and columns col0 .. col0 + 3 and
 // col0 + 16 .. col0 + 19 of them; the slot stores fragment row i as float4 words
 // (2 i) * NCT + tid and (2 i + 1) * NCT + tid.
-template <int MS, int NS, int WM>
+template <int MS_, int NS_, int WM>
 struct FragmentMap {
+    static constexpr int MS = MS_, NS = NS_;
     static constexpr int QT = NS / kVecLen;
     static constexpr int NCT = QT * (MS / WM) * 32;
     static constexpr int MT = WM / 8;
     __device__ static int vec(int tid) { return (tid >> 5) % QT; }
-    __device__ static int col0(int tid) { return vec(tid) * kVecLen + ((tid & 31) >> 4) * 8 + (tid & 1) * 4; }
+    __device__ static int col(int tid, int half) { return vec(tid) * kVecLen + ((tid & 31) >> 4) * 8 + (tid & 1) * 4 + 16 * half; }
     __device__ static int row(int tid, int i)
     {
         const int wm = (tid >> 5) / QT, lm = (tid & 15) >> 1;
         return wm * WM + ((MT == 8) ? ((i < 4) ? lm * 4 + i : 32 + lm * 4 + (i - 4)) : ((MT == 4) ? lm * 4 + i : lm * 2 + i));
+    }
+};
+
+// The same for the wide tiles (gemm_ffma_wide.cuh): WR x WV warps of WM rows x 128 / WM vectors, sixteen rows a thread.
+template <int WR, int WV, int WM>
+struct WideFragmentMap {
+    static constexpr int VPW = 128 / WM, MS = WR * WM, NS = WV * VPW * kVecLen;
+    static constexpr int NCT = WR * WV * 32;
+    static constexpr int MT = 16;
+    __device__ static int second(int tid) { return VPW == 2 ? (tid >> 3) & 1 : 0; }
+    __device__ static int vec(int tid) { return (tid >> 5) % WV * VPW + second(tid); }
+    __device__ static int col(int tid, int half)
+    {
+        return vec(tid) * kVecLen + ((tid & 31) >> 4) * 8 + (tid & 1) * 4 + 16 * (half ^ second(tid));
+    }
+    __device__ static int row(int tid, int i)
+    {
+        const int lm = (tid >> 1) & (VPW == 2 ? 3 : 7), group = (i >> 2) ^ second(tid);
+        return (tid >> 5) / WV * WM + lm * 4 + group * (VPW == 2 ? 16 : 32) + (i & 3);
     }
 };
 
@@ -52,12 +72,11 @@ constexpr int kReduceInFlight = 16;   // loads of one thread that are issued bef
 // trip to L2, so sixteen loads are in flight before the first is added.  CTAS_PER_ROW = 1: a
 // CTA adds both words, four loads of each in flight -- fewer, fuller CTAs for the common
 // case of a handful of pieces, where the launch is what costs.
-template <int MS, int NS, int WM, int CTAS_PER_ROW>
-__global__ void __launch_bounds__((FragmentMap<MS, NS, WM>::NCT))
+template <typename Map, int CTAS_PER_ROW>
+__global__ void __launch_bounds__((Map::NCT))
 nm_reduce_pieces_kernel(const GemmArgs g, const __grid_constant__ GemmOutputs outs, int first_tile)
 {
-    using Map = FragmentMap<MS, NS, WM>;
-    constexpr int NCT = Map::NCT, MT = Map::MT;
+    constexpr int NCT = Map::NCT, MT = Map::MT, MS = Map::MS, NS = Map::NS;
     constexpr int WORDS = 2 / CTAS_PER_ROW, FLIGHT = (CTAS_PER_ROW == 2) ? kReduceInFlight : 4;
     constexpr size_t kSlot = static_cast<size_t>(2 * MT) * NCT;       // float4 words per slot
     const int half = (CTAS_PER_ROW == 2) ? (blockIdx.x & 1) : 0;
@@ -71,7 +90,7 @@ nm_reduce_pieces_kernel(const GemmArgs g, const __grid_constant__ GemmOutputs ou
     int ty, tx;
     tile_coords(tile, g.tiles_x, (g.M + MS - 1) / MS, ty, tx);
     const int bj = tx * NS, bi = ty * MS;
-    const int r = bi + Map::row(tid, i), c = bj + Map::col0(tid) + 16 * half;
+    const int r = bi + Map::row(tid, i);
     if (Map::vec(tid) * kVecLen >= g.N - bj || r >= g.M) return;       // vectors past N, rows past M
     const float4* slots = reinterpret_cast<const float4*>(g.partial) + (2 * i + half) * NCT + tid;
     // Slot of range v's piece (piece_slot): one per range with an explicit split; with the
@@ -103,36 +122,37 @@ nm_reduce_pieces_kernel(const GemmArgs g, const __grid_constant__ GemmOutputs ou
             }
         }
     }
-    const size_t at = static_cast<size_t>(r) * outs.ldc + outs.col0 + c;
+    const size_t at = static_cast<size_t>(r) * outs.ldc + outs.col0 + bj;
     for (int o = 0; o < outs.n_out; ++o) {
         float* cp = output_of(g, outs, o) + at;
 #pragma unroll
-        for (int w = 0; w < WORDS; ++w) *reinterpret_cast<float4*>(cp + 16 * w) = sum[w];
+        for (int w = 0; w < WORDS; ++w) *reinterpret_cast<float4*>(cp + Map::col(tid, half + w)) = sum[w];
     }
 }
 
-template <int MS, int NS, int WM>
+template <typename Map>
 static cudaError_t launch_reduce(const GemmArgs& a, const GemmOutputs& outs, int first_tile, int n_tiles, cudaStream_t st)
 {
-    using Map = FragmentMap<MS, NS, WM>;
     // pieces per tile, about: the ranges that are not whole tiles over the tiles they cover
     const int pieces = a.sched.split_k > 0 ? a.sched.split_k : (a.sched.n_virtual - a.sched.n_dp) / (n_tiles > 0 ? n_tiles : 1) + 1;
     if (pieces > kReduceInFlight / 2)
-        return launch_after_multiply(nm_reduce_pieces_kernel<MS, NS, WM, 2>, n_tiles * Map::MT * 2, Map::NCT, st, a, outs, first_tile);
-    return launch_after_multiply(nm_reduce_pieces_kernel<MS, NS, WM, 1>, n_tiles * Map::MT, Map::NCT, st, a, outs, first_tile);
+        return launch_after_multiply(nm_reduce_pieces_kernel<Map, 2>, n_tiles * Map::MT * 2, Map::NCT, st, a, outs, first_tile);
+    return launch_after_multiply(nm_reduce_pieces_kernel<Map, 1>, n_tiles * Map::MT, Map::NCT, st, a, outs, first_tile);
 }
 
 cudaError_t launch_reduce_pieces(int tile_id, const GemmArgs& a, const GemmOutputs& outs, int first_tile, int n_tiles, cudaStream_t st)
 {
     if (n_tiles <= 0) return cudaSuccess;
     switch (tile_id) {
-    case kTile128x128: return launch_reduce<128, 128, 64>(a, outs, first_tile, n_tiles, st);
-    case kTile64x128: return launch_reduce<64, 128, 64>(a, outs, first_tile, n_tiles, st);
-    case kTile32x128: return launch_reduce<32, 128, 32>(a, outs, first_tile, n_tiles, st);
-    case kTile16x128: return launch_reduce<16, 128, 16>(a, outs, first_tile, n_tiles, st);
-    case kTile128x256: return launch_reduce<128, 256, 64>(a, outs, first_tile, n_tiles, st);
-    case kTile16x256: return launch_reduce<16, 256, 16>(a, outs, first_tile, n_tiles, st);
-    case kTile32x256: return launch_reduce<32, 256, 32>(a, outs, first_tile, n_tiles, st);
+    case kTile128x128: return launch_reduce<FragmentMap<128, 128, 64>>(a, outs, first_tile, n_tiles, st);
+    case kTile64x128: return launch_reduce<FragmentMap<64, 128, 64>>(a, outs, first_tile, n_tiles, st);
+    case kTile32x128: return launch_reduce<FragmentMap<32, 128, 32>>(a, outs, first_tile, n_tiles, st);
+    case kTile16x128: return launch_reduce<FragmentMap<16, 128, 16>>(a, outs, first_tile, n_tiles, st);
+    case kTile128x256: return launch_reduce<WideFragmentMap<1, 8, 128>>(a, outs, first_tile, n_tiles, st);
+    case kTile16x256: return launch_reduce<FragmentMap<16, 256, 16>>(a, outs, first_tile, n_tiles, st);
+    case kTile32x256: return launch_reduce<FragmentMap<32, 256, 32>>(a, outs, first_tile, n_tiles, st);
+    case kTile256x128: return launch_reduce<WideFragmentMap<2, 4, 128>>(a, outs, first_tile, n_tiles, st);
+    case kTile64x512: return launch_reduce<WideFragmentMap<1, 8, 64>>(a, outs, first_tile, n_tiles, st);
     default: return cudaErrorInvalidValue;
     }
 }

@@ -340,3 +340,27 @@ def test_row_major_scratch_is_what_the_call_writes(pkg):
     assert call(dense, pkg.DTYPE_F16) >= copy_a > call(dense, pkg.DTYPE_F32)
     assert lib.nmspmm_gemm_row_major_16_workspace_bytes(tf32) == own + copy_a       # whatever A is, without an FP32 C
     assert lib.nmspmm_gemm_row_major_workspace_bytes(tf32) == own + copy_a
+
+
+@pytest.mark.parametrize("M,N,K,n_keep,tile", [
+    (4096, 4096, 4096, 8, (128, 256)), (128, 1024, 131072, 4, (128, 256)), (64, 11008, 4096, 8, (64, 512)), (6512, 3200, 4096, 8, (256, 128)),
+    (32, 11008, 4096, 8, None), (5440, 1792, 640, 8, None), (128, 512, 1024, 16, None), (4096, 4096, 4096, 32, None)])
+def test_calls_take_a_wide_tile_where_it_pays_and_fits(pkg, M, N, K, n_keep, tile):
+    """148 SMs: the tile a call runs with all the scratch it asks for, and what it runs with less."""
+    d = pkg.make_desc(M, N, K, n_keep, pkg.format_of(n_keep), 128)
+    base, call = pkg.plan(d), pkg.call_plan(d)
+    assert (call.tile_m, call.tile_n) == (tile or (base.tile_m, base.tile_n))
+    need, more = pkg.workspace_bytes(d), pkg.call_workspace_bytes(d)
+    assert more >= need
+    own = pkg.make_desc(M, N, K, n_keep, pkg.format_of(n_keep), 128, 0, 0, call.tile)
+    for scratch in (0, need, more):                              # never a plan whose pieces do not fit
+        ran = pkg.call_plan(d, scratch)
+        assert ran.tile == base.tile or pkg.workspace_bytes(own) <= scratch
+    for named in (dict(tile=1), dict(split_k=2)):                # the caller's tile or split stays
+        e = pkg.make_desc(M, N, K, n_keep, pkg.format_of(n_keep), 128, 0, named.get("split_k", 0), named.get("tile", 0))
+        assert pkg.call_plan(e).tile == pkg.plan(e).tile
+    try:
+        pkg.set_tuned_plan(d, 2, 4)                              # so does a tuned entry
+        assert pkg.call_plan(d).tile == pkg.TILE_64x128
+    finally:
+        pkg.clear_tuned_plans()
