@@ -28,14 +28,24 @@
 //   warps 2-3   one elected thread each issues the products of half the tile's vectors
 //               (A = G from TMEM, B from shared memory, M128 N32 K8 each) once the gather's
 //               mbarrier has completed, and commits to the mbarrier that frees the stage and
-//               the result buffer.  One thread issues a tcgen05.mma every 26 cycles at best
-//               (measured), and a step has 12 to 20 of them: three issuing threads keep the
-//               tensor pipe, not the issue slot, the bound.
+//               the result buffer.  Measured alone (instruction chains, cycles): a product takes the pipe
+//               16 / 32 at N = 32 / 64, its arithmetic and no more; a gather 40 / 48 / 64 at N = 32 / 64 / 128,
+//               in TF32 (K = 8) and 16 bits (K = 16) alike; one thread issues an instruction every 27.
+//               Issuers are one elected thread each, from first wait to last commit, operand
+//               descriptors by addition: with a warp-wide wait, a vote and descriptors built anew
+//               per instruction a step of 8:32 took 600 cycles on the issuers' side alone (2048 x 9472 x 4096, 8:32,
+//               186 -> 138 us; 256 x 11008 x 4096, bfloat16, 42 -> 31.5).
 //   warps 4-11  (4-7 on the 128-column tile, at 16:32 and 12:32 with 32-wide vectors, and at 32:32) one
-//               thread per (vector, kept row) and turn: fetches its index two to four steps ahead
-//               with cp.async (through column_info on the 64-k format), keeps P's one-hot
+//               thread per (vector, kept row) and turn: loads its index two to four turns ahead
+//               into registers (through column_info on the 64-k format), keeps P's one-hot
 //               entry current, and after the last step reads the accumulators (tcgen05.ld),
 //               transposes them through shared memory and stores C in 128-byte row pieces.
+//
+// What bounds a step now is what feeds it: a tiled copy takes the SM about 2.1 cycles per row of its
+// box (128 bytes or fewer): 128 rows of A and 64 of B, 400 cycles, at 8:32, for FP32 and 16-bit
+// activations alike -- without any tensor-core instruction the kernel takes 126 us where it takes 138 (FP32)
+// and 125 (bfloat16) with them.  16:32 and 12:32 with 32-wide vectors have room for two gather results only, and
+// a result's way to its products and back, about 500 cycles each, is exposed (780 cycles a step with everything else left out).
 // n_keep = 32 (nothing pruned) has the identity as its index list and multiplies A_window by
 // the B rows directly.  12:32 gathers 16 columns per vector of which 4 are zero (P has no
 // entry for them), and loads 16 rows of B per vector of which the last 4 meet those zeros.
@@ -45,8 +55,7 @@
 // gathered in their own type (kind::f16, one-hot P of that type, FP32 result: exact), K = 16 per
 // instruction: half as many gather instructions per step and half of A's bytes, no transposing and
 // widening launch ahead of the multiply, and C is stored in the activations' type.
-// 256 x 11008 x 4096, bfloat16, 8:32: 59.5 us with a transposing and a rounding launch, 50.8 without, 42.5 with the
-// builder groups and stages below.
+// 256 x 11008 x 4096, bfloat16, 8:32: 59.5 us with a transposing and a rounding launch, 31.5 now.
 // Every wait is bounded; a wait that gives up raises the device status word.
 #include <cuda.h>
 
@@ -107,8 +116,7 @@ struct Tf32Cfg {
     static_assert(A_BYTES % 1024 == 0 && B_BYTES % 1024 == 0 && P_BYTES % 1024 == 0, "swizzle atoms stay aligned");
     static constexpr int CTAS_PER_SM = (QT == 8) ? 1 : 2;
     static constexpr int TMEM_COLS = 512 / CTAS_PER_SM;      // each resident CTA allocates its share
-    static constexpr int PD = 2;                             // index prefetch distance, in steps, per look-up
-    static constexpr int RING = 4 * PD;                      // slots of the per-thread index rings
+    static constexpr int PD = 2;                             // index prefetch distance, in turns, per look-up
     // One thread keeps one gathered column; the builder warps form GROUPS groups of N1 threads that take
     // turns with the steps.  A step is a chain of some 600 cycles for the warp that builds it (index
     // arrived, stage free, old entry, new entry, proxy fence, arrival): with one group that chain,
@@ -119,12 +127,10 @@ struct Tf32Cfg {
     static constexpr int GROUP_WARPS = N1 / 32;
     static constexpr int PRODUCT_WARPS = 2;
     static constexpr int THREADS = (2 + PRODUCT_WARPS) * 32 + BUILDERS;
-    // Every stage counts: a step's way through its stage -- copies, one-hot entries, gather, products and the
-    // barriers between them -- takes some 2400 cycles even with nothing to compute (bfloat16 activations,
-    // 2048 x 9472 x 4096, 8:32, four / six / eight stages: 202 / 185 / 171 us).  FP32 stages are larger; a seventh where
-    // it fits (64-wide vectors, 8:32) measured 2 % slower.
-    static constexpr int MAX_STAGES = (SRC == kTf32Rows16) ? 8 : 6;
-    static constexpr int AUX_BYTES = 2 * RING * BUILDERS * 4 + MAX_STAGES * 128 * 4;      // index rings; previous one-hot per stage and column
+    // Every stage counts (2048 x 9472 x 4096, 8:32, six / eight stages: 145 / 138 us, 64-wide vectors 141 / 130; 4096 cubed, 4:32,
+    // three / four: 142 / 121).
+    static constexpr int MAX_STAGES = 8;
+    static constexpr int AUX_BYTES = MAX_STAGES * 128;       // previous one-hot per stage and column (a byte each)
     static constexpr int CTRL_BYTES = 256;
     static constexpr int SMEM_LIMIT = (CTAS_PER_SM == 1 ? 227 : 113) * 1024;
     static constexpr int ST0 = (SMEM_LIMIT - 1024 - AUX_BYTES - CTRL_BYTES) / STAGE_BYTES;
@@ -167,6 +173,14 @@ __device__ __forceinline__ void sts_u16(uint32_t addr, unsigned v)
     asm volatile("st.shared.u16 [%0], %1;" ::"r"(addr), "h"(static_cast<unsigned short>(v)) : "memory");
 }
 
+__device__ __forceinline__ int lds_s8(uint32_t addr)
+{
+    int v;
+    asm volatile("ld.shared.s8 %0, [%1];" : "=r"(v) : "r"(addr));
+    return v;
+}
+__device__ __forceinline__ void sts_s8(uint32_t addr, int v) { asm volatile("st.shared.u8 [%0], %1;" ::"r"(addr), "r"(v) : "memory"); }
+
 // C16: C is stored in 16 bits (a parameter: see gemm_tf32_few_rows.cu).
 template <int NKEEP, int KW_, int MODE, int QT_, int VL_, int SRC_, bool C16>
 __global__ void __launch_bounds__((Tf32Cfg<NKEEP, KW_, MODE, QT_, VL_, SRC_>::THREADS), (Tf32Cfg<NKEEP, KW_, MODE, QT_, VL_, SRC_>::CTAS_PER_SM))
@@ -176,16 +190,13 @@ nm_gemm_tf32_kernel(const GemmArgs g, const __grid_constant__ CUtensorMap map_a,
     using Cfg = Tf32Cfg<NKEEP, KW_, MODE, QT_, VL_, SRC_>;
     constexpr int MS = Cfg::MS, NS = Cfg::NS, QT = Cfg::QT, KW = Cfg::KW, WS = Cfg::WS, WSP = Cfg::WSP;
     constexpr int VL = Cfg::VL, QV = Cfg::QV, BPV = VL / 32;              // 32-column blocks per vector
-    constexpr int STAGES = Cfg::STAGES, NBUF = Cfg::NBUF, RING = Cfg::RING, PD = Cfg::PD;
+    constexpr int STAGES = Cfg::STAGES, NBUF = Cfg::NBUF, PD = Cfg::PD;
     constexpr bool DIRECT = Cfg::DIRECT;
     constexpr int FIRST_BUILDER = 2 + Cfg::PRODUCT_WARPS;
 
     extern __shared__ unsigned char smem_raw[];
     const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u;          // swizzle atoms want 1024-byte alignment
-    const uint32_t idx_ring = ring + STAGES * Cfg::STAGE_BYTES;           // [RING][BUILDERS] raw index (rank on the 64-k format)
-    constexpr int SLOT = Cfg::BUILDERS * 4;
-    const uint32_t k_ring = idx_ring + RING * SLOT;                       // [RING][BUILDERS] k after the column_info look-up
-    const uint32_t prev_k = k_ring + RING * SLOT;                         // [STAGES][128] one-hot entry of each column now set in the stage
+    const uint32_t prev_k = ring + STAGES * Cfg::STAGE_BYTES;             // [STAGES][128] one-hot entry of each column now set in the stage
     const uint32_t bars = ring + STAGES * Cfg::STAGE_BYTES + Cfg::AUX_BYTES;
     const uint32_t bar_full = bars, bar_empty = bars + STAGES * 8;
     const uint32_t bar_gdone = bar_empty + STAGES * 8, bar_acc = bar_gdone + 4 * 8;
@@ -223,7 +234,7 @@ nm_gemm_tf32_kernel(const GemmArgs g, const __grid_constant__ CUtensorMap map_a,
     }
     if (warp == 1) tmem_alloc(tmem_word, Cfg::TMEM_COLS);
     if (!DIRECT) {
-        for (int o = tid * 4; o < Cfg::MAX_STAGES * 512; o += Cfg::THREADS * 4) sts_s32(prev_k + o, -1);
+        for (int o = tid * 4; o < Cfg::MAX_STAGES * 128; o += Cfg::THREADS * 4) sts_s32(prev_k + o, -1);
         // P starts as all zeros; 12:32 also wants the never-set columns of every vector zero
         const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
         for (int s = 0; s < STAGES; ++s)
@@ -239,149 +250,155 @@ nm_gemm_tf32_kernel(const GemmArgs g, const __grid_constant__ CUtensorMap map_a,
 
     if (warp == 0) {
         // ------------------------------------------------------------------ TMA producer
-        TF_DECL(p_empty = 0);
-        TF_T(p_start);
-        for (int it = 0; it < n_win; ++it) {
-            const int s = it % STAGES;
-            if (it >= STAGES) {
-                TF_T(t0);
-                const bool ok = mbar_wait_bounded(bar_empty + s * 8, ((it / STAGES) - 1) & 1, abort_word);
-                TF_ADD(p_empty, t0);
-                if (!__all_sync(0xffffffffu, ok)) {
-                    if (lane == 0) atomicMax(g.status, kDevTimeoutEmpty);
-                    break;
+        if (elect_one()) {
+            bool ok = true;
+            uint32_t st = ring, full = bar_full, parity = 1;           // stage of step `it`, its barrier, the parity of its last use
+            TF_DECL(p_empty = 0);
+            TF_T(p_start);
+            for (int it = 0, k = win0 * KW, w = win0 * WS; it < n_win; ++it, k += KW, w += WS) {
+                if (it >= STAGES) {
+                    TF_T(t0);
+                    ok = mbar_wait_bounded(full + (bar_empty - bar_full), parity, abort_word);
+                    TF_ADD(p_empty, t0);
+                    if (!ok) break;
                 }
-            }
-            const uint32_t st = ring + s * Cfg::STAGE_BYTES, full = bar_full + s * 8;
-            if (elect_one()) {
                 mbar_arrive_expect_tx(full, Cfg::A_BYTES + Cfg::B_BYTES);
                 if constexpr (Cfg::SRC == kTf32Rows32) {
-                    for (int kb = 0; kb < KW / 32; ++kb) tma_load_2d(st + kb * 16384, &map_a, (win0 + it) * KW + kb * 32, bi, full);
+                    for (int kb = 0; kb < KW / 32; ++kb) tma_load_2d(st + kb * 16384, &map_a, k + kb * 32, bi, full);
                 } else if constexpr (Cfg::SRC == kTf32Rows16) {
-                    tma_load_2d(st, &map_a, (win0 + it) * KW, bi, full);
+                    tma_load_2d(st, &map_a, k, bi, full);
                 } else if (a_form) {
-                    tma_load_3d(st, &map_a, 0, (win0 + it) * KW, bi >> 5, full);
+                    tma_load_3d(st, &map_a, 0, k, bi >> 5, full);
                 } else {                                   // rows not a multiple of 32: four boxes of 32 rows, the ragged one zero-filled
-                    for (int mb = 0; mb < 4; ++mb) tma_load_2d(st + mb * (KW * 128), &map_a, bi + mb * 32, (win0 + it) * KW, full);
+                    for (int mb = 0; mb < 4; ++mb) tma_load_2d(st + mb * (KW * 128), &map_a, bi + mb * 32, k, full);
                 }
-                tma_load_3d(st + Cfg::A_BYTES, &map_b, 0, (win0 + it) * WS, bj >> 5, full);
+                tma_load_3d(st + Cfg::A_BYTES, &map_b, 0, w, bj >> 5, full);
+                st += Cfg::STAGE_BYTES;
+                full += 8;
+                if (full == bar_full + STAGES * 8) { st = ring; full = bar_full; parity ^= 1; }
             }
-            __syncwarp();
-        }
 #ifdef NMSPMM_TF32_PROFILE
-        if (lane == 0) { TF_OUT(0, p_empty); TF_OUT(1, clock64() - p_start); }
+            TF_OUT(0, p_empty); TF_OUT(1, clock64() - p_start);
 #endif
+            if (!ok) atomicMax(g.status, kDevTimeoutEmpty);
+        }
+        __syncwarp();
     } else if (warp == 1) {
         // ------------------------------------------------------------------ gather issuer
         constexpr bool COLS = (Cfg::SRC == kTf32Cols);
         const uint32_t idesc_gather = Cfg::SRC == kTf32Rows16 ? umma_idesc_16(128, DIRECT ? 32 : Cfg::N1, a_form == kDtypeBF16)
                                                               : umma_idesc_tf32(128, DIRECT ? 32 : Cfg::N1, COLS);
         const uint32_t idesc_direct = umma_idesc_tf32(128, live_vecs * 32, COLS);
-        // A's descriptor for the ks-th 32 bytes of K (col-major: the ks-th eight rows of k)
-        auto a_desc = [](uint32_t st, int ks) {
-            if constexpr (Cfg::SRC == kTf32Cols) return umma_desc_mn_tf32(st + ks * 1024, KW * 128, 512);
-            else if constexpr (Cfg::SRC == kTf32Rows32) return umma_desc_k_major<128>(st + (ks >> 2) * 16384 + (ks & 3) * 32);
-            else return umma_desc_k_major<KW * 2>(st + ks * 32);
-        };
-        bool alive = true;
-        TF_DECL(m_full = 0, m_free = 0, m_issue = 0);
-        TF_T(m_start);
-        for (int t = 0; t < n_win; ++t) {
-            const int s = t % STAGES;
-            TF_T(t0);
-            bool ok = mbar_wait_bounded(bar_full + s * 8, (t / STAGES) & 1, abort_word);
-            TF_ADD(m_full, t0);
-            TF_T(t1);
-            // the result buffer is free once the products of step t - NBUF are done, which is when that
-            // step's stage is (the stage's next phase ends with step t - NBUF + STAGES, not before this one)
-            if (!DIRECT && t >= NBUF)
-                ok = ok && mbar_wait_bounded(bar_empty + ((t - NBUF) % STAGES) * 8, ((t - NBUF) / STAGES) & 1, abort_word);
-            TF_ADD(m_free, t1);
-            if (!__all_sync(0xffffffffu, ok)) { alive = false; break; }
-            TF_T(t2);
-            tc_fence_after_sync();
-            if (elect_one()) {
-                const uint32_t st = ring + s * Cfg::STAGE_BYTES;
+        // Low words of the operands' descriptors, 16-byte units: the next 32 bytes of K and the next stage are additions.
+        const uint64_t a0 = COLS ? umma_desc_mn_tf32(ring, KW * 128, 512)
+                                 : (Cfg::SRC == kTf32Rows32 ? umma_desc_k_major<128>(ring) : umma_desc_k_major<(KW * Cfg::EB < 128 ? 64 : 128)>(ring));
+        const uint64_t p0 = Cfg::SRC == kTf32Rows16 ? umma_desc_k_major<(KW * Cfg::EB < 128 ? 64 : 128)>(ring + Cfg::A_BYTES + Cfg::B_BYTES)
+                                                    : umma_desc_mn_tf32(ring + Cfg::A_BYTES + Cfg::B_BYTES, KW * 128, 512);
+        const uint64_t b0 = umma_desc_mn_tf32(ring + Cfg::A_BYTES, WSP * 128, 512);      // (unpruned only)
+        constexpr uint32_t P_STEP = (Cfg::SRC == kTf32Rows16) ? 2 : 64;
+        auto a_step = [](int ks) { return Cfg::SRC == kTf32Cols ? ks * 64 : (Cfg::SRC == kTf32Rows32 ? (ks >> 2) * 1024 + (ks & 3) * 2 : ks * 2); };
+        if (elect_one()) {
+            bool ok = true;
+            uint32_t at = 0, full = bar_full, parity = 0;              // stage of step t, as a descriptor offset; its barrier
+            uint32_t empty = bar_empty, empty_parity = 0;              // of step t - NBUF
+            int buf = 0;
+            TF_DECL(m_full = 0, m_free = 0, m_issue = 0);
+            TF_T(m_start);
+            for (int t = 0; t < n_win; ++t) {
+                TF_T(t0);
+                ok = mbar_spin_bounded(full, parity, abort_word);
+                TF_ADD(m_full, t0);
+                TF_T(t1);
+                // the result buffer is free once the products of step t - NBUF are done, which is when that
+                // step's stage is (the stage's next phase ends with step t - NBUF + STAGES, not before this one)
+                if (!DIRECT && t >= NBUF) {
+                    ok = ok && mbar_spin_bounded(empty, empty_parity, abort_word);
+                    empty += 8;
+                    if (empty == bar_empty + STAGES * 8) { empty = bar_empty; empty_parity ^= 1; }
+                }
+                TF_ADD(m_free, t1);
+                if (!ok) break;
+                TF_T(t2);
+                tc_fence_after_sync();
                 if (DIRECT) {
 #pragma unroll
                     for (int ks = 0; ks < Cfg::NKS; ++ks)
-                        umma_tf32_ss(tmem_addr(tmem, 0, 0), a_desc(st, ks),
-                                     umma_desc_mn_tf32(st + Cfg::A_BYTES + ks * 1024, WSP * 128, 512), idesc_direct,
+                        umma_tf32_ss(tmem_addr(tmem, 0, 0), umma_desc_plus(a0, at + a_step(ks)), umma_desc_plus(b0, at + ks * 64), idesc_direct,
                                      (t | ks) != 0);
-                    tc_commit(bar_empty + s * 8);
+                    tc_commit(full + (bar_empty - bar_full));
                 } else {
-                    const uint32_t gbuf = tmem_addr(tmem, 0, Cfg::ACOL0 + (t % NBUF) * Cfg::N1);
+                    const uint32_t gbuf = tmem_addr(tmem, 0, Cfg::ACOL0 + buf * Cfg::N1);
 #pragma unroll
                     for (int ks = 0; ks < Cfg::NKS; ++ks) {
-                        const uint32_t p = st + Cfg::A_BYTES + Cfg::B_BYTES;
                         if constexpr (Cfg::SRC == kTf32Rows16)
-                            umma_f16_ss(gbuf, a_desc(st, ks), umma_desc_k_major<KW * 2>(p + ks * 32), idesc_gather, ks != 0);
+                            umma_f16_ss(gbuf, umma_desc_plus(a0, at + a_step(ks)), umma_desc_plus(p0, at + ks * P_STEP), idesc_gather, ks != 0);
                         else
-                            umma_tf32_ss(gbuf, a_desc(st, ks), umma_desc_mn_tf32(p + ks * 1024, KW * 128, 512), idesc_gather, ks != 0);
+                            umma_tf32_ss(gbuf, umma_desc_plus(a0, at + a_step(ks)), umma_desc_plus(p0, at + ks * P_STEP), idesc_gather, ks != 0);
                     }
-                    tc_commit(bar_gdone + (t % NBUF) * 8);
+                    tc_commit(bar_gdone + buf * 8);
+                    if (++buf == NBUF) buf = 0;
                 }
+                at += Cfg::STAGE_BYTES / 16;
+                full += 8;
+                if (full == bar_full + STAGES * 8) { full = bar_full; at = 0; parity ^= 1; }
+                TF_ADD(m_issue, t2);
             }
-            __syncwarp();
-            TF_ADD(m_issue, t2);
-        }
 #ifdef NMSPMM_TF32_PROFILE
-        if (lane == 0) {
             TF_OUT(2, m_full); TF_OUT(3, m_free); TF_OUT(4, m_issue); TF_OUT(5, clock64() - m_start); TF_OUT(8, 1); TF_OUT(9, n_win);
-        }
 #endif
-        if (!alive && lane == 0) atomicMax(g.status, kDevTimeoutMma);
-        if (DIRECT) {
-            if (elect_one()) tc_commit(bar_acc);           // every MMA has completed: accumulators are final
-            __syncwarp();
+            if (!ok) atomicMax(g.status, kDevTimeoutMma);
+            if (DIRECT) tc_commit(bar_acc);                // every MMA has completed: accumulators are final
         }
+        __syncwarp();
     } else if (warp < FIRST_BUILDER) {
         // ------------------------------------------------------------------ product issuers
-        if (!DIRECT) {
+        if (!DIRECT && elect_one()) {
             constexpr uint32_t idesc_product = umma_idesc_tf32(128, VL, false);
             constexpr int VPI = QV / Cfg::PRODUCT_WARPS;   // vectors per issuer
-            const int v_begin = (warp - 2) * VPI, v_end = min(v_begin + VPI, live_vecs / BPV);
-            bool alive = true;
+            const int v_begin = (warp - 2) * VPI, v_live = min(VPI, live_vecs / BPV - v_begin);
+            const uint64_t b0 = umma_desc_mn_tf32(ring + Cfg::A_BYTES + v_begin * (BPV * WSP * 128), WSP * 128, 512);
+            bool ok = true;
+            uint32_t at = 0, empty = bar_empty;            // stage of step u, as a descriptor offset; its barrier
+            uint32_t done_parity = 0;
+            int buf = 0;
             TF_DECL(c_gdone = 0, c_issue = 0);
             TF_T(c_start);
             for (int u = 0; u < n_win; ++u) {
-                const int s = u % STAGES, b = u % NBUF;
                 TF_T(t0);
-                // the step's B rows have landed (their barrier completed before the gather was issued)
-                bool ok = mbar_wait_bounded(bar_full + s * 8, (u / STAGES) & 1, abort_word);
-                ok = ok && mbar_spin_bounded(bar_gdone + b * 8, (u / NBUF) & 1, abort_word);
+                // (the step's B rows have landed: the gather was issued after their barrier had completed)
+                ok = mbar_spin_bounded(bar_gdone + buf * 8, done_parity, abort_word);
                 TF_ADD(c_gdone, t0);
-                if (!__all_sync(0xffffffffu, ok)) { alive = false; break; }
+                if (!ok) break;
                 TF_T(t1);
                 tc_fence_after_sync();
-                if (elect_one()) {
-                    if (v_begin < v_end) {
-                        const uint32_t bs = ring + s * Cfg::STAGE_BYTES + Cfg::A_BYTES;
-                        const uint32_t gbuf = tmem_addr(tmem, 0, Cfg::ACOL0 + b * Cfg::N1);
-                        for (int v = v_begin; v < v_end; ++v) {
+                if (v_live > 0) {
+                    const uint32_t gbuf = tmem_addr(tmem, 0, Cfg::ACOL0 + buf * Cfg::N1 + v_begin * WSP), acc = tmem_addr(tmem, 0, v_begin * VL);
+#pragma unroll
+                    for (int v = 0; v < VPI; ++v) {
+                        if (v < v_live) {
 #pragma unroll
                             for (int gi = 0; gi < Cfg::G; ++gi)
-                                umma_tf32_ts(tmem_addr(tmem, 0, v * VL), gbuf + v * WSP + gi * 8,
-                                             umma_desc_mn_tf32(bs + v * (BPV * WSP * 128) + gi * 1024, WSP * 128, 512),
+                                umma_tf32_ts(acc + v * VL, gbuf + v * WSP + gi * 8, umma_desc_plus(b0, at + v * (BPV * WSP * 8) + gi * 64),
                                              idesc_product, (u | gi) != 0);
                         }
-                        tc_commit(bar_empty + s * 8);      // this half of the step's products has read the stage and the gather result
-                    } else {
-                        mbar_arrive(bar_empty + s * 8);    // no vector of this half exists; the gather itself has completed
                     }
+                    tc_commit(empty);                      // this half of the step's products has read the stage and the gather result
+                } else {
+                    mbar_arrive(empty);                    // no vector of this half exists; the gather itself has completed
                 }
-                __syncwarp();
+                if (++buf == NBUF) { buf = 0; done_parity ^= 1; }
+                at += Cfg::STAGE_BYTES / 16;
+                empty += 8;
+                if (empty == bar_empty + STAGES * 8) { empty = bar_empty; at = 0; }
                 TF_ADD(c_issue, t1);
             }
 #ifdef NMSPMM_TF32_PROFILE
-            if (lane == 0 && warp == 2) { TF_OUT(6, c_gdone); TF_OUT(7, c_issue); TF_OUT(15, clock64() - c_start); }
+            if (warp == 2) { TF_OUT(6, c_gdone); TF_OUT(7, c_issue); TF_OUT(15, clock64() - c_start); }
 #endif
-            if (!alive && lane == 0) atomicMax(g.status, kDevTimeoutMma);
-            if (elect_one()) {
-                if (v_begin < v_end) tc_commit(bar_acc); else mbar_arrive(bar_acc);
-            }
-            __syncwarp();
+            if (!ok) atomicMax(g.status, kDevTimeoutMma);
+            if (v_live > 0) tc_commit(bar_acc); else mbar_arrive(bar_acc);
         }
+        __syncwarp();
     } else {
         // ------------------------------------------------------------------ one-hot builders
         const int b = tid - FIRST_BUILDER * 32;
@@ -397,56 +414,59 @@ nm_gemm_tf32_kernel(const GemmArgs g, const __grid_constant__ CUtensorMap map_a,
                               (static_cast<size_t>(j) << qs_shift);
             const int n_merged = (KW == 64) ? g.sched.n_win : (g.sched.n_win >> 1);
             const int* ciptr = (MODE == kModeHigh) ? g.cinfo + static_cast<size_t>(q >> qs_shift) * n_merged * 64 : nullptr;
-            const uint32_t my_idx = idx_ring + b * 4, my_k = k_ring + b * 4, my_prev = prev_k + e * 4;
-            TF_DECL(b_cp = 0, b_empty = 0);
-            TF_T(b_start);
-            for (int turn = -2 * PD, i = group - 2 * PD * GROUPS; group < GROUPS && i < n_win; ++turn, i += GROUPS) {
-                TF_T(t0);
-                cp_async_wait<PD - 1>();                   // the copies issued PD turns ago and earlier have landed
-                TF_ADD(b_cp, t0);
-                int k = 0;
-                if (has && turn >= 0) {
-                    k = lds_s32((MODE == kModeHigh ? my_k : my_idx) + (turn & (RING - 1)) * SLOT);
+            const uint32_t my_prev = prev_k + e;
+            TF_DECL(b_empty = 0);
+            // Index loads run ahead in registers: idx[] two to four turns (through column_info on the 64-k
+            // format: k[] two turns behind them), each turn's value in a register of its own so that
+            // nothing waits for a load before its turn.
+            auto load_index = [&](int i) { return (has && i < n_win) ? __ldg(dptr + ((static_cast<size_t>(win0 + i) * WS) << qs_shift)) : 0; };
+            auto load_k = [&](int i, int rank) {
+                if constexpr (MODE != kModeHigh) return rank;
+                const int m = (KW == 64) ? (win0 + i) : ((win0 + i) >> 1);
+                return (has && i < n_win) ? __ldg(ciptr + static_cast<size_t>(m) * 64 + rank) : 0;
+            };
+            int idx[PD], kq[PD];
+#pragma unroll
+            for (int d = 0; d < PD; ++d) kq[d] = load_index(group + d * GROUPS);
+#pragma unroll
+            for (int d = 0; d < PD; ++d) idx[d] = load_index(group + (PD + d) * GROUPS);
+#pragma unroll
+            for (int d = 0; d < PD; ++d) kq[d] = load_k(group + d * GROUPS, kq[d]);
+            for (int i0 = group; group < GROUPS && alive && i0 < n_win; i0 += PD * GROUPS) {
+#pragma unroll
+                for (int d = 0; d < PD; ++d) {
+                    const int i = i0 + d * GROUPS;
+                    if (i >= n_win || !alive) break;
+                    int k = kq[d];
+                    kq[d] = load_k(i + PD * GROUPS, idx[d]);
+                    idx[d] = load_index(i + 2 * PD * GROUPS);
                     if (MODE == kModeHigh && KW == 32) k -= ((win0 + i) & 1) * 32;
-                }
-                if (has) {
-                    const int i2 = i + 2 * PD * GROUPS, i1 = i + PD * GROUPS;
-                    if (i2 < n_win)
-                        cp_async_4(my_idx + ((turn + 2 * PD) & (RING - 1)) * SLOT, dptr + ((static_cast<size_t>(win0 + i2) * WS) << qs_shift));
-                    if (MODE == kModeHigh && turn >= -PD && i1 < n_win) {
-                        const int rank = lds_s32(my_idx + ((turn + PD) & (RING - 1)) * SLOT);
-                        const int m = (KW == 64) ? (win0 + i1) : ((win0 + i1) >> 1);
-                        cp_async_4(my_k + ((turn + PD) & (RING - 1)) * SLOT, ciptr + static_cast<size_t>(m) * 64 + rank);
+                    const int s = i % STAGES;
+                    if (i >= STAGES) {
+                        TF_T(t1);
+                        const bool ok = mbar_wait_bounded(bar_empty + s * 8, ((i / STAGES) - 1) & 1, abort_word);
+                        TF_ADD(b_empty, t1);
+                        if (!__all_sync(0xffffffffu, ok)) { alive = false; break; }
                     }
-                }
-                cp_async_commit();
-                if (turn < 0) continue;
-                const int s = i % STAGES;
-                if (i >= STAGES) {
-                    TF_T(t1);
-                    const bool ok = mbar_wait_bounded(bar_empty + s * 8, ((i / STAGES) - 1) & 1, abort_word);
-                    TF_ADD(b_empty, t1);
-                    if (!__all_sync(0xffffffffu, ok)) { alive = false; break; }
-                }
-                if (has) {
-                    const uint32_t ps = ring + s * Cfg::STAGE_BYTES + Cfg::A_BYTES + Cfg::B_BYTES;
-                    const int old = lds_s32(my_prev + s * 512);
-                    if constexpr (Cfg::SRC == kTf32Rows16) {
-                        if (old >= 0) sts_u16(ps + p16_offset<KW>(e, old), 0u);
-                        sts_u16(ps + p16_offset<KW>(e, k), a_form == kDtypeBF16 ? 0x3F80u : 0x3C00u);      // 1.0
-                    } else {
-                        if (old >= 0) sts_f32(ps + p_offset<KW>(e, old), 0.f);
-                        sts_f32(ps + p_offset<KW>(e, k), 1.f);
+                    if (has) {
+                        const uint32_t ps = ring + s * Cfg::STAGE_BYTES + Cfg::A_BYTES + Cfg::B_BYTES;
+                        const int old = lds_s8(my_prev + s * 128);
+                        if constexpr (Cfg::SRC == kTf32Rows16) {
+                            if (old >= 0) sts_u16(ps + p16_offset<KW>(e, old), 0u);
+                            sts_u16(ps + p16_offset<KW>(e, k), a_form == kDtypeBF16 ? 0x3F80u : 0x3C00u);      // 1.0
+                        } else {
+                            if (old >= 0) sts_f32(ps + p_offset<KW>(e, old), 0.f);
+                            sts_f32(ps + p_offset<KW>(e, k), 1.f);
+                        }
+                        sts_s8(my_prev + s * 128, k);
                     }
-                    sts_s32(my_prev + s * 512, k);
+                    fence_proxy_async();                   // the tensor core reads P through the asynchronous proxy
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(bar_full + s * 8);
                 }
-                fence_proxy_async();                       // the tensor core reads P through the asynchronous proxy
-                __syncwarp();
-                if (lane == 0) mbar_arrive(bar_full + s * 8);
             }
-            cp_async_wait<0>();
 #ifdef NMSPMM_TF32_PROFILE
-            (void)b_cp; (void)b_empty; (void)b_start;
+            (void)b_empty;
 #endif
         }
         // ------------------------------------------------------------------ epilogue

@@ -92,6 +92,12 @@ __device__ __forceinline__ uint64_t umma_desc_k_major(uint32_t smem_addr)
     return d;
 }
 
+// The operand that starts `units` of 16 bytes further on (shared memory ends below the address field's 2^14 units).
+__device__ __forceinline__ uint64_t umma_desc_plus(uint64_t desc, uint32_t units)
+{
+    return (desc & 0xFFFFFFFF00000000ull) | (static_cast<uint32_t>(desc) + units);
+}
+
 // Instruction descriptor of kind::f16: FP32 accumulate, A and B both half (or both bfloat16), both K-major.
 __host__ __device__ constexpr uint32_t umma_idesc_16(int m, int n, bool bf16)
 {
