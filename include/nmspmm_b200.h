@@ -107,7 +107,7 @@ int nmspmm_preprocess_high_host(int* column_info_host, int pruning_M, int prunin
 /* ------------------------------------------------------------------ the multiply */
 
 /* CTA tiles compiled into the library (rows x columns of C).  The exact path has all of 1..7, 10 and 11;
- * the TF32 path 128 x 128 and 128 x 256, the latter in two forms: the tensor core gathers the
+ * the TF32 path 128 x 128, 128 x 192 and 128 x 256, the last in two forms: the tensor core gathers the
  * kept rows of A (every format and ratio), or B is expanded with zeros and the A window is
  * multiplied whole (32-k formats with 16, 12 or 8 kept rows).  NMSPMM_TILE_128x256 leaves the
  * form to the library.  On the TF32 path ids 4 / 3 / 2 are streaming tiles of 16 / 32 / 64 rows on
@@ -125,7 +125,8 @@ enum nmspmm_tile_id {
     NMSPMM_TILE_128x256_GATHER = 8,   /* TF32 path only */
     NMSPMM_TILE_128x256_EXPAND = 9,   /* TF32 path only */
     NMSPMM_TILE_256x128 = 10,         /* exact path only */
-    NMSPMM_TILE_64x512 = 11           /* exact path only */
+    NMSPMM_TILE_64x512 = 11,          /* exact path only */
+    NMSPMM_TILE_128x192 = 12          /* TF32 path only, 32-wide vectors, pruned ratios */
 };
 
 typedef struct nmspmm_gemm_desc {
@@ -156,7 +157,7 @@ typedef struct nmspmm_gemm_desc {
 size_t nmspmm_gemm_workspace_bytes(const nmspmm_gemm_desc* desc);
 /* Scratch with which a call runs its fastest form.  On the exact path, where tile and split_k are left to
  * the library and no tuned entry names them, a call may run one of the wide tiles (ids 5, 10 and 11: one CTA per SM)
- * instead of the tile that nmspmm_gemm_plan names, wherever the scratch it is handed holds that tile's
+ * instead of the tile that nmspmm_gemm_plan names (on the TF32 path 128 x 192 instead of 128 x 256), wherever the scratch it is handed holds that tile's
  * pieces; with nmspmm_gemm_workspace_bytes alone (never more than this) it runs the named one.  The wide
  * tiles write no counters. */
 size_t nmspmm_gemm_call_workspace_bytes(const nmspmm_gemm_desc* desc);

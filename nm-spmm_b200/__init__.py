@@ -28,7 +28,7 @@ LIB_PATH = os.environ.get("NMSPMM_LIBRARY") or os.path.join(_HERE, "libnmspmm_b2
 OK, INVALID_ARGUMENT, UNSUPPORTED, CUDA_ERROR, WORKSPACE_TOO_SMALL, DEVICE_TIMEOUT = range(6)
 PATH_FP32, PATH_TF32 = 0, 1
 (TILE_AUTO, TILE_128x128, TILE_64x128, TILE_32x128, TILE_16x128, TILE_128x256, TILE_16x256, TILE_32x256,
- TILE_128x256_GATHER, TILE_128x256_EXPAND, TILE_256x128, TILE_64x512) = range(12)   # nmspmm_tile_id
+ TILE_128x256_GATHER, TILE_128x256_EXPAND, TILE_256x128, TILE_64x512, TILE_128x192) = range(13)   # nmspmm_tile_id
 FORMAT_LOW, FORMAT_HIGH = 0, 1
 DTYPE_F32, DTYPE_F16, DTYPE_BF16 = 0, 1, 2               # nmspmm_dtype
 VEC_LEN = 32

@@ -318,7 +318,7 @@ static_assert(NMSPMM_TILE_128x128 == kTile128x128 && NMSPMM_TILE_64x128 == kTile
                   NMSPMM_TILE_16x128 == kTile16x128 && NMSPMM_TILE_128x256 == kTile128x256 && NMSPMM_TILE_16x256 == kTile16x256 &&
                   NMSPMM_TILE_32x256 == kTile32x256 && NMSPMM_TILE_128x256_GATHER == kTile128x256Gather &&
                   NMSPMM_TILE_128x256_EXPAND == kTile128x256Expand && NMSPMM_TILE_256x128 == kTile256x128 &&
-                  NMSPMM_TILE_64x512 == kTile64x512 && NMSPMM_TILE_64x512 + 1 == kTileCount,
+                  NMSPMM_TILE_64x512 == kTile64x512 && NMSPMM_TILE_128x192 == kTile128x192 && NMSPMM_TILE_128x192 + 1 == kTileCount,
               "the public tile ids are the library's");
 
 // Whether the TF32 path should expand B rather than gather A when the caller leaves the choice
@@ -440,6 +440,7 @@ static int make_plan(const nmspmm_gemm_desc* d_in, int sms, Plan* p, bool any_ro
         int want_ns = d->N >= 256 ? 256 : 128;
         if (d->tile == kTile128x256 || d->tile == kTile128x256Gather || d->tile == kTile128x256Expand) want_ns = 256;
         if (d->tile == kTile128x128) want_ns = 128;
+        if (d->tile == kTile128x192) want_ns = 192;
         // Two forms on tile 128 x 256 (gemm_tf32.cu, gemm_tf32_expand.cu).  With B expanded the
         // tensor core issues 32 / n_keep times the useful work at its fastest instruction
         // shape; with A gathered, twice the useful work in small instructions.
@@ -452,7 +453,7 @@ static int make_plan(const nmspmm_gemm_desc* d_in, int sms, Plan* p, bool any_ro
             if (!p->tv && d->tile == kTile128x256Expand) return NMSPMM_UNSUPPORTED;
         }
         // 64-wide vectors: the variants that gather once per 64 columns exist for tile 128 x 256
-        if (d->vec_len == 64 && d->tile != kTile128x128 && !p->tv)
+        if (d->vec_len == 64 && d->tile != kTile128x128 && d->tile != kTile128x192 && !p->tv)
             for (int i = 0; i < kTf32GatherVariantCount; ++i)
                 if (kTf32GatherVariants[i].n_keep == d->n_keep && kTf32GatherVariants[i].mode == mode && kTf32GatherVariants[i].vec_len == 64) {
                     p->tv = &kTf32GatherVariants[i];
@@ -478,7 +479,7 @@ static int make_plan(const nmspmm_gemm_desc* d_in, int sms, Plan* p, bool any_ro
         // tiles of a small problem) are cut into as many slices, of at least four windows,
         // as the free CTA slots allow -- with one CTA per SM a last wave that is 46 % full
         // (512 tiles on 148 SMs) otherwise costs as much as a full one.
-        const int resident = sms * (want_ns == 256 ? 1 : 2);
+        const int resident = sms * (want_ns == 128 ? 2 : 1);
         long long s = d->split_k, whole = 0;
         if (s <= 0) {
             whole = nt / resident * resident;
@@ -603,19 +604,36 @@ static int make_plan(const nmspmm_gemm_desc* d_in, int sms, Plan* p, bool any_ro
 
 static size_t scratch_bytes(const Plan& p) { return p.counters_bytes + p.partial_bytes; }
 
-// The plan a call runs that has `workspace_bytes` of scratch: make_plan's, or on the exact path, where the
-// description leaves tile and split to the library and no tuned entry names them, a wide tile's
-// (pick_wide_tile) if its scratch fits.
+// About how long a tensor-core plan of 256- or 192-column tiles (one CTA per SM, 32-wide vectors) takes, in
+// microseconds.  A step's time hardly depends on the width where the issuing threads bound it (8:32: 220 ns either
+// way) and follows it where two gather results at 256 columns against three at 192 do (16:32, 12:32: 423 / 320;
+// 4:32, a merged window: 418 / 365); a tile costs 6 us beside its steps (2048 x 9472 x 4096 and 4096 cubed, FP32).
+static double tf32_plan_us(const Plan& p, int sms)
+{
+    const bool narrow = p.tv->ns == 192;
+    const double step = (p.tv->n_keep == 8 ? 220 : (p.tv->n_keep == 4 ? (narrow ? 365 : 418) : (narrow ? 320 : 423))) * 1e-3;
+    double us = (p.n_dp + sms - 1) / sms * (p.n_win * step + (narrow ? 5.0 : 6.0));
+    if (p.grid > p.n_dp) us += (p.n_win + p.split_k - 1) / p.split_k * step + 9.0;       // the slices of the rest, and their sum
+    return us;
+}
+
+// The plan a call runs that has `workspace_bytes` of scratch: make_plan's, or where the description leaves tile and
+// split to the library and no tuned entry names them another's if its scratch fits: on the exact path a
+// wide tile's (pick_wide_tile); on the tensor cores that of 192-column tiles, where they leave fewer SMs
+// idle (256 x 11008 x 4096, bfloat16: 116 tiles instead of 86, 16:32 52.1 -> 35.1 us, 8:32 29.7 -> 27.8).
 static int plan_call(const nmspmm_gemm_desc* d, int sms, size_t workspace_bytes, Plan* p, bool any_rows = false)
 {
     const int rc = make_plan(d, sms, p, any_rows);
-    if (rc != NMSPMM_OK || !p->v || d->tile != 0 || d->split_k != 0) return rc;
+    if (rc != NMSPMM_OK || d->tile != 0 || d->split_k != 0) return rc;
+    const bool tensor = p->tv && p->tv->form == 0 && p->tv->ns == 256 && p->tv->vec_len == 32 && p->tv->n_keep != 32;
+    if (!p->v && !tensor) return rc;
     int tuned_tile, tuned_split;
     if (tuned_lookup(d, &tuned_tile, &tuned_split)) return rc;
     nmspmm_gemm_desc w = *d;
-    w.tile = pick_wide_tile(d, p->v->mode, sms);
+    w.tile = tensor ? kTile128x192 : pick_wide_tile(d, p->v->mode, sms);
     Plan wp;
-    if (w.tile != kTileAuto && make_plan(&w, sms, &wp, any_rows) == NMSPMM_OK && scratch_bytes(wp) <= workspace_bytes) *p = wp;
+    if (w.tile == kTileAuto || make_plan(&w, sms, &wp, any_rows) != NMSPMM_OK || scratch_bytes(wp) > workspace_bytes) return rc;
+    if (!tensor || tf32_plan_us(wp, sms) < 0.98 * tf32_plan_us(*p, sms)) *p = wp;
     return rc;
 }
 
@@ -855,7 +873,7 @@ static void describe_plan(const Plan& p, nmspmm_gemm_plan_info* out)
 {
     out->tile = p.v ? p.v->tile_id
                     : (p.tv->form == 2 ? (p.tv->ms == 16 ? kTile16x128 : (p.tv->ms == 32 ? kTile32x128 : kTile64x128))
-                                       : (p.tv->ns == 128 ? kTile128x128 : (p.tv->form == 1 ? kTile128x256Expand : kTile128x256)));
+                                       : (p.tv->ns == 128 ? kTile128x128 : (p.tv->ns == 192 ? kTile128x192 : (p.tv->form == 1 ? kTile128x256Expand : kTile128x256))));
     out->tile_m = p.v ? p.v->ms : (p.tv->ms ? p.tv->ms : 128);
     out->tile_n = p.v ? p.v->ns : p.tv->ns;
     out->split_k = p.split_k > 0 ? p.split_k

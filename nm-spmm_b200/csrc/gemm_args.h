@@ -28,6 +28,7 @@ enum nmspmm_tile {
     kTile128x256Expand = 9,   // TF32 path only: tile 128 x 256, the form that expands B with zeros (32-k formats, 16 / 12 / 8 kept)
     kTile256x128 = 10,    // exact path only
     kTile64x512 = 11,     // exact path only
+    kTile128x192 = 12,    // TF32 path only, vectors of 32 columns, pruned ratios
     kTileCount
 };
 

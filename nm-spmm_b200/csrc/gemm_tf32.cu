@@ -1,6 +1,6 @@
 // TF32 tensor-core path of the vector-wise N:M sparse GEMM (tcgen05, accumulators in TMEM).
 //
-// One CTA computes a 128 x NS tile of C (QT = NS / 32 vectors of 32 columns) over its k steps.
+// One CTA computes a 128 x NS tile of C (QT = NS / 32 vectors of 32 columns; NS = 256, 192 or 128) over its k steps.
 // A step is one 32-k window (one 64-k merged window for 4:32) with WS kept rows of B.  The
 // contraction is per vector, C[128 x 32] += A_gathered[128 x WS] . B[WS x 32], and A_gathered
 // (the WS columns of the step's A window that the vector's index list names) differs for
@@ -21,11 +21,11 @@
 //   warp 0      TMA producer: per step one tiled copy of the A window and one of the B rows,
 //               both as blocks of 32 floats along m / n with 32-byte chunks swizzled within
 //               128-byte rows (the one legal layout of an MN-major TF32 operand).
-//   warp 1      one elected thread issues the gathers (tcgen05.mma kind::tf32, A and P from
+//   warp 1      (and 2 where a step is short) one elected thread issues the gathers (tcgen05.mma kind::tf32, A and P from
 //               shared memory, M128 N=QT*WS, KW/8 instructions per step) into a ring of
 //               result buffers in TMEM, each followed by a tcgen05.commit to the buffer's
 //               mbarrier.
-//   warps 2-3   one elected thread each issues the products of half the tile's vectors
+//   next two    one elected thread each issues the products of half the tile's vectors
 //               (A = G from TMEM, B from shared memory, M128 N32 K8 each) once the gather's
 //               mbarrier has completed, and commits to the mbarrier that frees the stage and
 //               the result buffer.  Measured alone (instruction chains, cycles): a product takes the pipe
@@ -35,7 +35,7 @@
 //               descriptors by addition: with a warp-wide wait, a vote and descriptors built anew
 //               per instruction a step of 8:32 took 600 cycles on the issuers' side alone (2048 x 9472 x 4096, 8:32,
 //               186 -> 138 us; 256 x 11008 x 4096, bfloat16, 42 -> 31.5).
-//   warps 4-11  (4-7 on the 128-column tile, at 16:32 and 12:32 with 32-wide vectors, and at 32:32) one
+//   the others  (eight; four on the 128-column tile, at 16:32 and 12:32 with 32-wide vectors, and at 32:32) one
 //               thread per (vector, kept row) and turn: loads its index two to four turns ahead
 //               into registers (through column_info on the 64-k format), keeps P's one-hot
 //               entry current, and after the last step reads the accumulators (tcgen05.ld),
@@ -95,7 +95,7 @@ template <int NKEEP, int KW_, int MODE, int QT_, int VL_ = 32, int SRC_ = kTf32C
 struct Tf32Cfg {
     static constexpr int SRC = SRC_;
     static constexpr int EB = (SRC == kTf32Rows16) ? 2 : 4;  // bytes of a value of A and of P
-    static constexpr int MS = 128, QT = QT_, NS = QT * 32;   // QT = 8: one CTA per SM; QT = 4: two
+    static constexpr int MS = 128, QT = QT_, NS = QT * 32;   // QT = 8 and 6: one CTA per SM; QT = 4: two
     static constexpr int KW = KW_;                           // k per step
     static constexpr int WS = NKEEP * (KW / 32);             // rows of B per step
     static constexpr int WSP = (WS + 7) / 8 * 8;             // gathered columns per vector (K of the products)
@@ -106,15 +106,16 @@ struct Tf32Cfg {
     static constexpr int QV = NS / VL;                       // vectors per tile
     static constexpr int N1 = QV * WSP;                      // gathered columns per step
     static_assert(VL == 32 || (VL == 64 && NKEEP != 32), "vectors of 32 or 64 columns");
-    static_assert(DIRECT || (N1 <= 128 && N1 % 32 == 0), "one builder thread per gathered column, whole warps");
+    static constexpr int NT = (N1 + 31) / 32 * 32;           // threads that keep them, whole warps; columns of P's 32-bit layout
+    static_assert(DIRECT || (N1 <= 128 && N1 % 16 == 0), "one builder thread per gathered column");
     static_assert(MODE == kModeHigh || KW == 32, "only the 64-k format has merged windows");
     static_assert(!(DIRECT && SRC == kTf32Rows16), "the direct product multiplies A by FP32 rows of B");
     static constexpr int A_BYTES = 128 * KW * EB;            // col-major: [4 blocks of 32 rows of the tile][KW][32]; rows: [128][<= 128 bytes], blocks of 32 k if FP32
     static constexpr int B_BYTES = QT * WSP * 128;           // [QT][WSP][32]
-    static constexpr int P_BYTES = DIRECT ? 0 : N1 * KW * EB;  // [N1 / 32][KW][32]; 16 bits: K-major, [N1][KW]
+    static constexpr int P_BYTES = DIRECT ? 0 : (EB == 2 ? N1 : NT) * KW * EB;      // [NT / 32][KW][32]; 16 bits: K-major, [N1][KW]
     static constexpr int STAGE_BYTES = A_BYTES + B_BYTES + P_BYTES;
     static_assert(A_BYTES % 1024 == 0 && B_BYTES % 1024 == 0 && P_BYTES % 1024 == 0, "swizzle atoms stay aligned");
-    static constexpr int CTAS_PER_SM = (QT == 8) ? 1 : 2;
+    static constexpr int CTAS_PER_SM = (QT > 4) ? 1 : 2;
     static constexpr int TMEM_COLS = 512 / CTAS_PER_SM;      // each resident CTA allocates its share
     static constexpr int PD = 2;                             // index prefetch distance, in turns, per look-up
     // One thread keeps one gathered column; the builder warps form GROUPS groups of N1 threads that take
@@ -123,10 +124,15 @@ struct Tf32Cfg {
     // not the tensor pipe, was part of what an 8:32 step waited for: 4096 x 4096 x 11008, 8:32, 417 -> 404 us,
     // with bfloat16 activations 444 -> 405; 4096 x 28672 x 2048 with 64-wide vectors 667 -> 636 and 632 -> 578.
     // (16:32 and 12:32 with 32-wide vectors fill one group of 128: a second one gained nothing there, their steps are longer.)
-    static constexpr int BUILDERS = (QT == 8 && N1 < 128) ? 256 : 128;
-    static constexpr int GROUP_WARPS = N1 / 32;
+    static constexpr int BUILDERS = (QT > 4 && N1 < 128) ? 256 : 128;
+    static constexpr int GROUP_WARPS = NT / 32;
     static constexpr int PRODUCT_WARPS = 2;
-    static constexpr int THREADS = (2 + PRODUCT_WARPS) * 32 + BUILDERS;
+    // A wait costs the thread that issues some 150 to 190 cycles even when it is over already, and a gather
+    // has two of them ahead of it: where a step takes less, two threads take turns with the gathers (2048 x 9472 x 4096,
+    // bfloat16, 8:32, 125 -> 116 us, 64-wide vectors 121 -> 107, and in FP32 131 -> 125; FP32 8:32 with 32-wide vectors and 4:32 lose 2 - 4 %
+    // on 256 columns: the second gather only crowds the products).
+    static constexpr int GATHER_WARPS = (!DIRECT && KW == 32 && N1 <= 96 && (EB == 2 || VL == 64 || QT == 6)) ? 2 : 1;
+    static constexpr int THREADS = (1 + GATHER_WARPS + PRODUCT_WARPS) * 32 + BUILDERS;
     // Every stage counts (2048 x 9472 x 4096, 8:32, six / eight stages: 145 / 138 us, 64-wide vectors 141 / 130; 4096 cubed, 4:32,
     // three / four: 142 / 121).
     static constexpr int MAX_STAGES = 8;
@@ -138,7 +144,7 @@ struct Tf32Cfg {
     static_assert(STAGES >= 2, "at least two stages");
     // A group that has built step i - GROUPS knows that step i - GROUPS - STAGES has been consumed; its
     // wait for the stage of step i tells one phase from the next only if step i - 2 STAGES has been.
-    static constexpr int GROUPS = DIRECT ? 1 : (BUILDERS / N1 < STAGES ? BUILDERS / N1 : STAGES);
+    static constexpr int GROUPS = DIRECT ? 1 : (BUILDERS / NT < STAGES ? BUILDERS / NT : STAGES);
     static_assert(GROUPS >= 1 && GROUPS <= STAGES, "see above");
     // Ring of gather results beside the accumulators.  A gather's result is complete (and its
     // commit arrives) some hundreds of cycles after issue, and the products that free the
@@ -192,7 +198,7 @@ nm_gemm_tf32_kernel(const GemmArgs g, const __grid_constant__ CUtensorMap map_a,
     constexpr int VL = Cfg::VL, QV = Cfg::QV, BPV = VL / 32;              // 32-column blocks per vector
     constexpr int STAGES = Cfg::STAGES, NBUF = Cfg::NBUF, PD = Cfg::PD;
     constexpr bool DIRECT = Cfg::DIRECT;
-    constexpr int FIRST_BUILDER = 2 + Cfg::PRODUCT_WARPS;
+    constexpr int GW = Cfg::GATHER_WARPS, FIRST_PRODUCT = 1 + GW, FIRST_BUILDER = FIRST_PRODUCT + Cfg::PRODUCT_WARPS;
 
     extern __shared__ unsigned char smem_raw[];
     const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u;          // swizzle atoms want 1024-byte alignment
@@ -283,8 +289,8 @@ nm_gemm_tf32_kernel(const GemmArgs g, const __grid_constant__ CUtensorMap map_a,
             if (!ok) atomicMax(g.status, kDevTimeoutEmpty);
         }
         __syncwarp();
-    } else if (warp == 1) {
-        // ------------------------------------------------------------------ gather issuer
+    } else if (warp < FIRST_PRODUCT) {
+        // ------------------------------------------------------------------ gather issuers: they take turns with the steps
         constexpr bool COLS = (Cfg::SRC == kTf32Cols);
         const uint32_t idesc_gather = Cfg::SRC == kTf32Rows16 ? umma_idesc_16(128, DIRECT ? 32 : Cfg::N1, a_form == kDtypeBF16)
                                                               : umma_idesc_tf32(128, DIRECT ? 32 : Cfg::N1, COLS);
@@ -299,12 +305,13 @@ nm_gemm_tf32_kernel(const GemmArgs g, const __grid_constant__ CUtensorMap map_a,
         auto a_step = [](int ks) { return Cfg::SRC == kTf32Cols ? ks * 64 : (Cfg::SRC == kTf32Rows32 ? (ks >> 2) * 1024 + (ks & 3) * 2 : ks * 2); };
         if (elect_one()) {
             bool ok = true;
-            uint32_t at = 0, full = bar_full, parity = 0;              // stage of step t, as a descriptor offset; its barrier
-            uint32_t empty = bar_empty, empty_parity = 0;              // of step t - NBUF
-            int buf = 0;
+            // (the stages of this thread's next step and of the step NBUF before it)
+            uint32_t full = bar_full + (warp - 1) * 8, at = (warp - 1) * (Cfg::STAGE_BYTES / 16), parity = 0;
+            uint32_t empty = bar_empty + (GW == 1 ? 0 : (warp - 1 + NBUF) % GW) * 8, empty_parity = 0;
+            int buf = (warp - 1) % NBUF;
             TF_DECL(m_full = 0, m_free = 0, m_issue = 0);
             TF_T(m_start);
-            for (int t = 0; t < n_win; ++t) {
+            for (int t = warp - 1; t < n_win; t += GW) {
                 TF_T(t0);
                 ok = mbar_spin_bounded(full, parity, abort_word);
                 TF_ADD(m_full, t0);
@@ -313,8 +320,10 @@ nm_gemm_tf32_kernel(const GemmArgs g, const __grid_constant__ CUtensorMap map_a,
                 // step's stage is (the stage's next phase ends with step t - NBUF + STAGES, not before this one)
                 if (!DIRECT && t >= NBUF) {
                     ok = ok && mbar_spin_bounded(empty, empty_parity, abort_word);
-                    empty += 8;
-                    if (empty == bar_empty + STAGES * 8) { empty = bar_empty; empty_parity ^= 1; }
+                    empty += GW * 8;
+                    if (GW == 1) {
+                        if (empty == bar_empty + STAGES * 8) { empty = bar_empty; empty_parity ^= 1; }
+                    } else if (empty >= bar_empty + STAGES * 8) { empty -= STAGES * 8; empty_parity ^= 1; }
                 }
                 TF_ADD(m_free, t1);
                 if (!ok) break;
@@ -336,15 +345,18 @@ nm_gemm_tf32_kernel(const GemmArgs g, const __grid_constant__ CUtensorMap map_a,
                             umma_tf32_ss(gbuf, umma_desc_plus(a0, at + a_step(ks)), umma_desc_plus(p0, at + ks * P_STEP), idesc_gather, ks != 0);
                     }
                     tc_commit(bar_gdone + buf * 8);
-                    if (++buf == NBUF) buf = 0;
+                    if (GW == 1) { if (++buf == NBUF) buf = 0; }
+                    else buf = (buf + GW) % NBUF;
                 }
-                at += Cfg::STAGE_BYTES / 16;
-                full += 8;
-                if (full == bar_full + STAGES * 8) { full = bar_full; at = 0; parity ^= 1; }
+                at += GW * (Cfg::STAGE_BYTES / 16);
+                full += GW * 8;
+                if (GW == 1) {
+                    if (full == bar_full + STAGES * 8) { full = bar_full; at = 0; parity ^= 1; }
+                } else if (full >= bar_full + STAGES * 8) { full -= STAGES * 8; at -= STAGES * (Cfg::STAGE_BYTES / 16); parity ^= 1; }
                 TF_ADD(m_issue, t2);
             }
 #ifdef NMSPMM_TF32_PROFILE
-            TF_OUT(2, m_full); TF_OUT(3, m_free); TF_OUT(4, m_issue); TF_OUT(5, clock64() - m_start); TF_OUT(8, 1); TF_OUT(9, n_win);
+            TF_OUT(2, m_full); TF_OUT(3, m_free); TF_OUT(4, m_issue); TF_OUT(5, clock64() - m_start); if (warp == 1) { TF_OUT(8, 1); TF_OUT(9, n_win); }
 #endif
             if (!ok) atomicMax(g.status, kDevTimeoutMma);
             if (DIRECT) tc_commit(bar_acc);                // every MMA has completed: accumulators are final
@@ -355,7 +367,7 @@ nm_gemm_tf32_kernel(const GemmArgs g, const __grid_constant__ CUtensorMap map_a,
         if (!DIRECT && elect_one()) {
             constexpr uint32_t idesc_product = umma_idesc_tf32(128, VL, false);
             constexpr int VPI = QV / Cfg::PRODUCT_WARPS;   // vectors per issuer
-            const int v_begin = (warp - 2) * VPI, v_live = min(VPI, live_vecs / BPV - v_begin);
+            const int v_begin = (warp - FIRST_PRODUCT) * VPI, v_live = min(VPI, live_vecs / BPV - v_begin);
             const uint64_t b0 = umma_desc_mn_tf32(ring + Cfg::A_BYTES + v_begin * (BPV * WSP * 128), WSP * 128, 512);
             bool ok = true;
             uint32_t at = 0, empty = bar_empty;            // stage of step u, as a descriptor offset; its barrier
@@ -393,7 +405,7 @@ nm_gemm_tf32_kernel(const GemmArgs g, const __grid_constant__ CUtensorMap map_a,
                 TF_ADD(c_issue, t1);
             }
 #ifdef NMSPMM_TF32_PROFILE
-            if (warp == 2) { TF_OUT(6, c_gdone); TF_OUT(7, c_issue); TF_OUT(15, clock64() - c_start); }
+            if (warp == FIRST_PRODUCT) { TF_OUT(6, c_gdone); TF_OUT(7, c_issue); TF_OUT(15, clock64() - c_start); }
 #endif
             if (!ok) atomicMax(g.status, kDevTimeoutMma);
             if (v_live > 0) tc_commit(bar_acc); else mbar_arrive(bar_acc);
@@ -406,9 +418,9 @@ nm_gemm_tf32_kernel(const GemmArgs g, const __grid_constant__ CUtensorMap map_a,
         bool alive = true;
         if (!DIRECT) {
             constexpr int GROUPS = Cfg::GROUPS;
-            const int group = b / Cfg::N1, e = b % Cfg::N1;          // this thread keeps gathered column e of steps group, group + GROUPS, ...
+            const int group = b / Cfg::NT, e = b % Cfg::NT;          // this thread keeps gathered column e of steps group, group + GROUPS, ...
             const int v = e / WSP, j = e % WSP;
-            const bool has = j < WS && v * BPV < live_vecs;
+            const bool has = e < Cfg::N1 && j < WS && v * BPV < live_vecs;
             const int q = (bj >> 5) + v * BPV, qs_shift = g.qs_shift;       // the (first) 32-column index list of vector v
             const int* dptr = g.D + ((static_cast<size_t>(q >> qs_shift) * g.W) << qs_shift) + (q & ((1 << qs_shift) - 1)) +
                               (static_cast<size_t>(j) << qs_shift);
@@ -557,6 +569,8 @@ extern const SlicedVariant kTf32GatherVariants[] = {
     NMSPMM_TF32_VARIANT(8, 32, kModeLow, 8, 32),   NMSPMM_TF32_VARIANT(8, 32, kModeLow, 4, 32),
     NMSPMM_TF32_VARIANT(8, 32, kModeHigh, 8, 32),  NMSPMM_TF32_VARIANT(8, 32, kModeHigh, 4, 32),
     NMSPMM_TF32_VARIANT(4, 64, kModeHigh, 8, 32),  NMSPMM_TF32_VARIANT(4, 64, kModeHigh, 4, 32),
+    NMSPMM_TF32_VARIANT(16, 32, kModeLow, 6, 32),  NMSPMM_TF32_VARIANT(12, 32, kModeLow, 6, 32),  NMSPMM_TF32_VARIANT(8, 32, kModeLow, 6, 32),
+    NMSPMM_TF32_VARIANT(8, 32, kModeHigh, 6, 32),  NMSPMM_TF32_VARIANT(4, 64, kModeHigh, 6, 32),
     // vectors of 64 columns (two adjacent equal index lists): one gather and one N = 64 product per pair
     NMSPMM_TF32_VARIANT(16, 32, kModeLow, 8, 64),  NMSPMM_TF32_VARIANT(12, 32, kModeLow, 8, 64),
     NMSPMM_TF32_VARIANT(8, 32, kModeLow, 8, 64),   NMSPMM_TF32_VARIANT(8, 32, kModeHigh, 8, 64),

@@ -220,6 +220,8 @@ cudaError_t launch_reduce_slices(int ns, const GemmArgs& a, const GemmOutputs& o
     const bool many = a.sched.split_k > kReduceInFlight / 2;
     if (ns == 256 && ms == 128)
         return many ? launch_slices<256, 1, 128>(a, outs, first_tile, n_tiles, st) : launch_slices<256, 4, 128>(a, outs, first_tile, n_tiles, st);
+    if (ns == 192 && ms == 128)
+        return many ? launch_slices<192, 1, 128>(a, outs, first_tile, n_tiles, st) : launch_slices<192, 4, 128>(a, outs, first_tile, n_tiles, st);
     if (ns == 128 && ms == 128)
         return many ? launch_slices<128, 1, 128>(a, outs, first_tile, n_tiles, st) : launch_slices<128, 4, 128>(a, outs, first_tile, n_tiles, st);
     // the few-row tiles of gemm_tf32_few_rows.cu: slots of ms x 128

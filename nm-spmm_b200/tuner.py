@@ -19,7 +19,7 @@ from typing import Iterable, List, Sequence, Tuple
 Shape = Tuple[int, int, int, int, int, int, int]       # M, N, K, n_keep, format, path, vec_len
 
 FP32_TILES = (1, 2, 3, 4, 5, 6, 7, 10, 11)    # 128x128, 64x128, 32x128, 16x128, 128x256, 16x256, 32x256, 256x128, 64x512
-TF32_TILES = (1, 5)
+TF32_TILES = (1, 5, 12)
 SPLITS = (0, 1, 2, 4, 8, 16)          # 0 = the library's automatic schedule on that tile
 
 
