@@ -154,6 +154,15 @@ struct Tf32Cfg {
     static constexpr int NBUF1 = NBUF0 > 4 ? 4 : NBUF0;
     static constexpr int NBUF = NBUF1 > STAGES ? STAGES : NBUF1;     // (the barrier that frees a step's stage frees its buffer too)
     static_assert(NBUF >= 1, "no room for a gather result beside the accumulators");
+    // 16-bit activations: pairs of steps share one commit and one wait between gather and products where Tensor
+    // Memory holds three pairs of results or more -- their steps are the shortest, and the products' issuers spend
+    // them waiting (256 x 11008 x 4096, 8:32, 28.4 -> 25.4 us; 2048 x 9472 x 4096, 64-wide vectors, 107 -> 102; in FP32 125 -> 127).
+    // The buffers of a pair are free when the stage of its second step is; that stage's next phase may not end
+    // before they are asked for.
+    static constexpr int NP0 = DIRECT ? 0 : (TMEM_COLS - NS) / (2 * N1);
+    static constexpr int NP1 = NP0 > 4 ? 4 : NP0;
+    static constexpr int NP = NP1 > (STAGES + 1) / 2 ? (STAGES + 1) / 2 : NP1;
+    static constexpr bool PAIRS = EB == 2 && NP >= 3;
     static constexpr int EPI_BYTES = BUILDERS / 32 * kTf32PatchBytes;    // the builder warps' transposition patches
     static_assert(EPI_BYTES <= STAGES * STAGE_BYTES, "the epilogue reuses the stage ring");
     static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + AUX_BYTES + CTRL_BYTES + 1024;   // + alignment slack
@@ -309,6 +318,45 @@ nm_gemm_tf32_kernel(const GemmArgs g, const __grid_constant__ CUtensorMap map_a,
             uint32_t full = bar_full + (warp - 1) * 8, at = (warp - 1) * (Cfg::STAGE_BYTES / 16), parity = 0;
             uint32_t empty = bar_empty + (GW == 1 ? 0 : (warp - 1 + NBUF) % GW) * 8, empty_parity = 0;
             int buf = (warp - 1) % NBUF;
+            if constexpr (Cfg::PAIRS) {
+                constexpr int NP = Cfg::NP;
+                int st = 2 * (warp - 1), free_st = -1, pb = (warp - 1) % NP;       // stages of the pair's first step and of the second of the pair whose buffers it takes
+                uint32_t full_parity = 0, free_parity = 0;
+                auto gather = [&](int stage, int b) {
+                    const uint32_t off = stage * (Cfg::STAGE_BYTES / 16), gbuf = tmem_addr(tmem, 0, Cfg::ACOL0 + b * Cfg::N1);
+#pragma unroll
+                    for (int ks = 0; ks < Cfg::NKS; ++ks) {
+                        if constexpr (Cfg::SRC == kTf32Rows16)
+                            umma_f16_ss(gbuf, umma_desc_plus(a0, off + a_step(ks)), umma_desc_plus(p0, off + ks * P_STEP), idesc_gather, ks != 0);
+                        else
+                            umma_tf32_ss(gbuf, umma_desc_plus(a0, off + a_step(ks)), umma_desc_plus(p0, off + ks * P_STEP), idesc_gather, ks != 0);
+                    }
+                };
+                for (int t = 2 * (warp - 1), pair = warp - 1; t < n_win; t += 2 * GW, pair += GW) {
+                    const int st1 = (st + 1 == STAGES) ? 0 : st + 1;
+                    const uint32_t parity1 = (st + 1 == STAGES) ? full_parity ^ 1 : full_parity;
+                    if (pair >= NP) {
+                        if (free_st < 0) free_st = (2 * (pair - NP) + 1) % STAGES;
+                        ok = mbar_spin_bounded(bar_empty + free_st * 8, free_parity, abort_word);
+                        free_st += 2 * GW;
+                        if (free_st >= STAGES) { free_st -= STAGES; free_parity ^= 1; }
+                    }
+                    ok = ok && mbar_spin_bounded(bar_full + st * 8, full_parity, abort_word);
+                    if (!ok) break;
+                    tc_fence_after_sync();
+                    gather(st, 2 * pb);
+                    if (t + 1 < n_win) {
+                        ok = mbar_spin_bounded(bar_full + st1 * 8, parity1, abort_word);
+                        if (!ok) break;
+                        tc_fence_after_sync();
+                        gather(st1, 2 * pb + 1);
+                    }
+                    tc_commit(bar_gdone + pb * 8);
+                    pb = (pb + GW) % NP;
+                    st += 2 * GW;
+                    if (st >= STAGES) { st -= STAGES; full_parity ^= 1; }
+                }
+            } else {
             TF_DECL(m_full = 0, m_free = 0, m_issue = 0);
             TF_T(m_start);
             for (int t = warp - 1; t < n_win; t += GW) {
@@ -358,6 +406,7 @@ nm_gemm_tf32_kernel(const GemmArgs g, const __grid_constant__ CUtensorMap map_a,
 #ifdef NMSPMM_TF32_PROFILE
             TF_OUT(2, m_full); TF_OUT(3, m_free); TF_OUT(4, m_issue); TF_OUT(5, clock64() - m_start); if (warp == 1) { TF_OUT(8, 1); TF_OUT(9, n_win); }
 #endif
+            }
             if (!ok) atomicMax(g.status, kDevTimeoutMma);
             if (DIRECT) tc_commit(bar_acc);                // every MMA has completed: accumulators are final
         }
@@ -373,6 +422,36 @@ nm_gemm_tf32_kernel(const GemmArgs g, const __grid_constant__ CUtensorMap map_a,
             uint32_t at = 0, empty = bar_empty;            // stage of step u, as a descriptor offset; its barrier
             uint32_t done_parity = 0;
             int buf = 0;
+            if constexpr (Cfg::PAIRS) {
+                auto products = [&](int u, int b) {
+                    if (v_live > 0) {
+                        const uint32_t gbuf = tmem_addr(tmem, 0, Cfg::ACOL0 + b * Cfg::N1 + v_begin * WSP), acc = tmem_addr(tmem, 0, v_begin * VL);
+#pragma unroll
+                        for (int v = 0; v < VPI; ++v) {
+                            if (v < v_live) {
+#pragma unroll
+                                for (int gi = 0; gi < Cfg::G; ++gi)
+                                    umma_tf32_ts(acc + v * VL, gbuf + v * WSP + gi * 8, umma_desc_plus(b0, at + v * (BPV * WSP * 8) + gi * 64),
+                                                 idesc_product, (u | gi) != 0);
+                            }
+                        }
+                        tc_commit(empty);
+                    } else {
+                        mbar_arrive(empty);
+                    }
+                    at += Cfg::STAGE_BYTES / 16;
+                    empty += 8;
+                    if (empty == bar_empty + STAGES * 8) { empty = bar_empty; at = 0; }
+                };
+                for (int u = 0; u < n_win; u += 2) {
+                    ok = mbar_spin_bounded(bar_gdone + buf * 8, done_parity, abort_word);
+                    if (!ok) break;
+                    tc_fence_after_sync();
+                    products(u, 2 * buf);
+                    if (u + 1 < n_win) products(u + 1, 2 * buf + 1);
+                    if (++buf == Cfg::NP) { buf = 0; done_parity ^= 1; }
+                }
+            } else {
             TF_DECL(c_gdone = 0, c_issue = 0);
             TF_T(c_start);
             for (int u = 0; u < n_win; ++u) {
@@ -407,6 +486,7 @@ nm_gemm_tf32_kernel(const GemmArgs g, const __grid_constant__ CUtensorMap map_a,
 #ifdef NMSPMM_TF32_PROFILE
             if (warp == FIRST_PRODUCT) { TF_OUT(6, c_gdone); TF_OUT(7, c_issue); TF_OUT(15, clock64() - c_start); }
 #endif
+            }
             if (!ok) atomicMax(g.status, kDevTimeoutMma);
             if (v_live > 0) tc_commit(bar_acc); else mbar_arrive(bar_acc);
         }
