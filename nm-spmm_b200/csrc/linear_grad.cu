@@ -378,6 +378,222 @@ nm_grad_input_kernel(const GradArgs a, const __grid_constant__ CUtensorMap map_g
     }
 }
 
+// ------------------------------------------------------------- grad of the input, larger problems
+// The same sum with the register tile of the exact forward path (gemm_ffma_wide.cuh): 16 rows x 8 (6) kept rows
+// a thread, the packed FMA's pairs along m.  That wants both operands with n outermost, grad_y as
+// [N][m] and B as [N][W]: two transposing passes ahead (20 us at M = 2048, N = K = 4096), after which a column of a
+// vector costs six 128-bit shared loads per 64 packed FMAs (eight per 64 above, on half as many rows and kept rows).
+// A warp multiplies 128 rows by 32 (24) kept rows over a vector's 32 columns and adds the result to the accumulator
+// in shared memory, 64 accesses of 128 bits after 2048 packed FMAs (32 after 1024 above, a quarter of the vectors
+// later: groups of warps take the vectors in turn and hand the accumulator on in vector order).  A warpgroup
+// of 40 registers feeds each group through a ring of its own, sixteen columns a stage.
+// Bound by the FMA pipe, active 72 % of the time, its shared loads and the hand-overs: M = 2048, N = K = 4096, 12:32 and 8:32,
+// 672 and 455 us -> 552 and 372 with everything (340 of them this kernel at 8:32), 16:32 852 -> 709.
+template <int NKEEP>
+struct GradInputWideCfg {
+    static constexpr int MT = 128, KT = 256, WT = KT / 32 * NKEEP;
+    static constexpr int TR = (NKEEP == 12) ? 6 : 8, WROWS = 4 * TR;       // kept rows per thread / per warp: whole windows
+    static constexpr int AREAS = WT / WROWS, GROUPS = 8 / AREAS;
+    static constexpr int QN = 16, CHUNKS = 32 / QN;        // columns per stage
+    static constexpr int A_BYTES = QN * MT * 4, B_BYTES = QN * WT * 4, STAGE_BYTES = A_BYTES + B_BYTES;
+    static constexpr int ACC_BYTES = KT * MT * 4;
+    static constexpr int SPG = (227 * 1024 - 2048 - ACC_BYTES) / STAGE_BYTES / GROUPS;      // stages per group
+    static constexpr int STAGES = SPG * GROUPS;
+    static constexpr int CTRL_BYTES = 1024;
+    static constexpr int SMEM_BYTES = ACC_BYTES + STAGES * STAGE_BYTES + CTRL_BYTES + 1024;
+    static constexpr int THREADS = 384;
+    static constexpr int LAUNCH_REGS = 168, COMPUTE_REGS = 232, FEED_REGS = 40;
+    static_assert(2 * COMPUTE_REGS + FEED_REGS == 3 * LAUNCH_REGS, "the warpgroups share what the launch was given");
+    static_assert(WT % WROWS == 0 && WROWS % NKEEP == 0 && AREAS * GROUPS == 8 && (GROUPS == 2 || GROUPS == 4) && SPG >= 2, "eight warps");
+    static_assert(STAGES * 16 + 64 + 8 <= CTRL_BYTES && SMEM_BYTES <= 227 * 1024, "shared memory");
+};
+
+template <int NKEEP>
+__global__ void __launch_bounds__((GradInputWideCfg<NKEEP>::THREADS), 1)
+nm_grad_input_wide_kernel(const GradArgs a, const __grid_constant__ CUtensorMap map_g, const __grid_constant__ CUtensorMap map_b)
+{
+    using Cfg = GradInputWideCfg<NKEEP>;
+    constexpr int MT = Cfg::MT, KT = Cfg::KT, WT = Cfg::WT, TR = Cfg::TR, WROWS = Cfg::WROWS, AREAS = Cfg::AREAS, GROUPS = Cfg::GROUPS;
+    constexpr int QN = Cfg::QN, CHUNKS = Cfg::CHUNKS, SPG = Cfg::SPG;
+    extern __shared__ unsigned char smem_raw[];
+    const uint32_t sums = (smem_u32(smem_raw) + 1023u) & ~1023u, ring = sums + Cfg::ACC_BYTES;
+    const uint32_t full = ring + Cfg::STAGES * Cfg::STAGE_BYTES, empty = full + Cfg::STAGES * 8, tokens = empty + Cfg::STAGES * 8;
+    const uint32_t abort_word = tokens + 64;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+
+    const bool sliced = static_cast<int>(blockIdx.x) >= a.n_whole;
+    const int S = sliced ? a.slices : 1, slot = static_cast<int>(blockIdx.x) - a.n_whole;
+    const int tile = sliced ? a.n_whole + slot / S : static_cast<int>(blockIdx.x);
+    const int tm = tile / a.tiles_x, tk = tile - tm * a.tiles_x;
+    const int m0 = tm * MT, k0 = tk * KT, w0 = k0 / 32 * NKEEP;
+    int v0, T;                                             // this CTA's vectors: v0 .. v0 + T - 1
+    slice_range(a.N >> 5, S, sliced ? slot % S : 0, v0, T);
+
+    if (tid == 0) {
+        prefetch_tensor_map(&map_g);
+        prefetch_tensor_map(&map_b);
+        for (int s = 0; s < Cfg::STAGES; ++s) {
+            mbar_init(full + s * 8, 1);
+            mbar_init(empty + s * 8, AREAS);
+        }
+        for (int i = 0; i < 8; ++i) mbar_init(tokens + i * 8, 1);
+        sts_volatile_s32(abort_word, 0);
+        mbar_init_fence();
+    }
+    for (int o = tid * 16; o < Cfg::ACC_BYTES; o += Cfg::THREADS * 16) sts_f4(sums + o, make_float4(0.f, 0.f, 0.f, 0.f));
+    __syncthreads();
+    grid_dependency_wait();
+
+    if (warp >= 8) {
+        // ------------------------------------------------ copies: warp 8 + f feeds group f (of two or four)
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Cfg::FEED_REGS));
+        if (elect_one()) {
+            bool ok = true;
+            for (int r = 0; ok && r * GROUPS < T; ++r) {
+                for (int h = 0; ok && h < CHUNKS; ++h) {
+                    const int g = warp - 8, t = r * GROUPS + g;
+                    if (g >= GROUPS || t >= T) break;
+                    const int c = r * CHUNKS + h, s = g * SPG + c % SPG;
+                    if (c >= SPG) ok = mbar_sleep_bounded(empty + s * 8, (c / SPG - 1) & 1, abort_word);
+                    if (!ok) break;
+                    const uint32_t st = ring + s * Cfg::STAGE_BYTES;
+                    mbar_arrive_expect_tx(full + s * 8, Cfg::STAGE_BYTES);         // rows past M or W arrive as zeros
+                    tma_load_2d(st, &map_g, m0, (v0 + t) * 32 + h * QN, full + s * 8);
+                    tma_load_2d(st + Cfg::A_BYTES, &map_b, w0, (v0 + t) * 32 + h * QN, full + s * 8);
+                }
+            }
+            if (!ok) atomicMax(a.status, kDevTimeoutEmpty);
+        }
+        return;
+    }
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(Cfg::COMPUTE_REGS));
+
+    // Lanes as in gemm_ffma_wide.cuh: rows lm * 4 + 32 j .. + 3 (j < 4) of the tile, kept rows lw * 4 .. + 3 and 16 + lw * 4 .. + 3
+    // (12:32: 16 + lw * 2, + 1) of the warp's.
+    const int group = warp / AREAS, area = warp % AREAS;
+    const int lm = (lane >> 1) & 7, lw = (lane & 1) | ((lane >> 3) & 2);
+    const int nv = a.N >> 5;
+    const uint32_t a_rel = lm * 16, b_rel = Cfg::A_BYTES + (area * WROWS + lw * 4) * 4;
+    const uint32_t b_rel2 = (TR == 8) ? b_rel + 64 : Cfg::A_BYTES + (area * WROWS + 16 + lw * 2) * 4;
+    // lane p keeps the place in the accumulator of the warp's p-th kept row, -1: there is none
+    const int wp = w0 + area * WROWS + lane;
+    const bool has = lane < WROWS && wp < a.W;
+    const int* dt = a.DT + static_cast<size_t>(has ? wp : 0) * nv + v0;
+    auto place_of = [&](int t) { return has && t < T ? (area * WROWS + lane) / NKEEP * 32 + (__ldg(dt + t) & 31) : -1; };
+
+    float x[2][16], y[2][TR];
+    auto load = [&](int buf, uint32_t st, int n) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float4 v = lds_f4(st + a_rel + n * (MT * 4) + j * 128);
+            x[buf][4 * j] = v.x; x[buf][4 * j + 1] = v.y; x[buf][4 * j + 2] = v.z; x[buf][4 * j + 3] = v.w;
+        }
+        const float4 u = lds_f4(st + b_rel + n * (WT * 4));
+        y[buf][0] = u.x; y[buf][1] = u.y; y[buf][2] = u.z; y[buf][3] = u.w;
+        if constexpr (TR == 8) {
+            const float4 w = lds_f4(st + b_rel2 + n * (WT * 4));
+            y[buf][4] = w.x; y[buf][5] = w.y; y[buf][6] = w.z; y[buf][7] = w.w;
+        } else {
+            const float2 w = lds_f2(st + b_rel2 + n * (WT * 4));
+            y[buf][4] = w.x; y[buf][5] = w.y;
+        }
+    };
+
+    int s = 0;                                             // stage of the group's ring, and the parity of its next wait
+    uint32_t parity = 0;
+    int next = place_of(group);
+    bool alive = true;
+    auto wait_full = [&]() { return __all_sync(0xffffffffu, mbar_wait_bounded(full + (group * SPG + s) * 8, parity, abort_word)) != 0; };
+    for (int t = group; alive && t < T; t += GROUPS) {
+        const int place = next;
+        next = place_of(t + GROUPS);
+        float2 acc[8][TR];                                 // (rows 2 i, 2 i + 1) x kept row
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int r = 0; r < TR; ++r) acc[i][r] = make_float2(0.f, 0.f);
+        alive = wait_full();
+        if (!alive) break;
+        load(0, ring + (group * SPG + s) * Cfg::STAGE_BYTES, 0);
+#pragma unroll 1
+        for (int h = 0; h < CHUNKS; ++h) {
+            const int sc = s;
+            const uint32_t st = ring + (group * SPG + sc) * Cfg::STAGE_BYTES;
+            if (++s == SPG) { s = 0; parity ^= 1; }
+#pragma unroll
+            for (int n = 0; n < QN; ++n) {
+                if (n == QN - 2 && h + 1 < CHUNKS) alive = wait_full() && alive;
+                if (n + 1 < QN) load((n + 1) & 1, st, n + 1);
+                else load(0, ring + (group * SPG + s) * Cfg::STAGE_BYTES, 0);      // (after the last chunk: read once, not used)
+#pragma unroll
+                for (int r = 0; r < TR; ++r) {
+                    const float2 yy = make_float2(y[n & 1][r], y[n & 1][r]);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        const int q = (r & 1) ? 7 - i : i;
+                        acc[q][r] = __ffma2_rn(make_float2(x[n & 1][2 * q], x[n & 1][2 * q + 1]), yy, acc[q][r]);
+                    }
+                }
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(empty + (group * SPG + sc) * 8);
+        }
+        // this patch of the accumulator, after the vector before has been added to it
+        if (t > 0)
+            alive = __all_sync(0xffffffffu, mbar_wait_bounded(tokens + (area * GROUPS + (t - 1) % GROUPS) * 8, ((t - 1) / GROUPS) & 1, abort_word)) && alive;
+        if (!alive) break;
+#pragma unroll
+        for (int r0 = 0; r0 < TR; r0 += 2) {               // two kept rows at a time: eight loads in flight
+            float4 v[2][4];
+            uint32_t p[2];
+            bool there[2];
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                const int r = r0 + q, k = __shfl_sync(0xffffffffu, place, r < 4 ? lw * 4 + r : (TR == 8 ? 16 + lw * 4 + r - 4 : 16 + lw * 2 + r - 4));
+                there[q] = k >= 0;
+                p[q] = sums + (there[q] ? k : 0) * (MT * 4) + ((lm ^ (k & 7)) << 4);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) v[q][j] = lds_f4(p[q] + j * 128);
+            }
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                if (there[q]) {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const float2 lo = acc[2 * j][r0 + q], hi = acc[2 * j + 1][r0 + q];
+                        sts_f4(p[q] + j * 128, make_float4(v[q][j].x + lo.x, v[q][j].y + lo.y, v[q][j].z + hi.x, v[q][j].w + hi.y));
+                    }
+                }
+            }
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(tokens + (area * GROUPS + group) * 8);
+    }
+    asm volatile("bar.sync 1, 256;" ::: "memory");
+    grid_launch_dependents();
+    if (lds_volatile_s32(abort_word) != 0) {
+        if (tid == 0) atomicMax(a.status, kDevTimeoutFull);
+        return;
+    }
+    // a warp per row of the tile, lanes along k (four lanes of a load meet in a bank), eight loads in flight
+    for (int m = warp; m < MT; m += 8) {
+        if (m0 + m >= a.M) continue;
+        float val[KT / 32];
+#pragma unroll
+        for (int i = 0; i < KT / 32; ++i) {
+            const int k = lane + i * 32;
+            val[i] = __uint_as_float(lds_u32(sums + k * (MT * 4) + (m >> 5) * 128 + ((((m >> 2) & 7) ^ (k & 7)) << 4) + (m & 3) * 4));
+        }
+#pragma unroll
+        for (int i = 0; i < KT / 32; ++i) {
+            const int k = lane + i * 32;
+            if (k0 + k >= a.K) break;
+            if (sliced) a.partial[(static_cast<size_t>(slot) * MT + m) * KT + k] = val[i];
+            else store_as(a.out, static_cast<size_t>(m0 + m) * a.K + k0 + k, val[i], a.dtype);
+        }
+    }
+}
+
 // Adds the slices of split tiles (slots of rows x cols floats, one after the other) in order and
 // writes the elements that exist.  One float4 per thread.
 __global__ void __launch_bounds__(256) nm_grad_reduce_kernel(const GradArgs a, int rows, int cols, int out_rows, int out_cols)
@@ -467,6 +683,30 @@ static GradPlan plan_input(int M, int N, int K, int sms)
     return p;
 }
 
+// Whether the input's gradient takes the larger register tiles and the two transposing passes ahead of them: not at
+// 4:32, where one warp holds a vector's kept rows and eight in turn on one patch of the accumulator wait for one
+// another (2048 x 4096 x 4096: 250 -> 275 us), and not where the passes and their launches cost more than the tiles
+// save (20 us of products at the FMA peak: 256 x 4096 x 4096, 8:32, 29 us of them, 75.7 -> 68.7; 128 rows, 14 us, 45.9 -> 48.1).
+static bool wide_input_pays(int M, int N, int K, int n_keep)
+{
+    return n_keep != 4 && static_cast<double>(M) * N * (K / 32 * n_keep) >= 7.4e8;
+}
+
+template <int NKEEP>
+static GradPlan plan_input_wide(int M, int N, int K, int sms)
+{
+    using Cfg = GradInputWideCfg<NKEEP>;
+    GradPlan p;
+    p.rows = Cfg::MT;
+    p.cols = Cfg::KT;
+    p.tiles_x = (K + Cfg::KT - 1) / Cfg::KT;
+    p.tiles = p.tiles_x * ((M + Cfg::MT - 1) / Cfg::MT);
+    cut_tiles(p.tiles, sms, N / 32, 8, 4.0 / (N / 32 > 4 ? N / 32 : 4), &p.whole, &p.slices);
+    return p;
+}
+
+static size_t transposed_floats(int rows, int cols) { return static_cast<size_t>((rows + 3) / 4 * 4) * cols; }     // [cols][rows up to a multiple of 4]
+
 template <typename Kernel>
 static cudaError_t allow_smem(Kernel kernel, int bytes, bool* configured)
 {
@@ -534,6 +774,38 @@ static cudaError_t launch_input(GradArgs a, const GradPlan& p, const float* grad
     return e;
 }
 
+template <int NKEEP>
+static cudaError_t launch_input_wide(GradArgs a, const GradPlan& p, const float* grad_y, float* scratch, cudaStream_t st)
+{
+    using Cfg = GradInputWideCfg<NKEEP>;
+    static bool configured[64] = {};
+    cudaError_t e = allow_smem(nm_grad_input_wide_kernel<NKEEP>, Cfg::SMEM_BYTES, configured);
+    if (e != cudaSuccess) return e;
+    // the compute warps' share comes out of what the launch is given: less of it and they would wait
+    cudaFuncAttributes fa;
+    e = cudaFuncGetAttributes(&fa, nm_grad_input_wide_kernel<NKEEP>);
+    if (e != cudaSuccess) return e;
+    if (fa.numRegs < Cfg::LAUNCH_REGS) return cudaErrorInvalidKernelImage;
+    const int ldm = (a.M + 3) / 4 * 4, ldw = (a.W + 3) / 4 * 4;
+    float* g_cols = scratch;
+    float* b_cols = g_cols + transposed_floats(a.M, a.N);
+    a.partial = b_cols + transposed_floats(a.W, a.N);
+    e = launch_transpose_rows(kDtypeF32, grad_y, g_cols, a.M, a.N, ldm, st);
+    if (e == cudaSuccess) e = launch_transpose_rows(kDtypeF32, a.B, b_cols, a.W, a.N, ldw, st);
+    if (e != cudaSuccess) return e;
+    CUtensorMap map_g, map_b;
+    e = encode_tensor_map_2d(&map_g, g_cols, ldm, a.N, Cfg::MT, Cfg::QN);
+    if (e != cudaSuccess) return e;
+    e = encode_tensor_map_2d(&map_b, b_cols, ldw, a.N, Cfg::WT, Cfg::QN);
+    if (e != cudaSuccess) return e;
+    a.tiles_x = p.tiles_x;
+    a.n_whole = p.whole;
+    a.slices = p.slices;
+    e = launch_overlapped(nm_grad_input_wide_kernel<NKEEP>, p.ctas(), Cfg::THREADS, Cfg::SMEM_BYTES, st, a, map_g, map_b);
+    if (e == cudaSuccess && p.slices > 1) e = launch_grad_reduce(a, p, a.M, a.K, st);
+    return e;
+}
+
 #define NMSPMM_BY_RATIO(call)                       \
     switch (n_keep) {                               \
     case 16: return call(16);                       \
@@ -557,6 +829,10 @@ size_t grad_values_scratch_bytes(int M, int N, int K, int n_keep, int sms)
 
 size_t grad_input_scratch_bytes(int M, int N, int K, int n_keep, int sms)
 {
+    if (wide_input_pays(M, N, K, n_keep)) {
+        const GradPlan p = n_keep == 16 ? plan_input_wide<16>(M, N, K, sms) : (n_keep == 12 ? plan_input_wide<12>(M, N, K, sms) : plan_input_wide<8>(M, N, K, sms));
+        return (transposed_floats(M, N) + transposed_floats(K / 32 * n_keep, N) + p.partial_floats()) * sizeof(float);
+    }
 #define NMSPMM_CALL(R) plan_input<R>(M, N, K, sms).partial_floats() * sizeof(float)
     NMSPMM_BY_RATIO(NMSPMM_CALL)
 #undef NMSPMM_CALL
@@ -592,6 +868,14 @@ cudaError_t launch_grad_input(int dtype, const float* grad_y, const float* B, co
     a.status = status;
     a.dtype = dtype;
     a.M = M; a.N = N; a.K = K; a.W = K / 32 * n_keep;
+    if (wide_input_pays(M, N, K, n_keep)) {
+        switch (n_keep) {
+        case 16: return launch_input_wide<16>(a, plan_input_wide<16>(M, N, K, sms), grad_y, scratch, st);
+        case 12: return launch_input_wide<12>(a, plan_input_wide<12>(M, N, K, sms), grad_y, scratch, st);
+        case 8: return launch_input_wide<8>(a, plan_input_wide<8>(M, N, K, sms), grad_y, scratch, st);
+        default: return cudaErrorInvalidValue;
+        }
+    }
 #define NMSPMM_CALL(R) launch_input<R>(a, plan_input<R>(M, N, K, sms), grad_y, st)
     NMSPMM_BY_RATIO(NMSPMM_CALL)
 #undef NMSPMM_CALL
