@@ -95,6 +95,12 @@ int nmspmm_preprocess_high_device(const int* DT_dev, int* D_dev, int* column_inf
  * vec_len 64 adjacent pairs are equal) -- the inputs of nmspmm_preprocess_*_device. */
 int nmspmm_prune_device(const float* dense_dev, float* BT_dev, int* DT_dev,
                         int K, int N, int n_keep, int vec_len, void* stream);
+/* nmspmm_prune_device and the packing of its indices for layout_ns = 128 in one pass over the weight: BT as there, D_dev
+ * (W * N / 32 ints) and, for NMSPMM_FORMAT_HIGH (K % 64 == 0), column_info_dev ((N / 128) * (K / 64) * 64 ints and one more
+ * window of 64, all -1) as nmspmm_preprocess_low_device / _high_device (fused) write them.  N % 128 == 0.  The raw indices
+ * are not written. */
+int nmspmm_prune_pack_device(const float* dense_dev, float* BT_dev, int* D_dev, int* column_info_dev, int K, int N, int n_keep,
+                             int vec_len, int format, void* stream);
 
 /* Host-pointer forms with the reference's in-place semantics (H2D + kernel + D2H;
  * they allocate and free temporary device buffers).  The extra column_info window

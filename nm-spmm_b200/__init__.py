@@ -43,7 +43,7 @@ C_ABI_SYMBOLS = (
     "nmspmm_gemm_row_major_workspace_bytes", "nmspmm_gemm_row_major_call_bytes", "nmspmm_gemm_row_major_16", "nmspmm_gemm_row_major_16_workspace_bytes",
     "nmspmm_linear_grad", "nmspmm_linear_grad_workspace_bytes", "nmspmm_widen_device", "nmspmm_gemm_with_cached_workspace", "nmspmm_device_status",
     "nmspmm_gemm_plan", "nmspmm_gemm_host", "nmspmm_release_cached", "nmspmm_measure_ffma_peak",
-    "nmspmm_gemm_static_scratch", "nmspmm_gemm_gather", "nmspmm_prune_device",
+    "nmspmm_gemm_static_scratch", "nmspmm_gemm_gather", "nmspmm_prune_device", "nmspmm_prune_pack_device",
 )
 STATIC_SCRATCH_BYTES = 16 << 20     # NMSPMM_STATIC_SCRATCH_BYTES of include/nmspmm_b200.h
 
@@ -116,6 +116,7 @@ def load_library():
     lib.nmspmm_gemm_with_cached_workspace.argtypes = [ctypes.POINTER(GemmDesc), vp, vp, vp, vp, vp, vp]
     lib.nmspmm_gemm_static_scratch.argtypes = [ctypes.POINTER(GemmDesc), vp, vp, vp, vp, vp, vp]
     lib.nmspmm_prune_device.argtypes = [vp, vp, vp, ci, ci, ci, ci, vp]
+    lib.nmspmm_prune_pack_device.argtypes = [vp, vp, vp, vp, ci, ci, ci, ci, ci, vp]
     lib.nmspmm_gemm_gather.argtypes = [ctypes.POINTER(GemmDesc), vp, vp, vp, vp, ctypes.POINTER(vp), ci, ctypes.c_longlong, ci,
                                        vp, sz, vp]
     lib.nmspmm_device_status.argtypes = [ctypes.POINTER(ci), ci]
@@ -339,6 +340,22 @@ def prune_device(dense, n_keep: int, vec_len: int = 32, stream=None):
            load_library().nmspmm_prune_device(_dev_ptr(dense, torch.float32, "dense"), BT.data_ptr(), DT.data_ptr(),
                                               K, N, n_keep, vec_len, _stream_ptr(stream)))
     return BT, DT
+
+
+def prune_pack_device(dense, n_keep: int, fmt: int, vec_len: int = 32, stream=None):
+    """nmspmm_prune_pack_device: pruning and packing (layout_ns 128) in one pass.  Returns (BT (W, N) float32, packed D flat,
+    column_info flat or None) on the device."""
+    torch = _torch()
+    K, N = dense.shape
+    W = K // 32 * n_keep
+    BT = torch.empty((W, N), dtype=torch.float32, device=dense.device)
+    D = torch.empty(W * (N // VEC_LEN), dtype=torch.int32, device=dense.device)
+    ci = (torch.empty(formats.column_info_ints(W, N, 2 * n_keep, 64, 128), dtype=torch.int32, device=dense.device)
+          if fmt == FORMAT_HIGH else None)
+    _check("nmspmm_prune_pack_device",
+           load_library().nmspmm_prune_pack_device(_dev_ptr(dense, torch.float32, "dense"), BT.data_ptr(), D.data_ptr(),
+                                                   None if ci is None else ci.data_ptr(), K, N, n_keep, vec_len, fmt, _stream_ptr(stream)))
+    return BT, D, ci
 
 
 def gemm_gather(desc: GemmDesc, A, B, D, column_info, out_ptrs, ldc: int, col0: int, workspace=None, stream=None) -> None:
@@ -594,9 +611,19 @@ class NMSpMM:
     @classmethod
     def from_dense(cls, dense, n_keep: int, vec_len: int = 32, layout_ns: int = 128, fmt: Optional[int] = None):
         """Prune a dense (K, N) float32 CUDA weight to ``n_keep``:32 by per-vector L2 magnitude,
-        compress and pack it, all on the device (prune_device, then the packing kernels)."""
+        compress and pack it, all on the device (one pass where the layout is 128 columns; else prune_device, then the
+        packing kernels)."""
+        fmt = format_of(n_keep) if fmt is None else fmt
+        K, N = dense.shape
+        if cls is NMSpMM and layout_ns == 128 and N % 128 == 0 and K % (64 if fmt == FORMAT_HIGH else 32) == 0:
+            op = cls.__new__(cls)
+            op.K, op.n_keep, op.layout_ns, op.vec_len, op.format = K, n_keep, layout_ns, vec_len, fmt
+            op.B, op.D, op.column_info = prune_pack_device(dense, n_keep, fmt, vec_len)
+            op.W, op.N = op.B.shape
+            op._scratch = Scratch()
+            return op
         BT, DT = prune_device(dense, n_keep, vec_len)
-        return cls(BT, DT, dense.shape[0], n_keep, layout_ns, fmt, dense.device, vec_len=vec_len)
+        return cls(BT, DT, K, n_keep, layout_ns, fmt, dense.device, vec_len=vec_len)
 
     def desc(self, M: int, path: int = PATH_FP32, split_k: int = 0, tile: int = 0) -> GemmDesc:
         return make_desc(M, self.N, self.K, self.n_keep, self.format, self.layout_ns, path, split_k, tile, self.vec_len)

@@ -621,9 +621,10 @@ static double tf32_plan_us(const Plan& p, int sms)
 // split to the library and no tuned entry names them another's if its scratch fits: on the exact path a
 // wide tile's (pick_wide_tile); on the tensor cores that of 192-column tiles, where they leave fewer SMs
 // idle (256 x 11008 x 4096, bfloat16: 116 tiles instead of 86, 16:32 52.1 -> 35.1 us, 8:32 29.7 -> 27.8).
-static int plan_call(const nmspmm_gemm_desc* d, int sms, size_t workspace_bytes, Plan* p, bool any_rows = false)
+static int plan_call(const nmspmm_gemm_desc* d, int sms, size_t workspace_bytes, Plan* p, bool any_rows = false, size_t* own_bytes = nullptr)
 {
     const int rc = make_plan(d, sms, p, any_rows);
+    if (rc == NMSPMM_OK && own_bytes) *own_bytes = scratch_bytes(*p);      // of the description's own plan
     if (rc != NMSPMM_OK || d->tile != 0 || d->split_k != 0) return rc;
     const bool tensor = p->tv && p->tv->form == 0 && p->tv->ns == 256 && p->tv->vec_len == 32 && p->tv->n_keep != 32;
     if (!p->v && !tensor) return rc;
@@ -857,9 +858,10 @@ size_t nmspmm_gemm_workspace_bytes(const nmspmm_gemm_desc* desc)
 // The larger of what the description's plan and what the call's need.
 size_t nmspmm_gemm_call_workspace_bytes(const nmspmm_gemm_desc* desc)
 {
-    Plan p, c;
-    if (make_plan(desc, sm_count(), &p) != NMSPMM_OK || plan_call(desc, sm_count(), SIZE_MAX, &c) != NMSPMM_OK) return 0;
-    return scratch_bytes(p) > scratch_bytes(c) ? scratch_bytes(p) : scratch_bytes(c);
+    Plan c;
+    size_t own = 0;
+    if (plan_call(desc, sm_count(), SIZE_MAX, &c, false, &own) != NMSPMM_OK) return 0;
+    return own > scratch_bytes(c) ? own : scratch_bytes(c);
 }
 
 size_t nmspmm_gemm_counter_bytes(const nmspmm_gemm_desc* desc)
@@ -1027,13 +1029,15 @@ static size_t row_major_bytes(const Plan& p, const nmspmm_gemm_desc* d, int dtyp
 }
 
 // The larger of what the description's plan and what the call's takes (plan_call); copy_a < 0: by the addresses.
+// (The two differ in their scratch alone: both of the exact path, or both reading rows.)
 static size_t row_major_bytes_any(const nmspmm_gemm_desc* d, int dtype, int copy_a, const void* A_rows = nullptr, const void* C = nullptr)
 {
-    Plan p, c;
-    if (!d || make_plan(d, sm_count(), &p, true) != NMSPMM_OK || plan_call(d, sm_count(), SIZE_MAX, &c, true) != NMSPMM_OK) return 0;
-    const bool copy = copy_a < 0 ? !reads_rows(p, d, A_rows, C, dtype) : copy_a != 0;
-    const size_t x = row_major_bytes(p, d, dtype, copy), y = row_major_bytes(c, d, dtype, copy);
-    return x > y ? x : y;
+    Plan c;
+    size_t own = 0;
+    if (!d || plan_call(d, sm_count(), SIZE_MAX, &c, true, &own) != NMSPMM_OK) return 0;
+    const bool copy = copy_a < 0 ? !reads_rows(c, d, A_rows, C, dtype) : copy_a != 0;
+    const size_t head = own > 0 ? own : kCounterBlock, rest = row_major_bytes(c, d, dtype, copy) - row_major_head_bytes(c);
+    return (head > row_major_head_bytes(c) ? head : row_major_head_bytes(c)) + rest;
 }
 
 // The plan a row-major call with this much workspace runs.
