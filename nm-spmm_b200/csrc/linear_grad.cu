@@ -6,9 +6,9 @@
 // Both are 2 M N W useful FLOPs, n_keep / 32 of the dense products they replace (an expanded
 // B or an M x K x N product of which most is thrown away), and both are bound by the FP32
 // FMA pipe: 17.2 GFLOP at M = 2048, N = K = 4096, 8:32, against 0.1 GB of operands.  Measured
-// there: grad_B 331 us (51.8 TFLOP/s of the 74 the pipe has), grad_x 454 us (37.9), against 1169 and
-// 1136 us of the dense FP32 products (and 70 us of expanding B and picking the kept positions); at
-// 16:32 647 and 851 us, at 4:32 207 and 249 us.
+// there: grad_B 331 us (51.8 TFLOP/s of the 74 the pipe has), grad_x 372 us (46.2, two transposing passes
+// included), against 1169 and 1136 us of the dense FP32 products (and 70 us of expanding B and picking the kept
+// positions); at 16:32 647 and 709 us, at 4:32 207 and 235 us.
 //
 // The indices are the raw window-local ones, [W][N/32].  Every wait is bounded; one that
 // gives up raises the device status word and nothing of its tile is stored.
@@ -210,6 +210,8 @@ nm_grad_values_kernel(const GradArgs a, const __grid_constant__ CUtensorMap map_
 // Nothing is saturated: at M = 2048, N = K = 4096, 8:32 the FMA pipe is active 56 % of the time and half of the
 // shared-memory wavefronts there are go by, on two warps per scheduler whose own fixed latencies are the
 // largest stall.  (Thread tile 8 x 4 on sixteen warps took 481 us there.)
+// A tile's last stores go out eight at a time per lane: as pairs of load and store, one after the other, they cost
+// 5 % (2048 x 4096 x 4096, 4:32, 250 -> 235 us; 128 x 4096 x 4096, 8:32, 45.6 -> 42.2).
 // The accumulator is what limits the warps: 32 KB of it per warp at 8:32.  At 8:32 and 4:32 two
 // and four groups of warps therefore share it, each taking every second / fourth vector; a
 // token per patch of the accumulator hands it from group to group in vector order, so that the
@@ -365,15 +367,25 @@ nm_grad_input_kernel(const GradArgs a, const __grid_constant__ CUtensorMap map_g
         if (tid == 0) atomicMax(a.status, kDevTimeoutFull);
         return;
     }
-    // a warp per row of the tile, lanes along k (four lanes of a load meet in a bank: 1.5 % of a tile's time)
+    // a warp per row of the tile, lanes along k (four lanes of a load meet in a bank), eight loads in flight
     for (int m = warp; m < MT; m += Cfg::WARPS) {
         if (m0 + m >= a.M) continue;
         const int h = (m >> 5) & 1, x = (m >> 3) & 3;      // i = (m % 64) / 8 = 4 h + x
-        for (int k = lane; k < KT; k += 32) {
-            if (k0 + k >= a.K) break;
-            const float val = __uint_as_float(lds_u32(sums + k * (MT * 4) + (m >> 6) * 256 + h * 128 + (((m & 7) ^ (k & 7)) << 4) + x * 4));
-            if (sliced) a.partial[(static_cast<size_t>(slot) * MT + m) * KT + k] = val;
-            else store_as(a.out, static_cast<size_t>(m0 + m) * a.K + k0 + k, val, a.dtype);
+#pragma unroll 1
+        for (int kk = 0; kk < KT; kk += 256) {
+            float val[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const int k = kk + lane + i * 32;
+                val[i] = __uint_as_float(lds_u32(sums + k * (MT * 4) + (m >> 6) * 256 + h * 128 + (((m & 7) ^ (k & 7)) << 4) + x * 4));
+            }
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const int k = kk + lane + i * 32;
+                if (k0 + k >= a.K) break;
+                if (sliced) a.partial[(static_cast<size_t>(slot) * MT + m) * KT + k] = val[i];
+                else store_as(a.out, static_cast<size_t>(m0 + m) * a.K + k0 + k, val[i], a.dtype);
+            }
         }
     }
 }
