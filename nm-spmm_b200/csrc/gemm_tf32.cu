@@ -158,10 +158,10 @@ struct Tf32Cfg {
     // Memory holds three pairs of results or more -- their steps are the shortest, and the products' issuers spend
     // them waiting (256 x 11008 x 4096, 8:32, 28.4 -> 25.4 us; 2048 x 9472 x 4096, 64-wide vectors, 107 -> 102; in FP32 125 -> 127).
     // The buffers of a pair are free when the stage of its second step is; that stage's next phase may not end
-    // before they are asked for.
+    // before they are asked for; and a stage's last step is done by then, so that the wait on it is unmistakable.
     static constexpr int NP0 = DIRECT ? 0 : (TMEM_COLS - NS) / (2 * N1);
     static constexpr int NP1 = NP0 > 4 ? 4 : NP0;
-    static constexpr int NP = NP1 > (STAGES + 1) / 2 ? (STAGES + 1) / 2 : NP1;
+    static constexpr int NP = NP1 > STAGES / 2 ? STAGES / 2 : NP1;
     static constexpr bool PAIRS = EB == 2 && NP >= 3;
     static constexpr int EPI_BYTES = BUILDERS / 32 * kTf32PatchBytes;    // the builder warps' transposition patches
     static_assert(EPI_BYTES <= STAGES * STAGE_BYTES, "the epilogue reuses the stage ring");
@@ -360,20 +360,25 @@ nm_gemm_tf32_kernel(const GemmArgs g, const __grid_constant__ CUtensorMap map_a,
             TF_DECL(m_full = 0, m_free = 0, m_issue = 0);
             TF_T(m_start);
             for (int t = warp - 1; t < n_win; t += GW) {
-                TF_T(t0);
-                ok = mbar_spin_bounded(full, parity, abort_word);
-                TF_ADD(m_full, t0);
                 TF_T(t1);
                 // the result buffer is free once the products of step t - NBUF are done, which is when that
-                // step's stage is (the stage's next phase ends with step t - NBUF + STAGES, not before this one)
+                // step's stage is (the stage's next phase ends with step t - NBUF + STAGES, not before this one).
+                // This wait has to come before the one on the stage: with two gathering threads and an odd number
+                // of stages, the step before in this stage was the other thread's and may still wait to be filled,
+                // where a wait by parity would take the phase before that one for the awaited one. Products are in
+                // order, so past this wait every step up to t - NBUF, t - STAGES among them, has been used up.
+                static_assert(DIRECT || NBUF <= STAGES, "a stage's last step is done once the result buffer is free");
                 if (!DIRECT && t >= NBUF) {
-                    ok = ok && mbar_spin_bounded(empty, empty_parity, abort_word);
+                    ok = mbar_spin_bounded(empty, empty_parity, abort_word);
                     empty += GW * 8;
                     if (GW == 1) {
                         if (empty == bar_empty + STAGES * 8) { empty = bar_empty; empty_parity ^= 1; }
                     } else if (empty >= bar_empty + STAGES * 8) { empty -= STAGES * 8; empty_parity ^= 1; }
                 }
                 TF_ADD(m_free, t1);
+                TF_T(t0);
+                ok = ok && mbar_spin_bounded(full, parity, abort_word);
+                TF_ADD(m_full, t0);
                 if (!ok) break;
                 TF_T(t2);
                 tc_fence_after_sync();
