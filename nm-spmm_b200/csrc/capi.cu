@@ -416,6 +416,7 @@ static bool tf32_few_rows_pays(const nmspmm_gemm_desc* d)
 
 static int make_plan(const nmspmm_gemm_desc* d_in, int sms, Plan* p, bool any_rows = false)
 {
+    *p = Plan {};                                          // (a caller may hand in one that held another plan)
     int mode = 0;
     int rc = check_desc(d_in, &mode, any_rows);
     if (rc != NMSPMM_OK) return rc;

@@ -2,6 +2,8 @@
 rings: ragged rows, vectors past the last column, fewer windows than stages, pieces that cross tiles,
 every index layout, and the call that picks them by itself.  Against the oracle's float product; 1e-5 as for
 the other exact kernels (32-bit sums of up to 1024 products, 8e-7 seen)."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -53,6 +55,23 @@ def test_calls_that_take_a_wide_tile_by_themselves(pkg, M, N, K, n_keep):
         assert float((other.double() - planned.double()).norm() / planned.double().norm()) <= TOL
     assert bool((wide_buffer[:, :, :32] == -1).all()) and bool((wide_buffer[:, :, -32:] == -1).all())
     assert pkg.device_status() == 0
+
+
+@pytest.mark.parametrize("M,N,K,n_keep,path", [(2048, 5760, 1024, 16, 0), (2052, 5760, 1024, 8, 0), (512, 11008, 1024, 12, 0),
+                                               (132, 1024, 1024, 16, 1), (256, 1024, 1024, 12, 1)])
+def test_row_major_calls_with_the_named_plans_scratch(pkg, M, N, K, n_keep, path):
+    """Scratch for the plan that the description names and not a byte more: that plan runs, bit for bit."""
+    p = pkg.formats.make_random(M, N, K, n_keep, seed=19)
+    op = pkg.NMSpMM.from_problem(p)
+    d, x = op.desc(M, path=path), torch.from_numpy(p.A_km).cuda().t().contiguous()
+    own = pkg.workspace_bytes(d)
+    assert own < pkg.call_workspace_bytes(d) and pkg.call_plan(d, own).tile == pkg.plan(d).tile
+    less = max(own, 64 << 10) + (0 if path == pkg.PATH_TF32 else 4 * M * K)
+    got, ws = torch.full((M, N), float("nan"), device="cuda"), torch.zeros(less, dtype=torch.uint8, device="cuda")
+    rc = pkg.load_library().nmspmm_gemm_row_major(
+        ctypes.byref(d), x.data_ptr(), op.B.data_ptr(), op.D.data_ptr(), None if op.column_info is None else op.column_info.data_ptr(),
+        got.data_ptr(), ws.data_ptr(), less, torch.cuda.current_stream().cuda_stream)
+    assert rc == pkg.OK and torch.equal(got, op.matmul_rows(x, path=path, tile=pkg.plan(d).tile)) and pkg.device_status() == 0
 
 
 def test_non_finite_values_stay_where_they_belong(pkg):

@@ -364,3 +364,22 @@ def test_calls_take_a_wide_tile_where_it_pays_and_fits(pkg, M, N, K, n_keep, til
         assert pkg.call_plan(d).tile == pkg.TILE_64x128
     finally:
         pkg.clear_tuned_plans()
+
+
+@pytest.mark.parametrize("M,N,K,n_keep,path", [(4096, 4096, 4096, 8, 0), (4096, 4096, 4096, 16, 0), (2048, 5760, 1024, 16, 0),
+                                               (512, 11008, 1024, 12, 0), (132, 1024, 1024, 16, 1), (256, 1024, 1024, 12, 1)])
+def test_a_row_major_call_takes_the_named_plans_scratch(pkg, M, N, K, n_keep, path):
+    """Scratch for the plan that a description names, too little for the one a call prefers: planned all the same (the
+    launch then fails for want of a GPU).  Before the preferred plan was cleared away its sizes stayed and the call was refused."""
+    if pytest.importorskip("torch").cuda.is_available():
+        pytest.skip("the operands are made-up addresses; test_gpu_wide_tiles.py runs such calls")
+    d = pkg.make_desc(M, N, K, n_keep, pkg.format_of(n_keep), 128, path)
+    lib, ref, own = pkg.load_library(), ctypes.byref(d), pkg.workspace_bytes(d)
+    assert own < pkg.call_workspace_bytes(d)
+    copy_a = 0 if path == pkg.PATH_TF32 else 4 * M * K
+    less = max(own, 64 << 10) + copy_a
+    at = [ctypes.c_void_p((1 << 20) + (i << 32)) for i in range(6)]
+    assert lib.nmspmm_gemm_row_major(ref, *at[:4], at[4], at[5], less, None) == pkg.CUDA_ERROR
+    assert lib.nmspmm_gemm_row_major(ref, *at[:4], at[4], at[5], less - 1, None) == pkg.WORKSPACE_TOO_SMALL
+    if path == pkg.PATH_TF32:
+        assert lib.nmspmm_gemm_row_major_16(ref, pkg.DTYPE_BF16, *at[:4], at[4], at[5], less, None) == pkg.CUDA_ERROR
