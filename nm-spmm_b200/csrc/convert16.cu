@@ -48,7 +48,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) transpose_rows_kernel(const T* __restrict__ in, float* __restrict__ out, int M, int K, int ld, int aligned)
 {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int k = blockIdx.x * 128 + warp * 16 + (lane >> 3) * 4, m = blockIdx.y * 32 + (lane & 7) * 4;
+    const int k = blockIdx.x * 128 + warp * 16 + (lane >> 3) * 4, m = (blockIdx.z * gridDim.y + blockIdx.y) * 32 + (lane & 7) * 4;
     grid_dependency_wait();
     if (k < K && m < ld) {
         float4 r[4];
@@ -97,7 +97,9 @@ static unsigned flat_grid(size_t n4)
 template <typename T>
 static cudaError_t launch_transpose(const void* in, float* out, int M, int K, int ld, cudaStream_t st)
 {
-    const dim3 grid((K + 127) / 128, (ld + 31) / 32);
+    constexpr int kMaxY = 65535;                           // blocks of 32 rows along y; more of them (over 2097120 rows) go on along z
+    const int blocks = (ld + 31) / 32;
+    const dim3 grid((K + 127) / 128, blocks < kMaxY ? blocks : kMaxY, (blocks + kMaxY - 1) / kMaxY);
     const int aligned = reinterpret_cast<uintptr_t>(in) % (4 * sizeof(T)) == 0 ? 1 : 0;
     return launch_overlapped(transpose_rows_kernel<T>, grid, 256, 0, st, static_cast<const T*>(in), out, M, K, ld, aligned);
 }

@@ -26,3 +26,19 @@ def test_input_gradient(pkg, M, N, K, n_keep, dtype, tol):
     dense = torch.zeros((K, N), dtype=torch.float64, device="cuda").scatter_(0, pkg.linear._dense_rows(DT, n_keep), values.double())
     ref = g.double() @ dense.t()
     assert float((gx.double() - ref).norm() / ref.norm()) <= tol
+
+
+def test_more_rows_than_a_grid_has_blocks_along_y(pkg):
+    """The transposing pass over grad_y cuts the rows into blocks of 32, of which a grid holds 65535 along y."""
+    M, N, K, n_keep = 65535 * 32 + 100, 32, 64, 8
+    DT = torch.from_numpy(pkg.formats.random_indices(1, K, N // 32, n_keep)).cuda()
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(1)
+    values, g = torch.randn((K // 32 * n_keep, N), device="cuda", generator=gen), torch.randn((M, N), device="cuda", generator=gen)
+    assert M * N * values.shape[0] >= 7.4e8
+    gx, _ = pkg.linear._sparse_grads(pkg, torch.empty((M, K), device="cuda"), values, DT, n_keep, g, True, False)
+    dense = torch.zeros((K, N), dtype=torch.float64, device="cuda").scatter_(0, pkg.linear._dense_rows(DT, n_keep), values.double())
+    ref = g.double() @ dense.t()
+    for rows in (slice(0, 1 << 20), slice(1 << 20, 65535 * 32), slice(65535 * 32, M)):
+        assert float((gx[rows].double() - ref[rows]).norm() / ref[rows].norm()) <= 1e-5
+    assert pkg.device_status() == 0
