@@ -719,13 +719,20 @@ static GradPlan plan_input_wide(int M, int N, int K, int sms)
 
 static size_t transposed_floats(int rows, int cols) { return static_cast<size_t>((rows + 3) / 4 * 4) * cols; }     // [cols][rows up to a multiple of 4]
 
+// Once per device: the kernel's shared memory and, where its warpgroups share out registers, that the launch is given
+// as many a thread as the shares add up to (less of it and they would wait).
 template <typename Kernel>
-static cudaError_t allow_smem(Kernel kernel, int bytes, bool* configured)
+static cudaError_t allow_smem(Kernel kernel, int bytes, bool* configured, int launch_regs = 0)
 {
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess || dev >= 64 || configured[dev]) return e;
     e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess && launch_regs > 0) {
+        cudaFuncAttributes fa;
+        e = cudaFuncGetAttributes(&fa, kernel);
+        if (e == cudaSuccess && fa.numRegs < launch_regs) e = cudaErrorInvalidKernelImage;
+    }
     if (e == cudaSuccess) configured[dev] = true;
     return e;
 }
@@ -791,13 +798,8 @@ static cudaError_t launch_input_wide(GradArgs a, const GradPlan& p, const float*
 {
     using Cfg = GradInputWideCfg<NKEEP>;
     static bool configured[64] = {};
-    cudaError_t e = allow_smem(nm_grad_input_wide_kernel<NKEEP>, Cfg::SMEM_BYTES, configured);
+    cudaError_t e = allow_smem(nm_grad_input_wide_kernel<NKEEP>, Cfg::SMEM_BYTES, configured, Cfg::LAUNCH_REGS);
     if (e != cudaSuccess) return e;
-    // the compute warps' share comes out of what the launch is given: less of it and they would wait
-    cudaFuncAttributes fa;
-    e = cudaFuncGetAttributes(&fa, nm_grad_input_wide_kernel<NKEEP>);
-    if (e != cudaSuccess) return e;
-    if (fa.numRegs < Cfg::LAUNCH_REGS) return cudaErrorInvalidKernelImage;
     const int ldm = (a.M + 3) / 4 * 4, ldw = (a.W + 3) / 4 * 4;
     float* g_cols = scratch;
     float* b_cols = g_cols + transposed_floats(a.M, a.N);
