@@ -248,7 +248,10 @@ int nmspmm_gemm_gather(const nmspmm_gemm_desc* desc,
 
 /* Same, with scratch that the library allocates on first use and keeps per host thread
  * (cudaMalloc inside the first call that needs it).  For callers bound to the
- * reference's launcher signatures, which carry no workspace argument. */
+ * reference's launcher signatures, which carry no workspace argument.  The scratch is that of
+ * nmspmm_gemm_call_workspace_bytes; under stream capture, where nothing may be allocated, and where memory runs
+ * out, nmspmm_gemm_workspace_bytes of it are enough (none for most descriptions).  Scratch that was handed
+ * out under capture stays the graph's until nmspmm_release_cached. */
 int nmspmm_gemm_with_cached_workspace(const nmspmm_gemm_desc* desc,
                                       const float* A_dev, const float* B_dev, const int* D_dev,
                                       const int* column_info_dev, float* C_dev, void* stream);

@@ -647,34 +647,68 @@ static int sm_count()
 
 // ---- cached scratch for the entry points whose signature has no workspace ---------
 // One buffer per device and host thread: a thread that alternates between GPUs keeps each
-// GPU's buffer (and never frees one device's memory with another device current).
+// GPU's buffer (and never frees one device's memory with another device current).  A buffer that was
+// handed out under stream capture belongs to a graph, which may run as long as the process does: a
+// larger one takes its place but it is not freed (nmspmm_release_cached does).  What follows one is at
+// least twice as large, so that all such buffers together are smaller than the one in use.
 struct Scratch {
     void* ptr = nullptr;
     size_t bytes = 0;
+    size_t refused = SIZE_MAX;      // what memory did not suffice for: not asked for again
+    bool captured = false;
+    std::vector<void*> retired;
 };
 static thread_local Scratch tl_scratch[64];
 
-static int scratch_reserve(size_t bytes, void** out, size_t* have)
+static bool is_capturing(cudaStream_t st)
+{
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &status) == cudaSuccess) return status != cudaStreamCaptureStatusNone;
+    cudaGetLastError();                                    // the legacy stream while another one is captured
+    return true;
+}
+
+// At least `least` bytes, `wanted` where they can be had: not under capture, where nothing may be allocated, unless they are
+// there already, and not when memory runs out.
+static int scratch_reserve(size_t least, size_t wanted, cudaStream_t st, void** out, size_t* have)
 {
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return cuda_fail(e);
     if (dev < 0 || dev >= 64) return NMSPMM_UNSUPPORTED;
     Scratch& s = tl_scratch[dev];
-    if (s.bytes < bytes) {
+    const bool capturing = is_capturing(st);
+    if (s.bytes < (capturing || wanted >= s.refused ? least : wanted)) {
+        const size_t grown = s.captured ? 2 * s.bytes : 0;
         if (s.ptr) {
             cudaDeviceSynchronize();                       // launches that still use the old buffer
-            cudaFree(s.ptr);
+            if (s.captured) s.retired.push_back(s.ptr);
+            else cudaFree(s.ptr);
             s.ptr = nullptr;
             s.bytes = 0;
+            s.captured = false;
         }
-        size_t want = bytes < (size_t(8) << 20) ? (size_t(8) << 20) : bytes;
+        const size_t floor = grown > (size_t(8) << 20) ? grown : size_t(8) << 20;
+        size_t want = wanted > floor ? wanted : floor;
         e = cudaMalloc(&s.ptr, want);
-        if (e != cudaSuccess) return cuda_fail(e);
-        e = cudaMemset(s.ptr, 0, want);
-        if (e != cudaSuccess) return cuda_fail(e);
+        if (e == cudaErrorMemoryAllocation && least < want) {
+            cudaGetLastError();
+            s.refused = wanted;
+            want = least;
+            e = want > 0 ? cudaMalloc(&s.ptr, want) : cudaSuccess;
+        }
+        if (e != cudaSuccess) {
+            s.ptr = nullptr;
+            return cuda_fail(e);
+        }
+        if (want > 0 && (e = cudaMemset(s.ptr, 0, want)) != cudaSuccess) {
+            cudaFree(s.ptr);
+            s.ptr = nullptr;
+            return cuda_fail(e);
+        }
         s.bytes = want;
     }
+    if (capturing && s.ptr) s.captured = true;
     *out = s.ptr;
     *have = s.bytes;
     return NMSPMM_OK;
@@ -708,7 +742,10 @@ static int arena_reserve(size_t bytes, unsigned char** out, cudaStream_t* st, Ar
             a.bytes = 0;
         }
         e = cudaMalloc(&a.ptr, bytes);
-        if (e != cudaSuccess) return cuda_fail(e);
+        if (e != cudaSuccess) {
+            a.ptr = nullptr;
+            return cuda_fail(e);
+        }
         a.bytes = bytes;
         if (a.device != dev || !a.stream) {
             if ((e = cudaStreamCreateWithFlags(&a.stream, cudaStreamNonBlocking)) != cudaSuccess) return cuda_fail(e);
@@ -1210,11 +1247,11 @@ int nmspmm_device_status(int* status_out, int clear)
 int nmspmm_gemm_with_cached_workspace(const nmspmm_gemm_desc* desc, const float* A_dev, const float* B_dev,
                                       const int* D_dev, const int* column_info_dev, float* C_dev, void* stream)
 {
-    const size_t need = nmspmm_gemm_call_workspace_bytes(desc);
+    const size_t wanted = nmspmm_gemm_call_workspace_bytes(desc);
     void* ws = nullptr;
     size_t have = 0;
-    if (need > 0) {
-        int rc = scratch_reserve(need, &ws, &have);
+    if (wanted > 0) {
+        int rc = scratch_reserve(nmspmm_gemm_workspace_bytes(desc), wanted, static_cast<cudaStream_t>(stream), &ws, &have);
         if (rc != NMSPMM_OK) return rc;
     }
     return nmspmm_gemm(desc, A_dev, B_dev, D_dev, column_info_dev, C_dev, ws, have, stream);
@@ -1304,12 +1341,13 @@ int nmspmm_gemm_host(const nmspmm_gemm_desc* desc, const float* A_host, const fl
     if (n_chunks < 1) n_chunks = 1;
     const int chunk_rows = (M / n_chunks + 127) / 128 * 128;
     n_chunks = (M + chunk_rows - 1) / chunk_rows;
-    size_t ws_need = 0;
+    size_t ws_need = 0, ws_least = 0;
     for (int c = 0; c < n_chunks; ++c) {
         nmspmm_gemm_desc dc = *desc;
         dc.M = (c + 1 < n_chunks) ? chunk_rows : M - c * chunk_rows;
-        const size_t need = nmspmm_gemm_call_workspace_bytes(&dc);
+        const size_t need = nmspmm_gemm_call_workspace_bytes(&dc), least = nmspmm_gemm_workspace_bytes(&dc);
         if (need > ws_need) ws_need = need;
+        if (least > ws_least) ws_least = least;
     }
 
     const size_t a_b = round256(sizeof(float) * M * static_cast<size_t>(K));
@@ -1317,11 +1355,17 @@ int nmspmm_gemm_host(const nmspmm_gemm_desc* desc, const float* A_host, const fl
     const size_t d_b = round256(sizeof(int) * W * static_cast<size_t>(Q));
     const size_t c_b = round256(sizeof(float) * M * static_cast<size_t>(N));
     const size_t ci_b = high ? round256(sizeof(int) * (static_cast<size_t>(W / pn_m) * (N / desc->layout_ns) + 1) * pm_m) : 0;
-    const size_t ws_b = round256(ws_need);
+    const size_t operands = a_b + b_b + 2 * d_b + c_b + ci_b;
+    size_t ws_b = round256(ws_need);
     unsigned char* base = nullptr;
     cudaStream_t st = nullptr;
     Arena* arp = nullptr;
-    rc = arena_reserve(a_b + b_b + 2 * d_b + c_b + ci_b + ws_b, &base, &st, &arp);
+    rc = arena_reserve(operands + ws_b, &base, &st, &arp);
+    if (rc == NMSPMM_CUDA_ERROR && tl_last_cuda_error == cudaErrorMemoryAllocation && round256(ws_least) < ws_b) {
+        cudaGetLastError();                                // memory for the named plans' scratch, then
+        ws_b = round256(ws_least);
+        rc = arena_reserve(operands + ws_b, &base, &st, &arp);
+    }
     if (rc != NMSPMM_OK) return rc;
     Arena& ar = *arp;
     if (stream) st = static_cast<cudaStream_t>(stream);
@@ -1331,7 +1375,7 @@ int nmspmm_gemm_host(const nmspmm_gemm_desc* desc, const float* A_host, const fl
     int* dD = reinterpret_cast<int*>(base + a_b + b_b + d_b);
     float* dC = reinterpret_cast<float*>(base + a_b + b_b + 2 * d_b);
     int* dCI = reinterpret_cast<int*>(base + a_b + b_b + 2 * d_b + c_b);
-    unsigned char* dWS = base + a_b + b_b + 2 * d_b + c_b + ci_b;
+    unsigned char* dWS = base + operands;
     cudaError_t e;
 #define NMSPMM_TRY(call) do { if ((e = (call)) != cudaSuccess) return cuda_fail(e); } while (0)
     // the copy streams start where the caller's stream is now
@@ -1430,10 +1474,11 @@ int nmspmm_release_cached(void)
     for (int dev = 0; dev < 64; ++dev) {
         Scratch& s = tl_scratch[dev];
         Arena& a = tl_arena[dev];
-        if (!s.ptr && !a.ptr && !a.stream) continue;
+        if (!s.ptr && s.retired.empty() && !a.ptr && !a.stream) continue;
         cudaSetDevice(dev);
         cudaDeviceSynchronize();
         if (s.ptr) cudaFree(s.ptr);
+        for (void* p : s.retired) cudaFree(p);
         s = Scratch();
         if (a.ptr) cudaFree(a.ptr);
         if (a.stream) {
