@@ -268,18 +268,18 @@ int nmspmm_gemm_with_cached_workspace(const nmspmm_gemm_desc* desc,
  * held until the process exits.  The call is nmspmm_gemm with that array as workspace; it
  * calls no cudaMalloc, cudaFree or other allocating routine.
  *
- *  - With split_k = 0 the library first tries its automatic schedule; where that wants more
- *    than the array holds (it sizes its ranges for the machine: two slots per resident CTA)
- *    it falls back to the largest number of equal K slices per tile whose slots fit, down
+ *  - With split_k = 0 the library takes the plan that nmspmm_gemm takes with that much scratch; where that
+ *    wants more than the array holds (the automatic schedule sizes its ranges for the machine: two slots
+ *    per resident CTA) it falls back to the largest number of equal K slices per tile whose slots fit, down
  *    to whole tiles, which need no scratch.  The result is the same sum in a different
- *    order; it can be slower than nmspmm_gemm with caller scratch on skinny or deep-K shapes.
+ *    order; it can be slower than nmspmm_gemm with caller scratch: on skinny and deep-K shapes, and on
+ *    large ones, whose wide tiles (nmspmm_gemm_call_workspace_bytes) mostly want 39 MB.
  *  - An explicit split_k whose slots exceed NMSPMM_STATIC_SCRATCH_BYTES is rejected with
  *    NMSPMM_WORKSPACE_TOO_SMALL and a message on stderr (nothing is launched).
  *  - The first call on a device looks the array's address up (cudaGetSymbolAddress, with
  *    that device current) and keeps it; make that first call before any stream capture.
- *  - Every call uses the same array and it keeps the previous call's contents.  The
- *    arrival counters at its head are cleared on `stream` ahead of the kernel; the slots
- *    are written before they are read.  Two calls that overlap on the GPU (different
+ *  - Every call uses the same array and it keeps the previous call's contents.  It starts zero,
+ *    and every call leaves the arrival counters at its head so; the slots are written before they are read.  Two calls that overlap on the GPU (different
  *    streams, or different host threads) race on it: serialise them. */
 #define NMSPMM_STATIC_SCRATCH_BYTES (16u << 20)
 int nmspmm_gemm_static_scratch(const nmspmm_gemm_desc* desc,

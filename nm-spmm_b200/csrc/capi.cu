@@ -1275,25 +1275,23 @@ int nmspmm_gemm_static_scratch(const nmspmm_gemm_desc* desc, const float* A_dev,
     if (!desc) return NMSPMM_INVALID_ARGUMENT;
     nmspmm_gemm_desc d = *desc;
     size_t need = nmspmm_gemm_workspace_bytes(&d);
-    if (need > static_cast<size_t>(NMSPMM_STATIC_SCRATCH_BYTES) && desc->split_k == 0) {
+    Plan p;
+    if (desc->split_k == 0 && plan_call(desc, sm_count(), NMSPMM_STATIC_SCRATCH_BYTES, &p) == NMSPMM_OK) {
+        need = scratch_bytes(p);                           // of the plan that a call with this much scratch runs
         // The automatic schedule sizes its ranges for the machine, not for this array (two
         // slots per resident CTA).  Fall back to the largest number of equal K slices per
         // tile whose slots fit; a single slice is a whole tile and needs no scratch at all.
-        Plan p;
-        DeviceInfo* di = nullptr;
-        int rc = device_info(&di);
-        if (rc != NMSPMM_OK) return rc;
-        rc = make_plan(desc, di->sms, &p);
-        if (rc != NMSPMM_OK) return rc;
-        const size_t per_slot = p.slots > 0 ? p.partial_bytes / static_cast<size_t>(p.slots) : 0;
-        long long s = per_slot ? static_cast<long long>(NMSPMM_STATIC_SCRATCH_BYTES / (per_slot * static_cast<size_t>(p.n_tiles))) : 1;
-        if (s > p.n_win) s = p.n_win;
-        for (; s >= 1; --s) {
-            d.split_k = static_cast<int>(s);
-            need = nmspmm_gemm_workspace_bytes(&d);
-            if (need <= static_cast<size_t>(NMSPMM_STATIC_SCRATCH_BYTES)) break;
+        if (need > static_cast<size_t>(NMSPMM_STATIC_SCRATCH_BYTES)) {
+            const size_t per_slot = p.slots > 0 ? p.partial_bytes / static_cast<size_t>(p.slots) : 0;
+            long long s = per_slot ? static_cast<long long>(NMSPMM_STATIC_SCRATCH_BYTES / (per_slot * static_cast<size_t>(p.n_tiles))) : 1;
+            if (s > p.n_win) s = p.n_win;
+            for (; s >= 1; --s) {
+                d.split_k = static_cast<int>(s);
+                need = nmspmm_gemm_workspace_bytes(&d);
+                if (need <= static_cast<size_t>(NMSPMM_STATIC_SCRATCH_BYTES)) break;
+            }
+            if (s < 1) d.split_k = 1, need = nmspmm_gemm_workspace_bytes(&d);
         }
-        if (s < 1) d.split_k = 1, need = nmspmm_gemm_workspace_bytes(&d);
     }
     if (need > static_cast<size_t>(NMSPMM_STATIC_SCRATCH_BYTES)) {
         fprintf(stderr,
@@ -1314,9 +1312,9 @@ int nmspmm_gemm_static_scratch(const nmspmm_gemm_desc* desc, const float* A_dev,
         }
         scratch = g_static_scratch_ptr[dev];
     }
-    // (the arrival counters at the head of the scratch are cleared on the stream by the
-    // multiply itself; the slots behind them are fully written before they are read)
-    return nmspmm_gemm(&d, A_dev, B_dev, D_dev, column_info_dev, C_dev, need ? scratch : nullptr, need, stream);
+    // (the array starts zero and every multiply leaves the arrival counters at its head so; the
+    // slots behind them are fully written before they are read)
+    return nmspmm_gemm(&d, A_dev, B_dev, D_dev, column_info_dev, C_dev, scratch, NMSPMM_STATIC_SCRATCH_BYTES, stream);
 }
 
 int nmspmm_gemm_host(const nmspmm_gemm_desc* desc, const float* A_host, const float* B_host, const int* DT_host,

@@ -91,6 +91,18 @@ def test_static_scratch_takes_shapes_whose_automatic_plan_is_too_big(pkg, M, pat
         assert _rel(got, want) <= tol
 
 
+def test_static_scratch_holds_the_pieces_of_192_column_tiles(pkg):
+    """A plan that wants a little more than the named one and fits the array: the one that a caller with scratch gets."""
+    M, N, K, n_keep = 128, 1024, 1024, 16
+    op = pkg.NMSpMM.from_problem(pkg.formats.make_random(M, N, K, n_keep, seed=98))
+    desc = op.desc(M, path=pkg.PATH_TF32)
+    assert pkg.workspace_bytes(desc) < pkg.call_workspace_bytes(desc) <= pkg.STATIC_SCRATCH_BYTES
+    assert pkg.call_plan(desc, pkg.STATIC_SCRATCH_BYTES).tile == pkg.TILE_128x192
+    A, got = torch.randn((K, M), device="cuda"), torch.full((M, N), float("nan"), device="cuda")
+    pkg.gemm_static_scratch(desc, A, op.B, op.D, op.column_info, got)
+    assert torch.equal(got, op.matmul(A, path=pkg.PATH_TF32)) and pkg.device_status() == 0
+
+
 def test_static_scratch_rejects_sizes_beyond_the_array(pkg):
     p = pkg.formats.make_random(128, 1024, 4096, 8, seed=95)
     op = pkg.NMSpMM.from_problem(p)
