@@ -615,7 +615,8 @@ class NMSpMM:
         packing kernels)."""
         fmt = format_of(n_keep) if fmt is None else fmt
         K, N = dense.shape
-        if cls is NMSpMM and layout_ns == 128 and N % 128 == 0 and K % (64 if fmt == FORMAT_HIGH else 32) == 0:
+        if (cls is NMSpMM and layout_ns == 128 and N % 128 == 0 and fmt in (FORMAT_LOW, FORMAT_HIGH) and 1 <= n_keep <= 32
+                and K % (64 if fmt == FORMAT_HIGH else 32) == 0):
             op = cls.__new__(cls)
             op.K, op.n_keep, op.layout_ns, op.vec_len, op.format = K, n_keep, layout_ns, vec_len, fmt
             op.B, op.D, op.column_info = prune_pack_device(dense, n_keep, fmt, vec_len)

@@ -32,3 +32,13 @@ def test_same_as_apart(pkg, n_keep, fmt, K, N, vec_len, values):
     if values == "random":
         A = torch.randn((K, 8), device="cuda", generator=gen)
         assert torch.equal(op.matmul(A), apart.matmul(A))
+
+
+def test_what_one_pass_does_not_take_goes_the_two_step_way(pkg):
+    dense = torch.randn((128, 256), device="cuda")
+    for n_keep in (0, 33):
+        with pytest.raises(pkg.NMSpMMError) as e:
+            pkg.NMSpMM.from_dense(dense, n_keep, fmt=pkg.FORMAT_HIGH)
+        assert e.value.status == pkg.INVALID_ARGUMENT
+    other = pkg.NMSpMM.from_dense(dense, 8, fmt=2)               # no format of the multiply: packed as the 32-k one
+    assert torch.equal(other.D, pkg.NMSpMM.from_dense(dense, 8, fmt=pkg.FORMAT_LOW).D) and other.format == 2
