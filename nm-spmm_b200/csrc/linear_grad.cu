@@ -695,15 +695,6 @@ static GradPlan plan_input(int M, int N, int K, int sms)
     return p;
 }
 
-// Whether the input's gradient takes the larger register tiles and the two transposing passes ahead of them: not at
-// 4:32, where one warp holds a vector's kept rows and eight in turn on one patch of the accumulator wait for one
-// another (2048 x 4096 x 4096: 250 -> 275 us), and not where the passes and their launches cost more than the tiles
-// save (20 us of products at the FMA peak: 256 x 4096 x 4096, 8:32, 29 us of them, 75.7 -> 68.7; 128 rows, 14 us, 45.9 -> 48.1).
-static bool wide_input_pays(int M, int N, int K, int n_keep)
-{
-    return n_keep != 4 && static_cast<double>(M) * N * (K / 32 * n_keep) >= 7.4e8;
-}
-
 template <int NKEEP>
 static GradPlan plan_input_wide(int M, int N, int K, int sms)
 {
@@ -715,6 +706,36 @@ static GradPlan plan_input_wide(int M, int N, int K, int sms)
     p.tiles = p.tiles_x * ((M + Cfg::MT - 1) / Cfg::MT);
     cut_tiles(p.tiles, sms, N / 32, 8, 4.0 / (N / 32 > 4 ? N / 32 : 4), &p.whole, &p.slices);
     return p;
+}
+
+// About how long the input's gradient takes on a plan, in microseconds: the launches, the products of the busiest SM (at
+// the FMA peak of one, 128 a cycle at 1.965 GHz, times what the kernel takes of it: 55 % / 68 %), the slices' way through
+// scratch and, for the larger register tiles, the two transposing passes.
+static double input_us(const GradPlan& p, bool wide, int M, int N, int K, int n_keep, int sms)
+{
+    const long long cut = static_cast<long long>(p.tiles - p.whole) * p.slices;
+    const double rounds = (p.whole + sms - 1) / sms + (p.tiles > p.whole ? static_cast<double>((cut + sms - 1) / sms) / p.slices : 0.0);
+    const double slowdown = wide ? 1.47 : (n_keep == 8 ? 1.83 : (n_keep == 12 ? 1.74 : 1.75));
+    double us = (wide ? 17.3 : 12.1) + slowdown * rounds * (p.cols / 32 * n_keep) * N * p.rows / (128 * 1965.0);
+    if (p.slices > 1) us += (wide ? 0.5 : 1.9) + 0.16e-6 * 8.0 * cut * p.rows * p.cols;
+    if (wide) us += 0.107e-6 * 8.0 * N * (M + K / 32 * static_cast<double>(n_keep));
+    return us;
+}
+
+// Whether the input's gradient takes the larger register tiles and the two transposing passes ahead of them: not at
+// 4:32, where one warp holds a vector's kept rows and eight in turn on one patch of the accumulator wait for one
+// another (2048 x 4096 x 4096: 250 -> 275 us), and elsewhere where they are 2 % under the smaller tiles by the times
+// above: least squares over 120 shapes measured both ways (64 to 8192 rows, 20 to 850 us, each time within 11 %).  On 120
+// other shapes it takes 71, which are 1.10 times as fast in the mean, the slowest of them 0.974; the best of those it leaves would be
+// 1.013.  Few rows lose what transposing B costs (100 x 4224 x 4992, 12:32, 69.6 -> 74.8 us; 128 x 17792 x 9920, 16:32, 591 -> 630).
+static bool wide_input_pays(int M, int N, int K, int n_keep, int sms)
+{
+    switch (n_keep) {
+    case 16: return 1.02 * input_us(plan_input_wide<16>(M, N, K, sms), true, M, N, K, 16, sms) < input_us(plan_input<16>(M, N, K, sms), false, M, N, K, 16, sms);
+    case 12: return 1.02 * input_us(plan_input_wide<12>(M, N, K, sms), true, M, N, K, 12, sms) < input_us(plan_input<12>(M, N, K, sms), false, M, N, K, 12, sms);
+    case 8: return 1.02 * input_us(plan_input_wide<8>(M, N, K, sms), true, M, N, K, 8, sms) < input_us(plan_input<8>(M, N, K, sms), false, M, N, K, 8, sms);
+    default: return false;
+    }
 }
 
 static size_t transposed_floats(int rows, int cols) { return static_cast<size_t>((rows + 3) / 4 * 4) * cols; }     // [cols][rows up to a multiple of 4]
@@ -843,7 +864,7 @@ size_t grad_values_scratch_bytes(int M, int N, int K, int n_keep, int sms)
 
 size_t grad_input_scratch_bytes(int M, int N, int K, int n_keep, int sms)
 {
-    if (wide_input_pays(M, N, K, n_keep)) {
+    if (wide_input_pays(M, N, K, n_keep, sms)) {
         const GradPlan p = n_keep == 16 ? plan_input_wide<16>(M, N, K, sms) : (n_keep == 12 ? plan_input_wide<12>(M, N, K, sms) : plan_input_wide<8>(M, N, K, sms));
         return (transposed_floats(M, N) + transposed_floats(K / 32 * n_keep, N) + p.partial_floats()) * sizeof(float);
     }
@@ -882,7 +903,7 @@ cudaError_t launch_grad_input(int dtype, const float* grad_y, const float* B, co
     a.status = status;
     a.dtype = dtype;
     a.M = M; a.N = N; a.K = K; a.W = K / 32 * n_keep;
-    if (wide_input_pays(M, N, K, n_keep)) {
+    if (wide_input_pays(M, N, K, n_keep, sms)) {
         switch (n_keep) {
         case 16: return launch_input_wide<16>(a, plan_input_wide<16>(M, N, K, sms), grad_y, scratch, st);
         case 12: return launch_input_wide<12>(a, plan_input_wide<12>(M, N, K, sms), grad_y, scratch, st);
