@@ -1282,6 +1282,7 @@ int nmspmm_gemm_static_scratch(const nmspmm_gemm_desc* desc, const float* A_dev,
         // slots per resident CTA).  Fall back to the largest number of equal K slices per
         // tile whose slots fit; a single slice is a whole tile and needs no scratch at all.
         if (need > static_cast<size_t>(NMSPMM_STATIC_SCRATCH_BYTES)) {
+            if (p.v && p.n_tiles >= sm_count()) d.tile = p.v->tile_id;     // (a tuned entry's tile, where its whole tiles fill the SMs)
             const size_t per_slot = p.slots > 0 ? p.partial_bytes / static_cast<size_t>(p.slots) : 0;
             long long s = per_slot ? static_cast<long long>(NMSPMM_STATIC_SCRATCH_BYTES / (per_slot * static_cast<size_t>(p.n_tiles))) : 1;
             if (s > p.n_win) s = p.n_win;

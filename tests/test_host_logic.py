@@ -301,6 +301,20 @@ def test_tile_of_the_exact_path_follows_padding_and_pairs(pkg, M, K, n_keep, til
     assert pkg.plan(pkg.make_desc(M, 4096, K, n_keep, pkg.format_of(n_keep), 128)).tile_m == tile_m
 
 
+@pytest.mark.parametrize("M,N,K,n_keep", [(512, 24576, 8192, 4), (512, 24576, 8192, 8), (1024, 12288, 4096, 4), (1024, 12288, 4096, 8),
+                                          (1024, 22016, 8192, 8), (2048, 6144, 2048, 8)])
+def test_tuned_shapes_keep_an_entry_for_callers_with_the_named_scratch(pkg, M, N, K, n_keep):
+    """These ran a tuned tile on the scratch of nmspmm_gemm_workspace_bytes before calls took wide tiles by themselves: without an
+    entry that scratch is none, and a caller who sizes by it would be back on the untuned tile."""
+    d = pkg.make_desc(M, N, K, n_keep, 1, 128)
+    saved = pkg.tuned_plans_snapshot_and_clear()
+    try:
+        pkg.load_tuned_plans(pkg.tuner.default_table_path())
+        assert pkg.plan(d).tile == pkg.call_plan(d, pkg.workspace_bytes(d)).tile == pkg.TILE_128x256
+    finally:
+        pkg.tuned_plans_restore(saved)
+
+
 def test_the_few_rows_kernels_do_not_spill(pkg_host):
     """What ptxas said when the library was built: the 64-row tiles have 128 registers for four CTAs per SM."""
     report = os.path.join(pkg_host.build.OBJ, "gemm_tf32_few_rows.cu.o.ptxas.txt")
