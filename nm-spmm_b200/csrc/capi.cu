@@ -606,23 +606,33 @@ static int make_plan(const nmspmm_gemm_desc* d_in, int sms, Plan* p, bool any_ro
 static size_t scratch_bytes(const Plan& p) { return p.counters_bytes + p.partial_bytes; }
 
 // About how long a tensor-core plan of 256- or 192-column tiles (one CTA per SM, 32-wide vectors) takes, in
-// microseconds.  A step's time hardly depends on the width where the issuing threads bound it (8:32: 220 ns either
-// way) and follows it where two gather results at 256 columns against three at 192 do (16:32, 12:32: 423 / 320;
-// 4:32, a merged window: 418 / 365); a tile costs 6 us beside its steps (2048 x 9472 x 4096 and 4096 cubed, FP32).
-static double tf32_plan_us(const Plan& p, int sms)
+// microseconds: its steps, what a tile costs beside them, and for slices their way through scratch and the latency of the
+// kernel that adds them (four words a thread, four slices in flight, up to eight slices; one word, sixteen in flight, over
+// that).  Least squares over 590 calls (65 to 4096 rows, K to 11008, weights from HBM), 5.5 % standard deviation; three
+// constants for all activations, from three shapes, had made calls up to 20 % slower (73 x 512 x 9216 and other small ones,
+// 3242 x 640 x 6656, 4:32, bfloat16: 27.5 -> 29.3 us).
+static double tf32_plan_us(const Plan& p, int sms, bool rows16)
 {
-    const bool narrow = p.tv->ns == 192;
-    const double step = (p.tv->n_keep == 8 ? 220 : (p.tv->n_keep == 4 ? (narrow ? 365 : 418) : (narrow ? 320 : 423))) * 1e-3;
-    double us = (p.n_dp + sms - 1) / sms * (p.n_win * step + (narrow ? 5.0 : 6.0));
-    if (p.grid > p.n_dp) us += (p.n_win + p.split_k - 1) / p.split_k * step + 9.0;       // the slices of the rest, and their sum
+    static const double kStep[2][4][2] = { { { 0.429, 0.318 }, { 0.429, 0.316 }, { 0.220, 0.218 }, { 0.425, 0.399 } },      // FP32, 16 / 12 / 8 / 4 of 32: 256 and 192 columns
+                                           { { 0.347, 0.233 }, { 0.342, 0.233 }, { 0.193, 0.177 }, { 0.206, 0.227 } } };    // rows of 16 bits
+    static const double kTile[2][2] = { { 5.1, 4.7 }, { 4.7, 4.0 } };
+    const int narrow = p.tv->ns == 192, ratio = p.tv->n_keep == 16 ? 0 : (p.tv->n_keep == 12 ? 1 : (p.tv->n_keep == 8 ? 2 : 3));
+    const double step = kStep[rows16][ratio][narrow], tile = kTile[rows16][narrow];
+    double us = (p.n_dp + sms - 1) / sms * (p.n_win * step + tile);
+    if (p.grid > p.n_dp)
+        us += (p.n_win + p.split_k - 1) / p.split_k * step + tile + 0.18e-6 * p.partial_bytes +
+              (p.split_k <= 8 ? 1.0 + 1.7 * ((p.split_k + 3) / 4) : 0.7 + 0.9 * ((p.split_k + 15) / 16));
     return us;
 }
 
 // The plan a call runs that has `workspace_bytes` of scratch: make_plan's, or where the description leaves tile and
 // split to the library and no tuned entry names them another's if its scratch fits: on the exact path a
 // wide tile's (pick_wide_tile); on the tensor cores that of 192-column tiles, where they leave fewer SMs
-// idle (256 x 11008 x 4096, bfloat16: 116 tiles instead of 86, 16:32 52.1 -> 35.1 us, 8:32 29.7 -> 27.8).
-static int plan_call(const nmspmm_gemm_desc* d, int sms, size_t workspace_bytes, Plan* p, bool any_rows = false, size_t* own_bytes = nullptr)
+// idle (256 x 11008 x 4096, bfloat16: 116 tiles instead of 86, 16:32 52.1 -> 35.1 us, 8:32 29.7 -> 27.8) and are 3 % under by
+// the times above: of 395 calls that the times were not fitted to it takes 212, 1.14 times as fast in the mean, 0.90 the least,
+// nine under 0.98.  More than 16 slices of a few tiles take longer than the times say (84 x 512 x 6976, 16:32, 13.3 -> 15.8).
+// rows16: the activations are read as rows of 16-bit values.
+static int plan_call(const nmspmm_gemm_desc* d, int sms, size_t workspace_bytes, Plan* p, bool any_rows = false, bool rows16 = false, size_t* own_bytes = nullptr)
 {
     const int rc = make_plan(d, sms, p, any_rows);
     if (rc == NMSPMM_OK && own_bytes) *own_bytes = scratch_bytes(*p);      // of the description's own plan
@@ -635,7 +645,7 @@ static int plan_call(const nmspmm_gemm_desc* d, int sms, size_t workspace_bytes,
     w.tile = tensor ? kTile128x192 : pick_wide_tile(d, p->v->mode, sms);
     Plan wp;
     if (w.tile == kTileAuto || make_plan(&w, sms, &wp, any_rows) != NMSPMM_OK || scratch_bytes(wp) > workspace_bytes) return rc;
-    if (!tensor || tf32_plan_us(wp, sms) < 0.98 * tf32_plan_us(*p, sms)) *p = wp;
+    if (!tensor || (wp.split_k <= 16 && tf32_plan_us(wp, sms, rows16) < 0.97 * tf32_plan_us(*p, sms, rows16))) *p = wp;
     return rc;
 }
 
@@ -898,7 +908,7 @@ size_t nmspmm_gemm_call_workspace_bytes(const nmspmm_gemm_desc* desc)
 {
     Plan c;
     size_t own = 0;
-    if (plan_call(desc, sm_count(), SIZE_MAX, &c, false, &own) != NMSPMM_OK) return 0;
+    if (plan_call(desc, sm_count(), SIZE_MAX, &c, false, false, &own) != NMSPMM_OK) return 0;
     return own > scratch_bytes(c) ? own : scratch_bytes(c);
 }
 
@@ -956,7 +966,7 @@ static int gemm_launch(const nmspmm_gemm_desc* desc, const float* A_dev, const f
     int rc = device_info(&di);
     if (rc != NMSPMM_OK) return rc;
     Plan p;
-    rc = plan_call(desc, di->sms, aligned16(workspace_dev) && workspace_dev ? workspace_bytes : 0, &p, lda != 0 || a_rows != 0);
+    rc = plan_call(desc, di->sms, aligned16(workspace_dev) && workspace_dev ? workspace_bytes : 0, &p, lda != 0 || a_rows != 0, a_rows > 1 + kDtypeF32);
     if (rc != NMSPMM_OK) return rc;
     if (lda != 0 && (lda < desc->M || lda % 4 != 0)) return NMSPMM_INVALID_ARGUMENT;
     if (!A_dev || !B_dev || !D_dev || !C_out || n_out < 1 || n_out > kMaxOutputs) return NMSPMM_INVALID_ARGUMENT;
@@ -1047,11 +1057,15 @@ static bool overlap(const void* a, size_t a_bytes, const void* b, size_t b_bytes
 // they want them on 16 bytes); the others -- the exact path, the expanding form, and 16-bit rows of
 // an unpruned weight, whose product takes A and B in one type -- get a col-major copy.  So does a
 // call whose result overwrites its activations: the copy is complete before C is written.
-static bool reads_rows(const Plan& p, const nmspmm_gemm_desc* d, const void* A_rows, const void* C, int dtype)
+static bool rows_as_they_lie(const nmspmm_gemm_desc* d, const void* A_rows, const void* C, int dtype)
 {
     const size_t size = dtype == kDtypeF32 ? 4 : 2;
-    return p.tv && p.tv->form != 1 && aligned16(A_rows) && (dtype == kDtypeF32 || p.tv->n_keep != 32) &&
-           !overlap(A_rows, size * d->M * d->K, C, size * d->M * d->N);
+    return aligned16(A_rows) && !overlap(A_rows, size * d->M * d->K, C, size * d->M * d->N);
+}
+
+static bool reads_rows(const Plan& p, const nmspmm_gemm_desc* d, const void* A_rows, const void* C, int dtype)
+{
+    return p.tv && p.tv->form != 1 && (dtype == kDtypeF32 || p.tv->n_keep != 32) && rows_as_they_lie(d, A_rows, C, dtype);
 }
 
 static size_t result_copy_bytes(const nmspmm_gemm_desc* d)
@@ -1066,14 +1080,14 @@ static size_t row_major_bytes(const Plan& p, const nmspmm_gemm_desc* d, int dtyp
     return row_major_head_bytes(p) + (copy_a ? row_major_copy_bytes(d) : 0) + (dtype != kDtypeF32 && !p.tv ? result_copy_bytes(d) : 0);
 }
 
-// The larger of what the description's plan and what the call's takes (plan_call); copy_a < 0: by the addresses.
-// (The two differ in their scratch alone: both of the exact path, or both reading rows.)
-static size_t row_major_bytes_any(const nmspmm_gemm_desc* d, int dtype, int copy_a, const void* A_rows = nullptr, const void* C = nullptr)
+// The larger of what the description's plan and what the call's takes (plan_call), with room for the copy of A if
+// `copy`; rows16 as there.  (The two differ in their scratch alone: both of the exact path, or both reading rows.)
+static size_t row_major_bytes_any(const nmspmm_gemm_desc* d, int dtype, bool lies_well, bool copy)
 {
     Plan c;
     size_t own = 0;
-    if (!d || plan_call(d, sm_count(), SIZE_MAX, &c, true, &own) != NMSPMM_OK) return 0;
-    const bool copy = copy_a < 0 ? !reads_rows(c, d, A_rows, C, dtype) : copy_a != 0;
+    if (!d || plan_call(d, sm_count(), SIZE_MAX, &c, true, lies_well && dtype != kDtypeF32, &own) != NMSPMM_OK) return 0;
+    if (!copy) copy = !(c.tv && c.tv->form != 1 && (dtype == kDtypeF32 || c.tv->n_keep != 32));
     const size_t head = own > 0 ? own : kCounterBlock, rest = row_major_bytes(c, d, dtype, copy) - row_major_head_bytes(c);
     return (head > row_major_head_bytes(c) ? head : row_major_head_bytes(c)) + rest;
 }
@@ -1081,7 +1095,7 @@ static size_t row_major_bytes_any(const nmspmm_gemm_desc* d, int dtype, int copy
 // The plan a row-major call with this much workspace runs.
 static int plan_row_major(const nmspmm_gemm_desc* d, const void* A_rows, const void* C, int dtype, size_t workspace_bytes, Plan* p)
 {
-    int rc = plan_call(d, sm_count(), SIZE_MAX, p, true);
+    int rc = plan_call(d, sm_count(), SIZE_MAX, p, true, dtype != kDtypeF32 && rows_as_they_lie(d, A_rows, C, dtype));
     if (rc == NMSPMM_OK && workspace_bytes < row_major_bytes(*p, d, dtype, !reads_rows(*p, d, A_rows, C, dtype))) {
         rc = make_plan(d, sm_count(), p, true);
         if (rc == NMSPMM_OK && workspace_bytes < row_major_bytes(*p, d, dtype, !reads_rows(*p, d, A_rows, C, dtype))) rc = NMSPMM_WORKSPACE_TOO_SMALL;
@@ -1089,11 +1103,12 @@ static int plan_row_major(const nmspmm_gemm_desc* d, const void* A_rows, const v
     return rc;
 }
 
-size_t nmspmm_gemm_row_major_workspace_bytes(const nmspmm_gemm_desc* desc) { return row_major_bytes_any(desc, kDtypeF32, 1); }
+size_t nmspmm_gemm_row_major_workspace_bytes(const nmspmm_gemm_desc* desc) { return row_major_bytes_any(desc, kDtypeF32, true, true); }
 
 size_t nmspmm_gemm_row_major_call_bytes(const nmspmm_gemm_desc* desc, int dtype, const void* A_rows_dev, const void* C_dev)
 {
-    return row_major_bytes_any(desc, dtype, -1, A_rows_dev, C_dev);
+    const bool lies_well = desc && rows_as_they_lie(desc, A_rows_dev, C_dev, dtype);
+    return row_major_bytes_any(desc, dtype, lies_well, !lies_well);
 }
 
 int nmspmm_gemm_row_major(const nmspmm_gemm_desc* desc, const float* A_rows_dev, const float* B_dev, const int* D_dev,
@@ -1119,7 +1134,11 @@ int nmspmm_gemm_row_major(const nmspmm_gemm_desc* desc, const float* A_rows_dev,
 // ---- activations and result in 16-bit storage ---------------------------------------------
 static_assert(NMSPMM_DTYPE_F16 == kDtypeF16 && NMSPMM_DTYPE_BF16 == kDtypeBF16, "the public dtype ids are the library's");
 
-size_t nmspmm_gemm_row_major_16_workspace_bytes(const nmspmm_gemm_desc* desc) { return row_major_bytes_any(desc, kDtypeF16, 1); }
+size_t nmspmm_gemm_row_major_16_workspace_bytes(const nmspmm_gemm_desc* desc)
+{
+    const size_t rows = row_major_bytes_any(desc, kDtypeF16, true, true), copied = row_major_bytes_any(desc, kDtypeF16, false, true);
+    return rows > copied ? rows : copied;
+}
 
 int nmspmm_gemm_row_major_16(const nmspmm_gemm_desc* desc, int dtype, const void* A_rows_dev, const float* B_dev, const int* D_dev,
                              const int* column_info_dev, void* C_dev, void* workspace_dev, size_t workspace_bytes, void* stream)

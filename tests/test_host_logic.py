@@ -301,6 +301,29 @@ def test_tile_of_the_exact_path_follows_padding_and_pairs(pkg, M, K, n_keep, til
     assert pkg.plan(pkg.make_desc(M, 4096, K, n_keep, pkg.format_of(n_keep), 128)).tile_m == tile_m
 
 
+@pytest.mark.parametrize("M,N,K,n_keep,narrow", [(256, 11008, 4096, 16, True), (2048, 9472, 4096, 8, False), (1024, 640, 4096, 12, True),
+                                                 (168, 1664, 8320, 12, False), (84, 512, 6976, 16, False), (96, 640, 9152, 4, False), (1248, 1920, 2496, 8, False)])
+def test_calls_take_192_columns_where_they_are_faster(pkg, M, N, K, n_keep, narrow):
+    d = pkg.make_desc(M, N, K, n_keep, pkg.format_of(n_keep), 128, pkg.PATH_TF32)
+    assert pkg.plan(d).tile == pkg.TILE_128x256
+    assert pkg.call_plan(d).tile == (pkg.TILE_128x192 if narrow else pkg.TILE_128x256)
+
+
+def test_what_rows_of_16_bits_take_is_asked_for(pkg):
+    """Their steps have lengths of their own, so their plan may be another than that of FP32 rows or of a copy: what the
+    entries ask for holds either."""
+    lib, base, M = pkg.load_library(), 1 << 20, 256
+    differ = 0
+    for N in (640, 1024, 2560, 4096):
+        for n_keep in (16, 12, 8, 4):
+            d, K = ctypes.byref(pkg.make_desc(M, N, 2048, n_keep, pkg.format_of(n_keep), 128, pkg.PATH_TF32)), 2048
+            far = base + 4 * M * K
+            rows, copied = (lib.nmspmm_gemm_row_major_call_bytes(d, pkg.DTYPE_BF16, a, far) for a in (base, base + 2))
+            differ += rows != copied - 4 * M * K
+            assert lib.nmspmm_gemm_row_major_16_workspace_bytes(d) == max(rows + 4 * M * K, copied)
+    assert differ
+
+
 @pytest.mark.parametrize("M,N,K,n_keep", [(512, 24576, 8192, 4), (512, 24576, 8192, 8), (1024, 12288, 4096, 4), (1024, 12288, 4096, 8),
                                           (1024, 22016, 8192, 8), (2048, 6144, 2048, 8)])
 def test_tuned_shapes_keep_an_entry_for_callers_with_the_named_scratch(pkg, M, N, K, n_keep):
