@@ -34,7 +34,7 @@ def test_edges(pkg, orc, tile, n_keep, fmt, K, M, N, layout, split_k):
     assert pkg.device_status() == 0
 
 
-@pytest.mark.parametrize("M,N,K,n_keep", [(776, 2560, 2080, 12), (64, 11008, 4096, 8), (128, 1024, 65536, 4), (2048, 1152, 4096, 16)])
+@pytest.mark.parametrize("M,N,K,n_keep", [(776, 2560, 2080, 12), (1024, 5760, 1024, 12), (2048, 5760, 1024, 16), (64, 11008, 4096, 8), (128, 1024, 65536, 4), (2048, 1152, 4096, 16)])
 def test_calls_that_take_a_wide_tile_by_themselves(pkg, M, N, K, n_keep):
     """Whatever scratch the call is handed: the wide tile where its pieces fit, the planned one otherwise.
     Row-major callers and several outputs take the same route."""
@@ -42,12 +42,15 @@ def test_calls_that_take_a_wide_tile_by_themselves(pkg, M, N, K, n_keep):
     op = pkg.NMSpMM.from_problem(p)
     A = torch.from_numpy(p.A_km).cuda()
     d = op.desc(M)
-    assert pkg.call_plan(d).tile in TILES and pkg.call_plan(d, pkg.workspace_bytes(d)).n_virtual >= 1
-    planned = op.matmul(A, tile=pkg.plan(d).tile)
+    named, taken, own = pkg.plan(d).tile, pkg.call_plan(d).tile, pkg.workspace_bytes(d)
+    fits = pkg.workspace_bytes(op.desc(M, tile=taken)) <= own
+    assert taken in TILES and pkg.call_plan(d, own).tile == (taken if fits else named)
+    planned = op.matmul(A, tile=named)
     got = op.matmul(A)
-    small = torch.zeros(max(pkg.workspace_bytes(d), 16), dtype=torch.uint8, device="cuda")
+    small = torch.zeros(max(own, 16), dtype=torch.uint8, device="cuda")
     with_less = torch.empty_like(got)
     pkg.gemm(d, A, op.B, op.D, op.column_info, with_less, small)
+    assert torch.equal(got, op.matmul(A, tile=taken)) and torch.equal(with_less, got if fits else planned)
     rows = op.matmul_rows(A.t().contiguous())
     wide_buffer = torch.full((2, M, N + 64), -1.0, device="cuda")
     op.matmul_into(A, [wide_buffer[0].data_ptr(), wide_buffer[1].data_ptr()], N + 64, 32)
