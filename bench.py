@@ -275,6 +275,15 @@ def time_steps(torch, fn, steps: int, barrier=None):
     return start.elapsed_time(end)
 
 
+EXACT_CAPTURES = {"nm_gemm_wide_kernel": "nm_gemm_wide_128x256_high_4096cubed_8of32_4of32.md",
+                  "nm_gemm_ffma_kernel": "nm_gemm_ffma_128x128_high_4096cubed_8of32.md"}
+
+
+def exact_kernel(pkg, plan) -> str:
+    """The exact path's kernel that a plan runs."""
+    return "nm_gemm_wide_kernel" if plan.tile in (pkg.TILE_128x256, pkg.TILE_256x128, pkg.TILE_64x512) else "nm_gemm_ffma_kernel"
+
+
 def run_ours(args, rank: int, world: int, local_rank: int):
     import torch
     import torch.distributed as dist
@@ -393,13 +402,13 @@ def run_ours(args, rank: int, world: int, local_rank: int):
         "achieved": achieved, "peak": ffma_peak, "unit": "TFLOP/s", "frac": max(t_flop, t_mem) / (ms_per_step * 1e-3),
         "traffic": None,
         "traffic_source": "not measured in this run (DRAM counters need ncu); one capture of this kernel and workload is "
-                          "summarised in profiles/nm_gemm_ffma_128x128_high_4096cubed_8of32.md",
+                          f"summarised in profiles/{EXACT_CAPTURES[exact_kernel(pkg, plan)]}",
         "peak_source": "FP32 FMA rate measured live on this GPU by the library's register-only kernels, larger of "
                        f"scalar FFMA ({ffma_scalar:.1f}) and packed FFMA2 ({ffma_packed:.1f} TFLOP/s); "
                        "nominal 148 SMs x 128 lanes x 2 x SM clock",
         "algorithmic_bytes": abytes, "algorithmic_flops": useful,
         "hbm_time_us": t_mem * 1e6, "hbm_peak_gbs": hbm_gbs, "hbm_peak_source": hbm_src,
-        "kernel": f"nm_gemm_ffma_kernel tile {plan.tile_m}x{plan.tile_n}, "
+        "kernel": f"{exact_kernel(pkg, plan)} tile {plan.tile_m}x{plan.tile_n}, "
                   f"{'automatic schedule' if plan.stream_k else 'split_k ' + str(plan.split_k)}: "
                   f"{plan.tiles_x * plan.tiles_y} tiles ({plan.n_dp} whole) in {plan.n_virtual} unit ranges = CTAs, "
                   f"{plan.stages} stages, {plan.smem_bytes} B smem",
@@ -691,9 +700,8 @@ def measure_workload(pkg, torch, name: str, tile: int = 0, split_k: int = 0, ste
         out[pname] = {"ms": ms, "useful_tflops": useful / (ms * 1e-3) / 1e12, "bytes_per_s_gbs": abytes / (ms * 1e-3) / 1e9,
                       "roofline_frac": max(useful / peak, abytes / hbm) / (ms * 1e-3),
                       "bound": "hbm" if abytes / hbm > useful / peak else "flops",
-                      "kernel": (("nm_gemm_wide_kernel" if plan.tile in (pkg.TILE_128x256, pkg.TILE_256x128, pkg.TILE_64x512) else "nm_gemm_ffma_kernel")
-                                 if pname == "fp32" else
-                                 ("nm_gemm_tf32_few_rows_kernel" if plan.tile_m < 128 else "nm_gemm_tf32_kernel")),
+                      "kernel": (exact_kernel(pkg, plan) if pname == "fp32" else
+                                 "nm_gemm_tf32_few_rows_kernel" if plan.tile_m < 128 else "nm_gemm_tf32_kernel"),
                       "tile": [plan.tile_m, plan.tile_n], "ctas": plan.grid, "whole_tiles": plan.n_dp,
                       "rel_err_rows": err, "parity": bool(err <= (1e-5 if pname == "fp32" else 2e-3))}
     assert pkg.device_status() == 0
