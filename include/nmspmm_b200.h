@@ -98,7 +98,7 @@ int nmspmm_prune_device(const float* dense_dev, float* BT_dev, int* DT_dev,
 /* nmspmm_prune_device and the packing of its indices for layout_ns = 128 in one pass over the weight: BT as there, D_dev
  * (W * N / 32 ints) and, for NMSPMM_FORMAT_HIGH (K % 64 == 0), column_info_dev ((N / 128) * (K / 64) * 64 ints and one more
  * window of 64, all -1) as nmspmm_preprocess_low_device / _high_device (fused) write them.  N % 128 == 0.  The raw indices
- * are not written. */
+ * are not written (nmspmm_linear_grad wants them: then nmspmm_prune_device and the packing apart). */
 int nmspmm_prune_pack_device(const float* dense_dev, float* BT_dev, int* D_dev, int* column_info_dev, int K, int N, int n_keep,
                              int vec_len, int format, void* stream);
 
@@ -150,8 +150,9 @@ typedef struct nmspmm_gemm_desc {
                           and reads only the even list; the FP32 path computes the same either way. */
 } nmspmm_gemm_desc;
 
-/* Bytes of scratch the multiply needs for this description (0 when every unit range is a
- * whole tile).  The scratch starts with a block of per-tile arrival counters,
+/* Bytes of scratch the plan that nmspmm_gemm_plan names needs for this description (0 when every unit
+ * range is a whole tile): the least that nmspmm_gemm accepts.  A caller who has the memory gives
+ * nmspmm_gemm_call_workspace_bytes.  The scratch starts with a block of per-tile arrival counters,
  * NMSPMM_COUNTER_BYTES for every description of up to 16384 tiles, followed by slots for tile
  * pieces.  The counter block must be zero before the first use (cudaMemset once, e.g. of the
  * whole buffer); every multiply leaves it zero, and no multiply writes anything else there,
@@ -161,11 +162,14 @@ typedef struct nmspmm_gemm_desc {
  * multiply (a CTA that gave up did not arrive at its counter). */
 #define NMSPMM_COUNTER_BYTES (64u << 10)
 size_t nmspmm_gemm_workspace_bytes(const nmspmm_gemm_desc* desc);
-/* Scratch with which a call runs its fastest form.  On the exact path, where tile and split_k are left to
- * the library and no tuned entry names them, a call may run one of the wide tiles (ids 5, 10 and 11: one CTA per SM)
- * instead of the tile that nmspmm_gemm_plan names (on the TF32 path 128 x 192 instead of 128 x 256), wherever the scratch it is handed holds that tile's
- * pieces; with nmspmm_gemm_workspace_bytes alone (never more than this) it runs the named one.  The wide
- * tiles write no counters. */
+/* Scratch with which a call runs its fastest form (39 MB for most large exact calls).  On the exact path,
+ * where tile and split_k are left to the library and no tuned entry names them, a call may run one of the
+ * wide tiles (ids 5, 10 and 11: one CTA per SM) instead of the tile that nmspmm_gemm_plan names, on the TF32
+ * path 128 x 192 instead of 128 x 256, wherever the scratch it is handed holds that tile's pieces; with
+ * nmspmm_gemm_workspace_bytes (never more than this) it may have to run the named one: 4096 cubed, 8:32,
+ * 0.62 ms on no scratch, 0.565 on this.  So the size of the scratch decides the order of a result's
+ * sums: the same description and size give the same bits, another size may give others (within the path's
+ * tolerance).  The wide tiles write no counters. */
 size_t nmspmm_gemm_call_workspace_bytes(const nmspmm_gemm_desc* desc);
 /* How many bytes at the head of a workspace that no multiply has used yet have to be zero for this
  * description (any M; 0 for most): what a caller with fresh memory per call clears instead of all of it. */
@@ -224,7 +228,10 @@ int nmspmm_widen_device(int dtype, const void* src_dev, float* dst_dev, size_t n
  * M x K row-major and grad_y M x N row-major, both of `dtype`; B the compressed values and DT_dev
  * the raw window-local indices [W][N/32].  grad_x_dev (M x K, of dtype) receives
  * grad_y . B^T, grad_B_dev ([W][N], float) x^T . grad_y at the kept positions; either may be NULL
- * (then B resp. x may be too).  No result may overlap an operand.  The workspace needs no initial contents. */
+ * (then B resp. x may be too).  No result may overlap an operand.  The workspace needs no initial contents.  It holds
+ * an FP32 copy of a 16-bit grad_y, the slices of tiles that are cut, and where grad_x takes the larger register tiles
+ * (16, 12 and 8 of 32, all but small calls) transposed copies of grad_y and B: about 4 (M N + W N) bytes,
+ * 1.2 GB at 8192 x 28672 x 8192, 8:32. */
 size_t nmspmm_linear_grad_workspace_bytes(const nmspmm_gemm_desc* desc, int dtype, int want_x, int want_values);
 int nmspmm_linear_grad(const nmspmm_gemm_desc* desc, int dtype, const void* x_rows_dev, const void* grad_y_dev,
                        const float* B_dev, const int* DT_dev, void* grad_x_dev, float* grad_B_dev,

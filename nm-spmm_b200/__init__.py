@@ -315,8 +315,9 @@ def call_plan(desc: GemmDesc, scratch_bytes: Optional[int] = None) -> PlanInfo:
 
 def gemm(desc: GemmDesc, A, B, D, column_info, C, workspace=None, stream=None) -> None:
     """nmspmm_gemm on CUDA tensors.  ``A`` is (K, M) (col-major M x K), ``B`` (W, N),
-    ``C`` (M, N); ``workspace`` a uint8 tensor of at least workspace_bytes(desc)
-    whose first bytes (the counters) are zero."""
+    ``C`` (M, N); ``workspace`` a uint8 tensor of at least workspace_bytes(desc), better
+    call_workspace_bytes(desc) (the call's fastest plan; which plan runs, and so the order of the sums, follows
+    from its size), whose first bytes (the counters) are zero."""
     torch = _torch()
     ws_ptr, ws_bytes = ctypes.c_void_p(0), 0
     if workspace is not None:

@@ -34,7 +34,7 @@
 //               Issuers are one elected thread each, from first wait to last commit, operand
 //               descriptors by addition: with a warp-wide wait, a vote and descriptors built anew
 //               per instruction a step of 8:32 took 600 cycles on the issuers' side alone (2048 x 9472 x 4096, 8:32,
-//               186 -> 138 us; 256 x 11008 x 4096, bfloat16, 42 -> 31.5).
+//               186 -> 138 us; 256 x 11008 x 4096, bfloat16, 42 -> 31.5, and 28.0 with what GATHER_WARPS, PAIRS and 192 columns add).
 //   the others  (eight; four on the 128-column tile, at 16:32 and 12:32 with 32-wide vectors, and at 32:32) one
 //               thread per (vector, kept row) and turn: loads its index two to four turns ahead
 //               into registers (through column_info on the 64-k format), keeps P's one-hot
@@ -45,7 +45,9 @@
 // box (128 bytes or fewer): 128 rows of A and 64 of B, 400 cycles, at 8:32, for FP32 and 16-bit
 // activations alike -- without any tensor-core instruction the kernel takes 126 us where it takes 138 (FP32)
 // and 125 (bfloat16) with them.  16:32 and 12:32 with 32-wide vectors have room for two gather results only, and
-// a result's way to its products and back, about 500 cycles each, is exposed (780 cycles a step with everything else left out).
+// a result's way to its products and back, about 500 cycles each, is exposed (780 cycles a step with everything else left out;
+// at 4096 cubed the tensor pipe is active 59 % of an 8:32 call's cycles and 62 % of a 16:32 call's).  Long runs are also
+// under the power cap: 1.68 to 1.72 GHz there, 1.57 at 8192 x 28672 x 8192 (2817 us after a pause, 3242 back to back).
 // n_keep = 32 (nothing pruned) has the identity as its index list and multiplies A_window by
 // the B rows directly.  12:32 gathers 16 columns per vector of which 4 are zero (P has no
 // entry for them), and loads 16 rows of B per vector of which the last 4 meet those zeros.
@@ -55,7 +57,7 @@
 // gathered in their own type (kind::f16, one-hot P of that type, FP32 result: exact), K = 16 per
 // instruction: half as many gather instructions per step and half of A's bytes, no transposing and
 // widening launch ahead of the multiply, and C is stored in the activations' type.
-// 256 x 11008 x 4096, bfloat16, 8:32: 59.5 us with a transposing and a rounding launch, 31.5 now.
+// 256 x 11008 x 4096, bfloat16, 8:32: 59.5 us with a transposing and a rounding launch, 28.0 now.
 // Every wait is bounded; a wait that gives up raises the device status word.
 #include <cuda.h>
 
@@ -73,7 +75,8 @@ namespace nmspmm {
 // nmspmm_debug_tf32_profile (exported by that build only) reads and clears the sixteen sums:
 //   0 producer waits for a free stage, 1 producer total, 2 / 3 / 4 / 5 gather issuer: wait for the
 //   stage, wait for a result buffer, issue, total, 6 / 7 / 15 product issuer: wait for the gather,
-//   issue, total, 8 CTAs, 9 steps, 13 / 14 epilogue: wait for the accumulators, run.
+//   issue, total, 8 CTAs, 9 steps, 13 / 14 epilogue: wait for the accumulators, run.  The
+//   issuers of steps in pairs (Cfg::PAIRS) count nothing: 2 to 9 and 15 stay zero there.
 // Without the macro every TF_* below expands to nothing.
 #ifdef NMSPMM_TF32_PROFILE
 __device__ unsigned long long g_tf32_profile[16];
@@ -156,7 +159,7 @@ struct Tf32Cfg {
     static_assert(NBUF >= 1, "no room for a gather result beside the accumulators");
     // 16-bit activations: pairs of steps share one commit and one wait between gather and products where Tensor
     // Memory holds three pairs of results or more -- their steps are the shortest, and the products' issuers spend
-    // them waiting (256 x 11008 x 4096, 8:32, 28.4 -> 25.4 us; 2048 x 9472 x 4096, 64-wide vectors, 107 -> 102; in FP32 125 -> 127).
+    // them waiting (256 x 11008 x 4096, 8:32, 28.4 -> 27.8 us, 25.4 with the weights in L2; 2048 x 9472 x 4096, 64-wide vectors, 107 -> 102; in FP32 125 -> 127).
     // The buffers of a pair are free when the stage of its second step is; that stage's next phase may not end
     // before they are asked for; and a stage's last step is done by then, so that the wait on it is unmistakable.
     static constexpr int NP0 = DIRECT ? 0 : (TMEM_COLS - NS) / (2 * N1);
@@ -357,56 +360,56 @@ nm_gemm_tf32_kernel(const GemmArgs g, const __grid_constant__ CUtensorMap map_a,
                     if (st >= STAGES) { st -= STAGES; full_parity ^= 1; }
                 }
             } else {
-            TF_DECL(m_full = 0, m_free = 0, m_issue = 0);
-            TF_T(m_start);
-            for (int t = warp - 1; t < n_win; t += GW) {
-                TF_T(t1);
-                // the result buffer is free once the products of step t - NBUF are done, which is when that
-                // step's stage is (the stage's next phase ends with step t - NBUF + STAGES, not before this one).
-                // This wait has to come before the one on the stage: with two gathering threads and an odd number
-                // of stages, the step before in this stage was the other thread's and may still wait to be filled,
-                // where a wait by parity would take the phase before that one for the awaited one. Products are in
-                // order, so past this wait every step up to t - NBUF, t - STAGES among them, has been used up.
-                static_assert(DIRECT || NBUF <= STAGES, "a stage's last step is done once the result buffer is free");
-                if (!DIRECT && t >= NBUF) {
-                    ok = mbar_spin_bounded(empty, empty_parity, abort_word);
-                    empty += GW * 8;
-                    if (GW == 1) {
-                        if (empty == bar_empty + STAGES * 8) { empty = bar_empty; empty_parity ^= 1; }
-                    } else if (empty >= bar_empty + STAGES * 8) { empty -= STAGES * 8; empty_parity ^= 1; }
-                }
-                TF_ADD(m_free, t1);
-                TF_T(t0);
-                ok = ok && mbar_spin_bounded(full, parity, abort_word);
-                TF_ADD(m_full, t0);
-                if (!ok) break;
-                TF_T(t2);
-                tc_fence_after_sync();
-                if (DIRECT) {
-#pragma unroll
-                    for (int ks = 0; ks < Cfg::NKS; ++ks)
-                        umma_tf32_ss(tmem_addr(tmem, 0, 0), umma_desc_plus(a0, at + a_step(ks)), umma_desc_plus(b0, at + ks * 64), idesc_direct,
-                                     (t | ks) != 0);
-                    tc_commit(full + (bar_empty - bar_full));
-                } else {
-                    const uint32_t gbuf = tmem_addr(tmem, 0, Cfg::ACOL0 + buf * Cfg::N1);
-#pragma unroll
-                    for (int ks = 0; ks < Cfg::NKS; ++ks) {
-                        if constexpr (Cfg::SRC == kTf32Rows16)
-                            umma_f16_ss(gbuf, umma_desc_plus(a0, at + a_step(ks)), umma_desc_plus(p0, at + ks * P_STEP), idesc_gather, ks != 0);
-                        else
-                            umma_tf32_ss(gbuf, umma_desc_plus(a0, at + a_step(ks)), umma_desc_plus(p0, at + ks * P_STEP), idesc_gather, ks != 0);
+                TF_DECL(m_full = 0, m_free = 0, m_issue = 0);
+                TF_T(m_start);
+                for (int t = warp - 1; t < n_win; t += GW) {
+                    TF_T(t1);
+                    // the result buffer is free once the products of step t - NBUF are done, which is when that
+                    // step's stage is (the stage's next phase ends with step t - NBUF + STAGES, not before this one).
+                    // This wait has to come before the one on the stage: with two gathering threads and an odd number
+                    // of stages, the step before in this stage was the other thread's and may still wait to be filled,
+                    // where a wait by parity would take the phase before that one for the awaited one. Products are in
+                    // order, so past this wait every step up to t - NBUF, t - STAGES among them, has been used up.
+                    static_assert(DIRECT || NBUF <= STAGES, "a stage's last step is done once the result buffer is free");
+                    if (!DIRECT && t >= NBUF) {
+                        ok = mbar_spin_bounded(empty, empty_parity, abort_word);
+                        empty += GW * 8;
+                        if (GW == 1) {
+                            if (empty == bar_empty + STAGES * 8) { empty = bar_empty; empty_parity ^= 1; }
+                        } else if (empty >= bar_empty + STAGES * 8) { empty -= STAGES * 8; empty_parity ^= 1; }
                     }
-                    tc_commit(bar_gdone + buf * 8);
-                    if (GW == 1) { if (++buf == NBUF) buf = 0; }
-                    else buf = (buf + GW) % NBUF;
-                }
-                at += GW * (Cfg::STAGE_BYTES / 16);
-                full += GW * 8;
-                if (GW == 1) {
-                    if (full == bar_full + STAGES * 8) { full = bar_full; at = 0; parity ^= 1; }
-                } else if (full >= bar_full + STAGES * 8) { full -= STAGES * 8; at -= STAGES * (Cfg::STAGE_BYTES / 16); parity ^= 1; }
-                TF_ADD(m_issue, t2);
+                    TF_ADD(m_free, t1);
+                    TF_T(t0);
+                    ok = ok && mbar_spin_bounded(full, parity, abort_word);
+                    TF_ADD(m_full, t0);
+                    if (!ok) break;
+                    TF_T(t2);
+                    tc_fence_after_sync();
+                    if (DIRECT) {
+#pragma unroll
+                        for (int ks = 0; ks < Cfg::NKS; ++ks)
+                            umma_tf32_ss(tmem_addr(tmem, 0, 0), umma_desc_plus(a0, at + a_step(ks)), umma_desc_plus(b0, at + ks * 64), idesc_direct,
+                                         (t | ks) != 0);
+                        tc_commit(full + (bar_empty - bar_full));
+                    } else {
+                        const uint32_t gbuf = tmem_addr(tmem, 0, Cfg::ACOL0 + buf * Cfg::N1);
+#pragma unroll
+                        for (int ks = 0; ks < Cfg::NKS; ++ks) {
+                            if constexpr (Cfg::SRC == kTf32Rows16)
+                                umma_f16_ss(gbuf, umma_desc_plus(a0, at + a_step(ks)), umma_desc_plus(p0, at + ks * P_STEP), idesc_gather, ks != 0);
+                            else
+                                umma_tf32_ss(gbuf, umma_desc_plus(a0, at + a_step(ks)), umma_desc_plus(p0, at + ks * P_STEP), idesc_gather, ks != 0);
+                        }
+                        tc_commit(bar_gdone + buf * 8);
+                        if (GW == 1) { if (++buf == NBUF) buf = 0; }
+                        else buf = (buf + GW) % NBUF;
+                    }
+                    at += GW * (Cfg::STAGE_BYTES / 16);
+                    full += GW * 8;
+                    if (GW == 1) {
+                        if (full == bar_full + STAGES * 8) { full = bar_full; at = 0; parity ^= 1; }
+                    } else if (full >= bar_full + STAGES * 8) { full -= STAGES * 8; at -= STAGES * (Cfg::STAGE_BYTES / 16); parity ^= 1; }
+                    TF_ADD(m_issue, t2);
             }
 #ifdef NMSPMM_TF32_PROFILE
             TF_OUT(2, m_full); TF_OUT(3, m_free); TF_OUT(4, m_issue); TF_OUT(5, clock64() - m_start); if (warp == 1) { TF_OUT(8, 1); TF_OUT(9, n_win); }
@@ -457,36 +460,36 @@ nm_gemm_tf32_kernel(const GemmArgs g, const __grid_constant__ CUtensorMap map_a,
                     if (++buf == Cfg::NP) { buf = 0; done_parity ^= 1; }
                 }
             } else {
-            TF_DECL(c_gdone = 0, c_issue = 0);
-            TF_T(c_start);
-            for (int u = 0; u < n_win; ++u) {
-                TF_T(t0);
-                // (the step's B rows have landed: the gather was issued after their barrier had completed)
-                ok = mbar_spin_bounded(bar_gdone + buf * 8, done_parity, abort_word);
-                TF_ADD(c_gdone, t0);
-                if (!ok) break;
-                TF_T(t1);
-                tc_fence_after_sync();
-                if (v_live > 0) {
-                    const uint32_t gbuf = tmem_addr(tmem, 0, Cfg::ACOL0 + buf * Cfg::N1 + v_begin * WSP), acc = tmem_addr(tmem, 0, v_begin * VL);
+                TF_DECL(c_gdone = 0, c_issue = 0);
+                TF_T(c_start);
+                for (int u = 0; u < n_win; ++u) {
+                    TF_T(t0);
+                    // (the step's B rows have landed: the gather was issued after their barrier had completed)
+                    ok = mbar_spin_bounded(bar_gdone + buf * 8, done_parity, abort_word);
+                    TF_ADD(c_gdone, t0);
+                    if (!ok) break;
+                    TF_T(t1);
+                    tc_fence_after_sync();
+                    if (v_live > 0) {
+                        const uint32_t gbuf = tmem_addr(tmem, 0, Cfg::ACOL0 + buf * Cfg::N1 + v_begin * WSP), acc = tmem_addr(tmem, 0, v_begin * VL);
 #pragma unroll
-                    for (int v = 0; v < VPI; ++v) {
-                        if (v < v_live) {
+                        for (int v = 0; v < VPI; ++v) {
+                            if (v < v_live) {
 #pragma unroll
-                            for (int gi = 0; gi < Cfg::G; ++gi)
-                                umma_tf32_ts(acc + v * VL, gbuf + v * WSP + gi * 8, umma_desc_plus(b0, at + v * (BPV * WSP * 8) + gi * 64),
-                                             idesc_product, (u | gi) != 0);
+                                for (int gi = 0; gi < Cfg::G; ++gi)
+                                    umma_tf32_ts(acc + v * VL, gbuf + v * WSP + gi * 8, umma_desc_plus(b0, at + v * (BPV * WSP * 8) + gi * 64),
+                                                 idesc_product, (u | gi) != 0);
+                            }
                         }
+                        tc_commit(empty);                      // this half of the step's products has read the stage and the gather result
+                    } else {
+                        mbar_arrive(empty);                    // no vector of this half exists; the gather itself has completed
                     }
-                    tc_commit(empty);                      // this half of the step's products has read the stage and the gather result
-                } else {
-                    mbar_arrive(empty);                    // no vector of this half exists; the gather itself has completed
-                }
-                if (++buf == NBUF) { buf = 0; done_parity ^= 1; }
-                at += Cfg::STAGE_BYTES / 16;
-                empty += 8;
-                if (empty == bar_empty + STAGES * 8) { empty = bar_empty; at = 0; }
-                TF_ADD(c_issue, t1);
+                    if (++buf == NBUF) { buf = 0; done_parity ^= 1; }
+                    at += Cfg::STAGE_BYTES / 16;
+                    empty += 8;
+                    if (empty == bar_empty + STAGES * 8) { empty = bar_empty; at = 0; }
+                    TF_ADD(c_issue, t1);
             }
 #ifdef NMSPMM_TF32_PROFILE
             if (warp == FIRST_PRODUCT) { TF_OUT(6, c_gdone); TF_OUT(7, c_issue); TF_OUT(15, clock64() - c_start); }

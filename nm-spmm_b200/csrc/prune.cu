@@ -43,8 +43,9 @@ struct PruneCfg {
 // of one index block of 128 columns and writes the packed indices itself (the packing kernels read nothing else): 1: re-tiled,
 // [N / 128][W][4] (the 32-k formats); 2: the two windows' list of used columns to cinfo and every index's rank in it
 // (the 64-k formats; preprocess.cu::preprocess_high_kernel).  4096 x 11008, 4 of 32, with a packing launch behind it 39.6 us
-// (41.9 on another box), in one 38.3 (40.7): the warps of a block wait for one another, and what is left is this
-// kernel's own 34 us -- HBM at 61 %, beside the conversions to double and the ranking.
+// (41.9 on another box), in one 38.3 (40.7).  What is left is this kernel's own 37 us from cold (the profiler's): 197 MB
+// through DRAM at 5.3 TB/s, which is active 65 % of the time, beside the conversions to double, the ranking and
+// the warps of a block that wait for one another.
 template <int VEC, int PACK>
 __global__ void __launch_bounds__((PruneCfg<VEC>::WARPS * 32), 5)      // shared memory has room for five, whose copies are in flight together
 prune_magnitude_kernel(const float* __restrict__ dense, float* __restrict__ BT, int* __restrict__ DT, int* __restrict__ cinfo, int n_windows, int N,

@@ -49,8 +49,8 @@ def _dense_tf32_pays(M: int, N: int, K: int, n_keep: int) -> bool:
     """Whether the backward takes torch's dense products: only where the caller has allowed torch TF32
     matrix products, which are 32 / n_keep times the work at some twenty times the FP32 rate, and where
     the call is large enough for the expansion of B to pay.  Both gradients, B200, us: 4096 x 4096 x 4096 at
-    4 / 8 / 16:32 832 / 1493 / 2934 by the kernels, 419 / 444 / 495 dense in TF32; 1024 rows 241 / 416 / 819
-    against 177 / 202 / 254; 256 rows 90 / 127 / 226 against 123 / 147 / 200; 1024 x 1024 x 1024 at 8:32 56 against 109.
+    4 / 8 / 16:32 815 / 1332 / 2607 by the kernels, 436 / 457 / 509 dense in TF32; 1024 rows 239 / 375 / 730
+    against 219 / 222 / 258; 256 rows 91 / 127 / 223 against 128 / 148 / 204; 1024 x 1024 x 1024 at 8:32 56 against 97.
     (Dense in FP32 loses everywhere.)"""
     return (_torch().backends.cuda.matmul.fp32_precision == "tf32"        # whichever of torch's switches set it
             and M * n_keep >= 3000 and M * N * K * n_keep >= 3.4e10)
