@@ -22,8 +22,8 @@
 // barrier, waits and look-ups (82 / 78 / 75 / 62 % of the 74.1 TFLOP/s peak at 16 / 12 / 8 / 4 of 32, 4096 cubed); this one runs
 // at 85 / 82 / 82 / 74 %, of the 88 % that the inner loop reaches alone (its loads take register
 // ports from the FMAs).  What is left between the two is the waits and loop ends of a window (6 % at 8:32)
-// and the copies' writes to shared memory; at 4:32 half as many rows carry each, and the compute warps read about
-// two spilled registers per window (every variant spills 8 to 24 bytes; at 8:32 none of it is in the window loop).  Measured, us: 4096 cubed, 8:32, 620 -> 564; 128 x 1024 x 131072, 4:32, 107 -> 84;
+// and the copies' writes to shared memory; at 4:32 half as many rows carry each, and the compute warps read two or
+// three spilled registers per window (every variant spills 8 to 24 bytes; at 8:32 none of it is in the window loop).  Measured, us: 4096 cubed, 8:32, 620 -> 564; 128 x 1024 x 131072, 4:32, 107 -> 84;
 // 777 x 5760 x 2080, 12:32, row-major, 164 -> 153; 64 x 11008 x 4096, 8:32, 42.2 -> 40.3; 2368 x 4096 x 4096, 16:32, 671 -> 661.
 #pragma once
 #include <cuda.h>
