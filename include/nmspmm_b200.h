@@ -313,7 +313,8 @@ typedef struct nmspmm_gemm_plan_info {
     int stages;
 } nmspmm_gemm_plan_info;
 int nmspmm_gemm_plan(const nmspmm_gemm_desc* desc, nmspmm_gemm_plan_info* out);
-/* What a call of nmspmm_gemm with workspace_bytes of scratch runs (see nmspmm_gemm_call_workspace_bytes). */
+/* What a call of nmspmm_gemm with workspace_bytes of scratch runs (see nmspmm_gemm_call_workspace_bytes; rows of 16-bit
+ * activations may take the other width of tile on the TF32 path). */
 int nmspmm_gemm_call_plan(const nmspmm_gemm_desc* desc, size_t workspace_bytes, nmspmm_gemm_plan_info* out);
 
 /* End-to-end form on HOST buffers: copies A, B, the raw DT [W][Q] and nothing else
