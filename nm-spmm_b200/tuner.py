@@ -87,6 +87,21 @@ def tune_shape(pkg, shape: Shape, verbose: bool = False):
     return best[0], best[1], best[2], base
 
 
+def tile_for_less_scratch(pkg, shape: Shape) -> int:
+    """The tile that calls of this shape take by themselves, where scratch for the plan that its description names would not hold that
+    tile's pieces (0 elsewhere): with an entry for it a caller who sizes by workspace_bytes gets it too."""
+    M, N, K, n_keep, fmt, path, vec_len = shape
+    if path == pkg.PATH_TF32:                                # (whose choice follows the type of the activations, which an entry does not know)
+        return 0
+    saved = pkg.tuned_plans_snapshot_and_clear()
+    try:
+        d = pkg.make_desc(M, N, K, n_keep, fmt, 128 if N % 128 == 0 else 32, path, 0, 0, vec_len)
+        taken = pkg.call_plan(d).tile
+        return 0 if pkg.call_plan(d, pkg.workspace_bytes(d)).tile == taken else taken
+    finally:
+        pkg.tuned_plans_restore(saved)
+
+
 def tune(pkg, shapes: Iterable[Shape], out_path: str = "", verbose: bool = False):
     """Tunes ``shapes``, merges the winners that beat the heuristics into the table file and
     registers them in the running library.  Returns the list of result rows."""
@@ -94,6 +109,8 @@ def tune(pkg, shapes: Iterable[Shape], out_path: str = "", verbose: bool = False
     rows = []
     for shape in shapes:
         tile, split, ms, base = tune_shape(pkg, shape, verbose)
+        if (tile, split) == (0, 0):
+            tile = tile_for_less_scratch(pkg, shape)
         rows.append((shape, tile, split, ms, base))
         if verbose or True:
             print(f"{shape}: heuristic {base:.4f} ms, best tile {tile} split {split} {ms:.4f} ms ({base / ms:.3f}x)", flush=True)

@@ -334,6 +334,8 @@ def test_tuned_shapes_keep_an_entry_for_callers_with_the_named_scratch(pkg, M, N
     try:
         pkg.load_tuned_plans(pkg.tuner.default_table_path())
         assert pkg.plan(d).tile == pkg.call_plan(d, pkg.workspace_bytes(d)).tile == pkg.TILE_128x256
+        assert pkg.tuner.tile_for_less_scratch(pkg, (M, N, K, n_keep, 1, 0, 32)) == pkg.TILE_128x256      # tuning keeps it
+        assert pkg.tuner.tile_for_less_scratch(pkg, (256, 8192, 22016, 4, 1, 0, 32)) == 0                 # the named scratch is enough here
     finally:
         pkg.tuned_plans_restore(saved)
 
